@@ -20,14 +20,14 @@ static constexpr double kZeroThresh = (double)1e-8f;
 // ---------------------------------------------------------------------------
 struct SegDesc {
     long long tgt;    // first target row in the packed target arrays
-    long long src;    // first source row in the packed source arrays (TILE aligned)
+    long long src;    // first source row in the packed source arrays (a multiple of the fold, 32)
     long long part;   // first row of this segment in the partial-sum buffer
     int n_tgt;        // targets
-    int n_src_tiles;  // source tiles (sources zero-padded to a TILE multiple)
-    int n_tb;         // target blocks
-    int split;        // source chunks (one block per target block and chunk)
+    int n_folds;      // folds of 32 source records (sources zero-padded to a whole fold)
+    int n_tb;         // target groups
+    int split;        // source chunks (one block per target group and chunk)
     int item0;        // first block index of this segment
-    int sym_tiles;    // > 0: the first sym_tiles source tiles are the targets' own records and the
+    int sym_folds;    // > 0: the first sym_folds folds are the targets' own records and the
                       // sum is symmetric in (target, source): see sweep_kernel<Op, true>
 };
 

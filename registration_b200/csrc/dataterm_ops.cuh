@@ -48,13 +48,13 @@ struct DataLayout {
                                                       : D + 1;
 };
 
-template <class Real_, int KIND, int PDEG, int QDEG, int D, int MODE, bool SMALL = false>
+template <class Real_, int KIND, int PDEG, int QDEG, int D, int MODE>
 struct OpData {
     using Real = Real_;
     using L = DataLayout<MODE, D>;
     static constexpr bool F32 = sizeof(Real) == 4;
     static constexpr int TPS = 1;
-    static constexpr int BLOCK = SMALL ? 32 : 128, R = 2, TILE = SMALL ? 32 : 128, FOLD = F32 ? 32 : TILE;
+    static constexpr int R = 2;
     static constexpr int PP = PointPlanes<Real>::N;
     static constexpr int PW = Traits<Real>::PER_WORD;
     static constexpr int TVW = (L::TV + PW - 1) / PW;
@@ -64,6 +64,9 @@ struct OpData {
     static constexpr int NOUT = L::NOUT;
     using Params = KernelParamsBase<Real>;
     using Acc = typename AccFor<Real>::template type<NOUT>;
+    // K bounds the factor of K' as well (its polynomial Q is below P term by term)
+    static constexpr bool GRADX = MODE != M_VARI_VALUE;
+    static LDDMM_D float lgk(const Params& P, float d2) { return lg_factor<KIND, PDEG, F32>(P.pk, d2); }
     struct Tgt {
         Real x[D];
         Real u[L::TV > 0 ? L::TV : 1];
@@ -77,8 +80,8 @@ struct OpData {
         if constexpr (L::TV > 0) load_vals<Real, L::TV>(P.tgt4, P.tgt_stride, row, PP, t.u);
     }
     static LDDMM_D void load_source(const float4* S, int j, Src& s) {
-        load_vals_smem<Real, D, TILE>(S, j, 0, s.y);
-        load_vals_smem<Real, L::SV, TILE>(S, j, PP, s.v);
+        load_vals_smem<Real, D>(S, j, 0, s.y);
+        load_vals_smem<Real, L::SV>(S, j, PP, s.v);
     }
     static LDDMM_D void pair(const Params& P, const Tgt& t, const Src& s, Acc& acc) {
         Real dx[D], r2 = 0;
@@ -135,13 +138,15 @@ struct OpVariValue2 {
     static constexpr bool F32 = true;
     static constexpr bool DUP = true;
     static constexpr int TPS = 2;
-    static constexpr int BLOCK = 128, R = 4, TILE = 128, FOLD = 32;
+    static constexpr int R = 4;
     static constexpr int PP = 1;
     static constexpr int NV = 7;
     static constexpr int NS = (NV + 1) / 2;
     static constexpr int NOUT = 1;
     using Params = KernelParams2;
     using Acc = AccF32C2<1>;
+    static constexpr bool GRADX = false;
+    static LDDMM_D float lgk(const Params& P, float d2) { return lg_factor<KIND, PDEG, true>(P.pkd, d2); }
     struct Tgt {
         f2 x[3];
         f2 u[3];
@@ -153,7 +158,7 @@ struct OpVariValue2 {
         load_target_pair<3>(P.tgt4, P.tgt_stride, ra, rb, 0, t.x);
         load_target_pair<3>(P.tgt4, P.tgt_stride, ra, rb, 1, t.u);
     }
-    static LDDMM_D void load_source(const float4* S, int j, Src& s) { load_dup_source<NV, TILE>(S, j, s.val); }
+    static LDDMM_D void load_source(const float4* S, int j, Src& s) { load_dup_source<NV>(S, j, s.val); }
     static LDDMM_D void pair(const Params& P, const Tgt& t, const Src& s, Acc& a) {
         f2 r2;
 #pragma unroll
@@ -185,13 +190,15 @@ struct OpVariGrad2 {
     static constexpr bool F32 = true;
     static constexpr bool DUP = true;
     static constexpr int TPS = 2;
-    static constexpr int BLOCK = 128, R = 4, TILE = 128, FOLD = 32;
+    static constexpr int R = 4;
     static constexpr int PP = 1;
     static constexpr int NV = 7;
     static constexpr int NS = (NV + 1) / 2;
     static constexpr int NOUT = 7;
     using Params = KernelParams2;
     using Acc = AccF32C2<NOUT>;
+    static constexpr bool GRADX = true;
+    static LDDMM_D float lgk(const Params& P, float d2) { return lg_factor<KIND, PDEG, true>(P.pkd, d2); }
     struct Tgt {
         f2 x[3];
         f2 u[3];
@@ -203,7 +210,7 @@ struct OpVariGrad2 {
         load_target_pair<3>(P.tgt4, P.tgt_stride, ra, rb, 0, t.x);
         load_target_pair<3>(P.tgt4, P.tgt_stride, ra, rb, 1, t.u);
     }
-    static LDDMM_D void load_source(const float4* S, int j, Src& s) { load_dup_source<NV, TILE>(S, j, s.val); }
+    static LDDMM_D void load_source(const float4* S, int j, Src& s) { load_dup_source<NV>(S, j, s.val); }
     static LDDMM_D void pair(const Params& P, const Tgt& t, const Src& s, Acc& a) {
         f2 dx[3], r2;
 #pragma unroll
@@ -244,13 +251,15 @@ struct OpCurGrad2 {
     static constexpr bool F32 = true;
     static constexpr bool DUP = true;
     static constexpr int TPS = 2;
-    static constexpr int BLOCK = 128, R = 2, TILE = 128, FOLD = 32;
+    static constexpr int R = 2;
     static constexpr int PP = 1;
     static constexpr int NV = 6;
     static constexpr int NS = (NV + 1) / 2;
     static constexpr int NOUT = 6;
     using Params = KernelParams2;
     using Acc = AccF32C2<NOUT>;
+    static constexpr bool GRADX = true;
+    static LDDMM_D float lgk(const Params& P, float d2) { return lg_factor<KIND, PDEG, true>(P.pkd, d2); }
     struct Tgt {
         f2 x[3];
         f2 u[3];
@@ -262,7 +271,7 @@ struct OpCurGrad2 {
         load_target_pair<3>(P.tgt4, P.tgt_stride, ra, rb, 0, t.x);
         load_target_pair<3>(P.tgt4, P.tgt_stride, ra, rb, 1, t.u);
     }
-    static LDDMM_D void load_source(const float4* S, int j, Src& s) { load_dup_source<NV, TILE>(S, j, s.val); }
+    static LDDMM_D void load_source(const float4* S, int j, Src& s) { load_dup_source<NV>(S, j, s.val); }
     static LDDMM_D void pair(const Params& P, const Tgt& t, const Src& s, Acc& a) {
         f2 dx[3], r2;
 #pragma unroll
@@ -357,18 +366,28 @@ LDDMM_D double vec_norm_eps(const double* s, int d, double eps) {
 //   norm measure : target -, source a*sign              (value and gradient)
 //   norm varifold: target n, source (n, a*sign)         (value and gradient)
 // c == nullptr writes a zero (padding) record of nplanes planes.
+// bp, bw (sources): the packed position and the weight that bounds what the record adds (fold boxes).
 template <class Real>
 LDDMM_D void dt_pack_record(int norm, int grad, bool is_t, const double* c, const double* s, int d, double eps,
                             double sign, double scale, const double* center, float4* planes, long long stride,
-                            long long i, int nplanes, int slots, bool dup = false) {
+                            long long i, int nplanes, int slots, bool dup = false, Real* bp = nullptr,
+                            Real* bw = nullptr) {
     constexpr int PP = PointPlanes<Real>::N;
     if (c == nullptr) {
+        if (bp != nullptr) bp[0] = bp[1] = bp[2] = *bw = 0;
         for (int p = 0; p < nplanes; ++p) planes[(long long)p * stride + i] = make_float4(0.f, 0.f, 0.f, 0.f);
         return;
     }
     const double a = vec_norm_eps(s, d, eps);
     double pos[4] = {0, 0, 0, 0};
     for (int j = 0; j < d; ++j) pos[j] = (c[j] - center[j]) * scale;
+    if (bp != nullptr) {
+        Real w = (Real)(norm == NCURRENT ? 0.0 : a * sign);
+        for (int j = 0; j < 3; ++j) bp[j] = (Real)pos[j];
+        if (norm == NCURRENT)
+            for (int j = 0; j < d; ++j) w = max_nan(w, (Real)(s[j] * sign));
+        *bw = max_nan((Real)0, w);
+    }
     if (sizeof(Real) == 4 && dup) {
         // duplicated source record [pos0 pos1 pos2 vals...], two values per word (see ops2.cuh)
         double vals[4] = {0, 0, 0, 0};
@@ -431,9 +450,8 @@ static __global__ void dt_pack_kernel(int norm, int grad, const double* __restri
                                       long long n2, int d, double eps1, double eps2, double sign2, double scale,
                                       const double* __restrict__ center, float4* tgt, long long tstride, int tplanes,
                                       int tslots, float4* src, long long sstride, int splanes, int sslots,
-                                      int dup = 0, long long n1s = -1) {
-    // set-2 sources start at row n1s (n1 rounded up to a tile for symmetric sweeps)
-    if (n1s < 0) n1s = n1;
+                                      int dup, long long n1s, float4* boxes) {
+    // set-2 sources start at row n1s (n1 rounded up to a fold for symmetric sweeps)
     const long long npad = tstride > sstride ? tstride : sstride;
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < npad;
          i += (long long)gridDim.x * blockDim.x) {
@@ -444,8 +462,10 @@ static __global__ void dt_pack_kernel(int norm, int grad, const double* __restri
             const bool first = i < n1, second = i >= n1s && i < n1s + n2;
             const double* c = first ? c1 + i * d : (second ? c2 + (i - n1s) * d : nullptr);
             const double* sv = first ? s1 + i * d : (second ? s2 + (i - n1s) * d : nullptr);
+            Real bp[3], bw;
             dt_pack_record<Real>(norm, grad, false, c, sv, d, first ? eps1 : eps2, first ? 1.0 : sign2, scale, center,
-                                 src, sstride, i, splanes, sslots, dup != 0);
+                                 src, sstride, i, splanes, sslots, dup != 0, bp, &bw);
+            store_fold_box<Real>(boxes, i, c != nullptr, bp, bw);
         }
     }
 }

@@ -52,14 +52,15 @@ struct DataArgs {
 };
 
 // SYM (values): the cell-cell self part is evaluated once per unordered pair
-// (sweep_kernel<Op, true>); the target cells then start at a tile boundary.
+// (sweep_kernel<Op, true>); the target cells then start at a fold boundary.
 template <class Op, class Real, bool SYM = false>
 int dt_sweep(const DataArgs& a, Workspace& ws, cudaStream_t st, int grad, double sign2, const double* c1,
              const double* s1, double*& part, SinglePlan& pl, const KScale& ks, const double* center) {
-    const long long n1s = SYM ? (a.nc + Op::TILE - 1) / Op::TILE * Op::TILE : a.nc;
+    const long long n1s = SYM ? round_up(a.nc, kFold) : a.nc;
     pl = plan_single<Op>(a.nc, n1s + a.nc2);
     float4* tgt = ws.take<float4>((size_t)Op::NT_ * pl.n_tpad);
     float4* src = ws.take<float4>((size_t)Op::NS * pl.m_pad);
+    float4* boxes = ws.take<float4>(pl.box_words());
     part = ws.take<double>((size_t)pl.split * a.nc * Op::NOUT);
     if (ws.measuring()) return LDDMM_OK;
     typename Op::Params P{};
@@ -70,8 +71,8 @@ int dt_sweep(const DataArgs& a, Workspace& ws, cudaStream_t st, int grad, double
     set_data_poly<Op, Real>(P, ks);
     dt_pack_kernel<Real><<<grid_for(std::max(pl.n_tpad, pl.m_pad)), 256, 0, st>>>(
         a.norm, grad, c1, s1, a.nc, a.c2, a.s2, a.nc2, a.d, a.eps1, a.eps2, sign2, ks.scale, center, tgt, pl.n_tpad,
-        Op::NT_, Op::TSLOTS, src, pl.m_pad, Op::NS, Op::SSLOTS, op_dup<Op>::value ? 1 : 0, n1s);
-    return launch_single<Op, SYM>(pl, a.nc, P, part, st, (int)(n1s / Op::TILE));
+        Op::NT_, Op::TSLOTS, src, pl.m_pad, Op::NS, Op::SSLOTS, op_dup<Op>::value ? 1 : 0, n1s, boxes);
+    return launch_single<Op, SYM>(pl, a.nc, P, boxes, part, st, (int)(n1s / kFold));
 }
 
 // Adapters giving OpApplyK / OpData a uniform plane description.
@@ -82,8 +83,7 @@ struct DtOp : Base {
     static constexpr int SSLOTS = SSLOTS_;
 };
 
-// SMALL: the small tile shape for the unpacked operators (few target cells);
-// the packed FP32 surface operators keep their shape.
+// SMALL: the small groups of OpApplyK (few target cells); the other operators have one shape.
 template <class Real, int KIND, int PDEG, int QDEG, int D, bool SMALL = false>
 int dt_impl(const DataArgs& a, Workspace& ws, cudaStream_t st) {
     constexpr int PW = Traits<Real>::PER_WORD;
@@ -106,7 +106,7 @@ int dt_impl(const DataArgs& a, Workspace& ws, cudaStream_t st) {
         if (a.norm == NVARIFOLD) {
             // FP32: packed-pair operator (two targets per slot, duplicated sources)
             using Op = std::conditional_t<(sizeof(Real) == 4 && D == 3), DtOp<OpVariValue2<KIND, PDEG>, 3, 4, 2>,
-                                          DtOp<OpData<Real, KIND, PDEG, QDEG, D, M_VARI_VALUE, SMALL>, 3, 4,
+                                          DtOp<OpData<Real, KIND, PDEG, QDEG, D, M_VARI_VALUE>, 3, 4,
                                                PP + (3 + PW - 1) / PW>>;
             rc = dt_sweep<Op, Real, true>(a, ws, st, 0, -2.0, c1, s1, part, pl, ks, center);
             nout = Op::NOUT;
@@ -135,18 +135,18 @@ int dt_impl(const DataArgs& a, Workspace& ws, cudaStream_t st) {
         constexpr bool PACK = sizeof(Real) == 4 && D == 3;   // FP32 surfaces: packed-pair operators
         if (a.norm == NVARIFOLD) {
             using Op = std::conditional_t<PACK, DtOp<OpVariGrad2<KIND, PDEG, QDEG>, 3, 4, 2>,
-                                          DtOp<OpData<Real, KIND, PDEG, QDEG, D, M_VARI_GRAD, SMALL>, 3, 4,
+                                          DtOp<OpData<Real, KIND, PDEG, QDEG, D, M_VARI_GRAD>, 3, 4,
                                                PP + (3 + PW - 1) / PW>>;
             rc = dt_sweep<Op, Real>(a, ws, st, 1, -1.0, c1, s1, part, pl, ks, center);
             nout = Op::NOUT;
         } else if (a.norm == NCURRENT) {
             using Op = std::conditional_t<PACK, DtOp<OpCurGrad2<KIND, PDEG, QDEG>, D, D, 2>,
-                                          DtOp<OpData<Real, KIND, PDEG, QDEG, D, M_CUR_GRAD, SMALL>, D, D,
+                                          DtOp<OpData<Real, KIND, PDEG, QDEG, D, M_CUR_GRAD>, D, D,
                                                PP + (D + PW - 1) / PW>>;
             rc = dt_sweep<Op, Real>(a, ws, st, 1, -1.0, c1, s1, part, pl, ks, center);
             nout = Op::NOUT;
         } else {
-            using Op = DtOp<OpData<Real, KIND, PDEG, QDEG, D, M_MEAS_GRAD, SMALL>, 0, 1, PP>;
+            using Op = DtOp<OpData<Real, KIND, PDEG, QDEG, D, M_MEAS_GRAD>, 0, 1, PP>;
             rc = dt_sweep<Op, Real>(a, ws, st, 1, -1.0, c1, s1, part, pl, ks, center);
             nout = Op::NOUT;
         }

@@ -41,14 +41,16 @@ DeviceInfo device_info();
 // Maximum resident blocks per SM of a kernel (cached by the caller per kernel).
 int occupancy_blocks(const void* kernel, int block, size_t dyn_smem = 0);
 
-// Number of source chunks for a sweep: enough items (target blocks x chunks)
-// for about 8 waves of `slots` resident blocks, at least 2 source tiles per
-// chunk.  `slots` is taken as 8 blocks per SM for every operator, so the split
-// (and the workspace) depends only on the shape and the SM count.
-inline int choose_split(int n_tb, int n_src_tiles, int slots) {
-    if (n_tb <= 0 || n_src_tiles <= 0) return 1;
+// Number of source chunks for a sweep: enough items (target groups x chunks)
+// for about 8 waves of `slots` resident blocks, at least kMinFolds folds of 32
+// sources for each of a block's four warps.  `slots` is taken as 8 blocks per
+// SM for every operator, so the split (and the workspace) depends only on the
+// shape and the SM count.
+constexpr int kMinFolds = 4;
+inline int choose_split(int n_tb, int n_folds, int slots) {
+    if (n_tb <= 0 || n_folds <= 0) return 1;
     long long want = (8LL * slots + n_tb - 1) / n_tb;
-    int max_split = std::max(1, n_src_tiles / 2);
+    int max_split = std::max(1, n_folds / (4 * kMinFolds));
     return (int)std::max(1LL, std::min<long long>(want, max_split));
 }
 

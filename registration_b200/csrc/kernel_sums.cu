@@ -24,6 +24,7 @@ struct ApplyKArgs {
     int order;
     double* f;
     int split_cap;  // 0: no cap on the number of source chunks
+    bool boxed;     // keep fold boxes in the workspace (far folds are passed over)
 };
 
 template <class Real, int KIND, int DEG, int D, int DIMB>
@@ -34,6 +35,7 @@ int applyk_group(const ApplyKArgs& a, int col0, Workspace& ws, cudaStream_t st) 
     const SinglePlan pl = plan_single<Op>(a.n, a.m, a.split_cap);
     float4* tgt = ws.take<float4>((size_t)Op::PP * pl.n_tpad);
     float4* src = ws.take<float4>((size_t)Op::NS * pl.m_pad);
+    float4* boxes = a.boxed ? ws.take<float4>(pl.box_words()) : nullptr;
     double* part = ws.take<double>((size_t)pl.split * a.n * DIMB);
     double* center = ws.take<double>(kCenterWords);
     if (ws.measuring()) return LDDMM_OK;
@@ -60,15 +62,14 @@ int applyk_group(const ApplyKArgs& a, int col0, Workspace& ws, cudaStream_t st) 
         for (int j = 0; j < 5; ++j) P.pkd[j] = dup_coeff(ks.pk[j]);
         for (int j = 0; j < 4; ++j) P.pqd[j] = dup_coeff(ks.pq[j]);
         pack_dup_kernel<<<grid_for(pl.m_pad), 256, 0, st>>>(a.y, a.m, a.d, ks.scale, center, g, D, DIMB, src,
-                                                            pl.m_pad, pl.m_pad);
+                                                            pl.m_pad, pl.m_pad, boxes);
     } else {
         for (int j = 0; j < 5; ++j) P.pk[j] = (Real)ks.pk[j];
         for (int j = 0; j < 4; ++j) P.pq[j] = (Real)ks.pq[j];
-        pack_points_kernel<Real><<<grid_for(pl.m_pad), 256, 0, st>>>(a.y, a.m, a.d, ks.scale, center, src, pl.m_pad,
-                                                                     pl.m_pad);
-        pack_values_kernel<Real><<<grid_for(pl.m_pad), 256, 0, st>>>(g, a.m, src, pl.m_pad, pl.m_pad, Op::PP);
+        pack_records_kernel<Real><<<grid_for(pl.m_pad), 256, 0, st>>>(a.y, a.m, a.d, ks.scale, center, g, src,
+                                                                      pl.m_pad, pl.m_pad, boxes);
     }
-    LDDMM_TRY(launch_single<Op>(pl, a.n, P, part, st));
+    LDDMM_TRY(launch_single<Op>(pl, a.n, P, boxes, part, st));
     // combine writes only the group's own columns
     const int ncols = g.nvals;
     if (ncols == DIMB) {
@@ -125,7 +126,7 @@ static int applyk_validate(const ApplyKArgs& a) {
 
 template <class Real>
 size_t applyk_ws(int64_t n, int64_t m, int d, int dimb) {
-    ApplyKArgs a{nullptr, n, nullptr, m, nullptr, d, dimb, 1.0, 10, nullptr, 0};
+    ApplyKArgs a{nullptr, n, nullptr, m, nullptr, d, dimb, 1.0, 10, nullptr, 0, true};
     if (n <= 0 || m <= 0 || d < 1 || d > 3 || dimb < 1) return 0;
     Workspace ws;
     applyk_run<Real>(a, ws, 0);
@@ -179,6 +180,7 @@ int difft_impl(const DiffKTArgs& a, Workspace& ws, cudaStream_t st) {
     const SinglePlan pl = plan_single<Op>(a.n, a.m);
     float4* tgt = ws.take<float4>((size_t)NT * pl.n_tpad);
     float4* src = ws.take<float4>((size_t)Op::NS * pl.m_pad);
+    float4* boxes = ws.take<float4>(pl.box_words());
     double* part = ws.take<double>((size_t)pl.split * a.n * D);
     double* center = ws.take<double>(kCenterWords);
     if (ws.measuring()) return LDDMM_OK;
@@ -201,23 +203,20 @@ int difft_impl(const DiffKTArgs& a, Workspace& ws, cudaStream_t st) {
         gv.off[w] = (long long)i * a.m * a.dimb + c;
     }
     launch_bbox_center(a.x, a.n, a.y, a.m, a.d, center, st);
-    pack_points_kernel<Real><<<grid_for(pl.n_tpad), 256, 0, st>>>(a.x, a.n, a.d, ks.scale, center, tgt, pl.n_tpad,
-                                                                  pl.n_tpad);
-    pack_values_kernel<Real><<<grid_for(pl.n_tpad), 256, 0, st>>>(gu, a.n, tgt, pl.n_tpad, pl.n_tpad,
-                                                                  PointPlanes<Real>::N);
+    pack_records_kernel<Real><<<grid_for(pl.n_tpad), 256, 0, st>>>(a.x, a.n, a.d, ks.scale, center, gu, tgt,
+                                                                   pl.n_tpad, pl.n_tpad, nullptr);
     if constexpr (sizeof(Real) == 4) {
         for (int j = 0; j < 5; ++j) P.pkd[j] = dup_coeff(ks.pk[j]);
         for (int j = 0; j < 4; ++j) P.pqd[j] = dup_coeff(ks.pq[j]);
         pack_dup_kernel<<<grid_for(pl.m_pad), 256, 0, st>>>(a.y, a.m, a.d, ks.scale, center, gv, D, W, src,
-                                                            pl.m_pad, pl.m_pad);
+                                                            pl.m_pad, pl.m_pad, boxes);
     } else {
         for (int j = 0; j < 5; ++j) P.pk[j] = (Real)ks.pk[j];
         for (int j = 0; j < 4; ++j) P.pq[j] = (Real)ks.pq[j];
-        pack_points_kernel<Real><<<grid_for(pl.m_pad), 256, 0, st>>>(a.y, a.m, a.d, ks.scale, center, src, pl.m_pad,
-                                                                     pl.m_pad);
-        pack_values_kernel<Real><<<grid_for(pl.m_pad), 256, 0, st>>>(gv, a.m, src, pl.m_pad, pl.m_pad, Op::PP);
+        pack_records_kernel<Real><<<grid_for(pl.m_pad), 256, 0, st>>>(a.y, a.m, a.d, ks.scale, center, gv, src,
+                                                                      pl.m_pad, pl.m_pad, boxes);
     }
-    LDDMM_TRY(launch_single<Op>(pl, a.n, P, part, st));
+    LDDMM_TRY(launch_single<Op>(pl, a.n, P, boxes, part, st));
     const int dout = a.d;  // D may exceed d (d == 1 runs as D == 2)
     if (dout == D) {
         combine_kernel<<<grid_for(a.n * D), 256, 0, st>>>(part, a.n, D, pl.split, ks.dscale, a.f, a.d, 0);
@@ -322,16 +321,15 @@ int div_impl(const ApplyKArgs& a, Workspace& ws, cudaStream_t st) {
     launch_bbox_center(a.x, a.n, a.y, a.m, a.d, center, st);
     pack_points_kernel<Real><<<grid_for(pl.n_tpad), 256, 0, st>>>(a.x, a.n, a.d, ks.scale, center, tgt, pl.n_tpad,
                                                                   pl.n_tpad);
-    pack_points_kernel<Real><<<grid_for(pl.m_pad), 256, 0, st>>>(a.y, a.m, a.d, ks.scale, center, src, pl.m_pad,
-                                                                 pl.m_pad);
     Gather g{};
     g.src = a.beta;
     g.row_stride = a.d;
     g.nvals = a.d;
     for (int c = 0; c < a.d; ++c) g.off[c] = c;
     g.mult = 1.0;  // K' 2 <x-y, a> = dscale * F * <x'-y', a>
-    pack_values_kernel<Real><<<grid_for(pl.m_pad), 256, 0, st>>>(g, a.m, src, pl.m_pad, pl.m_pad, Op::PP);
-    LDDMM_TRY(launch_single<Op>(pl, a.n, P, part, st));
+    pack_records_kernel<Real><<<grid_for(pl.m_pad), 256, 0, st>>>(a.y, a.m, a.d, ks.scale, center, g, src, pl.m_pad,
+                                                                  pl.m_pad, nullptr);
+    LDDMM_TRY(launch_single<Op>(pl, a.n, P, nullptr, part, st));
     combine_kernel<<<grid_for(a.n), 256, 0, st>>>(part, a.n, 1, pl.split, ks.dscale, a.f, 1, 0);
     return cuda_check(cudaGetLastError(), "applydiv");
 }
@@ -348,7 +346,7 @@ int div_run(const ApplyKArgs& a, Workspace& ws, cudaStream_t st) {
 template <class Real>
 size_t div_ws(int64_t n, int64_t m, int d) {
     if (n <= 0 || m <= 0 || d < 1 || d > 3) return 0;
-    ApplyKArgs a{nullptr, n, nullptr, m, nullptr, d, d, 1.0, 10, nullptr, 0};
+    ApplyKArgs a{nullptr, n, nullptr, m, nullptr, d, d, 1.0, 10, nullptr, 0, true};
     Workspace ws;
     div_run<Real>(a, ws, 0);
     return ws.off + 256;
@@ -376,9 +374,9 @@ int div_entry(const ApplyKArgs& a, void* wsp, size_t wsb, cudaStream_t st) {
     return div_run<Real>(a, ws, st);
 }
 
-size_t applyk_f32c_scratch_bytes(int64_t n, int64_t m, int d, int dimb, int split_cap) {
+size_t applyk_f32c_scratch_bytes(int64_t n, int64_t m, int d, int dimb, int split_cap, bool boxed) {
     if (n <= 0 || m <= 0 || d < 1 || d > 3 || dimb < 1) return 0;
-    ApplyKArgs a{nullptr, n, nullptr, m, nullptr, d, dimb, 1.0, 10, nullptr, split_cap};
+    ApplyKArgs a{nullptr, n, nullptr, m, nullptr, d, dimb, 1.0, 10, nullptr, split_cap, boxed};
     size_t best = 0;
     for (int order : {10, 3}) {  // Gaussian and Laplacian plans
         a.order = order;
@@ -391,8 +389,8 @@ size_t applyk_f32c_scratch_bytes(int64_t n, int64_t m, int d, int dimb, int spli
 
 int applyk_f32c_in_workspace(const double* x, int64_t n, const double* y, int64_t m, const double* beta, int d,
                              int dimb, double sigma, int order, double* f, void* workspace, size_t workspace_bytes,
-                             cudaStream_t stream, int split_cap) {
-    ApplyKArgs a{x, n, y, m, beta, d, dimb, sigma, order, f, split_cap};
+                             cudaStream_t stream, int split_cap, bool boxed) {
+    ApplyKArgs a{x, n, y, m, beta, d, dimb, sigma, order, f, split_cap, boxed};
     return applyk_entry<float>(a, workspace, workspace_bytes, stream);
 }
 
@@ -408,14 +406,14 @@ size_t lddmm_applyk_f64_workspace(int64_t n, int64_t m, int d, int dimb) { retur
 int lddmm_applyk_f32c(const double* x, int64_t n, const double* y, int64_t m, const double* beta, int d, int dimb,
                       double sigma, int order, double* f, void* workspace, size_t workspace_bytes,
                       lddmm_stream_t stream) {
-    ApplyKArgs a{x, n, y, m, beta, d, dimb, sigma, order, f, 0};
+    ApplyKArgs a{x, n, y, m, beta, d, dimb, sigma, order, f, 0, true};
     return applyk_entry<float>(a, workspace, workspace_bytes, (cudaStream_t)stream);
 }
 
 int lddmm_applyk_f64(const double* x, int64_t n, const double* y, int64_t m, const double* beta, int d, int dimb,
                      double sigma, int order, double* f, void* workspace, size_t workspace_bytes,
                      lddmm_stream_t stream) {
-    ApplyKArgs a{x, n, y, m, beta, d, dimb, sigma, order, f, 0};
+    ApplyKArgs a{x, n, y, m, beta, d, dimb, sigma, order, f, 0, true};
     return applyk_entry<double>(a, workspace, workspace_bytes, (cudaStream_t)stream);
 }
 
@@ -445,13 +443,13 @@ size_t lddmm_applydiv_f64_workspace(int64_t n, int64_t m, int d) { return div_ws
 
 int lddmm_applydiv_f32c(const double* x, int64_t n, const double* y, int64_t m, const double* a, int d, double sigma,
                         int order, double* f, void* workspace, size_t workspace_bytes, lddmm_stream_t stream) {
-    ApplyKArgs q{x, n, y, m, a, d, d, sigma, order, f, 0};
+    ApplyKArgs q{x, n, y, m, a, d, d, sigma, order, f, 0, true};
     return div_entry<float>(q, workspace, workspace_bytes, (cudaStream_t)stream);
 }
 
 int lddmm_applydiv_f64(const double* x, int64_t n, const double* y, int64_t m, const double* a, int d, double sigma,
                        int order, double* f, void* workspace, size_t workspace_bytes, lddmm_stream_t stream) {
-    ApplyKArgs q{x, n, y, m, a, d, d, sigma, order, f, 0};
+    ApplyKArgs q{x, n, y, m, a, d, d, sigma, order, f, 0, true};
     return div_entry<double>(q, workspace, workspace_bytes, (cudaStream_t)stream);
 }
 

@@ -58,6 +58,25 @@ LDDMM_D float kdiff32(const float* pq, float r2) {
     }
 }
 
+// log2 of the kernel factor at a prescaled squared distance d2: K with its
+// polynomial P, or the factor of K' with Q (both fall with the distance).  A
+// few units of the last place are enough: it only bounds what far records add.
+LDDMM_D float coef32(float c) { return c; }
+LDDMM_D float coef32(double c) { return (float)c; }
+LDDMM_D float coef32(unsigned long long dup) { return __uint_as_float((unsigned)dup); }
+template <int KIND, int DEG, bool F32, class C>
+LDDMM_D float lg_factor(const C* c, float d2) {
+    if constexpr (KIND == KGAUSS) {
+        return F32 ? -d2 : -0.72134752f * d2;
+    } else {
+        const float u = sqrt_approx(d2);
+        float p = coef32(c[DEG]);
+#pragma unroll
+        for (int j = DEG - 1; j >= 0; --j) p = fmaf(p, u, coef32(c[j]));
+        return __log2f(p) - (F32 ? u : 1.44269504f * u);
+    }
+}
+
 // FP64 monomial-sum polynomial, evaluated like the Fortran expression
 // c0 + c1*u + c2*u**2 + ... (left-to-right).
 template <int DEG>

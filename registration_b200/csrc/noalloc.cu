@@ -75,9 +75,14 @@ extern "C" LDDMM_API int lddmm_applyk_f32c_noalloc(const double* x, int64_t n, c
         return LDDMM_ERR_ARG;
     }
     int cap = 0;
+    bool boxed = true;   // without the fold boxes where only they would not fit
     if (n > 0 && m > 0) {
         // largest chunk count whose workspace fits the static scratch
-        const size_t one = applyk_f32c_scratch_bytes(n, m, d, dimb, 1);
+        size_t one = applyk_f32c_scratch_bytes(n, m, d, dimb, 1, boxed);
+        if (one > kNoAllocScratchBytes) {
+            boxed = false;
+            one = applyk_f32c_scratch_bytes(n, m, d, dimb, 1, boxed);
+        }
         if (one == 0 || one > kNoAllocScratchBytes) {
             set_error("applyk_noalloc: n=%lld, m=%lld, dimb=%d needs %zu bytes of scratch; the static scratch holds "
                       "%zu (use lddmm_applyk_f32c with a workspace)",
@@ -86,10 +91,10 @@ extern "C" LDDMM_API int lddmm_applyk_f32c_noalloc(const double* x, int64_t n, c
         }
         const size_t per_chunk = (size_t)n * (size_t)std::min(dimb, 4) * sizeof(double) + 256;
         cap = 1 + (int)std::min<size_t>((kNoAllocScratchBytes - one) / per_chunk, 1 << 20);
-        while (cap > 1 && applyk_f32c_scratch_bytes(n, m, d, dimb, cap) > kNoAllocScratchBytes) --cap;
+        while (cap > 1 && applyk_f32c_scratch_bytes(n, m, d, dimb, cap, boxed) > kNoAllocScratchBytes) --cap;
     }
     void* scratch = nullptr;
     LDDMM_TRY(noalloc_scratch(&scratch));
     return applyk_f32c_in_workspace(x, n, y, m, beta, d, dimb, sigma, order, f, scratch, kNoAllocScratchBytes,
-                                    (cudaStream_t)stream, cap);
+                                    (cudaStream_t)stream, cap, boxed);
 }

@@ -18,55 +18,6 @@
 namespace lddmm {
 
 template <class Real>
-struct Traits;
-template <>
-struct Traits<float> {
-    static constexpr int PER_WORD = 4;  // values per 16-byte word
-};
-template <>
-struct Traits<double> {
-    static constexpr int PER_WORD = 2;
-};
-
-template <class Real>
-LDDMM_D Real word_get(const float4* w, int i) {
-    if constexpr (sizeof(Real) == 4) {
-        const float* f = reinterpret_cast<const float*>(w);
-        return f[i];
-    } else {
-        const double* f = reinterpret_cast<const double*>(w);
-        return f[i];
-    }
-}
-
-// Reads `n` consecutive values starting at value index 0 of a record that is
-// spread over planes: value i lives in plane (first_plane + i / PER_WORD).
-template <class Real, int N>
-LDDMM_D void load_vals(const float4* base, long long stride, long long row, int first_plane, Real* out) {
-    constexpr int PW = Traits<Real>::PER_WORD;
-#pragma unroll
-    for (int w = 0; w < (N + PW - 1) / PW; ++w) {
-        const float4 word = base[(long long)(first_plane + w) * stride + row];
-#pragma unroll
-        for (int i = 0; i < PW; ++i)
-            if (w * PW + i < N) out[w * PW + i] = word_get<Real>(&word, i);
-    }
-}
-
-// smem version: plane p of record j at S[p*TILE + j]
-template <class Real, int N, int TILE>
-LDDMM_D void load_vals_smem(const float4* S, int j, int first_plane, Real* out) {
-    constexpr int PW = Traits<Real>::PER_WORD;
-#pragma unroll
-    for (int w = 0; w < (N + PW - 1) / PW; ++w) {
-        const float4 word = S[(first_plane + w) * TILE + j];
-#pragma unroll
-        for (int i = 0; i < PW; ++i)
-            if (w * PW + i < N) out[w * PW + i] = word_get<Real>(&word, i);
-    }
-}
-
-template <class Real>
 struct AccFor;
 template <>
 struct AccFor<float> {
@@ -109,23 +60,21 @@ struct PointPlanes {
 // ---------------------------------------------------------------------------
 // f_k = sum_l K(x_k, y_l) beta_l
 // ---------------------------------------------------------------------------
-// SMALL: 32-thread blocks and 32-record tiles for a few thousand targets or
-// fewer (see OpApplyK2 in ops2.cuh)
+// SMALL: two targets per thread instead of four, for a few thousand targets or fewer
 template <class Real_, int KIND, int DEG, int D, int DIMB, bool SMALL = false>
 struct OpApplyK {
     using Real = Real_;
     static constexpr bool F32 = sizeof(Real) == 4;
     static constexpr int TPS = 1;
-    static constexpr int BLOCK = SMALL ? 32 : 128;
     static constexpr int R = (F32 && !SMALL) ? 4 : 2;
-    static constexpr int TILE = SMALL ? 32 : 128;
-    static constexpr int FOLD = F32 ? 32 : TILE;
     static constexpr int PP = PointPlanes<Real>::N;
     static constexpr int WP = (DIMB + Traits<Real>::PER_WORD - 1) / Traits<Real>::PER_WORD;
     static constexpr int NS = PP + WP;
     static constexpr int NOUT = DIMB;
     using Params = KernelParamsBase<Real>;
     using Acc = typename AccFor<Real>::template type<DIMB>;
+    static constexpr bool GRADX = false;
+    static LDDMM_D float lgk(const Params& P, float d2) { return lg_factor<KIND, DEG, F32>(P.pk, d2); }
     struct Tgt {
         Real x[D];
     };
@@ -137,8 +86,8 @@ struct OpApplyK {
         load_vals<Real, D>(P.tgt4, P.tgt_stride, row, 0, t.x);
     }
     static LDDMM_D void load_source(const float4* S, int j, Src& s) {
-        load_vals_smem<Real, D, TILE>(S, j, 0, s.y);
-        load_vals_smem<Real, DIMB, TILE>(S, j, PP, s.b);
+        load_vals_smem<Real, D>(S, j, 0, s.y);
+        load_vals_smem<Real, DIMB>(S, j, PP, s.b);
     }
     static LDDMM_D void pair(const Params& P, const Tgt& t, const Src& s, Acc& a) {
         Real r2 = 0;
@@ -156,21 +105,20 @@ struct OpApplyK {
 // ---------------------------------------------------------------------------
 // f_k = sum_l K'(x_k,y_l) 2 (x_k - y_l) <u_k, v_l>     (up to the combine scale)
 // ---------------------------------------------------------------------------
-template <class Real_, int KIND, int DEG, int D, int W, bool SMALL = false>
+template <class Real_, int KIND, int DEG, int D, int W>
 struct OpDiffKT {
     using Real = Real_;
     static constexpr bool F32 = sizeof(Real) == 4;
     static constexpr int TPS = 1;
-    static constexpr int BLOCK = SMALL ? 32 : 128;
     static constexpr int R = 2;
-    static constexpr int TILE = SMALL ? 32 : 128;
-    static constexpr int FOLD = F32 ? 32 : TILE;
     static constexpr int PP = PointPlanes<Real>::N;
     static constexpr int WP = (W + Traits<Real>::PER_WORD - 1) / Traits<Real>::PER_WORD;
     static constexpr int NS = PP + WP;
     static constexpr int NOUT = D;
     using Params = KernelParamsBase<Real>;
     using Acc = typename AccFor<Real>::template type<D>;
+    static constexpr bool GRADX = true;
+    static LDDMM_D float lgk(const Params& P, float d2) { return lg_factor<KIND, DEG, F32>(P.pq, d2); }
     struct Tgt {
         Real x[D];
         Real u[W];
@@ -184,8 +132,8 @@ struct OpDiffKT {
         load_vals<Real, W>(P.tgt4, P.tgt_stride, row, PP, t.u);
     }
     static LDDMM_D void load_source(const float4* S, int j, Src& s) {
-        load_vals_smem<Real, D, TILE>(S, j, 0, s.y);
-        load_vals_smem<Real, W, TILE>(S, j, PP, s.v);
+        load_vals_smem<Real, D>(S, j, 0, s.y);
+        load_vals_smem<Real, W>(S, j, PP, s.v);
     }
     static LDDMM_D void pair(const Params& P, const Tgt& t, const Src& s, Acc& a) {
         Real dx[D];
@@ -213,10 +161,7 @@ struct OpDivergence {
     using Real = Real_;
     static constexpr bool F32 = sizeof(Real) == 4;
     static constexpr int TPS = 1;
-    static constexpr int BLOCK = 128;
     static constexpr int R = 4;
-    static constexpr int TILE = 128;
-    static constexpr int FOLD = F32 ? 32 : TILE;
     static constexpr int PP = PointPlanes<Real>::N;
     static constexpr int WP = (D + Traits<Real>::PER_WORD - 1) / Traits<Real>::PER_WORD;
     static constexpr int NS = PP + WP;
@@ -234,8 +179,8 @@ struct OpDivergence {
         load_vals<Real, D>(P.tgt4, P.tgt_stride, row, 0, t.x);
     }
     static LDDMM_D void load_source(const float4* S, int j, Src& s) {
-        load_vals_smem<Real, D, TILE>(S, j, 0, s.y);
-        load_vals_smem<Real, D, TILE>(S, j, PP, s.a);
+        load_vals_smem<Real, D>(S, j, 0, s.y);
+        load_vals_smem<Real, D>(S, j, PP, s.a);
     }
     static LDDMM_D void pair(const Params& P, const Tgt& t, const Src& s, Acc& acc) {
         Real r2 = 0, dot = 0;

@@ -29,11 +29,11 @@ struct KernelParams2 {
 };
 
 // Source records with duplicated values: NV values -> (NV + 1) / 2 words.
-template <int NV, int TILE>
+template <int NV>
 LDDMM_D void load_dup_source(const float4* S, int j, f2* val) {
 #pragma unroll
     for (int w = 0; w < (NV + 1) / 2; ++w) {
-        const float4 word = S[w * TILE + j];
+        const float4 word = S[w * kFold + j];
         val[2 * w] = word_lo(word);
         if (2 * w + 1 < NV) val[2 * w + 1] = word_hi(word);
     }
@@ -78,22 +78,23 @@ LDDMM_D f2 kdiff2(const unsigned long long* pqd, f2 r2) {
     }
 }
 
-// SMALL: tile shape for a few thousand targets or fewer (64 targets per
-// 32-thread block, 32-source tiles), so that the (target block, source chunk)
-// items spread over the SMs instead of filling one or two 512-target blocks.
+// SMALL: groups of 64 targets instead of 128, for a few thousand targets or
+// fewer, so that the (target group, source chunk) items spread over the SMs.
 template <int KIND, int DEG, int D, int DIMB, bool SMALL = false>
 struct OpApplyK2 {
     using Real = float;
     static constexpr bool F32 = true;
     static constexpr bool DUP = true;
     static constexpr int TPS = 2;
-    static constexpr int BLOCK = SMALL ? 32 : 128, R = SMALL ? 2 : 4, TILE = SMALL ? 32 : 128, FOLD = 32;
+    static constexpr int R = SMALL ? 2 : 4;
     static constexpr int PP = 1;            // target planes: pos
     static constexpr int NV = D + DIMB;     // source values
     static constexpr int NS = (NV + 1) / 2; // source words (duplicated values)
     static constexpr int NOUT = DIMB;
     using Params = KernelParams2;
     using Acc = AccF32C2<DIMB>;
+    static constexpr bool GRADX = false;
+    static LDDMM_D float lgk(const Params& P, float d2) { return lg_factor<KIND, DEG, true>(P.pkd, d2); }
     struct Tgt {
         f2 x[D];
     };
@@ -103,7 +104,7 @@ struct OpApplyK2 {
     static LDDMM_D void load_target(const Params& P, long long ra, long long rb, Tgt& t) {
         load_target_pair<D>(P.tgt4, P.tgt_stride, ra, rb, 0, t.x);
     }
-    static LDDMM_D void load_source(const float4* S, int j, Src& s) { load_dup_source<NV, TILE>(S, j, s.val); }
+    static LDDMM_D void load_source(const float4* S, int j, Src& s) { load_dup_source<NV>(S, j, s.val); }
     static LDDMM_D void pair(const Params& P, const Tgt& t, const Src& s, Acc& a) {
         f2 r2;
 #pragma unroll
@@ -123,7 +124,7 @@ struct OpDiffKT2 {
     static constexpr bool F32 = true;
     static constexpr bool DUP = true;
     static constexpr int TPS = 2;
-    static constexpr int BLOCK = SMALL ? 32 : 128, R = SMALL ? 2 : 4, TILE = SMALL ? 32 : 128, FOLD = 32;
+    static constexpr int R = SMALL ? 2 : 4;
     static constexpr int PP = 1;
     static constexpr int NV = D + W;
     static constexpr int NS = (NV + 1) / 2;
@@ -131,6 +132,8 @@ struct OpDiffKT2 {
     static constexpr int NOUT = D;
     using Params = KernelParams2;
     using Acc = AccF32C2<D>;
+    static constexpr bool GRADX = true;
+    static LDDMM_D float lgk(const Params& P, float d2) { return lg_factor<KIND, DEG, true>(P.pqd, d2); }
     struct Tgt {
         f2 x[D];
         f2 u[W];
@@ -142,7 +145,7 @@ struct OpDiffKT2 {
         load_target_pair<D>(P.tgt4, P.tgt_stride, ra, rb, 0, t.x);
         load_target_pair<W>(P.tgt4, P.tgt_stride, ra, rb, 1, t.u);
     }
-    static LDDMM_D void load_source(const float4* S, int j, Src& s) { load_dup_source<NV, TILE>(S, j, s.val); }
+    static LDDMM_D void load_source(const float4* S, int j, Src& s) { load_dup_source<NV>(S, j, s.val); }
     static LDDMM_D void pair(const Params& P, const Tgt& t, const Src& s, Acc& a) {
         f2 dx[D], r2;
 #pragma unroll
@@ -167,11 +170,12 @@ inline unsigned long long dup_coeff(double c) {
     return ((unsigned long long)u << 32) | (unsigned long long)u;
 }
 
-// Packs sources into duplicated records: values [ (x_i - c) * s (D of them, zero
+// Packs sources into duplicated records (and the boxes of their folds): values [ (x_i - c) * s (D of them, zero
 // beyond d), gather values (V of them, zero beyond g.nvals) ], rows >= n zero.
 static __global__ void pack_dup_kernel(const double* __restrict__ x, long long n, int d, double scale,
                                        const double* __restrict__ center, const Gather g, int D, int V,
-                                       float4* __restrict__ out, long long stride, long long n_pad) {
+                                       float4* __restrict__ out, long long stride, long long n_pad,
+                                       float4* __restrict__ boxes) {
     const int nv = D + V;
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n_pad;
          i += (long long)gridDim.x * blockDim.x) {
@@ -184,6 +188,12 @@ static __global__ void pack_dup_kernel(const double* __restrict__ x, long long n
         for (int w = 0; w < (nv + 1) / 2; ++w) {
             const float a = v[2 * w], b = (2 * w + 1 < nv) ? v[2 * w + 1] : 0.f;
             out[(long long)w * stride + i] = make_float4(a, a, b, b);
+        }
+        if (boxes != nullptr) {
+            float p[3], w = 0.f;
+            for (int j = 0; j < 3; ++j) p[j] = j < D ? v[j] : 0.f;
+            for (int q = 0; q < V; ++q) w = max_nan(w, v[D + q]);
+            store_fold_box<float>(boxes, i, i < n, p, w);
         }
     }
 }

@@ -129,27 +129,42 @@ struct Gather {
     double mult;
 };
 
-// Writes `g.nvals` values per row into consecutive planes starting at first_plane.
+// Standard records: the position planes of pack_points_kernel, then `g.nvals`
+// values per row in the following planes; boxes (sources): the fold boxes.
 template <class Real>
-static __global__ void pack_values_kernel(const Gather g, long long n, float4* __restrict__ out, long long stride,
-                                   long long n_pad, int first_plane) {
-    constexpr int PW = Traits<Real>::PER_WORD;
+static __global__ void pack_records_kernel(const double* __restrict__ x, long long n, int d, double scale,
+                                           const double* __restrict__ center, const Gather g,
+                                           float4* __restrict__ out, long long stride, long long n_pad,
+                                           float4* __restrict__ boxes) {
+    constexpr int PW = Traits<Real>::PER_WORD, PP = PointPlanes<Real>::N;
     const int nwords = (g.nvals + PW - 1) / PW;
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n_pad;
          i += (long long)gridDim.x * blockDim.x) {
+        Real p[4] = {0, 0, 0, 0}, wmax = 0;
+        if (i < n)
+            for (int j = 0; j < d && j < 3; ++j) p[j] = (Real)((x[i * d + j] - center[j]) * scale);
+        if constexpr (sizeof(Real) == 4) {
+            out[i] = make_float4(p[0], p[1], p[2], p[3]);
+        } else {
+            double2* o = reinterpret_cast<double2*>(out);
+            o[i] = make_double2(p[0], p[1]);
+            o[stride + i] = make_double2(p[2], p[3]);
+        }
         for (int w = 0; w < nwords; ++w) {
             Real v[PW];
             for (int q = 0; q < PW; ++q) {
                 const int idx = w * PW + q;
                 v[q] = (i < n && idx < g.nvals) ? (Real)(g.src[i * g.row_stride + g.off[idx]] * g.mult) : (Real)0;
+                wmax = max_nan(wmax, v[q]);
             }
-            float4* dst = out + (long long)(first_plane + w) * stride + i;
+            float4* dst = out + (long long)(PP + w) * stride + i;
             if constexpr (sizeof(Real) == 4) {
                 *dst = make_float4(v[0], v[1], v[2], v[3]);
             } else {
                 *reinterpret_cast<double2*>(dst) = make_double2(v[0], v[1]);
             }
         }
+        if (boxes != nullptr) store_fold_box<Real>(boxes, i, i < n, p, wmax);
     }
 }
 

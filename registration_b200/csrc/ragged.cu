@@ -93,7 +93,7 @@ RagPlan<Op> rag_plan(const std::vector<long long>& n, const std::vector<long lon
         d.src = g.src;
         d.part = g.part;
         d.n_tgt = (int)n[s];
-        d.n_src_tiles = pl.n_src_tiles;
+        d.n_folds = pl.n_folds;
         d.n_tb = pl.n_tb;
         d.split = pl.split;
         d.item0 = p.items;
@@ -198,13 +198,22 @@ LDDMM_D void put_plain(float4* planes, long long stride, long long i, const floa
     }
 }
 
+// fold box of a packed source row: position v[0..D), weights v[D..NV) (whole warps: segments are padded to folds)
+template <int D>
+LDDMM_D void rag_box(float4* boxes, long long row, bool valid, const float* v, int NV) {
+    const float p[3] = {v[0], v[1], D > 2 ? v[2] : 0.f};
+    float w = 0.f;
+    for (int k = D; k < NV; ++k) w = max_nan(w, v[k]);
+    store_fold_box<float>(boxes, row, valid, p, w);
+}
+
 // ---- ragged shooting ---------------------------------------------------------------
 // xt / at of request s: blocks (T+1, n, d) / (T, n, d) at rows (T+1)*row0 / T*row0.
 template <int D>
 static __global__ void rag_shoot_pack_kernel(const RagSeg* __restrict__ segs, const long long* __restrict__ padoff,
                                              int nseg, const double* __restrict__ xt, const double* __restrict__ at,
                                              int T, int step, int d, float4* tgt, long long tstride, float4* src,
-                                             long long sstride) {
+                                             long long sstride, float4* boxes) {
     const long long total = padoff[nseg];
     for (long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x; q < total;
          q += (long long)gridDim.x * blockDim.x) {
@@ -223,7 +232,10 @@ static __global__ void rag_shoot_pack_kernel(const RagSeg* __restrict__ segs, co
             }
         }
         if (i < g.tpad) put_plain(tgt, tstride, g.tgt + i, pos, 3, 1);
-        if (i < g.spad) put_dup(src, sstride, g.src + i, vals, 2 * D);
+        if (i < g.spad) {
+            put_dup(src, sstride, g.src + i, vals, 2 * D);
+            rag_box<D>(boxes, g.src + i, i < g.n, vals, 2 * D);
+        }
     }
 }
 
@@ -297,6 +309,7 @@ int rag_shoot_impl(int nseg, const int64_t* v_off, int d, const double* x0, cons
     long long* dpad = ws.take<long long>(nseg + 1);
     float4* tgt = ws.take<float4>((size_t)Op::PP * pl.tt);
     float4* src = ws.take<float4>((size_t)Op::NS * pl.ss);
+    float4* boxes = ws.take<float4>(2 * (size_t)(pl.ss / kFold));
     double* part = ws.take<double>((size_t)pl.parts * D);
     double* epart = ws.take<double>((size_t)std::max<long long>(1, pl.eparts));
     if (ws.measuring()) return LDDMM_OK;
@@ -331,8 +344,8 @@ int rag_shoot_impl(int nseg, const int64_t* v_off, int d, const double* x0, cons
     grid.n_items = pl.items;
     for (int t = 0; t < T; ++t) {
         rag_shoot_pack_kernel<D><<<grid_for(padoff[nseg]), 256, 0, st>>>(dsegs, dpad, nseg, xt, at, T, t, d, tgt, pl.tt,
-                                                                        src, pl.ss);
-        sweep_kernel<Op><<<pl.items, Op::BLOCK, 0, st>>>(grid, P, part);
+                                                                        src, pl.ss, boxes);
+        sweep_kernel<Op><<<pl.items, 32 * kSweepWarps, 0, st>>>(grid, P, boxes, part);
         rag_shoot_combine_kernel<D><<<(int)pl.eparts, kRagThreads, 0, st>>>(dsegs, nseg, part, xt, at, T, t, d, epart);
     }
     if (energy) rag_energy_kernel<<<(nseg + 127) / 128, 128, 0, st>>>(dsegs, nseg, epart, 0.0, energy, 1);
@@ -345,7 +358,7 @@ template <int D>
 static __global__ void rag_cov_pack_kernel(const RagSeg* __restrict__ segs, const long long* __restrict__ padoff,
                                            int nseg, const double* __restrict__ xt, const double* __restrict__ at,
                                            const double* __restrict__ pxt, int T, int step, int d, float4* tgt,
-                                           long long tstride, float4* src, long long sstride) {
+                                           long long tstride, float4* src, long long sstride, float4* boxes) {
     const long long total = padoff[nseg];
     for (long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x; q < total;
          q += (long long)gridDim.x * blockDim.x) {
@@ -372,7 +385,10 @@ static __global__ void rag_cov_pack_kernel(const RagSeg* __restrict__ segs, cons
             put_plain(tgt, tstride, g.tgt + i, pos, 3, 1);
             put_plain(tgt + tstride, tstride, g.tgt + i, u, 2 * D, (2 * D + 3) / 4);
         }
-        if (i < g.spad) put_dup(src, sstride, g.src + i, v, 3 * D);
+        if (i < g.spad) {
+            put_dup(src, sstride, g.src + i, v, 3 * D);
+            rag_box<D>(boxes, g.src + i, i < g.n, v, 3 * D);
+        }
     }
 }
 
@@ -426,6 +442,7 @@ int rag_cov_impl(int nseg, const int64_t* v_off, int d, const double* xt, const 
     long long* drow = ws.take<long long>(nseg + 1);
     float4* tgt = ws.take<float4>((size_t)NT * pl.tt);
     float4* src = ws.take<float4>((size_t)Op::NS * pl.ss);
+    float4* boxes = ws.take<float4>(2 * (size_t)(pl.ss / kFold));
     double* part = ws.take<double>((size_t)pl.parts * D);
     if (ws.measuring()) return LDDMM_OK;
     for (int s = 0; s < nseg; ++s) {
@@ -458,8 +475,8 @@ int rag_cov_impl(int nseg, const int64_t* v_off, int d, const double* xt, const 
     grid.n_items = pl.items;
     for (int t = T - 1; t >= 0; --t) {
         rag_cov_pack_kernel<D><<<grid_for(padoff[nseg]), 256, 0, st>>>(dsegs, dpad, nseg, xt, at, pxt, T, t, d, tgt,
-                                                                      pl.tt, src, pl.ss);
-        sweep_kernel<Op><<<pl.items, Op::BLOCK, 0, st>>>(grid, P, part);
+                                                                      pl.tt, src, pl.ss, boxes);
+        sweep_kernel<Op><<<pl.items, 32 * kSweepWarps, 0, st>>>(grid, P, boxes, part);
         rag_cov_combine_kernel<D><<<grid_for(rowoff[nseg]), 256, 0, st>>>(dsegs, drow, nseg, part, at, pxt, dat, T, t,
                                                                          d);
     }
@@ -473,7 +490,7 @@ template <int D, int DIMB>
 static __global__ void rag_applyk_pack_kernel(const RagSeg* __restrict__ segs, const long long* __restrict__ padoff,
                                               int nseg, const double* __restrict__ x, const double* __restrict__ y,
                                               const double* __restrict__ beta, int d, int dimb, float4* tgt,
-                                              long long tstride, float4* src, long long sstride) {
+                                              long long tstride, float4* src, long long sstride, float4* boxes) {
     const long long total = padoff[nseg];
     for (long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x; q < total;
          q += (long long)gridDim.x * blockDim.x) {
@@ -494,6 +511,7 @@ static __global__ void rag_applyk_pack_kernel(const RagSeg* __restrict__ segs, c
                 for (int c = 0; c < dimb && c < DIMB; ++c) v[D + c] = (float)beta[(g.m0 + i) * dimb + c];
             }
             put_dup(src, sstride, g.src + i, v, D + DIMB);
+            rag_box<D>(boxes, g.src + i, i < g.m, v, D + DIMB);
         }
     }
 }
@@ -543,6 +561,7 @@ int rag_applyk_impl(int nseg, const int64_t* t_start, const int64_t* t_count, co
     long long* drow = ws.take<long long>(nseg + 1);
     float4* tgt = ws.take<float4>((size_t)Op::PP * pl.tt);
     float4* src = ws.take<float4>((size_t)Op::NS * pl.ss);
+    float4* boxes = ws.take<float4>(2 * (size_t)(pl.ss / kFold));
     double* part = ws.take<double>((size_t)pl.parts * DIMB);
     if (ws.measuring()) return LDDMM_OK;
     for (int s = 0; s < nseg; ++s) {
@@ -569,8 +588,8 @@ int rag_applyk_impl(int nseg, const int64_t* t_start, const int64_t* t_count, co
     grid.nseg = nseg;
     grid.n_items = pl.items;
     rag_applyk_pack_kernel<D, DIMB><<<grid_for(padoff[nseg]), 256, 0, st>>>(dsegs, dpad, nseg, x, y, beta, d, dimb,
-                                                                             tgt, pl.tt, src, pl.ss);
-    if (pl.items > 0) sweep_kernel<Op><<<pl.items, Op::BLOCK, 0, st>>>(grid, P, part);
+                                                                             tgt, pl.tt, src, pl.ss, boxes);
+    if (pl.items > 0) sweep_kernel<Op><<<pl.items, 32 * kSweepWarps, 0, st>>>(grid, P, boxes, part);
     rag_applyk_combine_kernel<DIMB><<<grid_for(rowoff[nseg]), 256, 0, st>>>(dsegs, drow, nseg, part, dimb, f);
     return cuda_check(cudaGetLastError(), "ragged applyk");
 }
@@ -585,7 +604,7 @@ static __global__ void rag_dt_pack_kernel(const RagSeg* __restrict__ segs, const
                                           const double* __restrict__ s2, int d, double eps1, double eps2,
                                           double sign2, float4* tgt, long long tstride, int tplanes, int tslots,
                                           float4* src, long long sstride, int splanes, int sslots, int dup,
-                                          int sym_align) {
+                                          int sym_align, float4* boxes) {
     const long long total = padoff[nseg];
     for (long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x; q < total;
          q += (long long)gridDim.x * blockDim.x) {
@@ -602,8 +621,10 @@ static __global__ void rag_dt_pack_kernel(const RagSeg* __restrict__ segs, const
             const bool first = i < g.n, second = i >= n1s && i < n1s + g.m;
             const double* c = first ? c1 + (g.row0 + i) * d : (second ? c2 + (g.m0 + i - n1s) * d : nullptr);
             const double* sv = first ? s1 + (g.row0 + i) * d : (second ? s2 + (g.m0 + i - n1s) * d : nullptr);
+            Real bp[3], bw;
             dt_pack_record<Real>(norm, grad, false, c, sv, d, first ? eps1 : eps2, first ? 1.0 : sign2, g.scale,
-                                 g.center, src, sstride, g.src + i, splanes, sslots, dup != 0);
+                                 g.center, src, sstride, g.src + i, splanes, sslots, dup != 0, bp, &bw);
+            store_fold_box<Real>(boxes, g.src + i, c != nullptr, bp, bw);
         }
     }
 }
@@ -682,7 +703,7 @@ struct RagDataArgs {
 };
 
 // SYM (values): each segment's cell-cell self part is evaluated once per
-// unordered pair (sweep_kernel<Op, true>); its target cells start at a tile.
+// unordered pair (sweep_kernel<Op, true>); its target cells start at a fold.
 template <class Real, class Op, int TSLOTS, int SSLOTS, int NT, bool SYM = false>
 int rag_dt_sweep(const RagDataArgs& a, int kind, int grad, double sign2, const double* c1, const double* s1,
                  Workspace& ws, cudaStream_t st, RagPlan<Op>& pl, RagSeg*& dsegs, long long*& drow, double*& part) {
@@ -690,11 +711,11 @@ int rag_dt_sweep(const RagDataArgs& a, int kind, int grad, double sign2, const d
     std::vector<long long> n(nseg), m(nseg), n1s(nseg);
     for (int s = 0; s < nseg; ++s) {
         n[s] = a.c_off[s + 1] - a.c_off[s];
-        n1s[s] = SYM ? (n[s] + Op::TILE - 1) / Op::TILE * Op::TILE : n[s];
+        n1s[s] = SYM ? round_up(n[s], kFold) : n[s];
         m[s] = n1s[s] + (a.c2_off[s + 1] - a.c2_off[s]);
     }
     pl = rag_plan<Op>(n, m);
-    for (int s = 0; s < nseg; ++s) pl.desc[s].sym_tiles = SYM ? (int)(n1s[s] / Op::TILE) : 0;
+    for (int s = 0; s < nseg; ++s) pl.desc[s].sym_folds = SYM ? (int)(n1s[s] / kFold) : 0;
     std::vector<long long> padoff(nseg + 1, 0), rowoff(nseg + 1, 0);
     for (int s = 0; s < nseg; ++s) {
         pl.segs[s].row0 = a.c_off[s];
@@ -709,6 +730,7 @@ int rag_dt_sweep(const RagDataArgs& a, int kind, int grad, double sign2, const d
     drow = ws.take<long long>(nseg + 1);
     float4* tgt = ws.take<float4>((size_t)NT * pl.tt);
     float4* src = ws.take<float4>((size_t)Op::NS * pl.ss);
+    float4* boxes = ws.take<float4>(2 * (size_t)(pl.ss / kFold));
     part = ws.take<double>((size_t)pl.parts * Op::NOUT);
     if (ws.measuring()) return LDDMM_OK;
     for (int s = 0; s < nseg; ++s) {
@@ -733,12 +755,12 @@ int rag_dt_sweep(const RagDataArgs& a, int kind, int grad, double sign2, const d
     set_data_poly<Op, Real>(P, ks0);
     rag_dt_pack_kernel<Real><<<grid_for(padoff[nseg]), 256, 0, st>>>(
         dsegs, dpad, nseg, a.norm, grad, c1, s1, a.c2, a.s2, a.d, a.eps1, a.eps2, sign2, tgt, pl.tt, NT, TSLOTS, src,
-        pl.ss, Op::NS, SSLOTS, op_dup<Op>::value ? 1 : 0, SYM ? Op::TILE : 0);
+        pl.ss, Op::NS, SSLOTS, op_dup<Op>::value ? 1 : 0, SYM ? kFold : 0, boxes);
     SweepGrid grid{};
     grid.segs = ddesc;
     grid.nseg = nseg;
     grid.n_items = pl.items;
-    if (pl.items > 0) sweep_kernel<Op, SYM><<<pl.items, Op::BLOCK, 0, st>>>(grid, P, part);
+    if (pl.items > 0) sweep_kernel<Op, SYM><<<pl.items, 32 * kSweepWarps, 0, st>>>(grid, P, boxes, part);
     return cuda_check(cudaGetLastError(), "ragged data sweep");
 }
 

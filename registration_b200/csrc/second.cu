@@ -80,7 +80,7 @@ struct OpSecond {
     using L = SecondLayout<MODE, D>;
     static constexpr bool F32 = sizeof(Real) == 4;
     static constexpr int TPS = 1;
-    static constexpr int BLOCK = 128, R = 2, TILE = 128, FOLD = F32 ? 32 : TILE;
+    static constexpr int R = 2;
     static constexpr int PP = PointPlanes<Real>::N;
     static constexpr int PW = Traits<Real>::PER_WORD;
     static constexpr int TVW = (L::TV + PW - 1) / PW;
@@ -103,8 +103,8 @@ struct OpSecond {
         if constexpr (L::TV > 0) load_vals<Real, L::TV>(P.tgt4, P.tgt_stride, row, PP, t.u);
     }
     static LDDMM_D void load_source(const float4* S, int j, Src& s) {
-        load_vals_smem<Real, D, TILE>(S, j, 0, s.y);
-        load_vals_smem<Real, L::SV, TILE>(S, j, PP, s.v);
+        load_vals_smem<Real, D>(S, j, 0, s.y);
+        load_vals_smem<Real, L::SV>(S, j, PP, s.v);
     }
     static LDDMM_D void pair(const Params& P, const Tgt& t, const Src& s, Acc& acc) {
         Real dx[D], r2 = 0;
@@ -266,7 +266,7 @@ int second_impl(const SecondArgs& a, Workspace& ws, cudaStream_t st) {
                                                                   pl.n_tpad, pl.n_tpad);
     second_pack_kernel<Real><<<grid_for(pl.m_pad), 256, 0, st>>>(a.x, a.n, a.d, ks.scale, center, sv0, sv1, D, src,
                                                                  pl.m_pad, pl.m_pad);
-    LDDMM_TRY(launch_single<Op>(pl, a.n, P, part, st));
+    LDDMM_TRY(launch_single<Op>(pl, a.n, P, nullptr, part, st));
     second_combine_kernel<MODE, D><<<grid_for(a.n), 256, 0, st>>>(part, a.n, pl.split, ks.dscale, d2scale, c1s, a.p,
                                                                   a.f, a.d);
     return cuda_check(cudaGetLastError(), "applykdiff");

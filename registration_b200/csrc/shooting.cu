@@ -82,6 +82,21 @@ LDDMM_D void store_dup(float4* planes, long long stride, long long i, const doub
     }
 }
 
+// Fold box of source row i (whole warps, see store_fold_box): packed position
+// of x and the largest of the values of a and (if given) b.
+template <class Real>
+LDDMM_D void store_box(float4* boxes, long long i, bool valid, const double* x, const double* a, const double* b,
+                       int d, double s, const double* c) {
+    Real p[3] = {0, 0, 0}, w = 0;
+    if (valid)
+        for (int j = 0; j < d; ++j) {
+            p[j] = (Real)((x[j] - c[j]) * s);
+            w = max_nan(w, (Real)a[j]);
+            if (b != nullptr) w = max_nan(w, (Real)b[j]);
+        }
+    store_fold_box<Real>(boxes, i, valid, p, w);
+}
+
 // block-level FP64 sum with a fixed tree; thread 0 writes out[blockIdx.x]
 LDDMM_D void block_sum_store(double v, double* out) {
     __shared__ double red[kCombineThreads];
@@ -114,10 +129,11 @@ template <class Real, bool DUP>
 static __global__ void shoot_pack_kernel(const double* __restrict__ x, const double* __restrict__ a, long long n,
                                          int d, double s, const double* __restrict__ c, float4* tgt,
                                          long long tstride, float4* src, long long sstride, int pp, int nslots,
-                                         int ns) {
+                                         int ns, float4* boxes) {
     const long long npad = tstride > sstride ? tstride : sstride;
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < npad;
          i += (long long)gridDim.x * blockDim.x) {
+        if (i < sstride) store_box<Real>(boxes, i, i < n, x + i * d, a + i * d, nullptr, d, s, c);
         if (i < n) {
             if (i < tstride) store_point<Real>(tgt, tstride, i, x + i * d, d, s, c);
             if (i < sstride) {
@@ -142,19 +158,21 @@ static __global__ void shoot_combine_kernel(const double* __restrict__ part, lon
                                             const double* __restrict__ a0, double* __restrict__ x1,
                                             const double* __restrict__ a1, double s, const double* __restrict__ c,
                                             float4* tgt, long long tstride, float4* src, long long sstride, int pp,
-                                            int nslots, double* __restrict__ epart) {
+                                            int nslots, float4* boxes, double* __restrict__ epart) {
     double e = 0.0;
-    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n;
+    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < sstride;   // whole warps: n padded to folds
          i += (long long)gridDim.x * blockDim.x) {
+        const bool valid = i < n;
         double xn[4];
-        for (int j = 0; j < d; ++j) {
+        for (int j = 0; j < d && valid; ++j) {
             double v = 0.0;
             for (int k = 0; k < split; ++k) v += part[((long long)k * n + i) * dout + j];
             e += a0[i * d + j] * v;
             xn[j] = x0[i * d + j] + dt * v;
             x1[i * d + j] = xn[j];
         }
-        if (a1 != nullptr) {
+        if (a1 != nullptr) store_box<Real>(boxes, i, valid, xn, a1 + i * d, nullptr, d, s, c);
+        if (a1 != nullptr && valid) {
             store_point<Real>(tgt, tstride, i, xn, d, s, c);
             if constexpr (DUP) {
                 store_dup(src, sstride, i, xn, d, nslots, s, c, a1 + i * d, d, nslots);
@@ -213,6 +231,7 @@ int shoot_impl(const ShootArgs& a, Workspace& ws, cudaStream_t st) {
     const SinglePlan pl = plan_single<Op>(a.n, a.n);
     float4* tgt = ws.take<float4>((size_t)Op::PP * pl.n_tpad);
     float4* src = ws.take<float4>((size_t)Op::NS * pl.m_pad);
+    float4* boxes = ws.take<float4>(pl.box_words());
     double* part = ws.take<double>((size_t)pl.split * a.n * D);
     const int nb = combine_blocks(a.n);
     double* epart = ws.take<double>((size_t)a.T * nb);
@@ -229,14 +248,14 @@ int shoot_impl(const ShootArgs& a, Workspace& ws, cudaStream_t st) {
     LDDMM_TRY(cuda_check(cudaMemcpyAsync(a.xt, a.x0, sizeof(double) * N, cudaMemcpyDeviceToDevice, st), "shoot copy"));
     launch_bbox_center(a.x0, a.n, nullptr, 0, a.d, center, st);
     shoot_pack_kernel<Real, DUP><<<grid_for(std::max(pl.n_tpad, pl.m_pad)), 256, 0, st>>>(
-        a.x0, a.at, a.n, a.d, ks.scale, center, tgt, pl.n_tpad, src, pl.m_pad, Op::PP, D, Op::NS);
+        a.x0, a.at, a.n, a.d, ks.scale, center, tgt, pl.n_tpad, src, pl.m_pad, Op::PP, D, Op::NS, boxes);
     const double dt = a.dt > 0 ? a.dt : 1.0 / a.T;
     for (int t = 0; t < a.T; ++t) {
-        LDDMM_TRY(launch_single<Op>(pl, a.n, P, part, st));
+        LDDMM_TRY(launch_single<Op>(pl, a.n, P, boxes, part, st));
         shoot_combine_kernel<Real, DUP><<<nb, kCombineThreads, 0, st>>>(
             part, a.n, a.d, D, pl.split, dt, a.xt + t * N, a.at + t * N, a.xt + (t + 1) * N,
             t + 1 < a.T ? a.at + (t + 1) * N : nullptr, ks.scale, center, tgt, pl.n_tpad, src, pl.m_pad, Op::PP,
-            D, epart + (long long)t * nb);
+            D, boxes, epart + (long long)t * nb);
     }
     if (a.energy != nullptr)
         finalize_sum_kernel<<<1, kCombineThreads, 0, st>>>(epart, (long long)a.T * nb, a.rw * dt, a.energy);
@@ -333,10 +352,12 @@ template <class Real, bool DUP>
 static __global__ void cov_pack_kernel(const double* __restrict__ x, const double* __restrict__ a,
                                        const double* __restrict__ p, long long n, int d, double s,
                                        const double* __restrict__ c, double rw, float4* tgt, long long tstride,
-                                       float4* src, long long sstride, int pp, int tplanes, int nplanes, int tw) {
+                                       float4* src, long long sstride, int pp, int tplanes, int nplanes, int tw,
+                                       float4* boxes) {
     const long long npad = tstride > sstride ? tstride : sstride;
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < npad;
          i += (long long)gridDim.x * blockDim.x) {
+        if (i < sstride) store_box<Real>(boxes, i, i < n, x + i * d, a + i * d, p + i * d, d, s, c);
         if (i < n) {
             cov_store<Real, DUP>(tgt, tstride, src, sstride, i, pp, x + i * d, a + i * d, p + i * d, d, s, c, rw, tw);
         } else {
@@ -354,11 +375,12 @@ static __global__ void cov_combine_kernel(const double* __restrict__ part, long 
                                           double* __restrict__ dat_t, const double* __restrict__ x_prev,
                                           const double* __restrict__ a_prev, double s, const double* __restrict__ c,
                                           float4* tgt, long long tstride, float4* src, long long sstride, int pp,
-                                          int tw) {
-    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n;
+                                          int tw, float4* boxes) {
+    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < sstride;   // whole warps: n padded to folds
          i += (long long)gridDim.x * blockDim.x) {
+        const bool valid = i < n;
         double pn[4];
-        for (int j = 0; j < d; ++j) {
+        for (int j = 0; j < d && valid; ++j) {
             double f = 0.0;
             for (int k = 0; k < split; ++k) f += part[((long long)k * n + i) * dout + j];
             const double pj = p_next[i * d + j];
@@ -366,7 +388,8 @@ static __global__ void cov_combine_kernel(const double* __restrict__ part, long 
             p_t[i * d + j] = pn[j];
             if (dat_t != nullptr) dat_t[i * d + j] = 2.0 * rw * a_t[i * d + j] - pj;
         }
-        if (x_prev != nullptr)
+        if (x_prev != nullptr) store_box<Real>(boxes, i, valid, x_prev + i * d, a_prev + i * d, pn, d, s, c);
+        if (x_prev != nullptr && valid)
             cov_store<Real, DUP>(tgt, tstride, src, sstride, i, pp, x_prev + i * d, a_prev + i * d, pn, d, s, c, rw,
                                  tw);
     }
@@ -391,11 +414,12 @@ template <class Real, int KIND, int DEG, int D, bool SMALL = false>
 int cov_impl(const CovArgs& a, Workspace& ws, cudaStream_t st) {
     constexpr int W = 2 * D;
     constexpr bool DUP = sizeof(Real) == 4;  // FP32: packed-pair operator with duplicated sources
-    using Op = std::conditional_t<DUP, OpDiffKT2<KIND, DEG, D, W, SMALL>, OpDiffKT<Real, KIND, DEG, D, W, SMALL>>;
+    using Op = std::conditional_t<DUP, OpDiffKT2<KIND, DEG, D, W, SMALL>, OpDiffKT<Real, KIND, DEG, D, W>>;
     constexpr int NT = DUP ? 1 + (W + 3) / 4 : Op::NS;  // target planes (standard layout)
     const SinglePlan pl = plan_single<Op>(a.n, a.n);
     float4* tgt = ws.take<float4>((size_t)NT * pl.n_tpad);
     float4* src = ws.take<float4>((size_t)Op::NS * pl.m_pad);
+    float4* boxes = ws.take<float4>(pl.box_words());
     double* part = ws.take<double>((size_t)pl.split * a.n * D);
     double* center = ws.take<double>(kCenterWords);
     if (ws.measuring()) return LDDMM_OK;
@@ -414,15 +438,15 @@ int cov_impl(const CovArgs& a, Workspace& ws, cudaStream_t st) {
     launch_bbox_center(a.xt, a.n, nullptr, 0, a.d, center, st);
     cov_pack_kernel<Real, DUP><<<grid_for(std::max(pl.n_tpad, pl.m_pad)), 256, 0, st>>>(
         a.xt + (long long)(T - 1) * N, a.at + (long long)(T - 1) * N, a.px1, a.n, a.d, ks.scale, center, a.rw,
-        tgt, pl.n_tpad, src, pl.m_pad, Op::PP, NT, Op::NS, W);
+        tgt, pl.n_tpad, src, pl.m_pad, Op::PP, NT, Op::NS, W, boxes);
     const int nb = combine_blocks(a.n);
     for (int t = T - 1; t >= 0; --t) {
-        LDDMM_TRY(launch_single<Op>(pl, a.n, P, part, st));
+        LDDMM_TRY(launch_single<Op>(pl, a.n, P, boxes, part, st));
         cov_combine_kernel<Real, DUP><<<nb, kCombineThreads, 0, st>>>(
             part, a.n, a.d, D, pl.split, dt, ks.dscale, a.rw, a.pxt + (long long)(t + 1) * N,
             a.at + (long long)t * N, a.pxt + (long long)t * N, a.dat ? a.dat + (long long)t * N : nullptr,
             t > 0 ? a.xt + (long long)(t - 1) * N : nullptr, t > 0 ? a.at + (long long)(t - 1) * N : nullptr,
-            ks.scale, center, tgt, pl.n_tpad, src, pl.m_pad, Op::PP, W);
+            ks.scale, center, tgt, pl.n_tpad, src, pl.m_pad, Op::PP, W, boxes);
     }
     return cuda_check(cudaGetLastError(), "covector");
 }
@@ -461,7 +485,7 @@ struct OpEPDiff {
     using Real = Real_;
     static constexpr bool F32 = sizeof(Real) == 4;
     static constexpr int TPS = 1;
-    static constexpr int BLOCK = 128, R = 2, TILE = 128, FOLD = F32 ? 32 : TILE;
+    static constexpr int R = 2;
     static constexpr int PP = PointPlanes<Real>::N;
     static constexpr int WP = (D + Traits<Real>::PER_WORD - 1) / Traits<Real>::PER_WORD;
     static constexpr int NS = PP + WP;
@@ -481,8 +505,8 @@ struct OpEPDiff {
         load_vals<Real, D>(P.tgt4, P.tgt_stride, row, PP, t.a);
     }
     static LDDMM_D void load_source(const float4* S, int j, Src& s) {
-        load_vals_smem<Real, D, TILE>(S, j, 0, s.y);
-        load_vals_smem<Real, D, TILE>(S, j, PP, s.a);
+        load_vals_smem<Real, D>(S, j, 0, s.y);
+        load_vals_smem<Real, D>(S, j, PP, s.a);
     }
     static LDDMM_D void pair(const Params& P, const Tgt& t, const Src& s, Acc& acc) {
         Real dx[D], r2 = 0, dot = 0;
@@ -583,7 +607,7 @@ int epd_impl(const EPDArgs& a, Workspace& ws, cudaStream_t st) {
         epd_pack_kernel<Real><<<grid_for(std::max(pl.n_tpad, pl.m_pad)), 256, 0, st>>>(
             a.xt + t * N, a.at + t * N, a.n, a.d, ks.scale, center, tgt, pl.n_tpad, src, pl.m_pad, Op::PP, D,
             Op::NS);
-        LDDMM_TRY(launch_single<Op>(pl, a.n, P, part, st));
+        LDDMM_TRY(launch_single<Op>(pl, a.n, P, nullptr, part, st));
         epd_combine_kernel<Real><<<nb, kCombineThreads, 0, st>>>(part, a.n, a.d, Op::NOUT, pl.split, dt, ks.dscale,
                                                                  a.xt + t * N, a.at + t * N, a.xt + (t + 1) * N,
                                                                  t + 1 < a.T ? a.at + (t + 1) * N : nullptr);

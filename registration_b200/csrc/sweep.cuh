@@ -1,30 +1,106 @@
-// Generic tiled N-body sweep over (target block, source chunk) items.
+// Generic N-body sweep over (target group, source chunk) items.
 //
-// Each block owns BLOCK*R targets (R per thread, kept in registers) and one
-// chunk of the source range.  Source records (NS 16-byte words each, packed
-// structure-of-arrays in global memory, see Op::Src) are streamed through
-// shared memory in tiles of TILE records with a two-stage cp.async pipeline;
-// every warp reads the same record at the same time (shared-memory broadcast).
-// Per-target accumulators: FP32 partials over FOLD sources, folded into a
-// TwoSum-compensated (sum, err) pair (FP32 ops), or plain FP64 sums.
-// The block writes its per-target sums as doubles into the partial buffer
+// A block owns GT = 32*R targets (R per thread, kept in registers; all four warps
+// hold the same targets) and one chunk of the source range.  Sources are
+// handled in folds of 32 consecutive records (NS 16-byte words each, packed
+// structure-of-arrays in global memory, see Op::Src).  The 4 * split warps
+// that share a target group take every (4 * split)-th fold each, so that the
+// folds a group needs (neighbours in memory, when the order of the points
+// follows the shape) spread evenly over them.  A warp streams its folds
+// through its own cp.async ring: it waits for nobody but itself
+// (`__syncwarp`), every lane reads the same record (shared-memory broadcast).
+// One fold is 4096 pairs against 1.5-2 KB from L2, about 5 bytes per clock
+// and SM, so sharing a tile between the warps would save nothing that counts.
+//
+// Per-target accumulators: FP32 partials over the 32 sources of a fold, in
+// order, folded into a TwoSum-compensated (sum, err) pair (FP32 ops), or plain
+// FP64 sums.  The block adds its warps in order and writes doubles into
 //   part[(seg.part + chunk * seg.n_tgt + t) * Op::NOUT + c]
 // and a separate combine kernel adds the chunks in a fixed order, so results
 // do not depend on scheduling.
 //
+// Far folds (operators with Op::lgk, `boxes` given).  The pack kernels leave
+// for each fold its bounding box and log2 of the sum of its weights.  With the
+// box of the target group these bound what a fold can add to any target of
+// the group, U = W_F K(dmin) (times dmax where the summand carries x - y), and
+// from below what the sum is made of, L = max_F W_F K(dmax).  A fold with
+//   U <= L 2^-MARGIN / (number of folds)
+// is passed over: all such folds together stay below 2^-MARGIN of the sum of
+// absolute terms of every target of the group, MARGIN = 36 for FP32 pairs (whose
+// own rounding is 2^-22 to 2^-24 of it) and 58 for FP64 (2^-53).  The test is
+// done in log2, so it holds as well for targets far from every source, where
+// the whole sum is tiny.  A fold or group with a non-finite coordinate or weight
+// is never passed over.  A lane tests one fold, a warp 32 at a time.
+// Measured against the sweep over every pair that this replaces (B200): FP32c
+// varifold gradient of a 20,480-cell sphere at sigma 0.1 0.97 -> 0.47 ms, its
+// FP64 value 1.63 -> 0.81 ms, the value of 98,000 cells at sigma 0.05 6.2 ->
+// 1.9 ms.  Where no fold is far (uniform random points) the test costs 0.5%.
+//
 // SYM (symmetric sums, used for energies <S,S> - 2 <S,T> whose summand is
-// symmetric in the target and the source): the first seg.sym_tiles source
-// tiles hold the targets' own records in target order.  A target block skips
-// those of its own records that precede it, counts its diagonal tiles once
-// and the later ones twice (per-tile weight applied to the FP32 fold partial,
-// exact for 1 and 2), so each unordered pair is evaluated once: the per-target
-// partial sums are no longer the per-target sums, their weighted total is.
+// symmetric in the target and the source): the first seg.sym_folds folds hold
+// the targets' own records in target order.  A group skips those of its own
+// records that precede it, counts its diagonal folds once and the later ones
+// twice (per-fold weight applied to the FP32 partial, exact for 1 and 2), so
+// each unordered pair is evaluated once: the per-target partial sums are no
+// longer the per-target sums, their weighted total is.
 #pragma once
 #include <type_traits>
 
 #include "common.cuh"
 
 namespace lddmm {
+
+constexpr int kSweepWarps = 4;     // warps of a sweep block
+constexpr int kFold = 32;          // source records per fold
+
+template <class Real>
+struct Traits;
+template <>
+struct Traits<float> {
+    static constexpr int PER_WORD = 4;  // values per 16-byte word
+};
+template <>
+struct Traits<double> {
+    static constexpr int PER_WORD = 2;
+};
+
+template <class Real>
+LDDMM_D Real word_get(const float4* w, int i) {
+    if constexpr (sizeof(Real) == 4) {
+        const float* f = reinterpret_cast<const float*>(w);
+        return f[i];
+    } else {
+        const double* f = reinterpret_cast<const double*>(w);
+        return f[i];
+    }
+}
+
+// Reads `n` consecutive values starting at value index 0 of a record that is
+// spread over planes: value i lives in plane (first_plane + i / PER_WORD).
+template <class Real, int N>
+LDDMM_D void load_vals(const float4* base, long long stride, long long row, int first_plane, Real* out) {
+    constexpr int PW = Traits<Real>::PER_WORD;
+#pragma unroll
+    for (int w = 0; w < (N + PW - 1) / PW; ++w) {
+        const float4 word = base[(long long)(first_plane + w) * stride + row];
+#pragma unroll
+        for (int i = 0; i < PW; ++i)
+            if (w * PW + i < N) out[w * PW + i] = word_get<Real>(&word, i);
+    }
+}
+
+// smem version: plane p of record j of a fold at S[p*kFold + j]
+template <class Real, int N>
+LDDMM_D void load_vals_smem(const float4* S, int j, int first_plane, Real* out) {
+    constexpr int PW = Traits<Real>::PER_WORD;
+#pragma unroll
+    for (int w = 0; w < (N + PW - 1) / PW; ++w) {
+        const float4 word = S[(first_plane + w) * kFold + j];
+#pragma unroll
+        for (int i = 0; i < PW; ++i)
+            if (w * PW + i < N) out[w * PW + i] = word_get<Real>(&word, i);
+    }
+}
 
 // An operator may accumulate some outputs scaled by a power of two (cheaper per
 // pair); Op::out_scale(c) is then the exact factor applied when they are written.
@@ -33,119 +109,353 @@ struct op_has_out_scale : std::false_type {};
 template <class Op>
 struct op_has_out_scale<Op, std::void_t<decltype(Op::out_scale(0))>> : std::true_type {};
 
-// An operator may ask for a minimum number of resident blocks per SM
-// (Op::MIN_BLOCKS), which caps its registers per thread.
-template <class Op, class = void>
-struct op_min_blocks : std::integral_constant<int, 1> {};
+// Resident blocks per SM that the register budget is cut for, and the unrolling
+// of the source loop.  Measured at n = m = 131,072 (FP32) and 32,768 (FP64):
+// FP32 runs best with 128 registers (4 blocks) and 8 sources in flight
+// (Gaussian applyK 2.69 -> 2.78e12 pairs/s against no bound and 4 sources,
+// Laplacian applyDiffKT 1.54 -> 1.62e12), FP64 with 128 registers and 4 sources
+// (varifold gradient 3.15 -> 3.35e11; 8 sources spill).  Operators with many
+// outputs or wide records keep 168 registers (3 blocks) instead of spilling.
 template <class Op>
-struct op_min_blocks<Op, std::void_t<decltype(Op::MIN_BLOCKS)>> : std::integral_constant<int, Op::MIN_BLOCKS> {};
+constexpr int op_min_blocks() {
+    return sizeof(typename Op::Real) == 4 ? (Op::NOUT * Op::R > 24 || Op::NS > 6 ? 3 : 4)
+                                          : (Op::NOUT > 4 || Op::NS > 5 ? 3 : 4);
+}
+template <class Op>
+constexpr int op_unroll() { return sizeof(typename Op::Real) == 4 ? 8 : 4; }
+
+// Operators that bound their kernel factor (Op::lgk) can pass over far folds.
+template <class Op, class = void>
+struct op_culls : std::false_type {};
+template <class Op>
+struct op_culls<Op, std::void_t<decltype(&Op::lgk)>> : std::true_type {};
+
+// Targets of one group.
+template <class Op>
+constexpr int op_group() { return 32 * Op::R; }
+
+// Squared distances between two boxes: the smallest and the largest, with
+// slack for the rounding of the pairs' own distances.
+struct Box {
+    float lo[3], hi[3];
+};
+LDDMM_D void box_dist2(const Box& a, const float4 lo, const float4 hi, float& dmin2, float& dmax2) {
+    const float l[3] = {lo.x, lo.y, lo.z}, h[3] = {hi.x, hi.y, hi.z};
+    float mn = 0.f, mx = 0.f;
+#pragma unroll
+    for (int j = 0; j < 3; ++j) {
+        const float g = fmaxf(0.f, fmaxf(l[j] - a.hi[j], a.lo[j] - h[j]));
+        const float f = fmaxf(h[j] - a.lo[j], a.hi[j] - l[j]);
+        mn = fmaf(g, g, mn);
+        mx = fmaf(f, f, mx);
+    }
+    dmin2 = mn * (1.f - 1.f / 65536.f);
+    dmax2 = mx * (1.f + 1.f / 65536.f);
+}
+
+LDDMM_D float warp_min(float v) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v = fminf(v, __shfl_xor_sync(0xffffffffu, v, o));
+    return v;
+}
+LDDMM_D float warp_max(float v) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, o));
+    return v;
+}
+
+// max(w, |v|) that keeps a NaN
+template <class Real>
+LDDMM_D Real max_nan(Real w, Real v) {
+    const Real a = v < (Real)0 ? -v : v;
+    return (a > w || !(a == a)) ? a : w;
+}
+
+// The box of a fold of packed source records and log2 of the sum of its
+// weights, written to boxes[2 fold] = (lo, lgw), boxes[2 fold + 1] = (hi, 0).
+// Called by whole warps, lane i holding record `row` = 32 fold + i; `valid`:
+// a real record (padding has none), p its packed position, w >= 0 its weight.
+// A non-finite value makes lgw +inf: such a fold is never passed over.
+template <class Real>
+LDDMM_D void store_fold_box(float4* boxes, long long row, bool valid, const Real* p, Real w) {
+    float lo[3], hi[3];
+    bool bad = false;
+#pragma unroll
+    for (int j = 0; j < 3; ++j) {
+        if constexpr (sizeof(Real) == 4) {
+            lo[j] = hi[j] = p[j];
+        } else {
+            lo[j] = __double2float_rd(p[j]);
+            hi[j] = __double2float_ru(p[j]);
+        }
+        bad = bad || !(fabsf(lo[j]) < INFINITY) || !(fabsf(hi[j]) < INFINITY);
+        lo[j] = warp_min(valid ? lo[j] : INFINITY);
+        hi[j] = warp_max(valid ? hi[j] : -INFINITY);
+    }
+    bad = bad || !(w < (Real)INFINITY);
+    Real sum = valid ? w : (Real)0;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+    const bool any = __any_sync(0xffffffffu, valid && bad);
+    if ((threadIdx.x & 31) == 0) {
+        const float lgw = any ? INFINITY : (sizeof(Real) == 4 ? log2f((float)sum) : (float)log2((double)sum));
+        boxes[2 * (row / kFold)] = make_float4(lo[0], lo[1], lo[2], lgw);
+        boxes[2 * (row / kFold) + 1] = make_float4(hi[0], hi[1], hi[2], 0.f);
+    }
+}
 
 template <class Op, bool SYM = false>
-__global__ void __launch_bounds__(Op::BLOCK, op_min_blocks<Op>::value) sweep_kernel(const SweepGrid grid, const typename Op::Params P,
-                                                           double* __restrict__ part) {
-    using Real = typename Op::Real;
-    constexpr int BLOCK = Op::BLOCK, R = Op::R, TILE = Op::TILE, NS = Op::NS, NOUT = Op::NOUT;
-    constexpr int WORDS_PER_REC = NS;                  // 16-byte words per source record
-    constexpr int WORDS_PER_TILE = WORDS_PER_REC * TILE;
-    static_assert(WORDS_PER_TILE % BLOCK == 0, "tile must split evenly over the block");
-    __shared__ __align__(16) float4 smem[2][WORDS_PER_TILE];
+__global__ void __launch_bounds__(32 * kSweepWarps, op_min_blocks<Op>())
+    sweep_kernel(const SweepGrid grid, const typename Op::Params P, const float4* __restrict__ boxes,
+                 double* __restrict__ part) {
+    constexpr int R = Op::R, TPS = Op::TPS, NS = Op::NS, NOUT = Op::NOUT, GT = op_group<Op>();
+    constexpr int STAGE = NS * kFold;   // 16-byte words of one fold
+    constexpr int STAGES = NS > 6 ? 2 : 3;   // folds of a warp's ring (at most 48 KB for the block)
+    constexpr int RING = kSweepWarps * STAGES * STAGE;
+    constexpr int RED = (GT * NOUT * 8 + 15) / 16;
+    __shared__ __align__(16) float4 smem[RING > RED ? RING : RED];
+    __shared__ float sbox[kSweepWarps][7];
 
     const int item = blockIdx.x;
     const SegDesc sg = find_segment(grid, item);
     const int local = item - sg.item0;
     const int tb = local % sg.n_tb;
     const int chunk = local / sg.n_tb;
-    int tile_lo = (int)(((long long)chunk * sg.n_src_tiles) / sg.split);
-    const int tile_hi = (int)(((long long)(chunk + 1) * sg.n_src_tiles) / sg.split);
-    int diag_hi = 0;   // SYM: own tiles at or after diag_hi (and before sym_tiles) count twice
-    if constexpr (SYM) {
-        static_assert((BLOCK * R) % TILE == 0, "symmetric sweeps need whole tiles per target block");
-        constexpr int TPB = (BLOCK * R) / TILE;
-        const int diag_lo = tb * TPB < sg.sym_tiles ? tb * TPB : sg.sym_tiles;
-        diag_hi = tb * TPB + TPB;
-        if (tile_lo < diag_lo) tile_lo = diag_lo < tile_hi ? diag_lo : tile_hi;
-    }
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 
-    // targets owned by this thread: t = tb*BLOCK*R + r*BLOCK + threadIdx.x (rows are padded);
-    // an operator with TPS == 2 keeps two of them per slot (packed FP32 pairs)
-    constexpr int TPS = Op::TPS;
+    // targets of this lane: t = tb*GT + r*32 + lane (rows are padded); an
+    // operator with TPS == 2 keeps two of them per slot (packed FP32 pairs)
     constexpr int SLOTS = R / TPS;
     static_assert(R % TPS == 0, "R must be a multiple of TPS");
     typename Op::Tgt tg[SLOTS];
 #pragma unroll
     for (int q = 0; q < SLOTS; ++q) {
-        const long long row = sg.tgt + (long long)tb * BLOCK * R + (q * TPS) * BLOCK + threadIdx.x;
+        const long long row = sg.tgt + (long long)tb * GT + (q * TPS) * 32 + lane;
         if constexpr (TPS == 1) Op::load_target(P, row, tg[q]);
-        else Op::load_target(P, row, row + BLOCK, tg[q]);
+        else Op::load_target(P, row, row + 32, tg[q]);
     }
     typename Op::Acc acc[SLOTS];
 #pragma unroll
     for (int q = 0; q < SLOTS; ++q) acc[q].zero();
 
-    // global source words: Op lays a record out as NS planes of float4 words,
-    // plane p of record j at P.src4[p * P.src_stride + j]
-    auto load_tile = [&](int tile, int stage) {
-        const long long rec0 = sg.src + (long long)tile * TILE;
+    const int n_folds = sg.n_folds;
+    int f_lo = 0, diag_hi = 0;   // SYM: own folds at or after diag_hi (and before sym_folds) count twice
+    if constexpr (SYM) {
+        f_lo = min(tb * (GT / kFold), sg.sym_folds);
+        diag_hi = tb * (GT / kFold) + GT / kFold;
+    }
+
+    // the group's box and the threshold below which a fold is passed over
+    Box wb{};
+    float thr = 0.f;
+    bool cull = false;
+    const float4* fbox = nullptr;
+    if constexpr (op_culls<Op>::value) {
+        if (boxes != nullptr) {
+            fbox = boxes + 2 * (sg.src / kFold);
+            using Real = typename Op::Real;
+            float lo[3] = {INFINITY, INFINITY, INFINITY}, hi[3] = {-INFINITY, -INFINITY, -INFINITY};
+            bool bad = false;
+            if (threadIdx.x < GT && tb * GT + (int)threadIdx.x < sg.n_tgt) {
+                Real x[3];
+                load_vals<Real, 3>(P.tgt4, P.tgt_stride, sg.tgt + (long long)tb * GT + threadIdx.x, 0, x);
 #pragma unroll
-        for (int w = threadIdx.x; w < WORDS_PER_TILE; w += BLOCK) {
-            const int plane = w / TILE;
-            const int j = w - plane * TILE;
-            cp_async16(&smem[stage][w], P.src4 + (long long)plane * P.src_stride + rec0 + j);
+                for (int j = 0; j < 3; ++j) {
+                    if constexpr (sizeof(Real) == 4) {
+                        lo[j] = hi[j] = x[j];
+                    } else {
+                        lo[j] = __double2float_rd(x[j]);
+                        hi[j] = __double2float_ru(x[j]);
+                    }
+                    bad = bad || !(fabsf(lo[j]) < INFINITY) || !(fabsf(hi[j]) < INFINITY);
+                }
+            }
+#pragma unroll
+            for (int j = 0; j < 3; ++j) {
+                lo[j] = warp_min(lo[j]);
+                hi[j] = warp_max(hi[j]);
+            }
+            if (lane == 0) {
+#pragma unroll
+                for (int j = 0; j < 3; ++j) {
+                    sbox[warp][j] = lo[j];
+                    sbox[warp][3 + j] = hi[j];
+                }
+            }
+            cull = !__syncthreads_or(bad);
+#pragma unroll
+            for (int j = 0; j < 3; ++j) {
+                wb.lo[j] = sbox[0][j];
+                wb.hi[j] = sbox[0][3 + j];
+                for (int w = 1; w < kSweepWarps; ++w) {
+                    wb.lo[j] = fminf(wb.lo[j], sbox[w][j]);
+                    wb.hi[j] = fmaxf(wb.hi[j], sbox[w][3 + j]);
+                }
+            }
+            // L from at most kLSamples folds spread over the range and the group's own rows (any fold
+            // gives a valid lower bound; the nearest heavy one gives a good one)
+            constexpr int kLSamples = 512;
+            float lgl = -INFINITY;
+            const int step = max(1, n_folds / kLSamples);
+            for (int f = threadIdx.x * step; f < n_folds; f += 32 * kSweepWarps * step) {
+                float d0, d1;
+                const float4 bl = fbox[2 * f];
+                box_dist2(wb, bl, fbox[2 * f + 1], d0, d1);
+                if (bl.w < INFINITY) lgl = fmaxf(lgl, bl.w + Op::lgk(P, d1));
+            }
+            {
+                const int f = tb * (GT / kFold) + (int)threadIdx.x;
+                if (step > 1 && threadIdx.x < GT / kFold && f < n_folds) {
+                    float d0, d1;
+                    const float4 bl = fbox[2 * f];
+                    box_dist2(wb, bl, fbox[2 * f + 1], d0, d1);
+                    if (bl.w < INFINITY) lgl = fmaxf(lgl, bl.w + Op::lgk(P, d1));
+                }
+            }
+            lgl = warp_max(lgl);
+            if (lane == 0) sbox[warp][6] = lgl;
+            __syncthreads();
+            for (int w = 0; w < kSweepWarps; ++w) lgl = fmaxf(lgl, sbox[w][6]);
+            constexpr float kMargin = sizeof(Real) == 4 ? 36.f : 58.f;
+            thr = lgl - kMargin - log2f((float)n_folds) - (SYM ? 1.f : 0.f);
+        }
+    }
+
+    // this warp's folds: f_lo + c, f_lo + c + C, ...; next() gives the next one that counts, -1 after the last
+    const int C = sg.split * kSweepWarps;
+    int f_base = f_lo + chunk * kSweepWarps + warp, f_cur = 0;
+    unsigned f_mask = 0;
+    auto next = [&]() -> int {
+        while (f_mask == 0) {
+            if (f_base >= n_folds) return -1;
+            const long long f = (long long)f_base + (long long)lane * C;
+            bool act = f < n_folds;
+            if constexpr (op_culls<Op>::value) {
+                if (cull && act) {
+                    float d0, d1;
+                    const float4 bl = fbox[2 * f];
+                    box_dist2(wb, bl, fbox[2 * f + 1], d0, d1);
+                    float u = bl.w + Op::lgk(P, d0);
+                    if (Op::GRADX) u += 0.5f * __log2f(fmaxf(1.f, d1));
+                    act = !(u <= thr);
+                }
+            }
+            f_mask = __ballot_sync(0xffffffffu, act);
+            f_cur = f_base;
+            f_base = (int)min((long long)f_base + 32LL * C, (long long)n_folds);
+        }
+        const int b = __ffs(f_mask) - 1;
+        f_mask &= f_mask - 1;
+        return f_cur + b * C;
+    };
+
+    // source words: Op lays a record out as NS planes of 16-byte words, plane
+    // p of record j at P.src4[p * P.src_stride + j]; a fold's stage is plane-major
+    float4* ring = smem + warp * STAGES * STAGE;
+    auto load_fold = [&](int f, int st) {
+        if (f >= 0) {
+            const float4* g = P.src4 + sg.src + (long long)f * kFold + lane;
+#pragma unroll
+            for (int w = 0; w < NS; ++w) cp_async16(ring + st * STAGE + w * kFold + lane, g + (long long)w * P.src_stride);
         }
         cp_async_commit();
     };
 
-    if (tile_lo < tile_hi) load_tile(tile_lo, 0);
-    for (int tile = tile_lo; tile < tile_hi; ++tile) {
-        const int stage = (tile - tile_lo) & 1;
-        if (tile + 1 < tile_hi) {
-            load_tile(tile + 1, stage ^ 1);
-            cp_async_wait<1>();
-        } else {
-            cp_async_wait<0>();
+    int fa = next(), fb = -1;   // the fold to do, and (three stages) the one after it
+    load_fold(fa, 0);
+    if constexpr (STAGES == 3) {
+        if (fa >= 0) fb = next();
+        load_fold(fb, 1);
+    }
+    int st = 0;
+    while (fa >= 0) {
+        const int fn = (STAGES == 2 || fb >= 0) ? next() : -1;
+        load_fold(fn, st >= 1 ? st - 1 : STAGES - 1);
+        cp_async_wait<STAGES - 1>();
+        __syncwarp();
+        const float4* S = ring + st * STAGE;
+#pragma unroll
+        for (int q = 0; q < SLOTS; ++q) acc[q].begin_fold();
+#pragma unroll op_unroll<Op>()
+        for (int j = 0; j < kFold; ++j) {
+            typename Op::Src s;
+            Op::load_source(S, j, s);
+#pragma unroll
+            for (int q = 0; q < SLOTS; ++q) Op::pair(P, tg[q], s, acc[q]);
         }
-        __syncthreads();
-        const float4* S = smem[stage];
-        const float wt = (SYM && tile >= diag_hi && tile < sg.sym_tiles) ? 2.f : 1.f;
-        (void)wt;
-#pragma unroll 1
-        for (int j0 = 0; j0 < TILE; j0 += Op::FOLD) {
 #pragma unroll
-            for (int q = 0; q < SLOTS; ++q) acc[q].begin_fold();
-#pragma unroll 4
-            for (int j = j0; j < j0 + Op::FOLD; ++j) {
-                typename Op::Src s;
-                Op::load_source(S, j, s);
-#pragma unroll
-                for (int q = 0; q < SLOTS; ++q) Op::pair(P, tg[q], s, acc[q]);
-            }
+        for (int q = 0; q < SLOTS; ++q) {
+            if constexpr (SYM) acc[q].end_fold_w(fa >= diag_hi && fa < sg.sym_folds ? 2.f : 1.f);
+            else acc[q].end_fold();
+        }
+        __syncwarp();
+        fa = STAGES == 3 ? fb : fn;
+        fb = fn;
+        st = st == STAGES - 1 ? 0 : st + 1;
+    }
+    cp_async_wait<0>();
+    __syncthreads();
+
+    // add the warps in order, then one coalesced row block of doubles
+    double* red = reinterpret_cast<double*>(smem);
+    for (int w = 0; w < kSweepWarps; ++w) {
+        if (warp == w) {
 #pragma unroll
             for (int q = 0; q < SLOTS; ++q) {
-                if constexpr (SYM) acc[q].end_fold_w(wt);
-                else acc[q].end_fold();
-            }
-        }
-        __syncthreads();
-    }
-
 #pragma unroll
-    for (int q = 0; q < SLOTS; ++q) {
+                for (int l = 0; l < TPS; ++l) {
+                    const int t = (q * TPS + l) * 32 + lane;
 #pragma unroll
-        for (int lane = 0; lane < TPS; ++lane) {
-            const int t = tb * BLOCK * R + (q * TPS + lane) * BLOCK + threadIdx.x;
-            if (t < sg.n_tgt) {
-                double* dst = part + (sg.part + (long long)chunk * sg.n_tgt + t) * NOUT;
-#pragma unroll
-                for (int c = 0; c < NOUT; ++c) {
-                    double v;
-                    if constexpr (TPS == 1) v = acc[q].value(c);
-                    else v = acc[q].value(c, lane);
-                    if constexpr (op_has_out_scale<Op>::value) v *= Op::out_scale(c);
-                    dst[c] = v;
+                    for (int c = 0; c < NOUT; ++c) {
+                        double v;
+                        if constexpr (TPS == 1) v = acc[q].value(c);
+                        else v = acc[q].value(c, l);
+                        if constexpr (op_has_out_scale<Op>::value) v *= Op::out_scale(c);
+                        red[t * NOUT + c] = w == 0 ? v : red[t * NOUT + c] + v;
+                    }
                 }
             }
         }
+        __syncthreads();
     }
+    const int rows = min(GT, sg.n_tgt - tb * GT);
+    double* dst = part + (sg.part + (long long)chunk * sg.n_tgt + (long long)tb * GT) * NOUT;
+    for (int i = threadIdx.x; i < rows * NOUT; i += 32 * kSweepWarps) dst[i] = red[i];
+}
+
+// FP64 sums over at most kSeqFolds folds: one thread per target adds all sources
+// in their order, as the reference's loop does.  An optimiser run on a few
+// hundred points amplifies the last bits of its FP64 sums by 1e7 over 50
+// iterations, so these keep the reference's order to the bit; the sums are too
+// small for the split of the sweep above to gain anything (256 x 256 points: 8
+// blocks, one source after the other, 10 us).
+constexpr int kSeqFolds = 15;
+template <class Op>
+__global__ void __launch_bounds__(32) sweep_seq_kernel(const SegDesc sg, const typename Op::Params P,
+                                                       double* __restrict__ part) {
+    static_assert(Op::TPS == 1, "unpacked operators");
+    constexpr int NS = Op::NS, NOUT = Op::NOUT;
+    __shared__ __align__(16) float4 S[NS * kFold];
+    const long long t = (long long)blockIdx.x * 32 + threadIdx.x;   // rows are padded to whole groups
+    typename Op::Tgt tg;
+    Op::load_target(P, sg.tgt + t, tg);
+    typename Op::Acc acc;
+    acc.zero();
+    for (int f = 0; f < sg.n_folds; ++f) {
+        const float4* g = P.src4 + sg.src + (long long)f * kFold + threadIdx.x;
+        __syncwarp();
+#pragma unroll
+        for (int w = 0; w < NS; ++w) S[w * kFold + threadIdx.x] = g[(long long)w * P.src_stride];
+        __syncwarp();
+#pragma unroll 4
+        for (int j = 0; j < kFold; ++j) {
+            typename Op::Src s;
+            Op::load_source(S, j, s);
+            Op::pair(P, tg, s, acc);
+        }
+    }
+    if (t < sg.n_tgt)
+        for (int c = 0; c < NOUT; ++c) part[(sg.part + t) * NOUT + c] = acc.value(c);
 }
 
 // ---------------------------------------------------------------------------

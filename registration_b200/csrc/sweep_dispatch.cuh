@@ -19,9 +19,8 @@ int sweep_slots() {
     return 8 * device_info().sms;
 }
 
-// Problems with at most this many targets use the SMALL tile shape of the
-// packed operators that have one (more, smaller items: the large shape would
-// leave most SMs idle).
+// Problems with at most this many targets use the SMALL shape of the operators
+// that have one (groups of 64 targets: more, smaller items).
 #ifndef LDDMM_SMALL_TARGETS
 #define LDDMM_SMALL_TARGETS 4096
 #endif
@@ -29,36 +28,44 @@ constexpr long long kSmallTargets = LDDMM_SMALL_TARGETS;
 
 struct SinglePlan {
     long long n_tpad, m_pad;
-    int n_tb, n_src_tiles, split;
+    int n_tb, n_folds, split;
+    size_t box_words() const { return 2 * (size_t)(m_pad / kFold); }   // float4 words of the fold boxes
 };
 
 template <class Op>
 SinglePlan plan_single(long long n, long long m, int split_cap = 0) {
     SinglePlan p;
-    const long long per_block = (long long)Op::BLOCK * Op::R;
-    p.n_tb = (int)((n + per_block - 1) / per_block);
-    p.n_tpad = (long long)std::max(p.n_tb, 1) * per_block;
-    p.n_src_tiles = (int)((m + Op::TILE - 1) / Op::TILE);
-    p.m_pad = (long long)std::max(p.n_src_tiles, 1) * Op::TILE;
-    p.split = choose_split(p.n_tb, p.n_src_tiles, sweep_slots<Op>());
+    const long long per_group = op_group<Op>();
+    p.n_tb = (int)((n + per_group - 1) / per_group);
+    p.n_tpad = (long long)std::max(p.n_tb, 1) * per_group;
+    p.n_folds = (int)((m + kFold - 1) / kFold);
+    p.m_pad = (long long)std::max(p.n_folds, 1) * kFold;
+    p.split = choose_split(p.n_tb, p.n_folds, sweep_slots<Op>());
     if (split_cap > 0 && p.split > split_cap) p.split = split_cap;
     return p;
 }
 
-// SYM: symmetric sweep over sym_tiles own source tiles (see sweep_kernel<Op, true>)
+// boxes: fold boxes written with the packed sources, or NULL (every fold counts).
+// SYM: symmetric sweep over sym_folds own folds (see sweep_kernel<Op, true>)
 template <class Op, bool SYM = false>
-int launch_single(const SinglePlan& pl, long long n, const typename Op::Params& P, double* part, cudaStream_t st,
-                  int sym_tiles = 0) {
+int launch_single(const SinglePlan& pl, long long n, const typename Op::Params& P, const float4* boxes, double* part,
+                  cudaStream_t st, int sym_folds = 0) {
     SweepGrid g{};
     g.seg0.n_tgt = (int)n;
-    g.seg0.n_src_tiles = pl.n_src_tiles;
+    g.seg0.n_folds = pl.n_folds;
     g.seg0.n_tb = pl.n_tb;
     g.seg0.split = pl.split;
-    g.seg0.sym_tiles = sym_tiles;
+    g.seg0.sym_folds = sym_folds;
     g.nseg = 0;
     g.n_items = pl.n_tb * pl.split;
     if (g.n_items <= 0) return LDDMM_OK;
-    sweep_kernel<Op, SYM><<<g.n_items, Op::BLOCK, 0, st>>>(g, P, part);
+    if constexpr (sizeof(typename Op::Real) == 8 && !SYM) {
+        if (pl.n_folds <= kSeqFolds) {   // split is 1 for so few folds
+            sweep_seq_kernel<Op><<<(unsigned)((n + 31) / 32), 32, 0, st>>>(g.seg0, P, part);
+            return cuda_check(cudaGetLastError(), "sweep launch");
+        }
+    }
+    sweep_kernel<Op, SYM><<<g.n_items, 32 * kSweepWarps, 0, st>>>(g, P, boxes, part);
     return cuda_check(cudaGetLastError(), "sweep launch");
 }
 

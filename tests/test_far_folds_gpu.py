@@ -1,0 +1,122 @@
+"""Sweeps pass over folds of 32 sources that are too far from a target group to count.
+
+Every target's sum must stay what the sum over all pairs gives: the far part
+that is left out is bounded by 2^-36 (FP32c) or 2^-58 (FP64) of the sum of the
+absolute terms, so a row's error is compared with that sum.
+
+Tolerances.  FP32c: packed coordinates below 16 (the cloud spans at most 1.6 =
+27 units of the Gaussian's frame, 46 of the Laplacian's) carry 2^-21 each, so a
+difference is off by 2^-20 and the exponent of a term at distance r by
+2 sqrt(3) r 2^-20 + 4 r^2 2^-24; rows count while their largest terms have r^2 <=
+110, which gives 0.69 (3.5e-5 + 2.6e-5) = 4.2e-5, and half of that for the
+Laplacian: 1e-4.  FP64: the same with 2^-53 in place of 2^-24 and r^2 / 2 up to
+700, on both sides: 1e-12.
+"""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+SIGMA = 0.05
+
+
+def _points(layout, n, m, rng):
+    """Targets and sources whose memory order follows the shape (so that folds are compact) or not."""
+    t = np.linspace(0, 1, max(n, m))
+    line = np.stack([t, 0.2 * np.sin(9 * t), 0.1 * np.cos(7 * t)], axis=1)
+    if layout == "line":           # a curve of 20 kernel widths
+        return line[:n].copy(), line[:m].copy()
+    if layout == "clusters":       # targets twelve widths away from either cluster of sources
+        y = line[:m] * 0.1
+        y[m // 2:, 0] += 1.5
+        return line[:n] * 0.2 + np.array([0.7, 0.0, 0.0]), y
+    return rng.uniform(0, 1, (n, 3)), rng.uniform(0, 1, (m, 3))   # no order at all
+
+
+def _weights(kind, m, rng):
+    b = rng.standard_normal((m, 3))
+    if kind == "steep":            # the first sources weigh next to nothing, the last a lot
+        b *= np.exp(np.linspace(-40, 10, m))[:, None]
+    if kind == "zero":
+        b[: m // 2] = 0.0
+    if kind == "tiny":
+        b *= 1e-30
+    return b
+
+
+@pytest.mark.parametrize("precision,tol", [("fp32c", 1e-4), ("fp64", 1e-12)])
+@pytest.mark.parametrize("name,order", [("gauss", 10), ("laplacian", 3)])
+@pytest.mark.parametrize("layout", ["line", "clusters", "random"])
+@pytest.mark.parametrize("n,m,kind", [(129, 1023, "plain"), (1, 1057, "steep"), (640, 31, "plain"),
+                                      (300, 1600, "zero"), (65, 992, "tiny")])
+def test_rows_keep_their_sums(oracle_lib, precision, tol, name, order, layout, n, m, kind):
+    import torch
+    from oracle import lddmm_ref as ref
+    from registration_b200 import kernelFunctions as kf
+    rng = np.random.default_rng(n + m)
+    x, y = _points(layout, n, m, rng)
+    b, p = _weights(kind, m, rng), rng.standard_normal((n, 3))
+    K = kf.Kernel(name=name, sigma=SIGMA, order=order, precision=precision)
+    xd, yd, bd, pd = (torch.from_numpy(t).cuda() for t in (x, y, b, p))
+    dense = ref.kernel_matrix(ref.Kernel(name=name, sigma=SIGMA, order=order), x, y)
+    dist = np.linalg.norm(x[:, None] - y[None], axis=2)
+    bmax, pmax = np.abs(b).max(axis=1), np.abs(p).max(axis=1)
+    cond = dense @ bmax
+    # FP32 holds no digits of rows whose terms all lie below 2^-100 of the weights or near the smallest float
+    rows = cond > (max(1e-30 * bmax.max(), 1e-36) if precision == "fp32c" else 0.0)
+    f = K.applyK(yd, bd, firstVar=xd).cpu().numpy()
+    err = np.abs(f - oracle_lib.applyk(x, y, b, SIGMA, K.order)).max(axis=1)
+    assert (err[rows] <= tol * cond[rows]).all()
+    g = K.applyDiffKT(yd, [pd], [bd], firstVar=xd).cpu().numpy()
+    err = np.abs(g - oracle_lib.applykdifft(x, y, p[None], b[None], SIGMA, K.order)).max(axis=1)
+    gcond = 3 * pmax * (((dense * dist) @ bmax) / SIGMA ** 2 + cond / SIGMA)
+    assert (err[rows] <= tol * gcond[rows]).all()
+
+
+@pytest.mark.parametrize("precision", ["fp32c", "fp64"])
+@pytest.mark.parametrize("bad", [np.nan, np.inf])
+def test_non_finite_weights_are_never_passed_over(precision, bad):
+    """As in the sum over all pairs a bad weight reaches every row of its column, and no other column."""
+    import torch
+    from registration_b200 import kernelFunctions as kf
+    n, m = 300, 2000
+    x, y = _points("line", n, m, None)
+    b = np.ones((m, 3))
+    b[m - 7, 1] = bad
+    K = kf.Kernel(name="gauss", sigma=SIGMA, precision=precision)
+    f = K.applyK(torch.from_numpy(y).cuda(), torch.from_numpy(b).cuda(), firstVar=torch.from_numpy(x).cuda())
+    f = f.cpu().numpy()
+    assert not np.isfinite(f[:, 1]).any() and np.isfinite(f[:, [0, 2]]).all()
+
+
+@pytest.mark.parametrize("precision,tol", [("fp32c", 2e-5), ("fp64", 1e-11)])
+@pytest.mark.parametrize("norm", ["varifold", "current", "measure"])
+@pytest.mark.parametrize("level", [3, 4])
+def test_data_terms_of_narrow_kernels(oracle_lib, precision, tol, norm, level):
+    """Values and gradients where most of the sphere is far (1280 and 5120 cells, sigma 0.06), within `tol` of the
+    sums of the absolute terms."""
+    from oracle import lddmm_ref as ref
+    from registration_b200 import geometry as geo
+    from registration_b200 import kernelFunctions as kf
+    from registration_b200 import surfaces as sf
+    rng = np.random.default_rng(level)
+    sigma = 0.06
+    v, f = geo.icosphere(level)
+    vt = geo.bumped_sphere(v, f, 5, 0.3, 0.1, rng)
+    K, RK = kf.Kernel(name="gauss", sigma=sigma, precision=precision), ref.Kernel(name="gauss", sigma=sigma)
+    S, T = sf.Surface(FV=[f, v]), sf.Surface(FV=[f, vt])
+    RS, RT = ref.Surface(FV=[f, v]), ref.Surface(FV=[f, vt])
+    sfx = "_pairs" if norm == "varifold" else ""
+    area = np.linalg.norm(S.surfel, axis=1)
+    y = np.concatenate([S.centers, T.centers])
+    w = np.concatenate([area, np.linalg.norm(T.surfel, axis=1)])
+    vmag, gmag = 0.0, np.zeros(len(area))
+    for k in range(len(area)):
+        d = np.linalg.norm(S.centers[k] - y, axis=1)
+        kw = 2 * np.exp(-d ** 2 / (2 * sigma ** 2)) * w
+        vmag += area[k] * kw.sum()
+        gmag[k] = (kw * (area[k] * d / sigma ** 2 + 2 * np.sqrt(area[k]))).sum()
+    want = getattr(ref, norm + "NormDef" + sfx)(RS, RT, RK)
+    assert abs(getattr(sf, norm + "NormDef")(S, T, K) - want) <= tol * vmag
+    g, gw = getattr(sf, norm + "NormGradient")(S, T, K), getattr(ref, norm + "NormGradient" + sfx)(RS, RT, RK)
+    assert np.linalg.norm(g - gw) <= tol * 6 * np.linalg.norm(gmag)
