@@ -130,18 +130,18 @@ struct OpData {
 // Packed-pair FP32 varifold VALUE operator (two targets per thread slot, see
 // ops2.cuh): the per-pair arithmetic of OpData<float, ..., M_VARI_VALUE>
 //   acc += K(c_k, c_l) (1 + <n_k, n_l>^2) w_l
-// with sources stored as duplicated records [y0 y1 y2 n0 n1 n2 w] (4 words)
+// with sources stored as list records [y0 y1 y2 n0 n1 n2 w] (2 words)
 // and targets in the standard planes (pos word, normal word).  d = 3 only.
 template <int KIND, int PDEG>
 struct OpVariValue2 {
     using Real = float;
     static constexpr bool F32 = true;
-    static constexpr bool DUP = true;
+    static constexpr bool LIST = true;
     static constexpr int TPS = 2;
     static constexpr int R = 4;
     static constexpr int PP = 1;
     static constexpr int NV = 7;
-    static constexpr int NS = (NV + 1) / 2;
+    static constexpr int NS = (NV + 3) / 4;
     static constexpr int NOUT = 1;
     using Params = KernelParams2;
     using Acc = AccF32C2<1>;
@@ -158,7 +158,7 @@ struct OpVariValue2 {
         load_target_pair<3>(P.tgt4, P.tgt_stride, ra, rb, 0, t.x);
         load_target_pair<3>(P.tgt4, P.tgt_stride, ra, rb, 1, t.u);
     }
-    static LDDMM_D void load_source(const float4* S, int j, Src& s) { load_dup_source<NV>(S, j, s.val); }
+    static LDDMM_D void load_source(const float4* S, int j, Src& s) { load_list_source<NV>(S, j, s.val); }
     static LDDMM_D void pair(const Params& P, const Tgt& t, const Src& s, Acc& a) {
         f2 r2;
 #pragma unroll
@@ -181,19 +181,18 @@ struct OpVariValue2 {
 // 21 packed instructions per slot and source (Gaussian): acc[0..3) is summed
 // without its factor 2 (restored exactly by out_scale when written), and
 // 1 - <n,n'>^2 is formed as 2 - (1 + <n,n'>^2) from the factor the K' part needs.
-// Two packed slots per thread (R = 4): each 4-word source record read from
-// shared memory serves four target cells (11.6% faster than one slot at
-// F = 100k, 200k sources).
+// Two packed slots per thread (R = 4): each 2-word source record read from
+// shared memory serves four target cells.
 template <int KIND, int PDEG, int QDEG>
 struct OpVariGrad2 {
     using Real = float;
     static constexpr bool F32 = true;
-    static constexpr bool DUP = true;
+    static constexpr bool LIST = true;
     static constexpr int TPS = 2;
     static constexpr int R = 4;
     static constexpr int PP = 1;
     static constexpr int NV = 7;
-    static constexpr int NS = (NV + 1) / 2;
+    static constexpr int NS = (NV + 3) / 4;
     static constexpr int NOUT = 7;
     using Params = KernelParams2;
     using Acc = AccF32C2<NOUT>;
@@ -210,7 +209,7 @@ struct OpVariGrad2 {
         load_target_pair<3>(P.tgt4, P.tgt_stride, ra, rb, 0, t.x);
         load_target_pair<3>(P.tgt4, P.tgt_stride, ra, rb, 1, t.u);
     }
-    static LDDMM_D void load_source(const float4* S, int j, Src& s) { load_dup_source<NV>(S, j, s.val); }
+    static LDDMM_D void load_source(const float4* S, int j, Src& s) { load_list_source<NV>(S, j, s.val); }
     static LDDMM_D void pair(const Params& P, const Tgt& t, const Src& s, Acc& a) {
         f2 dx[3], r2;
 #pragma unroll
@@ -243,18 +242,18 @@ struct OpVariGrad2 {
 };
 
 // Packed-pair FP32 current GRADIENT operator (OpData<float, ..., M_CUR_GRAD>,
-// d = 3): sources [y0 y1 y2 s0 s1 s2] duplicated, targets (pos, s_k):
+// d = 3): sources [y0 y1 y2 s0 s1 s2], targets (pos, s_k):
 //   acc[0..3) += K s_l,  acc[3..6) += K' <s_k, s_l> (c_k - c_l)'
 template <int KIND, int PDEG, int QDEG>
 struct OpCurGrad2 {
     using Real = float;
     static constexpr bool F32 = true;
-    static constexpr bool DUP = true;
+    static constexpr bool LIST = true;
     static constexpr int TPS = 2;
     static constexpr int R = 2;
     static constexpr int PP = 1;
     static constexpr int NV = 6;
-    static constexpr int NS = (NV + 1) / 2;
+    static constexpr int NS = (NV + 3) / 4;
     static constexpr int NOUT = 6;
     using Params = KernelParams2;
     using Acc = AccF32C2<NOUT>;
@@ -271,7 +270,7 @@ struct OpCurGrad2 {
         load_target_pair<3>(P.tgt4, P.tgt_stride, ra, rb, 0, t.x);
         load_target_pair<3>(P.tgt4, P.tgt_stride, ra, rb, 1, t.u);
     }
-    static LDDMM_D void load_source(const float4* S, int j, Src& s) { load_dup_source<NV>(S, j, s.val); }
+    static LDDMM_D void load_source(const float4* S, int j, Src& s) { load_list_source<NV>(S, j, s.val); }
     static LDDMM_D void pair(const Params& P, const Tgt& t, const Src& s, Acc& a) {
         f2 dx[3], r2;
 #pragma unroll
@@ -298,16 +297,16 @@ struct OpCurGrad2 {
     }
 };
 
-// Operators with duplicated source records (DUP) take duplicated polynomial
-// coefficients and a duplicated source layout from the pack.
+// Packed operators (LIST) take duplicated polynomial coefficients and list
+// source records from the pack.
 template <class Op, class = void>
-struct op_dup : std::false_type {};
+struct op_list : std::false_type {};
 template <class Op>
-struct op_dup<Op, std::void_t<decltype(Op::DUP)>> : std::bool_constant<Op::DUP> {};
+struct op_list<Op, std::void_t<decltype(Op::LIST)>> : std::bool_constant<Op::LIST> {};
 
 template <class Op, class Real>
 inline void set_data_poly(typename Op::Params& P, const KScale& ks) {
-    if constexpr (op_dup<Op>::value) {
+    if constexpr (op_list<Op>::value) {
         for (int j = 0; j < 5; ++j) P.pkd[j] = dup_coeff(ks.pk[j]);
         for (int j = 0; j < 4; ++j) P.pqd[j] = dup_coeff(ks.pq[j]);
     } else {
@@ -370,7 +369,7 @@ LDDMM_D double vec_norm_eps(const double* s, int d, double eps) {
 template <class Real>
 LDDMM_D void dt_pack_record(int norm, int grad, bool is_t, const double* c, const double* s, int d, double eps,
                             double sign, double scale, const double* center, float4* planes, long long stride,
-                            long long i, int nplanes, int slots, bool dup = false, Real* bp = nullptr,
+                            long long i, int nplanes, int slots, bool list = false, Real* bp = nullptr,
                             Real* bw = nullptr) {
     constexpr int PP = PointPlanes<Real>::N;
     if (c == nullptr) {
@@ -388,8 +387,8 @@ LDDMM_D void dt_pack_record(int norm, int grad, bool is_t, const double* c, cons
             for (int j = 0; j < d; ++j) w = max_nan(w, (Real)(s[j] * sign));
         *bw = max_nan((Real)0, w);
     }
-    if (sizeof(Real) == 4 && dup) {
-        // duplicated source record [pos0 pos1 pos2 vals...], two values per word (see ops2.cuh)
+    if (sizeof(Real) == 4 && list) {
+        // list source record [pos0 pos1 pos2 vals...] (see ops2.cuh)
         double vals[4] = {0, 0, 0, 0};
         if (norm == NVARIFOLD) {
             for (int j = 0; j < 3; ++j) vals[j] = s[j] / a;
@@ -403,7 +402,7 @@ LDDMM_D void dt_pack_record(int norm, int grad, bool is_t, const double* c, cons
         for (int j = 0; j < 3; ++j) q[j] = (float)pos[j];
         for (int j = 0; j < slots && j < 4; ++j) q[3 + j] = (float)vals[j];
         for (int w = 0; w < nplanes; ++w)
-            planes[(long long)w * stride + i] = make_float4(q[2 * w], q[2 * w], q[2 * w + 1], q[2 * w + 1]);
+            planes[(long long)w * stride + i] = make_float4(q[4 * w], q[4 * w + 1], q[4 * w + 2], q[4 * w + 3]);
         return;
     }
     if constexpr (sizeof(Real) == 4) {
@@ -450,7 +449,7 @@ static __global__ void dt_pack_kernel(int norm, int grad, const double* __restri
                                       long long n2, int d, double eps1, double eps2, double sign2, double scale,
                                       const double* __restrict__ center, float4* tgt, long long tstride, int tplanes,
                                       int tslots, float4* src, long long sstride, int splanes, int sslots,
-                                      int dup, long long n1s, float4* boxes) {
+                                      int list, long long n1s, float4* boxes) {
     // set-2 sources start at row n1s (n1 rounded up to a fold for symmetric sweeps)
     const long long npad = tstride > sstride ? tstride : sstride;
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < npad;
@@ -464,7 +463,7 @@ static __global__ void dt_pack_kernel(int norm, int grad, const double* __restri
             const double* sv = first ? s1 + i * d : (second ? s2 + (i - n1s) * d : nullptr);
             Real bp[3], bw;
             dt_pack_record<Real>(norm, grad, false, c, sv, d, first ? eps1 : eps2, first ? 1.0 : sign2, scale, center,
-                                 src, sstride, i, splanes, sslots, dup != 0, bp, &bw);
+                                 src, sstride, i, splanes, sslots, list != 0, bp, &bw);
             store_fold_box<Real>(boxes, i, c != nullptr, bp, bw);
         }
     }

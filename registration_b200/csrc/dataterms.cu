@@ -71,7 +71,7 @@ int dt_sweep(const DataArgs& a, Workspace& ws, cudaStream_t st, int grad, double
     set_data_poly<Op, Real>(P, ks);
     dt_pack_kernel<Real><<<grid_for(std::max(pl.n_tpad, pl.m_pad)), 256, 0, st>>>(
         a.norm, grad, c1, s1, a.nc, a.c2, a.s2, a.nc2, a.d, a.eps1, a.eps2, sign2, ks.scale, center, tgt, pl.n_tpad,
-        Op::NT_, Op::TSLOTS, src, pl.m_pad, Op::NS, Op::SSLOTS, op_dup<Op>::value ? 1 : 0, n1s, boxes);
+        Op::NT_, Op::TSLOTS, src, pl.m_pad, Op::NS, Op::SSLOTS, op_list<Op>::value ? 1 : 0, n1s, boxes);
     return launch_single<Op, SYM>(pl, a.nc, P, boxes, part, st, (int)(n1s / kFold));
 }
 
@@ -104,7 +104,7 @@ int dt_impl(const DataArgs& a, Workspace& ws, cudaStream_t st) {
         int rc = LDDMM_OK;
         int nout = 1;
         if (a.norm == NVARIFOLD) {
-            // FP32: packed-pair operator (two targets per slot, duplicated sources)
+            // FP32: packed-pair operator (two targets per slot, list records)
             using Op = std::conditional_t<(sizeof(Real) == 4 && D == 3), DtOp<OpVariValue2<KIND, PDEG>, 3, 4, 2>,
                                           DtOp<OpData<Real, KIND, PDEG, QDEG, D, M_VARI_VALUE>, 3, 4,
                                                PP + (3 + PW - 1) / PW>>;

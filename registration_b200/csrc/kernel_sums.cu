@@ -29,7 +29,7 @@ struct ApplyKArgs {
 
 template <class Real, int KIND, int DEG, int D, int DIMB>
 int applyk_group(const ApplyKArgs& a, int col0, Workspace& ws, cudaStream_t st) {
-    // FP32: packed-pair operator (two targets per slot, duplicated source records);
+    // FP32: packed-pair operator (two targets per slot, list source records);
     // FP64: the plain operator on double records.
     using Op = std::conditional_t<sizeof(Real) == 4, OpApplyK2<KIND, DEG, D, DIMB>, OpApplyK<Real, KIND, DEG, D, DIMB>>;
     const SinglePlan pl = plan_single<Op>(a.n, a.m, a.split_cap);
@@ -61,7 +61,7 @@ int applyk_group(const ApplyKArgs& a, int col0, Workspace& ws, cudaStream_t st) 
     if constexpr (sizeof(Real) == 4) {
         for (int j = 0; j < 5; ++j) P.pkd[j] = dup_coeff(ks.pk[j]);
         for (int j = 0; j < 4; ++j) P.pqd[j] = dup_coeff(ks.pq[j]);
-        pack_dup_kernel<<<grid_for(pl.m_pad), 256, 0, st>>>(a.y, a.m, a.d, ks.scale, center, g, D, DIMB, src,
+        pack_list_kernel<<<grid_for(pl.m_pad), 256, 0, st>>>(a.y, a.m, a.d, ks.scale, center, g, D, DIMB, src,
                                                             pl.m_pad, pl.m_pad, boxes);
     } else {
         for (int j = 0; j < 5; ++j) P.pk[j] = (Real)ks.pk[j];
@@ -208,7 +208,7 @@ int difft_impl(const DiffKTArgs& a, Workspace& ws, cudaStream_t st) {
     if constexpr (sizeof(Real) == 4) {
         for (int j = 0; j < 5; ++j) P.pkd[j] = dup_coeff(ks.pk[j]);
         for (int j = 0; j < 4; ++j) P.pqd[j] = dup_coeff(ks.pq[j]);
-        pack_dup_kernel<<<grid_for(pl.m_pad), 256, 0, st>>>(a.y, a.m, a.d, ks.scale, center, gv, D, W, src,
+        pack_list_kernel<<<grid_for(pl.m_pad), 256, 0, st>>>(a.y, a.m, a.d, ks.scale, center, gv, D, W, src,
                                                             pl.m_pad, pl.m_pad, boxes);
     } else {
         for (int j = 0; j < 5; ++j) P.pk[j] = (Real)ks.pk[j];

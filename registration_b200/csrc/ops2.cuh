@@ -6,10 +6,20 @@
 // Same arithmetic as OpApplyK / OpDiffKT<float> (ops.cuh), evaluated for two
 // targets at once with `f32x2` instructions.  Layouts:
 //   targets : the standard planes (pos word, then values 4 per word);
-//   sources : "duplicated" records, the value list [y_0..y_{D-1}, v_0..v_{V-1}]
-//             with every value stored twice, two values per 16-byte word
-//             (v_a, v_a, v_b, v_b), so one shared-memory load yields two packed
-//             operands ready for the f32x2 instructions.
+//   sources : "list" records, the value list [y_0..y_{D-1}, v_0..v_{V-1}], four
+//             values per 16-byte word; splat2 makes the packed operand (v, v) of
+//             the f32x2 instructions from each.
+//
+// A record read by a warp returns its words to all 32 lanes at 128 bytes per
+// clock and SM, broadcast or not: a record of values stored twice (v, v), which
+// needs no splat, took 3 words = 12 clocks for the 128 pairs of a Gaussian applyK
+// whose FP32 arithmetic takes 9, so the sweep was bound by shared memory.  Two
+// words (6 values) take 8.  Measured at n = m = 131,072 (pairs/s, before ->
+// after): Gaussian applyK 2.78 -> 3.02e12, Laplacian 1.84 -> 1.93e12, Gaussian
+// applyDiffKT 2.02 -> 2.15e12, adjoint (W = 6) 1.62 -> 1.73e12, varifold value
+// 2.36 -> 2.47e12, varifold gradient 1.25 -> 1.33e12, current gradient 1.51 ->
+// 1.63e12.  Eight targets per thread instead of four gain nothing more and make
+// the groups coarser.
 #pragma once
 #include <cstring>
 
@@ -28,14 +38,16 @@ struct KernelParams2 {
     unsigned long long pqd[4];  // K' polynomial, duplicated
 };
 
-// Source records with duplicated values: NV values -> (NV + 1) / 2 words.
+// List record j of a fold: NV values, each splat over the two lanes.
 template <int NV>
-LDDMM_D void load_dup_source(const float4* S, int j, f2* val) {
+LDDMM_D void load_list_source(const float4* S, int j, f2* val) {
 #pragma unroll
-    for (int w = 0; w < (NV + 1) / 2; ++w) {
+    for (int w = 0; w < (NV + 3) / 4; ++w) {
         const float4 word = S[w * kFold + j];
-        val[2 * w] = word_lo(word);
-        if (2 * w + 1 < NV) val[2 * w + 1] = word_hi(word);
+        const float f[4] = {word.x, word.y, word.z, word.w};
+#pragma unroll
+        for (int q = 0; q < 4; ++q)
+            if (4 * w + q < NV) val[4 * w + q] = splat2(f[q]);
     }
 }
 
@@ -84,12 +96,12 @@ template <int KIND, int DEG, int D, int DIMB, bool SMALL = false>
 struct OpApplyK2 {
     using Real = float;
     static constexpr bool F32 = true;
-    static constexpr bool DUP = true;
+    static constexpr bool LIST = true;
     static constexpr int TPS = 2;
     static constexpr int R = SMALL ? 2 : 4;
     static constexpr int PP = 1;            // target planes: pos
     static constexpr int NV = D + DIMB;     // source values
-    static constexpr int NS = (NV + 1) / 2; // source words (duplicated values)
+    static constexpr int NS = (NV + 3) / 4; // source words
     static constexpr int NOUT = DIMB;
     using Params = KernelParams2;
     using Acc = AccF32C2<DIMB>;
@@ -104,7 +116,7 @@ struct OpApplyK2 {
     static LDDMM_D void load_target(const Params& P, long long ra, long long rb, Tgt& t) {
         load_target_pair<D>(P.tgt4, P.tgt_stride, ra, rb, 0, t.x);
     }
-    static LDDMM_D void load_source(const float4* S, int j, Src& s) { load_dup_source<NV>(S, j, s.val); }
+    static LDDMM_D void load_source(const float4* S, int j, Src& s) { load_list_source<NV>(S, j, s.val); }
     static LDDMM_D void pair(const Params& P, const Tgt& t, const Src& s, Acc& a) {
         f2 r2;
 #pragma unroll
@@ -122,12 +134,12 @@ template <int KIND, int DEG, int D, int W, bool SMALL = false>
 struct OpDiffKT2 {
     using Real = float;
     static constexpr bool F32 = true;
-    static constexpr bool DUP = true;
+    static constexpr bool LIST = true;
     static constexpr int TPS = 2;
     static constexpr int R = SMALL ? 2 : 4;
     static constexpr int PP = 1;
     static constexpr int NV = D + W;
-    static constexpr int NS = (NV + 1) / 2;
+    static constexpr int NS = (NV + 3) / 4;
     static constexpr int NT = 1 + (W + 3) / 4;  // target planes: pos, u values
     static constexpr int NOUT = D;
     using Params = KernelParams2;
@@ -145,7 +157,7 @@ struct OpDiffKT2 {
         load_target_pair<D>(P.tgt4, P.tgt_stride, ra, rb, 0, t.x);
         load_target_pair<W>(P.tgt4, P.tgt_stride, ra, rb, 1, t.u);
     }
-    static LDDMM_D void load_source(const float4* S, int j, Src& s) { load_dup_source<NV>(S, j, s.val); }
+    static LDDMM_D void load_source(const float4* S, int j, Src& s) { load_list_source<NV>(S, j, s.val); }
     static LDDMM_D void pair(const Params& P, const Tgt& t, const Src& s, Acc& a) {
         f2 dx[D], r2;
 #pragma unroll
@@ -170,9 +182,9 @@ inline unsigned long long dup_coeff(double c) {
     return ((unsigned long long)u << 32) | (unsigned long long)u;
 }
 
-// Packs sources into duplicated records (and the boxes of their folds): values [ (x_i - c) * s (D of them, zero
+// Packs sources into list records (and the boxes of their folds): values [ (x_i - c) * s (D of them, zero
 // beyond d), gather values (V of them, zero beyond g.nvals) ], rows >= n zero.
-static __global__ void pack_dup_kernel(const double* __restrict__ x, long long n, int d, double scale,
+static __global__ void pack_list_kernel(const double* __restrict__ x, long long n, int d, double scale,
                                        const double* __restrict__ center, const Gather g, int D, int V,
                                        float4* __restrict__ out, long long stride, long long n_pad,
                                        float4* __restrict__ boxes) {
@@ -180,15 +192,13 @@ static __global__ void pack_dup_kernel(const double* __restrict__ x, long long n
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n_pad;
          i += (long long)gridDim.x * blockDim.x) {
         float v[16];
-        for (int q = 0; q < nv && q < 16; ++q) v[q] = 0.f;
+        for (int q = 0; q < 16; ++q) v[q] = 0.f;
         if (i < n) {
             for (int j = 0; j < d && j < D; ++j) v[j] = (float)((x[i * d + j] - (center ? center[j] : 0.0)) * scale);
             for (int q = 0; q < V && q < g.nvals; ++q) v[D + q] = (float)(g.src[i * g.row_stride + g.off[q]] * g.mult);
         }
-        for (int w = 0; w < (nv + 1) / 2; ++w) {
-            const float a = v[2 * w], b = (2 * w + 1 < nv) ? v[2 * w + 1] : 0.f;
-            out[(long long)w * stride + i] = make_float4(a, a, b, b);
-        }
+        for (int w = 0; w < (nv + 3) / 4; ++w)
+            out[(long long)w * stride + i] = make_float4(v[4 * w], v[4 * w + 1], v[4 * w + 2], v[4 * w + 3]);
         if (boxes != nullptr) {
             float p[3], w = 0.f;
             for (int j = 0; j < 3; ++j) p[j] = j < D ? v[j] : 0.f;

@@ -183,13 +183,6 @@ static void rag_bbox_launch(RagSeg* dsegs, int nseg, int nbb, const double* x, c
     rag_bbox_finish_kernel<<<(nseg + 127) / 128, 128, 0, st>>>(dsegs, nseg, d, y != nullptr ? 1 : 0);
 }
 
-LDDMM_D void put_dup(float4* planes, long long stride, long long i, const float* v, int NV) {
-    for (int w = 0; w < (NV + 1) / 2; ++w) {
-        const float a = v[2 * w], b = (2 * w + 1 < NV) ? v[2 * w + 1] : 0.f;
-        planes[(long long)w * stride + i] = make_float4(a, a, b, b);
-    }
-}
-
 LDDMM_D void put_plain(float4* planes, long long stride, long long i, const float* v, int nv, int nwords) {
     for (int w = 0; w < nwords; ++w) {
         float q[4];
@@ -233,7 +226,7 @@ static __global__ void rag_shoot_pack_kernel(const RagSeg* __restrict__ segs, co
         }
         if (i < g.tpad) put_plain(tgt, tstride, g.tgt + i, pos, 3, 1);
         if (i < g.spad) {
-            put_dup(src, sstride, g.src + i, vals, 2 * D);
+            put_plain(src, sstride, g.src + i, vals, 2 * D, (2 * D + 3) / 4);
             rag_box<D>(boxes, g.src + i, i < g.n, vals, 2 * D);
         }
     }
@@ -386,7 +379,7 @@ static __global__ void rag_cov_pack_kernel(const RagSeg* __restrict__ segs, cons
             put_plain(tgt + tstride, tstride, g.tgt + i, u, 2 * D, (2 * D + 3) / 4);
         }
         if (i < g.spad) {
-            put_dup(src, sstride, g.src + i, v, 3 * D);
+            put_plain(src, sstride, g.src + i, v, 3 * D, (3 * D + 3) / 4);
             rag_box<D>(boxes, g.src + i, i < g.n, v, 3 * D);
         }
     }
@@ -510,7 +503,7 @@ static __global__ void rag_applyk_pack_kernel(const RagSeg* __restrict__ segs, c
                 for (int j = 0; j < d; ++j) v[j] = (float)((y[(g.m0 + i) * d + j] - g.center[j]) * g.scale);
                 for (int c = 0; c < dimb && c < DIMB; ++c) v[D + c] = (float)beta[(g.m0 + i) * dimb + c];
             }
-            put_dup(src, sstride, g.src + i, v, D + DIMB);
+            put_plain(src, sstride, g.src + i, v, D + DIMB, (D + DIMB + 3) / 4);
             rag_box<D>(boxes, g.src + i, i < g.m, v, D + DIMB);
         }
     }
@@ -603,7 +596,7 @@ static __global__ void rag_dt_pack_kernel(const RagSeg* __restrict__ segs, const
                                           const double* __restrict__ s1, const double* __restrict__ c2,
                                           const double* __restrict__ s2, int d, double eps1, double eps2,
                                           double sign2, float4* tgt, long long tstride, int tplanes, int tslots,
-                                          float4* src, long long sstride, int splanes, int sslots, int dup,
+                                          float4* src, long long sstride, int splanes, int sslots, int list,
                                           int sym_align, float4* boxes) {
     const long long total = padoff[nseg];
     for (long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x; q < total;
@@ -623,7 +616,7 @@ static __global__ void rag_dt_pack_kernel(const RagSeg* __restrict__ segs, const
             const double* sv = first ? s1 + (g.row0 + i) * d : (second ? s2 + (g.m0 + i - n1s) * d : nullptr);
             Real bp[3], bw;
             dt_pack_record<Real>(norm, grad, false, c, sv, d, first ? eps1 : eps2, first ? 1.0 : sign2, g.scale,
-                                 g.center, src, sstride, g.src + i, splanes, sslots, dup != 0, bp, &bw);
+                                 g.center, src, sstride, g.src + i, splanes, sslots, list != 0, bp, &bw);
             store_fold_box<Real>(boxes, g.src + i, c != nullptr, bp, bw);
         }
     }
@@ -755,7 +748,7 @@ int rag_dt_sweep(const RagDataArgs& a, int kind, int grad, double sign2, const d
     set_data_poly<Op, Real>(P, ks0);
     rag_dt_pack_kernel<Real><<<grid_for(padoff[nseg]), 256, 0, st>>>(
         dsegs, dpad, nseg, a.norm, grad, c1, s1, a.c2, a.s2, a.d, a.eps1, a.eps2, sign2, tgt, pl.tt, NT, TSLOTS, src,
-        pl.ss, Op::NS, SSLOTS, op_dup<Op>::value ? 1 : 0, SYM ? kFold : 0, boxes);
+        pl.ss, Op::NS, SSLOTS, op_list<Op>::value ? 1 : 0, SYM ? kFold : 0, boxes);
     SweepGrid grid{};
     grid.segs = ddesc;
     grid.nseg = nseg;
@@ -781,7 +774,7 @@ int rag_dt_impl(const RagDataArgs& a, Workspace& ws, cudaStream_t st) {
         int nout = 1, rc = LDDMM_OK;
         long long eparts = 0;
         if (a.norm == NVARIFOLD) {
-            // FP32: packed-pair operator (two targets per slot, duplicated sources)
+            // FP32: packed-pair operator (two targets per slot, list records)
             using Op = std::conditional_t<(sizeof(Real) == 4 && D == 3), OpVariValue2<KIND, PDEG>,
                                           OpData<Real, KIND, PDEG, QDEG, D, M_VARI_VALUE>>;
             RagPlan<Op> pl;

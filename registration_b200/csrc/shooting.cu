@@ -67,19 +67,16 @@ LDDMM_D void zero_record(float4* planes, long long stride, long long i, int npla
     for (int p = 0; p < nplanes; ++p) planes[(long long)p * stride + i] = make_float4(0.f, 0.f, 0.f, 0.f);
 }
 
-// Duplicated source record (packed-pair FP32 operators, ops2.cuh): values
-// [(x - c) * s for D coordinates, vals[0..nv) padded to V], each value twice.
-LDDMM_D void store_dup(float4* planes, long long stride, long long i, const double* x, int d, int D, double s,
-                       const double* c, const double* vals, int nv, int V) {
+// List source record (packed-pair FP32 operators, ops2.cuh): values
+// [(x - c) * s for D coordinates, vals[0..nv) padded to V].
+LDDMM_D void store_list(float4* planes, long long stride, long long i, const double* x, int d, int D, double s,
+                        const double* c, const double* vals, int nv, int V) {
     float v[16];
-    const int NV = D + V;
-    for (int q = 0; q < NV; ++q) v[q] = 0.f;
+    for (int q = 0; q < 16; ++q) v[q] = 0.f;
     for (int j = 0; j < d; ++j) v[j] = (float)((x[j] - c[j]) * s);
     for (int q = 0; q < nv && q < V; ++q) v[D + q] = (float)vals[q];
-    for (int w = 0; w < (NV + 1) / 2; ++w) {
-        const float a = v[2 * w], b = (2 * w + 1 < NV) ? v[2 * w + 1] : 0.f;
-        planes[(long long)w * stride + i] = make_float4(a, a, b, b);
-    }
+    for (int w = 0; w < (D + V + 3) / 4; ++w)
+        planes[(long long)w * stride + i] = make_float4(v[4 * w], v[4 * w + 1], v[4 * w + 2], v[4 * w + 3]);
 }
 
 // Fold box of source row i (whole warps, see store_fold_box): packed position
@@ -125,7 +122,7 @@ inline void set_poly(KernelParams2& P, const KScale& ks) {
 
 // ---- shooting ---------------------------------------------------------------
 // Packs step-0 planes: targets (pos) and sources (pos, a).
-template <class Real, bool DUP>
+template <class Real, bool LIST>
 static __global__ void shoot_pack_kernel(const double* __restrict__ x, const double* __restrict__ a, long long n,
                                          int d, double s, const double* __restrict__ c, float4* tgt,
                                          long long tstride, float4* src, long long sstride, int pp, int nslots,
@@ -137,8 +134,8 @@ static __global__ void shoot_pack_kernel(const double* __restrict__ x, const dou
         if (i < n) {
             if (i < tstride) store_point<Real>(tgt, tstride, i, x + i * d, d, s, c);
             if (i < sstride) {
-                if constexpr (DUP) {
-                    store_dup(src, sstride, i, x + i * d, d, nslots, s, c, a + i * d, d, nslots);
+                if constexpr (LIST) {
+                    store_list(src, sstride, i, x + i * d, d, nslots, s, c, a + i * d, d, nslots);
                 } else {
                     store_point<Real>(src, sstride, i, x + i * d, d, s, c);
                     store_vals<Real>(src, sstride, i, pp, a + i * d, d, nslots);
@@ -152,7 +149,7 @@ static __global__ void shoot_pack_kernel(const double* __restrict__ x, const dou
 }
 
 // v = sum of chunks; x1 = x0 + dt v; energy partial <a, v>; pack next step.
-template <class Real, bool DUP>
+template <class Real, bool LIST>
 static __global__ void shoot_combine_kernel(const double* __restrict__ part, long long n, int d, int dout,
                                             int split, double dt, const double* __restrict__ x0,
                                             const double* __restrict__ a0, double* __restrict__ x1,
@@ -174,8 +171,8 @@ static __global__ void shoot_combine_kernel(const double* __restrict__ part, lon
         if (a1 != nullptr) store_box<Real>(boxes, i, valid, xn, a1 + i * d, nullptr, d, s, c);
         if (a1 != nullptr && valid) {
             store_point<Real>(tgt, tstride, i, xn, d, s, c);
-            if constexpr (DUP) {
-                store_dup(src, sstride, i, xn, d, nslots, s, c, a1 + i * d, d, nslots);
+            if constexpr (LIST) {
+                store_list(src, sstride, i, xn, d, nslots, s, c, a1 + i * d, d, nslots);
             } else {
                 store_point<Real>(src, sstride, i, xn, d, s, c);
                 store_vals<Real>(src, sstride, i, pp, a1 + i * d, d, nslots);
@@ -226,8 +223,8 @@ static __global__ void trial_momenta_kernel(const double* __restrict__ at, const
 
 template <class Real, int KIND, int DEG, int D, bool SMALL = false>
 int shoot_impl(const ShootArgs& a, Workspace& ws, cudaStream_t st) {
-    constexpr bool DUP = sizeof(Real) == 4;  // FP32: packed-pair operator with duplicated sources
-    using Op = std::conditional_t<DUP, OpApplyK2<KIND, DEG, D, D, SMALL>, OpApplyK<Real, KIND, DEG, D, D, SMALL>>;
+    constexpr bool LIST = sizeof(Real) == 4;  // FP32: packed-pair operator with list records
+    using Op = std::conditional_t<LIST, OpApplyK2<KIND, DEG, D, D, SMALL>, OpApplyK<Real, KIND, DEG, D, D, SMALL>>;
     const SinglePlan pl = plan_single<Op>(a.n, a.n);
     float4* tgt = ws.take<float4>((size_t)Op::PP * pl.n_tpad);
     float4* src = ws.take<float4>((size_t)Op::NS * pl.m_pad);
@@ -247,12 +244,12 @@ int shoot_impl(const ShootArgs& a, Workspace& ws, cudaStream_t st) {
     const long long N = a.n * a.d;
     LDDMM_TRY(cuda_check(cudaMemcpyAsync(a.xt, a.x0, sizeof(double) * N, cudaMemcpyDeviceToDevice, st), "shoot copy"));
     launch_bbox_center(a.x0, a.n, nullptr, 0, a.d, center, st);
-    shoot_pack_kernel<Real, DUP><<<grid_for(std::max(pl.n_tpad, pl.m_pad)), 256, 0, st>>>(
+    shoot_pack_kernel<Real, LIST><<<grid_for(std::max(pl.n_tpad, pl.m_pad)), 256, 0, st>>>(
         a.x0, a.at, a.n, a.d, ks.scale, center, tgt, pl.n_tpad, src, pl.m_pad, Op::PP, D, Op::NS, boxes);
     const double dt = a.dt > 0 ? a.dt : 1.0 / a.T;
     for (int t = 0; t < a.T; ++t) {
         LDDMM_TRY(launch_single<Op>(pl, a.n, P, boxes, part, st));
-        shoot_combine_kernel<Real, DUP><<<nb, kCombineThreads, 0, st>>>(
+        shoot_combine_kernel<Real, LIST><<<nb, kCombineThreads, 0, st>>>(
             part, a.n, a.d, D, pl.split, dt, a.xt + t * N, a.at + t * N, a.xt + (t + 1) * N,
             t + 1 < a.T ? a.at + (t + 1) * N : nullptr, ks.scale, center, tgt, pl.n_tpad, src, pl.m_pad, Op::PP,
             D, boxes, epart + (long long)t * nb);
@@ -323,7 +320,7 @@ int shoot_run(const ShootArgs& a0, Workspace& ws, cudaStream_t st) {
 
 // ---- covector ---------------------------------------------------------------
 // planes of step t: targets (pos, u = (p - 2 rw a, a)), sources (pos, v = (a, p))
-template <class Real, bool DUP>
+template <class Real, bool LIST>
 LDDMM_D void cov_store(float4* tgt, long long tstride, float4* src, long long sstride, long long i, int pp,
                        const double* x, const double* a, const double* p, int d, double s, const double* c,
                        double rw, int tw) {
@@ -339,8 +336,8 @@ LDDMM_D void cov_store(float4* tgt, long long tstride, float4* src, long long ss
         store_vals<Real>(tgt, tstride, i, pp, u, 2 * d, tw);
     }
     if (i < sstride) {
-        if constexpr (DUP) {
-            store_dup(src, sstride, i, x, d, tw / 2, s, c, v, 2 * d, tw);
+        if constexpr (LIST) {
+            store_list(src, sstride, i, x, d, tw / 2, s, c, v, 2 * d, tw);
         } else {
             store_point<Real>(src, sstride, i, x, d, s, c);
             store_vals<Real>(src, sstride, i, pp, v, 2 * d, tw);
@@ -348,7 +345,7 @@ LDDMM_D void cov_store(float4* tgt, long long tstride, float4* src, long long ss
     }
 }
 
-template <class Real, bool DUP>
+template <class Real, bool LIST>
 static __global__ void cov_pack_kernel(const double* __restrict__ x, const double* __restrict__ a,
                                        const double* __restrict__ p, long long n, int d, double s,
                                        const double* __restrict__ c, double rw, float4* tgt, long long tstride,
@@ -359,7 +356,7 @@ static __global__ void cov_pack_kernel(const double* __restrict__ x, const doubl
          i += (long long)gridDim.x * blockDim.x) {
         if (i < sstride) store_box<Real>(boxes, i, i < n, x + i * d, a + i * d, p + i * d, d, s, c);
         if (i < n) {
-            cov_store<Real, DUP>(tgt, tstride, src, sstride, i, pp, x + i * d, a + i * d, p + i * d, d, s, c, rw, tw);
+            cov_store<Real, LIST>(tgt, tstride, src, sstride, i, pp, x + i * d, a + i * d, p + i * d, d, s, c, rw, tw);
         } else {
             if (i < tstride) zero_record<Real>(tgt, tstride, i, tplanes);
             if (i < sstride) zero_record<Real>(src, sstride, i, nplanes);
@@ -368,7 +365,7 @@ static __global__ void cov_pack_kernel(const double* __restrict__ x, const doubl
 }
 
 // p_t = p_{t+1} + dt * dscale * sum(chunks); dat_t = 2 rw a_t - p_{t+1}; pack step t-1.
-template <class Real, bool DUP>
+template <class Real, bool LIST>
 static __global__ void cov_combine_kernel(const double* __restrict__ part, long long n, int d, int dout, int split,
                                           double dt, double dscale, double rw, const double* __restrict__ p_next,
                                           const double* __restrict__ a_t, double* __restrict__ p_t,
@@ -390,7 +387,7 @@ static __global__ void cov_combine_kernel(const double* __restrict__ part, long 
         }
         if (x_prev != nullptr) store_box<Real>(boxes, i, valid, x_prev + i * d, a_prev + i * d, pn, d, s, c);
         if (x_prev != nullptr && valid)
-            cov_store<Real, DUP>(tgt, tstride, src, sstride, i, pp, x_prev + i * d, a_prev + i * d, pn, d, s, c, rw,
+            cov_store<Real, LIST>(tgt, tstride, src, sstride, i, pp, x_prev + i * d, a_prev + i * d, pn, d, s, c, rw,
                                  tw);
     }
 }
@@ -413,9 +410,9 @@ struct CovArgs {
 template <class Real, int KIND, int DEG, int D, bool SMALL = false>
 int cov_impl(const CovArgs& a, Workspace& ws, cudaStream_t st) {
     constexpr int W = 2 * D;
-    constexpr bool DUP = sizeof(Real) == 4;  // FP32: packed-pair operator with duplicated sources
-    using Op = std::conditional_t<DUP, OpDiffKT2<KIND, DEG, D, W, SMALL>, OpDiffKT<Real, KIND, DEG, D, W>>;
-    constexpr int NT = DUP ? 1 + (W + 3) / 4 : Op::NS;  // target planes (standard layout)
+    constexpr bool LIST = sizeof(Real) == 4;  // FP32: packed-pair operator with list records
+    using Op = std::conditional_t<LIST, OpDiffKT2<KIND, DEG, D, W, SMALL>, OpDiffKT<Real, KIND, DEG, D, W>>;
+    constexpr int NT = LIST ? 1 + (W + 3) / 4 : Op::NS;  // target planes (standard layout)
     const SinglePlan pl = plan_single<Op>(a.n, a.n);
     float4* tgt = ws.take<float4>((size_t)NT * pl.n_tpad);
     float4* src = ws.take<float4>((size_t)Op::NS * pl.m_pad);
@@ -436,13 +433,13 @@ int cov_impl(const CovArgs& a, Workspace& ws, cudaStream_t st) {
                                          cudaMemcpyDeviceToDevice, st), "covector copy"));
     const int T = a.T;
     launch_bbox_center(a.xt, a.n, nullptr, 0, a.d, center, st);
-    cov_pack_kernel<Real, DUP><<<grid_for(std::max(pl.n_tpad, pl.m_pad)), 256, 0, st>>>(
+    cov_pack_kernel<Real, LIST><<<grid_for(std::max(pl.n_tpad, pl.m_pad)), 256, 0, st>>>(
         a.xt + (long long)(T - 1) * N, a.at + (long long)(T - 1) * N, a.px1, a.n, a.d, ks.scale, center, a.rw,
         tgt, pl.n_tpad, src, pl.m_pad, Op::PP, NT, Op::NS, W, boxes);
     const int nb = combine_blocks(a.n);
     for (int t = T - 1; t >= 0; --t) {
         LDDMM_TRY(launch_single<Op>(pl, a.n, P, boxes, part, st));
-        cov_combine_kernel<Real, DUP><<<nb, kCombineThreads, 0, st>>>(
+        cov_combine_kernel<Real, LIST><<<nb, kCombineThreads, 0, st>>>(
             part, a.n, a.d, D, pl.split, dt, ks.dscale, a.rw, a.pxt + (long long)(t + 1) * N,
             a.at + (long long)t * N, a.pxt + (long long)t * N, a.dat ? a.dat + (long long)t * N : nullptr,
             t > 0 ? a.xt + (long long)(t - 1) * N : nullptr, t > 0 ? a.at + (long long)(t - 1) * N : nullptr,
