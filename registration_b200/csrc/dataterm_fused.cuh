@@ -333,7 +333,7 @@ __global__ void __launch_bounds__(kFusedThreads)
                         r2 = q == 0 ? dx[q] * dx[q] : r2 + dx[q] * dx[q];
                     }
                     Real kv, fv;
-                    kboth<Real, KIND, PDEG, QDEG>(pk, pq, r2, kv, fv);
+                    kboth<Real, KIND, PDEG, QDEG, true>(pk, pq, r2, kv, fv);
                     if (norm == NVARIFOLD) {
                         const Real dn = uk[0] * w[0] + uk[1] * w[1] + uk[2] * w[2];
                         const Real wk = kv * w[3];

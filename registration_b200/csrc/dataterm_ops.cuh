@@ -15,10 +15,10 @@ enum DataNorm : int { NCURRENT = 0, NMEASURE = 1, NVARIFOLD = 2 };
 enum DataMode : int { M_VARI_VALUE = 0, M_VARI_GRAD = 1, M_CUR_GRAD = 2, M_MEAS_GRAD = 3 };
 
 // Gaussian K' uses the same exponential as K.
-template <class Real, int KIND, int PDEG, int QDEG>
+template <class Real, int KIND, int PDEG, int QDEG, bool LIB>
 LDDMM_D void kboth(const Real* pk, const Real* pq, Real r2, Real& k, Real& f) {
     if constexpr (KIND == KGAUSS) {
-        k = kval<Real, KIND, 0>(pk, r2);
+        k = kval<Real, KIND, 0, LIB>(pk, r2);
         f = k;
     } else if constexpr (sizeof(Real) == 4) {
         const float u = sqrt_approx(r2);
@@ -27,14 +27,10 @@ LDDMM_D void kboth(const Real* pk, const Real* pq, Real r2, Real& k, Real& f) {
         f = (QDEG == 0 ? pq[0] : horner<QDEG>(pq, u)) * e;
     } else {
         const double u = sqrt(r2);
-        if (u < kZeroThresh) {
-            k = 1.0;
-            f = pq[0];
-        } else {
-            const double e = exp(-1.0 * u);
-            k = poly64<PDEG>(pk, u) * e;
-            f = poly64<QDEG>(pq, u) * e;
-        }
+        const bool zero = LIB ? u < kZeroThresh : less_nonneg(u, kZero2Lap);
+        const double e = LIB ? exp(-1.0 * u) : exp2neg(u);
+        k = zero ? 1.0 : poly64<PDEG>(pk, u) * e;
+        f = zero ? pq[0] : poly64<QDEG>(pq, u) * e;
     }
 }
 
@@ -66,7 +62,7 @@ struct OpData {
     using Acc = typename AccFor<Real>::template type<NOUT>;
     // K bounds the factor of K' as well (its polynomial Q is below P term by term)
     static constexpr bool GRADX = MODE != M_VARI_VALUE;
-    static LDDMM_D float lgk(const Params& P, float d2) { return lg_factor<KIND, PDEG, F32>(P.pk, d2); }
+    static LDDMM_D float lgk(const Params& P, float d2) { return lg_factor<KIND, PDEG>(P.pk, d2); }
     struct Tgt {
         Real x[D];
         Real u[L::TV > 0 ? L::TV : 1];
@@ -83,6 +79,7 @@ struct OpData {
         load_vals_smem<Real, D>(S, j, 0, s.y);
         load_vals_smem<Real, L::SV>(S, j, PP, s.v);
     }
+    template <bool LIB = false>
     static LDDMM_D void pair(const Params& P, const Tgt& t, const Src& s, Acc& acc) {
         Real dx[D], r2 = 0;
 #pragma unroll
@@ -91,12 +88,12 @@ struct OpData {
             r2 = j == 0 ? dx[j] * dx[j] : r2 + dx[j] * dx[j];
         }
         if constexpr (MODE == M_VARI_VALUE) {
-            const Real k = kval<Real, KIND, PDEG>(P.pk, r2);
+            const Real k = kval<Real, KIND, PDEG, LIB>(P.pk, r2);
             const Real dn = t.u[0] * s.v[0] + t.u[1] * s.v[1] + t.u[2] * s.v[2];
             acc.fma(0, k * s.v[3], (Real)1 + dn * dn);
         } else {
             Real k, f;
-            kboth<Real, KIND, PDEG, QDEG>(P.pk, P.pq, r2, k, f);
+            kboth<Real, KIND, PDEG, QDEG, LIB>(P.pk, P.pq, r2, k, f);
             if constexpr (MODE == M_VARI_GRAD) {
                 const Real dn = t.u[0] * s.v[0] + t.u[1] * s.v[1] + t.u[2] * s.v[2];
                 const Real wk = k * s.v[3];
@@ -146,7 +143,7 @@ struct OpVariValue2 {
     using Params = KernelParams2;
     using Acc = AccF32C2<1>;
     static constexpr bool GRADX = false;
-    static LDDMM_D float lgk(const Params& P, float d2) { return lg_factor<KIND, PDEG, true>(P.pkd, d2); }
+    static LDDMM_D float lgk(const Params& P, float d2) { return lg_factor<KIND, PDEG>(P.pkd, d2); }
     struct Tgt {
         f2 x[3];
         f2 u[3];
@@ -197,7 +194,7 @@ struct OpVariGrad2 {
     using Params = KernelParams2;
     using Acc = AccF32C2<NOUT>;
     static constexpr bool GRADX = true;
-    static LDDMM_D float lgk(const Params& P, float d2) { return lg_factor<KIND, PDEG, true>(P.pkd, d2); }
+    static LDDMM_D float lgk(const Params& P, float d2) { return lg_factor<KIND, PDEG>(P.pkd, d2); }
     struct Tgt {
         f2 x[3];
         f2 u[3];
@@ -258,7 +255,7 @@ struct OpCurGrad2 {
     using Params = KernelParams2;
     using Acc = AccF32C2<NOUT>;
     static constexpr bool GRADX = true;
-    static LDDMM_D float lgk(const Params& P, float d2) { return lg_factor<KIND, PDEG, true>(P.pkd, d2); }
+    static LDDMM_D float lgk(const Params& P, float d2) { return lg_factor<KIND, PDEG>(P.pkd, d2); }
     struct Tgt {
         f2 x[3];
         f2 u[3];

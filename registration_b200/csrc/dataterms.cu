@@ -58,6 +58,7 @@ int dt_sweep(const DataArgs& a, Workspace& ws, cudaStream_t st, int grad, double
              const double* s1, double*& part, SinglePlan& pl, const KScale& ks, const double* center) {
     const long long n1s = SYM ? round_up(a.nc, kFold) : a.nc;
     pl = plan_single<Op>(a.nc, n1s + a.nc2);
+    pl.seq = false;   // shapes of so few cells take the single-cluster kernels
     float4* tgt = ws.take<float4>((size_t)Op::NT_ * pl.n_tpad);
     float4* src = ws.take<float4>((size_t)Op::NS * pl.m_pad);
     float4* boxes = ws.take<float4>(pl.box_words());
@@ -91,7 +92,7 @@ int dt_impl(const DataArgs& a, Workspace& ws, cudaStream_t st) {
     double* c1 = ws.take<double>((size_t)a.nc * a.d);
     double* s1 = ws.take<double>((size_t)a.nc * a.d);
     double* center = ws.take<double>(kCenterWords);
-    const KScale ks = kernel_scale<Real>(KIND, a.order, a.sigma);
+    const KScale ks = kernel_scale(KIND, a.order, a.sigma, true);
     const int nb = (int)std::min<long long>(1024, (a.nc + kDtThreads - 1) / kDtThreads);
     if (!ws.measuring()) {
         cell_geometry_kernel<<<grid_for(a.nc), 256, 0, st>>>(a.ncorner, a.v, a.nv, a.d, a.cells, a.nc, c1, s1);
@@ -171,7 +172,7 @@ int dt_value_fused(const DataArgs& a, Workspace& ws, cudaStream_t st) {
     const FusedShape fs = fused_shape(a.nc);
     double* epart = ws.take<double>((size_t)kFusedMaxCluster * a.nbatch);
     if (ws.measuring()) return LDDMM_OK;
-    const KScale ks = kernel_scale<Real>(KIND, a.order, a.sigma);
+    const KScale ks = kernel_scale(KIND, a.order, a.sigma, sizeof(Real) == 4);
     FusedCoef cf{};
     for (int j = 0; j < 5; ++j) cf.pk[j] = ks.pk[j];
     for (int j = 0; j < 4; ++j) cf.pq[j] = ks.pq[j];
@@ -190,7 +191,7 @@ int dt_grad_fused(const DataArgs& a, Workspace& ws, cudaStream_t st) {
     double* z1 = ws.take<double>((size_t)a.nc * a.d);
     double* dz1 = ws.take<double>((size_t)a.nc * a.d);
     if (ws.measuring()) return LDDMM_OK;
-    const KScale ks = kernel_scale<Real>(KIND, a.order, a.sigma);
+    const KScale ks = kernel_scale(KIND, a.order, a.sigma, sizeof(Real) == 4);
     FusedCoef cf{};
     for (int j = 0; j < 5; ++j) cf.pk[j] = ks.pk[j];
     for (int j = 0; j < 4; ++j) cf.pq[j] = ks.pq[j];

@@ -77,7 +77,7 @@ static __global__ void __launch_bounds__(kMatThreads) kmat_kernel(const double* 
         for (long long l = threadIdx.x; l < m; l += blockDim.x) {
             double K;
             if constexpr (F32) K = (double)kval32<KIND, DEG>(P.pk32, mat_r2<true>(xk, y + l * d, d, P.scale));
-            else K = kval64<KIND, DEG>(P.pk64, mat_r2<false>(xk, y + l * d, d, P.scale));
+            else K = kval64<KIND, DEG, true>(P.pk64, mat_r2<false>(xk, y + l * d, d, P.scale));
             for (int c = 0; c < dimb; ++c) acc[c] += K * brow[l * dimb + c];
         }
         mat_block_sum(acc, dimb);
@@ -100,7 +100,7 @@ static __global__ void __launch_bounds__(kMatThreads) kdiffmat_kernel(const doub
             const double* yl = y + l * d;
             double F;
             if constexpr (F32) F = (double)kdiff32<KIND, QDEG>(P.pq32, mat_r2<true>(xk, yl, d, P.scale));
-            else F = kdiff64<KIND, QDEG>(P.pq64, mat_r2<false>(xk, yl, d, P.scale));
+            else F = kdiff64<KIND, QDEG, true>(P.pq64, mat_r2<false>(xk, yl, d, P.scale));
             F *= brow[l];
             for (int j = 0; j < d; ++j) acc[j] += F * ((xk[j] - yl[j]) * P.scale);
         }
@@ -112,7 +112,7 @@ static __global__ void __launch_bounds__(kMatThreads) kdiffmat_kernel(const doub
 
 template <bool F32>
 static MatParams mat_params(int kind, int order, double sigma) {
-    const KScale ks = F32 ? kernel_scale<float>(kind, order, sigma) : kernel_scale<double>(kind, order, sigma);
+    const KScale ks = kernel_scale(kind, order, sigma, F32);
     MatParams P{};
     P.scale = ks.scale;
     P.dscale = ks.dscale;

@@ -131,7 +131,7 @@ int dots_impl(const DotArgs& a, Workspace& ws, cudaStream_t st) {
     const int nb = (int)((a.n + kDotTargets - 1) / kDotTargets);
     double* partial = ws.take<double>((size_t)nb * a.T * a.m);
     if (ws.measuring()) return LDDMM_OK;
-    const KScale ks = kernel_scale<Real>(KIND, a.order, a.sigma);
+    const KScale ks = kernel_scale(KIND, a.order, a.sigma, sizeof(Real) == 4);
     FusedCoef cf{};
     for (int j = 0; j < 5; ++j) cf.pk[j] = ks.pk[j];
     for (int j = 0; j < 4; ++j) cf.pq[j] = ks.pq[j];

@@ -194,12 +194,12 @@ LDDMM_D void fused_vals(const FusedRec<Real>& r, Real* v) {
 template <class Real, int KIND, int DEG>
 LDDMM_D Real fused_k(const Real* pk, Real r2) {
     if constexpr (sizeof(Real) == 4) return kval32<KIND, DEG>(pk, r2);
-    else return kval64<KIND, DEG>(pk, r2);
+    else return kval64<KIND, DEG, true>(pk, r2);
 }
 template <class Real, int KIND, int QDEG>
 LDDMM_D Real fused_kd(const Real* pq, Real r2) {
     if constexpr (sizeof(Real) == 4) return kdiff32<KIND, QDEG>(pq, r2);
-    else return kdiff64<KIND, QDEG>(pq, r2);
+    else return kdiff64<KIND, QDEG, true>(pq, r2);
 }
 
 template <class Real, int N>

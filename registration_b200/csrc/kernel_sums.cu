@@ -43,7 +43,7 @@ int applyk_group(const ApplyKArgs& a, int col0, Workspace& ws, cudaStream_t st) 
         set_error("workspace too small: need %zu bytes, got %zu", ws.off, ws.cap);
         return LDDMM_ERR_WORKSPACE;
     }
-    const KScale ks = kernel_scale<Real>(KIND, a.order, a.sigma);
+    const KScale ks = kernel_scale(KIND, a.order, a.sigma, !pl.seq);
     typename Op::Params P{};
     P.src4 = src;
     P.src_stride = pl.m_pad;
@@ -184,7 +184,7 @@ int difft_impl(const DiffKTArgs& a, Workspace& ws, cudaStream_t st) {
     double* part = ws.take<double>((size_t)pl.split * a.n * D);
     double* center = ws.take<double>(kCenterWords);
     if (ws.measuring()) return LDDMM_OK;
-    const KScale ks = kernel_scale<Real>(KIND, a.order, a.sigma);
+    const KScale ks = kernel_scale(KIND, a.order, a.sigma, !pl.seq);
     typename Op::Params P{};
     P.src4 = src;
     P.src_stride = pl.m_pad;
@@ -308,7 +308,7 @@ int div_impl(const ApplyKArgs& a, Workspace& ws, cudaStream_t st) {
     double* part = ws.take<double>((size_t)pl.split * a.n);
     double* center = ws.take<double>(kCenterWords);
     if (ws.measuring()) return LDDMM_OK;
-    const KScale ks = kernel_scale<Real>(KIND, a.order, a.sigma, /*exact_tables=*/true);
+    const KScale ks = kernel_scale(KIND, a.order, a.sigma, !pl.seq, /*exact_tables=*/true);
     // (the reference's applyDivergence runs on its dense numpy matrices, which
     //  use the exact rational polynomials, kernelFunctions.py:75-88)
     typename Op::Params P{};

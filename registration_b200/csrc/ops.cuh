@@ -30,15 +30,16 @@ struct AccFor<double> {
     using type = AccF64<N>;
 };
 
-template <class Real, int KIND, int DEG>
+// LIB (FP64): exp() of the CUDA library in the x/s frame, see kfun.cuh
+template <class Real, int KIND, int DEG, bool LIB>
 LDDMM_D Real kval(const Real* pk, Real r2) {
     if constexpr (sizeof(Real) == 4) return kval32<KIND, DEG>(pk, r2);
-    else return kval64<KIND, DEG>(pk, r2);
+    else return kval64<KIND, DEG, LIB>(pk, r2);
 }
-template <class Real, int KIND, int DEG>
+template <class Real, int KIND, int DEG, bool LIB>
 LDDMM_D Real kdiff(const Real* pq, Real r2) {
     if constexpr (sizeof(Real) == 4) return kdiff32<KIND, DEG>(pq, r2);
-    else return kdiff64<KIND, DEG>(pq, r2);
+    else return kdiff64<KIND, DEG, LIB>(pq, r2);
 }
 
 template <class Real>
@@ -74,7 +75,7 @@ struct OpApplyK {
     using Params = KernelParamsBase<Real>;
     using Acc = typename AccFor<Real>::template type<DIMB>;
     static constexpr bool GRADX = false;
-    static LDDMM_D float lgk(const Params& P, float d2) { return lg_factor<KIND, DEG, F32>(P.pk, d2); }
+    static LDDMM_D float lgk(const Params& P, float d2) { return lg_factor<KIND, DEG>(P.pk, d2); }
     struct Tgt {
         Real x[D];
     };
@@ -89,6 +90,7 @@ struct OpApplyK {
         load_vals_smem<Real, D>(S, j, 0, s.y);
         load_vals_smem<Real, DIMB>(S, j, PP, s.b);
     }
+    template <bool LIB = false>
     static LDDMM_D void pair(const Params& P, const Tgt& t, const Src& s, Acc& a) {
         Real r2 = 0;
 #pragma unroll
@@ -96,7 +98,7 @@ struct OpApplyK {
             const Real dj = t.x[j] - s.y[j];
             r2 = j == 0 ? dj * dj : r2 + dj * dj;
         }
-        const Real k = kval<Real, KIND, DEG>(P.pk, r2);
+        const Real k = kval<Real, KIND, DEG, LIB>(P.pk, r2);
 #pragma unroll
         for (int c = 0; c < DIMB; ++c) a.fma(c, k, s.b[c]);
     }
@@ -118,7 +120,7 @@ struct OpDiffKT {
     using Params = KernelParamsBase<Real>;
     using Acc = typename AccFor<Real>::template type<D>;
     static constexpr bool GRADX = true;
-    static LDDMM_D float lgk(const Params& P, float d2) { return lg_factor<KIND, DEG, F32>(P.pq, d2); }
+    static LDDMM_D float lgk(const Params& P, float d2) { return lg_factor<KIND, DEG>(P.pq, d2); }
     struct Tgt {
         Real x[D];
         Real u[W];
@@ -135,6 +137,7 @@ struct OpDiffKT {
         load_vals_smem<Real, D>(S, j, 0, s.y);
         load_vals_smem<Real, W>(S, j, PP, s.v);
     }
+    template <bool LIB = false>
     static LDDMM_D void pair(const Params& P, const Tgt& t, const Src& s, Acc& a) {
         Real dx[D];
         Real r2 = 0;
@@ -146,7 +149,7 @@ struct OpDiffKT {
         Real dot = 0;
 #pragma unroll
         for (int w = 0; w < W; ++w) dot = w == 0 ? t.u[0] * s.v[0] : dot + t.u[w] * s.v[w];
-        const Real g = kdiff<Real, KIND, DEG>(P.pq, r2) * dot;
+        const Real g = kdiff<Real, KIND, DEG, LIB>(P.pq, r2) * dot;
 #pragma unroll
         for (int j = 0; j < D; ++j) a.fma(j, g, dx[j]);
     }
@@ -182,6 +185,7 @@ struct OpDivergence {
         load_vals_smem<Real, D>(S, j, 0, s.y);
         load_vals_smem<Real, D>(S, j, PP, s.a);
     }
+    template <bool LIB = false>
     static LDDMM_D void pair(const Params& P, const Tgt& t, const Src& s, Acc& acc) {
         Real r2 = 0, dot = 0;
 #pragma unroll
@@ -190,7 +194,7 @@ struct OpDivergence {
             r2 = j == 0 ? dj * dj : r2 + dj * dj;
             dot = j == 0 ? dj * s.a[j] : dot + dj * s.a[j];
         }
-        acc.fma(0, kdiff<Real, KIND, DEG>(P.pq, r2), dot);
+        acc.fma(0, kdiff<Real, KIND, DEG, LIB>(P.pq, r2), dot);
     }
 };
 

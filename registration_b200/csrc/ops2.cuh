@@ -106,7 +106,7 @@ struct OpApplyK2 {
     using Params = KernelParams2;
     using Acc = AccF32C2<DIMB>;
     static constexpr bool GRADX = false;
-    static LDDMM_D float lgk(const Params& P, float d2) { return lg_factor<KIND, DEG, true>(P.pkd, d2); }
+    static LDDMM_D float lgk(const Params& P, float d2) { return lg_factor<KIND, DEG>(P.pkd, d2); }
     struct Tgt {
         f2 x[D];
     };
@@ -145,7 +145,7 @@ struct OpDiffKT2 {
     using Params = KernelParams2;
     using Acc = AccF32C2<D>;
     static constexpr bool GRADX = true;
-    static LDDMM_D float lgk(const Params& P, float d2) { return lg_factor<KIND, DEG, true>(P.pqd, d2); }
+    static LDDMM_D float lgk(const Params& P, float d2) { return lg_factor<KIND, DEG>(P.pqd, d2); }
     struct Tgt {
         f2 x[D];
         f2 u[W];

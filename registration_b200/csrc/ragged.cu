@@ -307,7 +307,7 @@ int rag_shoot_impl(int nseg, const int64_t* v_off, int d, const double* x0, cons
     double* epart = ws.take<double>((size_t)std::max<long long>(1, pl.eparts));
     if (ws.measuring()) return LDDMM_OK;
     for (int s = 0; s < nseg; ++s) {
-        const KScale ks = kernel_scale<float>(KIND, order, sigma[s]);
+        const KScale ks = kernel_scale(KIND, order, sigma[s], true);
         pl.segs[s].scale = ks.scale;
         pl.segs[s].dscale = ks.dscale;
         pl.segs[s].rw = rw[s];
@@ -328,7 +328,7 @@ int rag_shoot_impl(int nseg, const int64_t* v_off, int d, const double* x0, cons
     P.src_stride = pl.ss;
     P.tgt4 = tgt;
     P.tgt_stride = pl.tt;
-    const KScale ks0 = kernel_scale<float>(KIND, order, sigma[0]);
+    const KScale ks0 = kernel_scale(KIND, order, sigma[0], true);
     for (int j = 0; j < 5; ++j) P.pkd[j] = dup_coeff(ks0.pk[j]);
     for (int j = 0; j < 4; ++j) P.pqd[j] = dup_coeff(ks0.pq[j]);
     SweepGrid grid{};
@@ -439,7 +439,7 @@ int rag_cov_impl(int nseg, const int64_t* v_off, int d, const double* xt, const 
     double* part = ws.take<double>((size_t)pl.parts * D);
     if (ws.measuring()) return LDDMM_OK;
     for (int s = 0; s < nseg; ++s) {
-        const KScale ks = kernel_scale<float>(KIND, order, sigma[s]);
+        const KScale ks = kernel_scale(KIND, order, sigma[s], true);
         pl.segs[s].scale = ks.scale;
         pl.segs[s].dscale = ks.dscale;
         pl.segs[s].rw = rw[s];
@@ -459,7 +459,7 @@ int rag_cov_impl(int nseg, const int64_t* v_off, int d, const double* xt, const 
     P.src_stride = pl.ss;
     P.tgt4 = tgt;
     P.tgt_stride = pl.tt;
-    const KScale ks0 = kernel_scale<float>(KIND, order, sigma[0]);
+    const KScale ks0 = kernel_scale(KIND, order, sigma[0], true);
     for (int j = 0; j < 5; ++j) P.pkd[j] = dup_coeff(ks0.pk[j]);
     for (int j = 0; j < 4; ++j) P.pqd[j] = dup_coeff(ks0.pq[j]);
     SweepGrid grid{};
@@ -558,7 +558,7 @@ int rag_applyk_impl(int nseg, const int64_t* t_start, const int64_t* t_count, co
     double* part = ws.take<double>((size_t)pl.parts * DIMB);
     if (ws.measuring()) return LDDMM_OK;
     for (int s = 0; s < nseg; ++s) {
-        const KScale ks = kernel_scale<float>(KIND, order, sigma[s]);
+        const KScale ks = kernel_scale(KIND, order, sigma[s], true);
         pl.segs[s].scale = ks.scale;
         pl.segs[s].dscale = ks.dscale;
     }
@@ -573,7 +573,7 @@ int rag_applyk_impl(int nseg, const int64_t* t_start, const int64_t* t_count, co
     P.src_stride = pl.ss;
     P.tgt4 = tgt;
     P.tgt_stride = pl.tt;
-    const KScale ks0 = kernel_scale<float>(KIND, order, sigma[0]);
+    const KScale ks0 = kernel_scale(KIND, order, sigma[0], true);
     for (int j = 0; j < 5; ++j) P.pkd[j] = dup_coeff(ks0.pk[j]);
     for (int j = 0; j < 4; ++j) P.pqd[j] = dup_coeff(ks0.pq[j]);
     SweepGrid grid{};
@@ -727,7 +727,7 @@ int rag_dt_sweep(const RagDataArgs& a, int kind, int grad, double sign2, const d
     part = ws.take<double>((size_t)pl.parts * Op::NOUT);
     if (ws.measuring()) return LDDMM_OK;
     for (int s = 0; s < nseg; ++s) {
-        const KScale ks = kernel_scale<Real>(kind, a.order, a.sigma[s]);
+        const KScale ks = kernel_scale(kind, a.order, a.sigma[s], true);
         pl.segs[s].scale = ks.scale;
         pl.segs[s].dscale = ks.dscale;
         if (a.frame)
@@ -744,7 +744,7 @@ int rag_dt_sweep(const RagDataArgs& a, int kind, int grad, double sign2, const d
     P.src_stride = pl.ss;
     P.tgt4 = tgt;
     P.tgt_stride = pl.tt;
-    const KScale ks0 = kernel_scale<Real>(kind, a.order, a.sigma[0]);
+    const KScale ks0 = kernel_scale(kind, a.order, a.sigma[0], true);
     set_data_poly<Op, Real>(P, ks0);
     rag_dt_pack_kernel<Real><<<grid_for(padoff[nseg]), 256, 0, st>>>(
         dsegs, dpad, nseg, a.norm, grad, c1, s1, a.c2, a.s2, a.d, a.eps1, a.eps2, sign2, tgt, pl.tt, NT, TSLOTS, src,

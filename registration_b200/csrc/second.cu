@@ -50,10 +50,10 @@ struct SecondParams : KernelParamsBase<Real> {
 };
 
 // F (first-derivative factor) and G (second) from the prescaled squared distance
-template <class Real, int KIND, int QDEG, int RDEG, bool SECOND>
+template <class Real, int KIND, int QDEG, int RDEG, bool SECOND, bool LIB>
 LDDMM_D void kfactors(const Real* pq, const Real* pr, Real r2, Real& F, Real& G) {
     if constexpr (KIND == KGAUSS) {
-        F = kdiff<Real, KIND, 0>(pq, r2);
+        F = kdiff<Real, KIND, 0, LIB>(pq, r2);
         G = F;
     } else if constexpr (sizeof(Real) == 4) {
         const float u = sqrt_approx(r2);
@@ -63,14 +63,10 @@ LDDMM_D void kfactors(const Real* pq, const Real* pr, Real r2, Real& F, Real& G)
         else G = 0.f;
     } else {
         const double u = sqrt(r2);
-        if (u < kZeroThresh) {
-            F = pq[0];
-            G = SECOND ? pr[0] : 0.0;
-        } else {
-            const double e = exp(-1.0 * u);
-            F = poly64<QDEG>(pq, u) * e;
-            G = SECOND ? poly64<RDEG>(pr, u) * e : 0.0;
-        }
+        const bool zero = LIB ? u < kZeroThresh : less_nonneg(u, kZero2Lap);
+        const double e = LIB ? exp(-1.0 * u) : exp2neg(u);
+        F = zero ? pq[0] : poly64<QDEG>(pq, u) * e;
+        G = !SECOND ? 0.0 : zero ? pr[0] : poly64<RDEG>(pr, u) * e;
     }
 }
 
@@ -106,6 +102,7 @@ struct OpSecond {
         load_vals_smem<Real, D>(S, j, 0, s.y);
         load_vals_smem<Real, L::SV>(S, j, PP, s.v);
     }
+    template <bool LIB = false>
     static LDDMM_D void pair(const Params& P, const Tgt& t, const Src& s, Acc& acc) {
         Real dx[D], r2 = 0;
 #pragma unroll
@@ -114,7 +111,7 @@ struct OpSecond {
             r2 = j == 0 ? dx[j] * dx[j] : r2 + dx[j] * dx[j];
         }
         Real F, G;
-        kfactors<Real, KIND, QDEG, RDEG, L::SECOND>(P.pq, P.pr, r2, F, G);
+        kfactors<Real, KIND, QDEG, RDEG, L::SECOND, LIB>(P.pq, P.pr, r2, F, G);
         if constexpr (MODE == S_D1 || MODE == S_D2 || MODE == S_D12) {
             // a1 of the <dx, .> product: target (D1), source (D2), difference (D12)
             Real dot = 0;
@@ -237,7 +234,8 @@ int second_impl(const SecondArgs& a, Workspace& ws, cudaStream_t st) {
     double* part = ws.take<double>((size_t)pl.split * a.n * Op::NOUT);
     double* center = ws.take<double>(kCenterWords);
     if (ws.measuring()) return LDDMM_OK;
-    const KScale ks = kernel_scale<Real>(KIND, a.order, a.sigma);
+    const bool base2 = !pl.seq;
+    const KScale ks = kernel_scale(KIND, a.order, a.sigma, base2);
     double Pp[5], Qq[4], Rr[3];
     laplacian_tables(a.order, Pp, Qq, Rr, false);
     typename Op::Params P{};
@@ -250,7 +248,7 @@ int second_impl(const SecondArgs& a, Workspace& ws, cudaStream_t st) {
     for (int j = 0; j < 5; ++j) P.pk[j] = (Real)ks.pk[j];
     for (int j = 0; j < 4; ++j) P.pq[j] = (Real)ks.pq[j];
     for (int j = 0; j < 3; ++j) {
-        P.pr[j] = (Real)(sizeof(Real) == 4 ? Rr[j] / Lj : Rr[j]);
+        P.pr[j] = (Real)(base2 ? Rr[j] / Lj : Rr[j]);
         Lj *= Lg;
     }
     const double s2 = a.sigma * a.sigma;

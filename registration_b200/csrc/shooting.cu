@@ -234,7 +234,7 @@ int shoot_impl(const ShootArgs& a, Workspace& ws, cudaStream_t st) {
     double* epart = ws.take<double>((size_t)a.T * nb);
     double* center = ws.take<double>(kCenterWords);
     if (ws.measuring()) return LDDMM_OK;
-    const KScale ks = kernel_scale<Real>(KIND, a.order, a.sigma);
+    const KScale ks = kernel_scale(KIND, a.order, a.sigma, !pl.seq);
     typename Op::Params P{};
     P.src4 = src;
     P.src_stride = pl.m_pad;
@@ -265,7 +265,7 @@ int shoot_fused(const ShootArgs& a, Workspace& ws, cudaStream_t st) {
     const FusedShape fs = fused_shape(a.n);
     double* epart = ws.take<double>((size_t)kFusedMaxCluster * a.nbatch);
     if (ws.measuring()) return LDDMM_OK;
-    const KScale ks = kernel_scale<Real>(KIND, a.order, a.sigma);
+    const KScale ks = kernel_scale(KIND, a.order, a.sigma, sizeof(Real) == 4);
     FusedCoef cf{};
     for (int j = 0; j < 5; ++j) cf.pk[j] = ks.pk[j];
     for (int j = 0; j < 4; ++j) cf.pq[j] = ks.pq[j];
@@ -420,7 +420,7 @@ int cov_impl(const CovArgs& a, Workspace& ws, cudaStream_t st) {
     double* part = ws.take<double>((size_t)pl.split * a.n * D);
     double* center = ws.take<double>(kCenterWords);
     if (ws.measuring()) return LDDMM_OK;
-    const KScale ks = kernel_scale<Real>(KIND, a.order, a.sigma);
+    const KScale ks = kernel_scale(KIND, a.order, a.sigma, !pl.seq);
     typename Op::Params P{};
     P.src4 = src;
     P.src_stride = pl.m_pad;
@@ -452,7 +452,7 @@ template <class Real, int KIND, int QDEG, int D>
 int cov_fused(const CovArgs& a, Workspace& ws, cudaStream_t st) {
     const FusedShape fs = fused_shape(a.n);
     if (ws.measuring()) return LDDMM_OK;
-    const KScale ks = kernel_scale<Real>(KIND, a.order, a.sigma);
+    const KScale ks = kernel_scale(KIND, a.order, a.sigma, sizeof(Real) == 4);
     FusedCoef cf{};
     for (int j = 0; j < 5; ++j) cf.pk[j] = ks.pk[j];
     for (int j = 0; j < 4; ++j) cf.pq[j] = ks.pq[j];
@@ -505,6 +505,7 @@ struct OpEPDiff {
         load_vals_smem<Real, D>(S, j, 0, s.y);
         load_vals_smem<Real, D>(S, j, PP, s.a);
     }
+    template <bool LIB = false>
     static LDDMM_D void pair(const Params& P, const Tgt& t, const Src& s, Acc& acc) {
         Real dx[D], r2 = 0, dot = 0;
 #pragma unroll
@@ -513,8 +514,8 @@ struct OpEPDiff {
             r2 = j == 0 ? dx[j] * dx[j] : r2 + dx[j] * dx[j];
             dot = j == 0 ? t.a[j] * s.a[j] : dot + t.a[j] * s.a[j];
         }
-        const Real k = kval<Real, KIND, PDEG>(P.pk, r2);
-        const Real g = kdiff<Real, KIND, QDEG>(P.pq, r2) * dot;
+        const Real k = kval<Real, KIND, PDEG, LIB>(P.pk, r2);
+        const Real g = kdiff<Real, KIND, QDEG, LIB>(P.pq, r2) * dot;
 #pragma unroll
         for (int j = 0; j < D; ++j) {
             acc.fma(j, k, s.a[j]);
@@ -586,7 +587,7 @@ int epd_impl(const EPDArgs& a, Workspace& ws, cudaStream_t st) {
     double* part = ws.take<double>((size_t)pl.split * a.n * Op::NOUT);
     double* center = ws.take<double>(kCenterWords);
     if (ws.measuring()) return LDDMM_OK;
-    const KScale ks = kernel_scale<Real>(KIND, a.order, a.sigma);
+    const KScale ks = kernel_scale(KIND, a.order, a.sigma, !pl.seq);
     typename Op::Params P{};
     P.src4 = src;
     P.src_stride = pl.m_pad;

@@ -111,18 +111,17 @@ struct op_has_out_scale<Op, std::void_t<decltype(Op::out_scale(0))>> : std::true
 
 // Resident blocks per SM that the register budget is cut for, and the unrolling
 // of the source loop.  Measured at n = m = 131,072 (FP32) and 32,768 (FP64):
-// FP32 runs best with 128 registers (4 blocks) and 8 sources in flight
-// (Gaussian applyK 2.69 -> 2.78e12 pairs/s against no bound and 4 sources,
-// Laplacian applyDiffKT 1.54 -> 1.62e12), FP64 with 128 registers and 4 sources
-// (varifold gradient 3.15 -> 3.35e11; 8 sources spill).  Operators with many
-// outputs or wide records keep 168 registers (3 blocks) instead of spilling.
+// both run best with 128 registers (4 blocks) and 8 sources in flight (FP32
+// Gaussian applyK 2.69 -> 2.78e12 pairs/s against no bound and 4 sources,
+// Laplacian applyDiffKT 1.54 -> 1.62e12; FP64 applyK 6.35 -> 6.5e11, varifold
+// gradient 4.1 -> 4.2e11).  Operators with many outputs or wide records keep 168
+// registers (3 blocks) instead of spilling.
 template <class Op>
 constexpr int op_min_blocks() {
     return sizeof(typename Op::Real) == 4 ? (Op::NOUT * Op::R > 24 || Op::NS > 6 ? 3 : 4)
                                           : (Op::NOUT > 4 || Op::NS > 5 ? 3 : 4);
 }
-template <class Op>
-constexpr int op_unroll() { return sizeof(typename Op::Real) == 4 ? 8 : 4; }
+constexpr int kSweepUnroll = 8;
 
 // Operators that bound their kernel factor (Op::lgk) can pass over far folds.
 template <class Op, class = void>
@@ -376,7 +375,7 @@ __global__ void __launch_bounds__(32 * kSweepWarps, op_min_blocks<Op>())
         const float4* S = ring + st * STAGE;
 #pragma unroll
         for (int q = 0; q < SLOTS; ++q) acc[q].begin_fold();
-#pragma unroll op_unroll<Op>()
+#pragma unroll kSweepUnroll
         for (int j = 0; j < kFold; ++j) {
             typename Op::Src s;
             Op::load_source(S, j, s);
@@ -451,7 +450,7 @@ __global__ void __launch_bounds__(32) sweep_seq_kernel(const SegDesc sg, const t
         for (int j = 0; j < kFold; ++j) {
             typename Op::Src s;
             Op::load_source(S, j, s);
-            Op::pair(P, tg, s, acc);
+            Op::template pair<true>(P, tg, s, acc);
         }
     }
     if (t < sg.n_tgt)

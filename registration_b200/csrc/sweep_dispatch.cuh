@@ -29,6 +29,7 @@ constexpr long long kSmallTargets = LDDMM_SMALL_TARGETS;
 struct SinglePlan {
     long long n_tpad, m_pad;
     int n_tb, n_folds, split;
+    bool seq;   // FP64 sums over few sources: sweep_seq_kernel, coordinates in the x/s frame (kfun.cuh)
     size_t box_words() const { return 2 * (size_t)(m_pad / kFold); }   // float4 words of the fold boxes
 };
 
@@ -41,6 +42,7 @@ SinglePlan plan_single(long long n, long long m, int split_cap = 0) {
     p.n_folds = (int)((m + kFold - 1) / kFold);
     p.m_pad = (long long)std::max(p.n_folds, 1) * kFold;
     p.split = choose_split(p.n_tb, p.n_folds, sweep_slots<Op>());
+    p.seq = sizeof(typename Op::Real) == 8 && p.n_folds <= kSeqFolds;   // split is 1 for so few folds
     if (split_cap > 0 && p.split > split_cap) p.split = split_cap;
     return p;
 }
@@ -59,8 +61,8 @@ int launch_single(const SinglePlan& pl, long long n, const typename Op::Params& 
     g.nseg = 0;
     g.n_items = pl.n_tb * pl.split;
     if (g.n_items <= 0) return LDDMM_OK;
-    if constexpr (sizeof(typename Op::Real) == 8 && !SYM) {
-        if (pl.n_folds <= kSeqFolds) {   // split is 1 for so few folds
+    if constexpr (sizeof(typename Op::Real) == 8) {
+        if (pl.seq) {
             sweep_seq_kernel<Op><<<(unsigned)((n + 31) / 32), 32, 0, st>>>(g.seg0, P, part);
             return cuda_check(cudaGetLastError(), "sweep launch");
         }
@@ -78,13 +80,13 @@ struct KScale {
     double dscale;  // sum_l K' 2 (x-y) <u,v> = dscale * sum_l F (x'-y') <u,v>
 };
 
-template <class Real>
-KScale kernel_scale(int kind, int order, double sigma, bool exact_tables = false) {
+// base2: the frame of the sweep kernels; otherwise x/s (see kfun.cuh).
+inline KScale kernel_scale(int kind, int order, double sigma, bool base2, bool exact_tables = false) {
     KScale k{};
     double P[5], Q[4], Rr[3];
     laplacian_tables(order, P, Q, Rr, exact_tables);
     const double L = 1.4426950408889634;  // log2(e)
-    if (sizeof(Real) == 4) {
+    if (base2) {
         k.scale = (kind == KGAUSS) ? std::sqrt(0.5 * L) / sigma : L / sigma;
         double Lj = 1.0;
         for (int j = 0; j < 5; ++j) {
