@@ -23,7 +23,7 @@ PROBE_SRC = os.path.join(HERE, "probe", "probe.cu")
 PROBE_LIB = os.path.join(HERE, "probe", "liblddmm_probe.so")
 NVCC = os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc")
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
-FLAGS = ["-O3", "-lineinfo", "-std=c++17", "-Xcompiler", "-fPIC", "-Xcompiler", "-fvisibility=hidden",
+FLAGS = ["-O3", "--split-compile", "0", "-lineinfo", "-std=c++17", "-Xcompiler", "-fPIC", "-Xcompiler", "-fvisibility=hidden",
          "--expt-relaxed-constexpr", "-I", os.path.join(ROOT, "include")]
 HOSTCC = "/usr/bin/g++" if os.path.exists("/usr/bin/g++") else None
 

@@ -29,6 +29,8 @@ struct SegDesc {
     int item0;        // first block index of this segment
     int sym_folds;    // > 0: the first sym_folds folds are the targets' own records and the
                       // sum is symmetric in (target, source): see sweep_kernel<Op, true>
+    int id;           // segment number (ragged launches)
+    int cnt;          // first counter of this segment's groups (see sweep_kernel)
 };
 
 struct SweepGrid {

@@ -301,17 +301,6 @@ struct op_list : std::false_type {};
 template <class Op>
 struct op_list<Op, std::void_t<decltype(Op::LIST)>> : std::bool_constant<Op::LIST> {};
 
-template <class Op, class Real>
-inline void set_data_poly(typename Op::Params& P, const KScale& ks) {
-    if constexpr (op_list<Op>::value) {
-        for (int j = 0; j < 5; ++j) P.pkd[j] = dup_coeff(ks.pk[j]);
-        for (int j = 0; j < 4; ++j) P.pqd[j] = dup_coeff(ks.pq[j]);
-    } else {
-        for (int j = 0; j < 5; ++j) P.pk[j] = (Real)ks.pk[j];
-        for (int j = 0; j < 4; ++j) P.pq[j] = (Real)ks.pq[j];
-    }
-}
-
 // ---- geometry -----------------------------------------------------------------
 // centres (nc, d), vectors (nc, d) (surfels or tangents) of set 1; invalid cell
 // indices give zero geometry (host code validates them before the call).
@@ -446,11 +435,13 @@ static __global__ void dt_pack_kernel(int norm, int grad, const double* __restri
                                       long long n2, int d, double eps1, double eps2, double sign2, double scale,
                                       const double* __restrict__ center, float4* tgt, long long tstride, int tplanes,
                                       int tslots, float4* src, long long sstride, int splanes, int sslots,
-                                      int list, long long n1s, float4* boxes) {
+                                      int list, long long n1s, float4* boxes, int* __restrict__ counters,
+                                      int n_counters) {
     // set-2 sources start at row n1s (n1 rounded up to a fold for symmetric sweeps)
     const long long npad = tstride > sstride ? tstride : sstride;
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < npad;
          i += (long long)gridDim.x * blockDim.x) {
+        if (i < n_counters) counters[i] = 0;
         if (i < tstride)
             dt_pack_record<Real>(norm, grad, true, i < n1 ? c1 + i * d : nullptr, i < n1 ? s1 + i * d : nullptr, d,
                                  eps1, 1.0, scale, center, tgt, tstride, i, tplanes, tslots);
@@ -466,7 +457,7 @@ static __global__ void dt_pack_kernel(int norm, int grad, const double* __restri
     }
 }
 
-// per-cell z1, dz1 of row i from the chunk sums (see dt_grad_combine_kernel)
+// per-cell z1, dz1 of row i from the chunk sums of its sums
 LDDMM_D void dt_grad_row(int norm, const double* acc, const double* s, int d, double eps1, double dzscale, double* z1,
                          double* dz1) {
     if (norm == NCURRENT) {
@@ -489,59 +480,56 @@ LDDMM_D void dt_grad_row(int norm, const double* acc, const double* s, int d, do
     }
 }
 
-constexpr int kDtThreads = 256;
-
-LDDMM_D void dt_block_sum(double v, double* out) {
-    __shared__ double red[kDtThreads];
-    red[threadIdx.x] = v;
-    __syncthreads();
-    for (int s = kDtThreads / 2; s > 0; s >>= 1) {
-        if (threadIdx.x < s) red[threadIdx.x] += red[threadIdx.x + s];
-        __syncthreads();
-    }
-    if (threadIdx.x == 0) out[blockIdx.x] = red[0];
+// what a cell adds to the energy: w1 . z (current: s1 . z, measure and varifold: a1 z)
+LDDMM_D double dt_value_row(int norm, const double* z, const double* s, int d, double eps1) {
+    if (norm != NCURRENT) return vec_norm_eps(s, d, eps1) * z[0];
+    double e = 0.0;
+    for (int j = 0; j < d; ++j) e += s[j] * z[j];
+    return e;
 }
 
-// energy partial: sum_k w1_k . acc_k (current: s1 . z, measure: a1 z, varifold: a1 z)
-static __global__ void dt_value_combine_kernel(int norm, const double* __restrict__ part, long long n1, int nout,
-                                               int split, const double* __restrict__ s1, int d, double eps1,
-                                               double* __restrict__ epart) {
-    double e = 0.0;
-    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n1;
-         i += (long long)gridDim.x * blockDim.x) {
-        double z[4] = {0, 0, 0, 0};
-        for (int c = 0; c < nout; ++c)
-            for (int k = 0; k < split; ++k) z[c] += part[((long long)k * n1 + i) * nout + c];
-        const double* s = s1 + i * d;
-        if (norm == NCURRENT) {
-            for (int j = 0; j < d; ++j) e += s[j] * z[j];
-        } else {
-            e += vec_norm_eps(s, d, eps1) * z[0];
+// Epilogue of the value sweeps: energy partial of the group's cells; the last group adds them.
+struct EpiDtValue {
+    static constexpr bool NONE = false;
+    int norm;
+    const double* s1;
+    int d;
+    double eps1;
+    double* epart;
+    int groups, op_rows;   // groups, and rows of one
+    int* counter;
+    double* energy;
+    template <int NOUT>
+    LDDMM_D void run(const SegDesc&, int row0, int rows, const double* red) const {
+        double e = 0.0;
+        for (int r = threadIdx.x; r < rows; r += blockDim.x)
+            e += dt_value_row(norm, red + r * NOUT, s1 + (long long)(row0 + r) * d, d, eps1);
+        e = block_sum_all(e);
+        if (threadIdx.x == 0) epart[row0 / op_rows] = e;
+        if (!last_block(counter, groups)) return;
+        e = 0.0;
+        for (int q = threadIdx.x; q < groups; q += blockDim.x) e += __ldcg(epart + q);
+        e = block_sum_all(e);
+        if (threadIdx.x == 0) *energy = e;
+    }
+};
+
+// Epilogue of the gradient sweeps: per-cell z1, dz1.
+struct EpiDtGrad {
+    static constexpr bool NONE = false;
+    int norm;
+    const double* s1;
+    int d;
+    double eps1, dzscale;
+    double *z1, *dz1;
+    template <int NOUT>
+    LDDMM_D void run(const SegDesc&, int row0, int rows, const double* red) const {
+        for (int r = threadIdx.x; r < rows; r += blockDim.x) {
+            const long long q = (long long)(row0 + r) * d;
+            dt_grad_row(norm, red + r * NOUT, s1 + q, d, eps1, dzscale, z1 + q, dz1 + q);
         }
     }
-    dt_block_sum(e, epart);
-}
-
-static __global__ void dt_finalize_kernel(const double* __restrict__ vals, long long count, double scale,
-                                          double* __restrict__ out) {
-    double v = 0.0;
-    for (long long i = threadIdx.x; i < count; i += blockDim.x) v += vals[i];
-    dt_block_sum(v, out);
-    if (threadIdx.x == 0) out[0] = scale * out[0];
-}
-
-// per-cell z1, dz1 from the gradient sweep
-static __global__ void dt_grad_combine_kernel(int norm, const double* __restrict__ part, long long n1, int nout,
-                                              int split, const double* __restrict__ s1, int d, double eps1,
-                                              double dzscale, double* __restrict__ z1, double* __restrict__ dz1) {
-    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n1;
-         i += (long long)gridDim.x * blockDim.x) {
-        double acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-        for (int c = 0; c < nout; ++c)
-            for (int k = 0; k < split; ++k) acc[c] += part[((long long)k * n1 + i) * nout + c];
-        dt_grad_row(norm, acc, s1 + i * d, d, eps1, dzscale, z1 + i * d, dz1 + i * d);
-    }
-}
+};
 
 // px[q] = 2 sum over the (cell, corner) entries of vertex q of the corner contribution.
 // L2ONLY: z1 / dz1 were written by other CTAs of the same launch (loads bypass L1).

@@ -51,31 +51,6 @@ struct DataArgs {
     long long vstride = 0;
 };
 
-// SYM (values): the cell-cell self part is evaluated once per unordered pair
-// (sweep_kernel<Op, true>); the target cells then start at a fold boundary.
-template <class Op, class Real, bool SYM = false>
-int dt_sweep(const DataArgs& a, Workspace& ws, cudaStream_t st, int grad, double sign2, const double* c1,
-             const double* s1, double*& part, SinglePlan& pl, const KScale& ks, const double* center) {
-    const long long n1s = SYM ? round_up(a.nc, kFold) : a.nc;
-    pl = plan_single<Op>(a.nc, n1s + a.nc2);
-    pl.seq = false;   // shapes of so few cells take the single-cluster kernels
-    float4* tgt = ws.take<float4>((size_t)Op::NT_ * pl.n_tpad);
-    float4* src = ws.take<float4>((size_t)Op::NS * pl.m_pad);
-    float4* boxes = ws.take<float4>(pl.box_words());
-    part = ws.take<double>((size_t)pl.split * a.nc * Op::NOUT);
-    if (ws.measuring()) return LDDMM_OK;
-    typename Op::Params P{};
-    P.src4 = src;
-    P.src_stride = pl.m_pad;
-    P.tgt4 = tgt;
-    P.tgt_stride = pl.n_tpad;
-    set_data_poly<Op, Real>(P, ks);
-    dt_pack_kernel<Real><<<grid_for(std::max(pl.n_tpad, pl.m_pad)), 256, 0, st>>>(
-        a.norm, grad, c1, s1, a.nc, a.c2, a.s2, a.nc2, a.d, a.eps1, a.eps2, sign2, ks.scale, center, tgt, pl.n_tpad,
-        Op::NT_, Op::TSLOTS, src, pl.m_pad, Op::NS, Op::SSLOTS, op_list<Op>::value ? 1 : 0, n1s, boxes);
-    return launch_single<Op, SYM>(pl, a.nc, P, boxes, part, st, (int)(n1s / kFold));
-}
-
 // Adapters giving OpApplyK / OpData a uniform plane description.
 template <class Base, int TSLOTS_, int SSLOTS_, int NT>
 struct DtOp : Base {
@@ -84,83 +59,91 @@ struct DtOp : Base {
     static constexpr int SSLOTS = SSLOTS_;
 };
 
+// One sweep over the cell pairs: the value into a.energy, or (GRAD) the cells' z1, dz1.
+// Values are SYM: the cell-cell self part is evaluated once per unordered pair
+// (sweep_kernel<Op, true>); the target cells then start at a fold boundary.
+template <class Op, class Real, bool GRAD>
+int dt_sweep(const DataArgs& a, Workspace& ws, cudaStream_t st, const double* c1, const double* s1, const KScale& ks,
+             const double* center, double* z1, double* dz1) {
+    constexpr bool SYM = !GRAD;
+    const long long n1s = SYM ? round_up(a.nc, kFold) : a.nc;
+    SinglePlan pl = plan_single<Op>(a.nc, n1s + a.nc2);
+    pl.seq = false;   // shapes of so few cells take the single-cluster kernels
+    float4* tgt = ws.take<float4>((size_t)Op::NT_ * pl.n_tpad);
+    float4* src = ws.take<float4>((size_t)Op::NS * pl.m_pad);
+    float4* boxes = ws.take<float4>(pl.box_words());
+    double* part = ws.take<double>(pl.part_doubles(a.nc, Op::NOUT));
+    int* counters = ws.take<int>(pl.counters());
+    double* epart = ws.take<double>(GRAD ? 0 : pl.n_tb);
+    if (ws.measuring()) return LDDMM_OK;
+    typename Op::Params P{};
+    P.src4 = src;
+    P.src_stride = pl.m_pad;
+    P.tgt4 = tgt;
+    P.tgt_stride = pl.n_tpad;
+    set_poly(P, ks);
+    dt_pack_kernel<Real><<<grid_for(std::max(pl.n_tpad, pl.m_pad)), 256, 0, st>>>(
+        a.norm, GRAD ? 1 : 0, c1, s1, a.nc, a.c2, a.s2, a.nc2, a.d, a.eps1, a.eps2, GRAD ? -1.0 : -2.0, ks.scale,
+        center, tgt, pl.n_tpad, Op::NT_, Op::TSLOTS, src, pl.m_pad, Op::NS, Op::SSLOTS, op_list<Op>::value ? 1 : 0,
+        n1s, boxes, counters, (int)pl.counters());
+    if constexpr (GRAD) {
+        const double fac = a.ncorner == 3 ? 1.0 / 3.0 : 0.5;
+        const EpiDtGrad E{a.norm, s1, a.d, a.eps1, fac * ks.dscale, z1, dz1};
+        return launch_single<Op, false>(pl, a.nc, P, boxes, part, st, 0, counters, E);
+    } else {
+        const EpiDtValue E{a.norm, s1, a.d, a.eps1, epart, pl.n_tb, op_group<Op>(), counters + pl.n_tb, a.energy};
+        return launch_single<Op, true>(pl, a.nc, P, boxes, part, st, (int)(n1s / kFold), counters, E);
+    }
+}
+
 // SMALL: the small groups of OpApplyK (few target cells); the other operators have one shape.
 template <class Real, int KIND, int PDEG, int QDEG, int D, bool SMALL = false>
 int dt_impl(const DataArgs& a, Workspace& ws, cudaStream_t st) {
     constexpr int PW = Traits<Real>::PER_WORD;
     constexpr int PP = PointPlanes<Real>::N;
+    constexpr bool PACK = sizeof(Real) == 4 && D == 3;   // FP32 surfaces: packed-pair operators with list records
     double* c1 = ws.take<double>((size_t)a.nc * a.d);
     double* s1 = ws.take<double>((size_t)a.nc * a.d);
     double* center = ws.take<double>(kCenterWords);
     const KScale ks = kernel_scale(KIND, a.order, a.sigma, true);
-    const int nb = (int)std::min<long long>(1024, (a.nc + kDtThreads - 1) / kDtThreads);
     if (!ws.measuring()) {
         cell_geometry_kernel<<<grid_for(a.nc), 256, 0, st>>>(a.ncorner, a.v, a.nv, a.d, a.cells, a.nc, c1, s1);
         launch_bbox_center(c1, a.nc, a.c2, a.nc2, a.d, center, st);
     }
     if (a.energy != nullptr) {
-        double* part = nullptr;
-        SinglePlan pl{};
-        double* epart = nullptr;
-        int rc = LDDMM_OK;
-        int nout = 1;
         if (a.norm == NVARIFOLD) {
-            // FP32: packed-pair operator (two targets per slot, list records)
-            using Op = std::conditional_t<(sizeof(Real) == 4 && D == 3), DtOp<OpVariValue2<KIND, PDEG>, 3, 4, 2>,
+            using Op = std::conditional_t<PACK, DtOp<OpVariValue2<KIND, PDEG>, 3, 4, 2>,
                                           DtOp<OpData<Real, KIND, PDEG, QDEG, D, M_VARI_VALUE>, 3, 4,
                                                PP + (3 + PW - 1) / PW>>;
-            rc = dt_sweep<Op, Real, true>(a, ws, st, 0, -2.0, c1, s1, part, pl, ks, center);
-            nout = Op::NOUT;
+            LDDMM_TRY((dt_sweep<Op, Real, false>(a, ws, st, c1, s1, ks, center, nullptr, nullptr)));
         } else if (a.norm == NCURRENT) {
             using Op = DtOp<OpApplyK<Real, KIND, PDEG, D, D, SMALL>, 0, D, PP>;
-            rc = dt_sweep<Op, Real, true>(a, ws, st, 0, -2.0, c1, s1, part, pl, ks, center);
-            nout = Op::NOUT;
+            LDDMM_TRY((dt_sweep<Op, Real, false>(a, ws, st, c1, s1, ks, center, nullptr, nullptr)));
         } else {
             using Op = DtOp<OpApplyK<Real, KIND, PDEG, D, 1, SMALL>, 0, 1, PP>;
-            rc = dt_sweep<Op, Real, true>(a, ws, st, 0, -2.0, c1, s1, part, pl, ks, center);
-            nout = Op::NOUT;
-        }
-        if (rc != LDDMM_OK) return rc;
-        epart = ws.take<double>((size_t)nb);
-        if (!ws.measuring()) {
-            dt_value_combine_kernel<<<nb, kDtThreads, 0, st>>>(a.norm, part, a.nc, nout, pl.split, s1, a.d, a.eps1,
-                                                               epart);
-            dt_finalize_kernel<<<1, kDtThreads, 0, st>>>(epart, nb, 1.0, a.energy);
+            LDDMM_TRY((dt_sweep<Op, Real, false>(a, ws, st, c1, s1, ks, center, nullptr, nullptr)));
         }
     }
     if (a.px != nullptr) {
-        double* part = nullptr;
-        SinglePlan pl{};
-        int rc = LDDMM_OK;
-        int nout = 1;
-        constexpr bool PACK = sizeof(Real) == 4 && D == 3;   // FP32 surfaces: packed-pair operators
+        double* z1 = ws.take<double>((size_t)a.nc * a.d);
+        double* dz1 = ws.take<double>((size_t)a.nc * a.d);
         if (a.norm == NVARIFOLD) {
             using Op = std::conditional_t<PACK, DtOp<OpVariGrad2<KIND, PDEG, QDEG>, 3, 4, 2>,
                                           DtOp<OpData<Real, KIND, PDEG, QDEG, D, M_VARI_GRAD>, 3, 4,
                                                PP + (3 + PW - 1) / PW>>;
-            rc = dt_sweep<Op, Real>(a, ws, st, 1, -1.0, c1, s1, part, pl, ks, center);
-            nout = Op::NOUT;
+            LDDMM_TRY((dt_sweep<Op, Real, true>(a, ws, st, c1, s1, ks, center, z1, dz1)));
         } else if (a.norm == NCURRENT) {
             using Op = std::conditional_t<PACK, DtOp<OpCurGrad2<KIND, PDEG, QDEG>, D, D, 2>,
                                           DtOp<OpData<Real, KIND, PDEG, QDEG, D, M_CUR_GRAD>, D, D,
                                                PP + (D + PW - 1) / PW>>;
-            rc = dt_sweep<Op, Real>(a, ws, st, 1, -1.0, c1, s1, part, pl, ks, center);
-            nout = Op::NOUT;
+            LDDMM_TRY((dt_sweep<Op, Real, true>(a, ws, st, c1, s1, ks, center, z1, dz1)));
         } else {
             using Op = DtOp<OpData<Real, KIND, PDEG, QDEG, D, M_MEAS_GRAD>, 0, 1, PP>;
-            rc = dt_sweep<Op, Real>(a, ws, st, 1, -1.0, c1, s1, part, pl, ks, center);
-            nout = Op::NOUT;
+            LDDMM_TRY((dt_sweep<Op, Real, true>(a, ws, st, c1, s1, ks, center, z1, dz1)));
         }
-        if (rc != LDDMM_OK) return rc;
-        double* z1 = ws.take<double>((size_t)a.nc * a.d);
-        double* dz1 = ws.take<double>((size_t)a.nc * a.d);
-        if (!ws.measuring()) {
-            const double fac = a.ncorner == 3 ? 1.0 / 3.0 : 0.5;
-            dt_grad_combine_kernel<<<grid_for(a.nc), 256, 0, st>>>(a.norm, part, a.nc, nout, pl.split, s1, a.d,
-                                                                   a.eps1, fac * ks.dscale, z1, dz1);
+        if (!ws.measuring())
             dt_gather_kernel<<<grid_for(a.nv), 256, 0, st>>>(a.ncorner, a.v, a.nv, a.d, a.cells, a.nc, a.vptr,
                                                              a.vidx, z1, dz1, a.px);
-        }
     }
     if (ws.measuring()) return LDDMM_OK;
     return cuda_check(cudaGetLastError(), "dataterm");

@@ -41,17 +41,37 @@ DeviceInfo device_info();
 // Maximum resident blocks per SM of a kernel (cached by the caller per kernel).
 int occupancy_blocks(const void* kernel, int block, size_t dyn_smem = 0);
 
-// Number of source chunks for a sweep: enough items (target groups x chunks)
-// for about 8 waves of `slots` resident blocks, at least kMinFolds folds of 32
-// sources for each of a block's four warps.  `slots` is taken as 8 blocks per
-// SM for every operator, so the split (and the workspace) depends only on the
-// shape and the SM count.
-constexpr int kMinFolds = 4;
-inline int choose_split(int n_tb, int n_folds, int slots) {
+// Number of source chunks of a sweep over n_tb target groups and n_folds folds
+// of 32 sources; `resident` blocks fit the device at once, a block's four warps
+// share the folds of its chunk.  A function of the operator, the shape and the
+// SM count only (workspace queries run the same code).
+//   Many blocks (four waves and more): up to 64 blocks per SM, at least 16 folds
+// per warp, so that groups whose far folds are passed over balance out.
+//   Fewer: waves count.  The chunks that make ceil(blocks / resident) (folds per
+// warp + kBlockFolds) smallest, kBlockFolds being what a block's start and end
+// cost in folds (3,166 points, 11 / 8 / 5 chunks: 404 / 392 / 420 us per shot and
+// adjoint; 10,242 points, adjoint sweeps with 444 resident blocks: 5 chunks = 405
+// blocks 1421 us, 6 chunks = 486 blocks 1542 us).
+//   A segment of a ragged launch (`shared`) has the other segments beside it: 8
+// folds per warp (template step of 8 x 2,562 points with 4 / 8 / 16: 2792 / 2778 /
+// 2945 us, with a lone problem's chunks 3231).
+// Varifold gradient of 20,480 cells, 4 / 8 / 16 folds per warp: 431 / 422 / 382 us.
+constexpr int kBlockFolds = 3;
+inline int choose_split(int n_tb, int n_folds, int sms, int resident, bool shared) {
     if (n_tb <= 0 || n_folds <= 0) return 1;
-    long long want = (8LL * slots + n_tb - 1) / n_tb;
-    int max_split = std::max(1, n_folds / (4 * kMinFolds));
-    return (int)std::max(1LL, std::min<long long>(want, max_split));
+    const long long want = (64LL * sms + n_tb - 1) / n_tb;
+    const long long many = std::max(1LL, std::min<long long>(want, n_folds / (4 * (shared ? 8 : 16))));
+    if (shared || many * n_tb >= 4LL * resident) return (int)many;
+    long long best = 1, best_cost = -1;
+    for (long long s = 1; s <= (n_folds + 3) / 4 && s * n_tb <= 4LL * resident + n_tb; ++s) {
+        const long long waves = (s * n_tb + resident - 1) / resident;
+        const long long cost = waves * ((n_folds + 4 * s - 1) / (4 * s) + kBlockFolds);
+        if (best_cost < 0 || cost < best_cost) {
+            best = s;
+            best_cost = cost;
+        }
+    }
+    return (int)best;
 }
 
 inline long long round_up(long long v, long long m) { return (v + m - 1) / m * m; }

@@ -36,7 +36,8 @@ int applyk_group(const ApplyKArgs& a, int col0, Workspace& ws, cudaStream_t st) 
     float4* tgt = ws.take<float4>((size_t)Op::PP * pl.n_tpad);
     float4* src = ws.take<float4>((size_t)Op::NS * pl.m_pad);
     float4* boxes = a.boxed ? ws.take<float4>(pl.box_words()) : nullptr;
-    double* part = ws.take<double>((size_t)pl.split * a.n * DIMB);
+    double* part = ws.take<double>(pl.part_doubles(a.n, DIMB));
+    int* counters = ws.take<int>(pl.split > 1 ? pl.counters() : 0);
     double* center = ws.take<double>(kCenterWords);
     if (ws.measuring()) return LDDMM_OK;
     if (ws.overflow()) {
@@ -49,6 +50,7 @@ int applyk_group(const ApplyKArgs& a, int col0, Workspace& ws, cudaStream_t st) 
     P.src_stride = pl.m_pad;
     P.tgt4 = tgt;
     P.tgt_stride = pl.n_tpad;
+    set_poly(P, ks);
     Gather g{};
     g.src = a.beta;
     g.row_stride = a.dimb;
@@ -56,29 +58,12 @@ int applyk_group(const ApplyKArgs& a, int col0, Workspace& ws, cudaStream_t st) 
     for (int c = 0; c < g.nvals; ++c) g.off[c] = col0 + c;
     g.mult = 1.0;
     launch_bbox_center(a.x, a.n, a.y, a.m, a.d, center, st);
-    pack_points_kernel<Real><<<grid_for(pl.n_tpad), 256, 0, st>>>(a.x, a.n, a.d, ks.scale, center, tgt, pl.n_tpad,
-                                                                  pl.n_tpad);
-    if constexpr (sizeof(Real) == 4) {
-        for (int j = 0; j < 5; ++j) P.pkd[j] = dup_coeff(ks.pk[j]);
-        for (int j = 0; j < 4; ++j) P.pqd[j] = dup_coeff(ks.pq[j]);
-        pack_list_kernel<<<grid_for(pl.m_pad), 256, 0, st>>>(a.y, a.m, a.d, ks.scale, center, g, D, DIMB, src,
-                                                            pl.m_pad, pl.m_pad, boxes);
-    } else {
-        for (int j = 0; j < 5; ++j) P.pk[j] = (Real)ks.pk[j];
-        for (int j = 0; j < 4; ++j) P.pq[j] = (Real)ks.pq[j];
-        pack_records_kernel<Real><<<grid_for(pl.m_pad), 256, 0, st>>>(a.y, a.m, a.d, ks.scale, center, g, src,
-                                                                      pl.m_pad, pl.m_pad, boxes);
-    }
-    LDDMM_TRY(launch_single<Op>(pl, a.n, P, boxes, part, st));
-    // combine writes only the group's own columns
-    const int ncols = g.nvals;
-    if (ncols == DIMB) {
-        combine_kernel<<<grid_for(a.n * DIMB), 256, 0, st>>>(part, a.n, DIMB, pl.split, 1.0, a.f, a.dimb, col0);
-    } else {
-        combine_cols_kernel<<<grid_for(a.n * ncols), 256, 0, st>>>(part, a.n, DIMB, ncols, pl.split, 1.0, a.f,
-                                                                  a.dimb, col0);
-    }
-    return cuda_check(cudaGetLastError(), "applyk");
+    pack_sum_kernel<Real, sizeof(Real) == 4><<<grid_for(pl.n_tpad + pl.m_pad), 256, 0, st>>>(
+        a.x, a.n, Gather{}, 0, tgt, pl.n_tpad, a.y, a.m, g, D, DIMB, src, pl.m_pad, a.d, ks.scale, center, boxes,
+        counters, pl.split > 1 ? (int)pl.counters() : 0);
+    // the epilogue writes only the group's own columns
+    const EpiSum E{a.f, a.dimb, col0, g.nvals, 1.0};
+    return launch_single<Op, false>(pl, a.n, P, boxes, part, st, 0, counters, E);
 }
 
 template <class Real>
@@ -181,7 +166,8 @@ int difft_impl(const DiffKTArgs& a, Workspace& ws, cudaStream_t st) {
     float4* tgt = ws.take<float4>((size_t)NT * pl.n_tpad);
     float4* src = ws.take<float4>((size_t)Op::NS * pl.m_pad);
     float4* boxes = ws.take<float4>(pl.box_words());
-    double* part = ws.take<double>((size_t)pl.split * a.n * D);
+    double* part = ws.take<double>(pl.part_doubles(a.n, D));
+    int* counters = ws.take<int>(pl.counters());
     double* center = ws.take<double>(kCenterWords);
     if (ws.measuring()) return LDDMM_OK;
     const KScale ks = kernel_scale(KIND, a.order, a.sigma, !pl.seq);
@@ -190,6 +176,7 @@ int difft_impl(const DiffKTArgs& a, Workspace& ws, cudaStream_t st) {
     P.src_stride = pl.m_pad;
     P.tgt4 = tgt;
     P.tgt_stride = pl.n_tpad;
+    set_poly(P, ks);
     // u_k / v_l: value w = c*na + i  <->  a[i, row, c]  (the Fortran sum order)
     Gather gu{}, gv{};
     gu.src = a.a1;
@@ -203,28 +190,11 @@ int difft_impl(const DiffKTArgs& a, Workspace& ws, cudaStream_t st) {
         gv.off[w] = (long long)i * a.m * a.dimb + c;
     }
     launch_bbox_center(a.x, a.n, a.y, a.m, a.d, center, st);
-    pack_records_kernel<Real><<<grid_for(pl.n_tpad), 256, 0, st>>>(a.x, a.n, a.d, ks.scale, center, gu, tgt,
-                                                                   pl.n_tpad, pl.n_tpad, nullptr);
-    if constexpr (sizeof(Real) == 4) {
-        for (int j = 0; j < 5; ++j) P.pkd[j] = dup_coeff(ks.pk[j]);
-        for (int j = 0; j < 4; ++j) P.pqd[j] = dup_coeff(ks.pq[j]);
-        pack_list_kernel<<<grid_for(pl.m_pad), 256, 0, st>>>(a.y, a.m, a.d, ks.scale, center, gv, D, W, src,
-                                                            pl.m_pad, pl.m_pad, boxes);
-    } else {
-        for (int j = 0; j < 5; ++j) P.pk[j] = (Real)ks.pk[j];
-        for (int j = 0; j < 4; ++j) P.pq[j] = (Real)ks.pq[j];
-        pack_records_kernel<Real><<<grid_for(pl.m_pad), 256, 0, st>>>(a.y, a.m, a.d, ks.scale, center, gv, src,
-                                                                      pl.m_pad, pl.m_pad, boxes);
-    }
-    LDDMM_TRY(launch_single<Op>(pl, a.n, P, boxes, part, st));
-    const int dout = a.d;  // D may exceed d (d == 1 runs as D == 2)
-    if (dout == D) {
-        combine_kernel<<<grid_for(a.n * D), 256, 0, st>>>(part, a.n, D, pl.split, ks.dscale, a.f, a.d, 0);
-    } else {
-        combine_cols_kernel<<<grid_for(a.n * dout), 256, 0, st>>>(part, a.n, D, dout, pl.split, ks.dscale, a.f,
-                                                                 a.d, 0);
-    }
-    return cuda_check(cudaGetLastError(), "applykdifft");
+    pack_sum_kernel<Real, sizeof(Real) == 4><<<grid_for(pl.n_tpad + pl.m_pad), 256, 0, st>>>(
+        a.x, a.n, gu, W, tgt, pl.n_tpad, a.y, a.m, gv, D, W, src, pl.m_pad, a.d, ks.scale, center, boxes, counters,
+        (int)pl.counters());
+    const EpiSum E{a.f, a.d, 0, a.d, ks.dscale};   // D may exceed d (d == 1 runs as D == 2)
+    return launch_single<Op, false>(pl, a.n, P, boxes, part, st, 0, counters, E);
 }
 
 template <class Real>
@@ -305,7 +275,8 @@ int div_impl(const ApplyKArgs& a, Workspace& ws, cudaStream_t st) {
     const SinglePlan pl = plan_single<Op>(a.n, a.m);
     float4* tgt = ws.take<float4>((size_t)Op::PP * pl.n_tpad);
     float4* src = ws.take<float4>((size_t)Op::NS * pl.m_pad);
-    double* part = ws.take<double>((size_t)pl.split * a.n);
+    double* part = ws.take<double>(pl.part_doubles(a.n, 1));
+    int* counters = ws.take<int>(pl.counters());
     double* center = ws.take<double>(kCenterWords);
     if (ws.measuring()) return LDDMM_OK;
     const KScale ks = kernel_scale(KIND, a.order, a.sigma, !pl.seq, /*exact_tables=*/true);
@@ -316,22 +287,19 @@ int div_impl(const ApplyKArgs& a, Workspace& ws, cudaStream_t st) {
     P.src_stride = pl.m_pad;
     P.tgt4 = tgt;
     P.tgt_stride = pl.n_tpad;
-    for (int j = 0; j < 5; ++j) P.pk[j] = (Real)ks.pk[j];
-    for (int j = 0; j < 4; ++j) P.pq[j] = (Real)ks.pq[j];
-    launch_bbox_center(a.x, a.n, a.y, a.m, a.d, center, st);
-    pack_points_kernel<Real><<<grid_for(pl.n_tpad), 256, 0, st>>>(a.x, a.n, a.d, ks.scale, center, tgt, pl.n_tpad,
-                                                                  pl.n_tpad);
+    set_poly(P, ks);
     Gather g{};
     g.src = a.beta;
     g.row_stride = a.d;
     g.nvals = a.d;
     for (int c = 0; c < a.d; ++c) g.off[c] = c;
     g.mult = 1.0;  // K' 2 <x-y, a> = dscale * F * <x'-y', a>
-    pack_records_kernel<Real><<<grid_for(pl.m_pad), 256, 0, st>>>(a.y, a.m, a.d, ks.scale, center, g, src, pl.m_pad,
-                                                                  pl.m_pad, nullptr);
-    LDDMM_TRY(launch_single<Op>(pl, a.n, P, nullptr, part, st));
-    combine_kernel<<<grid_for(a.n), 256, 0, st>>>(part, a.n, 1, pl.split, ks.dscale, a.f, 1, 0);
-    return cuda_check(cudaGetLastError(), "applydiv");
+    launch_bbox_center(a.x, a.n, a.y, a.m, a.d, center, st);
+    pack_sum_kernel<Real, false><<<grid_for(pl.n_tpad + pl.m_pad), 256, 0, st>>>(
+        a.x, a.n, Gather{}, 0, tgt, pl.n_tpad, a.y, a.m, g, D, D, src, pl.m_pad, a.d, ks.scale, center, nullptr,
+        counters, (int)pl.counters());
+    const EpiSum E{a.f, 1, 0, 1, ks.dscale};
+    return launch_single<Op, false>(pl, a.n, P, nullptr, part, st, 0, counters, E);
 }
 
 template <class Real>

@@ -141,6 +141,7 @@ struct OpDiffKT2 {
     static constexpr int NV = D + W;
     static constexpr int NS = (NV + 3) / 4;
     static constexpr int NT = 1 + (W + 3) / 4;  // target planes: pos, u values
+    static constexpr int MIN_BLOCKS = 3;        // see op_min_blocks
     static constexpr int NOUT = D;
     using Params = KernelParams2;
     using Acc = AccF32C2<D>;
@@ -180,32 +181,6 @@ inline unsigned long long dup_coeff(double c) {
     unsigned int u;
     memcpy(&u, &f, 4);
     return ((unsigned long long)u << 32) | (unsigned long long)u;
-}
-
-// Packs sources into list records (and the boxes of their folds): values [ (x_i - c) * s (D of them, zero
-// beyond d), gather values (V of them, zero beyond g.nvals) ], rows >= n zero.
-static __global__ void pack_list_kernel(const double* __restrict__ x, long long n, int d, double scale,
-                                       const double* __restrict__ center, const Gather g, int D, int V,
-                                       float4* __restrict__ out, long long stride, long long n_pad,
-                                       float4* __restrict__ boxes) {
-    const int nv = D + V;
-    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n_pad;
-         i += (long long)gridDim.x * blockDim.x) {
-        float v[16];
-        for (int q = 0; q < 16; ++q) v[q] = 0.f;
-        if (i < n) {
-            for (int j = 0; j < d && j < D; ++j) v[j] = (float)((x[i * d + j] - (center ? center[j] : 0.0)) * scale);
-            for (int q = 0; q < V && q < g.nvals; ++q) v[D + q] = (float)(g.src[i * g.row_stride + g.off[q]] * g.mult);
-        }
-        for (int w = 0; w < (nv + 3) / 4; ++w)
-            out[(long long)w * stride + i] = make_float4(v[4 * w], v[4 * w + 1], v[4 * w + 2], v[4 * w + 3]);
-        if (boxes != nullptr) {
-            float p[3], w = 0.f;
-            for (int j = 0; j < 3; ++j) p[j] = j < D ? v[j] : 0.f;
-            for (int q = 0; q < V; ++q) w = max_nan(w, v[D + q]);
-            store_fold_box<float>(boxes, i, i < n, p, w);
-        }
-    }
 }
 
 }  // namespace lddmm

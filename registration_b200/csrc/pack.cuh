@@ -11,11 +11,15 @@ namespace lddmm {
 // centre halves the magnitude (and so the FP32 rounding error) of the packed
 // coordinates.
 //
-// Many blocks reduce min / max of order-preserving 64-bit keys of the
-// coordinates with atomicMin / atomicMax: min and max are exact, so the result
-// does not depend on the order of the blocks.  The centre buffer holds
-// kCenterWords doubles: the centre in [0, 4) and the six keys in [4, 10).
-constexpr int kCenterWords = 16;
+// Blocks reduce min / max of order-preserving 64-bit keys of the coordinates
+// (exact, so the result does not depend on their order): one block up to
+// kBboxOneBlock points (one launch, 3 us; a launch that zeroes atomics and one
+// that reads them back cost 2 us each), otherwise a block per 2048 points leaves
+// its six keys for a second, one-block launch.  Ragged launches commit with
+// atomicMin / atomicMax into their segment's keys.
+constexpr long long kBboxOneBlock = 8192;
+constexpr int kBboxMaxBlocks = 592;
+constexpr int kCenterWords = 4 + 6 * kBboxMaxBlocks;   // doubles: the centre in [0, 4), then the blocks' keys
 constexpr long long kKeyMax = 0x7FFFFFFFFFFFFFFFLL;
 constexpr long long kKeyMin = -kKeyMax - 1;
 
@@ -27,9 +31,8 @@ LDDMM_D long long bbox_key(double v) {
 
 LDDMM_D double bbox_val(long long k) { return __longlong_as_double(k >= 0 ? k : (k ^ kKeyMax)); }
 
-// warp + block reduction of per-thread key bounds, then one atomic per block
-// and component into keys[0..3) (min) and keys[3..6) (max)
-LDDMM_D void bbox_block_commit(long long (&l)[3], long long (&h)[3], long long* keys) {
+// warp + block reduction of per-thread key bounds; thread 0 gets the block's (min in l, max in h)
+LDDMM_D void bbox_block_reduce(long long (&l)[3], long long (&h)[3]) {
     __shared__ long long sl[3][32], sh[3][32];
     for (int off = 16; off > 0; off >>= 1)
         for (int j = 0; j < 3; ++j) {
@@ -53,21 +56,29 @@ LDDMM_D void bbox_block_commit(long long (&l)[3], long long (&h)[3], long long* 
                 l[j] = min(l[j], __shfl_down_sync(0xffffffffu, l[j], off));
                 h[j] = max(h[j], __shfl_down_sync(0xffffffffu, h[j], off));
             }
-        if (lane == 0)
-            for (int j = 0; j < 3; ++j) {
-                if (l[j] != kKeyMax) atomicMin(keys + j, l[j]);
-                if (h[j] != kKeyMin) atomicMax(keys + 3 + j, h[j]);
-            }
     }
 }
 
-static __global__ void bbox_init_kernel(long long* __restrict__ keys) {
-    if (threadIdx.x < 6) keys[threadIdx.x] = threadIdx.x < 3 ? kKeyMax : kKeyMin;
+// one atomic per block and component into keys[0..3) (min) and keys[3..6) (max)
+LDDMM_D void bbox_block_commit(long long (&l)[3], long long (&h)[3], long long* keys) {
+    bbox_block_reduce(l, h);
+    if (threadIdx.x == 0)
+        for (int j = 0; j < 3; ++j) {
+            if (l[j] != kKeyMax) atomicMin(keys + j, l[j]);
+            if (h[j] != kKeyMin) atomicMax(keys + 3 + j, h[j]);
+        }
 }
 
-static __global__ void bbox_keys_kernel(const double* __restrict__ x, long long n, const double* __restrict__ y,
-                                        long long m, int d, long long* __restrict__ keys) {
+LDDMM_D void bbox_write_center(const long long (&l)[3], const long long (&h)[3], int d, bool nonempty,
+                               double* center) {
+    for (int j = 0; j < 3; ++j) center[j] = (j < d && nonempty) ? 0.5 * (bbox_val(l[j]) + bbox_val(h[j])) : 0.0;
+}
+
+// gridDim 1: the centre; otherwise each block's keys
+static __global__ void bbox_part_kernel(const double* __restrict__ x, long long n, const double* __restrict__ y,
+                                        long long m, int d, double* __restrict__ center) {
     long long l[3] = {kKeyMax, kKeyMax, kKeyMax}, h[3] = {kKeyMin, kKeyMin, kKeyMin};
+#pragma unroll 4
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n + m;
          i += (long long)gridDim.x * blockDim.x) {
         const double* p = i < n ? x + i * d : y + (i - n) * d;
@@ -77,47 +88,42 @@ static __global__ void bbox_keys_kernel(const double* __restrict__ x, long long 
             h[j] = max(h[j], k);
         }
     }
-    bbox_block_commit(l, h, keys);
+    bbox_block_reduce(l, h);
+    if (threadIdx.x != 0) return;
+    if (gridDim.x == 1) {
+        bbox_write_center(l, h, d, n + m > 0, center);
+    } else {
+        long long* keys = reinterpret_cast<long long*>(center + 4) + 6 * blockIdx.x;
+        for (int j = 0; j < 3; ++j) {
+            keys[j] = l[j];
+            keys[3 + j] = h[j];
+        }
+    }
 }
 
-static __global__ void bbox_finish_kernel(const long long* __restrict__ keys, int d, int nonempty,
-                                          double* __restrict__ center) {
-    if (threadIdx.x < 3) {
-        const int j = threadIdx.x;
-        center[j] = (j < d && nonempty) ? 0.5 * (bbox_val(keys[j]) + bbox_val(keys[3 + j])) : 0.0;
-    }
+static __global__ void bbox_finish_kernel(int blocks, int d, double* __restrict__ center) {
+    long long l[3] = {kKeyMax, kKeyMax, kKeyMax}, h[3] = {kKeyMin, kKeyMin, kKeyMin};
+    const long long* keys = reinterpret_cast<const long long*>(center + 4);
+    for (int b = threadIdx.x; b < blocks; b += blockDim.x)
+        for (int j = 0; j < 3; ++j) {
+            l[j] = min(l[j], keys[6 * b + j]);
+            h[j] = max(h[j], keys[6 * b + 3 + j]);
+        }
+    bbox_block_reduce(l, h);
+    if (threadIdx.x == 0) bbox_write_center(l, h, d, true, center);
 }
 
 // center: kCenterWords doubles of device memory (see above)
 inline void launch_bbox_center(const double* x, long long n, const double* y, long long m, int d, double* center,
                                cudaStream_t st) {
-    long long* keys = reinterpret_cast<long long*>(center + 4);
     const long long tot = n + m;
-    const int blocks = (int)std::max<long long>(1, std::min<long long>(148 * 4, (tot + 2047) / 2048));
-    bbox_init_kernel<<<1, 32, 0, st>>>(keys);
-    bbox_keys_kernel<<<blocks, 256, 0, st>>>(x, n, y, m, d, keys);
-    bbox_finish_kernel<<<1, 32, 0, st>>>(keys, d, tot > 0 ? 1 : 0, center);
-}
-
-// Points: value j of row i is (x[i*d + j] - center[j]) * scale (zero for j >= d or i >= n).
-// FP32: one float4 word per row in plane 0.  FP64: two double2 words (planes 0, 1).
-template <class Real>
-static __global__ void pack_points_kernel(const double* __restrict__ x, long long n, int d, double scale,
-                                          const double* __restrict__ center, float4* __restrict__ out,
-                                          long long stride, long long n_pad) {
-    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n_pad;
-         i += (long long)gridDim.x * blockDim.x) {
-        double v[4] = {0, 0, 0, 0};
-        if (i < n)
-            for (int j = 0; j < d && j < 4; ++j) v[j] = (x[i * d + j] - (center ? center[j] : 0.0)) * scale;
-        if constexpr (sizeof(Real) == 4) {
-            out[i] = make_float4((float)v[0], (float)v[1], (float)v[2], (float)v[3]);
-        } else {
-            double2* o = reinterpret_cast<double2*>(out);
-            o[i] = make_double2(v[0], v[1]);
-            o[stride + i] = make_double2(v[2], v[3]);
-        }
+    if (tot <= kBboxOneBlock) {
+        bbox_part_kernel<<<1, 1024, 0, st>>>(x, n, y, m, d, center);
+        return;
     }
+    const int blocks = (int)std::min<long long>(kBboxMaxBlocks, (tot + 2047) / 2048);
+    bbox_part_kernel<<<blocks, 256, 0, st>>>(x, n, y, m, d, center);
+    bbox_finish_kernel<<<1, 256, 0, st>>>(blocks, d, center);
 }
 
 // Gather spec for value planes: value w of row i is src[i*row_stride + off[w]] * mult.
@@ -129,72 +135,53 @@ struct Gather {
     double mult;
 };
 
-// Standard records: the position planes of pack_points_kernel, then `g.nvals`
-// values per row in the following planes; boxes (sources): the fold boxes.
-template <class Real>
-static __global__ void pack_records_kernel(const double* __restrict__ x, long long n, int d, double scale,
-                                           const double* __restrict__ center, const Gather g,
-                                           float4* __restrict__ out, long long stride, long long n_pad,
-                                           float4* __restrict__ boxes) {
-    constexpr int PW = Traits<Real>::PER_WORD, PP = PointPlanes<Real>::N;
-    const int nwords = (g.nvals + PW - 1) / PW;
-    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n_pad;
-         i += (long long)gridDim.x * blockDim.x) {
-        Real p[4] = {0, 0, 0, 0}, wmax = 0;
-        if (i < n)
-            for (int j = 0; j < d && j < 3; ++j) p[j] = (Real)((x[i * d + j] - center[j]) * scale);
-        if constexpr (sizeof(Real) == 4) {
-            out[i] = make_float4(p[0], p[1], p[2], p[3]);
-        } else {
-            double2* o = reinterpret_cast<double2*>(out);
-            o[i] = make_double2(p[0], p[1]);
-            o[stride + i] = make_double2(p[2], p[3]);
+// Packed row i of a kernel sum: the position (x_i - center) * scale, then the
+// gather's values (V of them at most, zero beyond g.nvals).  LIST (packed FP32
+// sources, ops2.cuh): one list of D + V values; otherwise the standard planes,
+// position first (FP32: one float4 word; FP64: two double2 words).  boxes
+// (sources): the fold's box.  Rows >= n are zero.
+template <class Real, bool LIST>
+LDDMM_D void pack_row(const double* __restrict__ x, long long n, int d, double scale,
+                      const double* __restrict__ center, const Gather& g, int D, int V, float4* __restrict__ out,
+                      long long stride, long long i, float4* boxes) {
+    constexpr int PW = Traits<Real>::PER_WORD;
+    Real v[16], w = 0;
+#pragma unroll
+    for (int q = 0; q < 16; ++q) v[q] = 0;
+    const int V0 = LIST ? D : 4;   // first value
+    if (i < n) {
+        for (int j = 0; j < d && j < 3; ++j) v[j] = (Real)((x[i * d + j] - center[j]) * scale);
+        for (int q = 0; q < V && q < g.nvals; ++q) {
+            v[V0 + q] = (Real)(g.src[i * g.row_stride + g.off[q]] * g.mult);
+            w = max_nan(w, v[V0 + q]);
         }
-        for (int w = 0; w < nwords; ++w) {
-            Real v[PW];
-            for (int q = 0; q < PW; ++q) {
-                const int idx = w * PW + q;
-                v[q] = (i < n && idx < g.nvals) ? (Real)(g.src[i * g.row_stride + g.off[idx]] * g.mult) : (Real)0;
-                wmax = max_nan(wmax, v[q]);
-            }
-            float4* dst = out + (long long)(PP + w) * stride + i;
-            if constexpr (sizeof(Real) == 4) {
-                *dst = make_float4(v[0], v[1], v[2], v[3]);
-            } else {
-                *reinterpret_cast<double2*>(dst) = make_double2(v[0], v[1]);
-            }
-        }
-        if (boxes != nullptr) store_fold_box<Real>(boxes, i, i < n, p, wmax);
+    }
+    const int nwords = LIST ? (D + V + PW - 1) / PW : 4 / PW + (V + PW - 1) / PW;
+    for (int k = 0; k < nwords; ++k) {
+        float4* dst = out + (long long)k * stride + i;
+        if constexpr (sizeof(Real) == 4) *dst = make_float4(v[4 * k], v[4 * k + 1], v[4 * k + 2], v[4 * k + 3]);
+        else *reinterpret_cast<double2*>(dst) = make_double2(v[2 * k], v[2 * k + 1]);
+    }
+    if (boxes != nullptr) {
+        const Real p[3] = {v[0], v[1], D > 2 ? v[2] : (Real)0};
+        store_fold_box<Real>(boxes, i, i < n, p, w);
     }
 }
 
-// out[i*out_ld + col0 + c] = scale * sum_{chunk < split} part[(chunk*n + i)*nout + c]
-static __global__ void combine_kernel(const double* __restrict__ part, long long n, int nout, int split,
-                                      double scale, double* __restrict__ out, long long out_ld, int col0) {
-    const long long total = n * nout;
-    for (long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x; q < total;
+// Targets (standard planes), then sources of a kernel sum, one launch; zeroes the sweep's counters.
+template <class Real, bool LIST>
+static __global__ void pack_sum_kernel(const double* __restrict__ x, long long n, const Gather gt, int Vt,
+                                       float4* __restrict__ tgt, long long n_tpad, const double* __restrict__ y,
+                                       long long m, const Gather gs, int D, int Vs, float4* __restrict__ src,
+                                       long long m_pad, int d, double scale, const double* __restrict__ center,
+                                       float4* __restrict__ boxes, int* __restrict__ counters, int n_counters) {
+    for (long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x; q < n_tpad + m_pad;
          q += (long long)gridDim.x * blockDim.x) {
-        const long long i = q / nout;
-        const int c = (int)(q - i * nout);
-        double s = 0.0;
-        for (int k = 0; k < split; ++k) s += part[((long long)k * n + i) * nout + c];
-        out[i * out_ld + col0 + c] = scale * s;
-    }
-}
-
-// Like combine_kernel but the partial rows hold `nout` values of which only
-// the first `ncols` are written out.
-static __global__ void combine_cols_kernel(const double* __restrict__ part, long long n, int nout, int ncols,
-                                           int split, double scale, double* __restrict__ out, long long out_ld,
-                                           int col0) {
-    const long long total = n * ncols;
-    for (long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x; q < total;
-         q += (long long)gridDim.x * blockDim.x) {
-        const long long i = q / ncols;
-        const int c = (int)(q - i * ncols);
-        double s = 0.0;
-        for (int k = 0; k < split; ++k) s += part[((long long)k * n + i) * nout + c];
-        out[i * out_ld + col0 + c] = scale * s;
+        if (q < n_counters) counters[q] = 0;
+        if (q < n_tpad)
+            pack_row<Real, false>(x, n, d, scale, center, gt, D, Vt, tgt, n_tpad, q, nullptr);
+        else
+            pack_row<Real, LIST>(y, m, d, scale, center, gs, D, Vs, src, m_pad, q - n_tpad, boxes);
     }
 }
 

@@ -46,7 +46,7 @@ struct RagSeg {
     long long tpad, spad;  // packed rows of this segment (targets, sources)
     long long part;      // first row of the partial-sum buffer
     int split;
-    int nb;              // reduction blocks of this segment
+    int nb;              // target groups of this segment (one energy partial each)
     long long eoff;      // first energy partial of this segment
     double scale;        // coordinate prescale
     double dscale;       // derivative constant
@@ -62,7 +62,7 @@ template <class Op>
 struct RagPlan {
     std::vector<RagSeg> segs;
     std::vector<SegDesc> desc;
-    long long tt = 0, ss = 0, parts = 0, eparts = 0;
+    long long tt = 0, ss = 0, parts = 0, eparts = 0;   // eparts: energy partials = groups = counters
     int items = 0;
 };
 
@@ -74,7 +74,7 @@ RagPlan<Op> rag_plan(const std::vector<long long>& n, const std::vector<long lon
     p.desc.resize(nseg);
     long long row = 0, mrow = 0;
     for (int s = 0; s < nseg; ++s) {
-        const SinglePlan pl = plan_single<Op>(n[s], m[s]);
+        const SinglePlan pl = plan_single<Op>(n[s], m[s], 0, true);
         RagSeg& g = p.segs[s];
         g.row0 = row;
         g.n = n[s];
@@ -86,7 +86,7 @@ RagPlan<Op> rag_plan(const std::vector<long long>& n, const std::vector<long lon
         g.spad = pl.m_pad;
         g.part = p.parts;
         g.split = pl.split;
-        g.nb = (int)std::max<long long>(1, std::min<long long>(1024, (n[s] + kRagThreads - 1) / kRagThreads));
+        g.nb = pl.n_tb;
         g.eoff = p.eparts;
         SegDesc& d = p.desc[s];
         d.tgt = g.tgt;
@@ -97,6 +97,8 @@ RagPlan<Op> rag_plan(const std::vector<long long>& n, const std::vector<long lon
         d.n_tb = pl.n_tb;
         d.split = pl.split;
         d.item0 = p.items;
+        d.id = s;
+        d.cnt = (int)p.eparts;
         p.items += pl.n_tb * pl.split;
         p.tt += pl.n_tpad;
         p.ss += pl.m_pad;
@@ -109,19 +111,6 @@ RagPlan<Op> rag_plan(const std::vector<long long>& n, const std::vector<long lon
 }
 
 // ---- segment-local reductions ----------------------------------------------------
-LDDMM_D double rag_block_sum(double v) {
-    __shared__ double red[kRagThreads];
-    red[threadIdx.x] = v;
-    __syncthreads();
-    for (int s = kRagThreads / 2; s > 0; s >>= 1) {
-        if (threadIdx.x < s) red[threadIdx.x] += red[threadIdx.x + s];
-        __syncthreads();
-    }
-    const double r = red[0];
-    __syncthreads();
-    return r;
-}
-
 // Centre of the bounding box of each segment's rows: rows [row0, row0 + n) of x
 // (x0 of a trajectory block when XT0: rows (T+1) row0 + i) and, if y, rows
 // [m0, m0 + m) of y.  nbb blocks per segment reduce order-preserving keys with
@@ -202,85 +191,96 @@ LDDMM_D void rag_box(float4* boxes, long long row, bool valid, const float* v, i
 
 // ---- ragged shooting ---------------------------------------------------------------
 // xt / at of request s: blocks (T+1, n, d) / (T, n, d) at rows (T+1)*row0 / T*row0.
+struct RagPlanes {
+    float4 *tgt, *src, *boxes;
+};
+
+// packed row i of segment g from its position x, momentum a (NULL: padding)
+template <int D>
+LDDMM_D void rag_shoot_row(const RagSeg& g, long long i, const double* x, const double* a, int d, const RagPlanes& p,
+                           long long tstride, long long sstride) {
+    float pos[3] = {0, 0, 0}, vals[2 * D];
+    for (int k = 0; k < 2 * D; ++k) vals[k] = 0.f;
+    if (x != nullptr)
+        for (int j = 0; j < d; ++j) {
+            pos[j] = (float)((x[j] - g.center[j]) * g.scale);
+            vals[j] = pos[j];
+            vals[D + j] = (float)a[j];
+        }
+    if (i < g.tpad) put_plain(p.tgt, tstride, g.tgt + i, pos, 3, 1);
+    if (i < g.spad) {
+        put_plain(p.src, sstride, g.src + i, vals, 2 * D, (2 * D + 3) / 4);
+        rag_box<D>(p.boxes, g.src + i, x != nullptr, vals, 2 * D);
+    }
+}
+
+// planes of step 0, the padding of both sets
 template <int D>
 static __global__ void rag_shoot_pack_kernel(const RagSeg* __restrict__ segs, const long long* __restrict__ padoff,
                                              int nseg, const double* __restrict__ xt, const double* __restrict__ at,
-                                             int T, int step, int d, float4* tgt, long long tstride, float4* src,
-                                             long long sstride, float4* boxes) {
+                                             int T, int d, RagPlanes p0, RagPlanes p1, long long tstride,
+                                             long long sstride) {
     const long long total = padoff[nseg];
     for (long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x; q < total;
          q += (long long)gridDim.x * blockDim.x) {
         const int s = seg_lookup(padoff, nseg, q);
         const RagSeg& g = segs[s];
         const long long i = q - padoff[s];
-        float pos[3] = {0, 0, 0}, vals[2 * D];
-        for (int k = 0; k < 2 * D; ++k) vals[k] = 0.f;
-        if (i < g.n) {
-            const double* x = xt + (((long long)(T + 1) * g.row0 + (long long)step * g.n + i) * d);
-            const double* a = at + (((long long)T * g.row0 + (long long)step * g.n + i) * d);
-            for (int j = 0; j < d; ++j) {
-                pos[j] = (float)((x[j] - g.center[j]) * g.scale);
-                vals[j] = pos[j];
-                vals[D + j] = (float)a[j];
-            }
-        }
-        if (i < g.tpad) put_plain(tgt, tstride, g.tgt + i, pos, 3, 1);
-        if (i < g.spad) {
-            put_plain(src, sstride, g.src + i, vals, 2 * D, (2 * D + 3) / 4);
-            rag_box<D>(boxes, g.src + i, i < g.n, vals, 2 * D);
-        }
+        const double* x = i < g.n ? xt + ((long long)(T + 1) * g.row0 + i) * d : nullptr;
+        const double* a = i < g.n ? at + ((long long)T * g.row0 + i) * d : nullptr;
+        rag_shoot_row<D>(g, i, x, a, d, p0, tstride, sstride);
+        rag_shoot_row<D>(g, i, x, a, d, p1, tstride, sstride);
     }
 }
 
-// v = sum of chunks, x_{t+1} = x_t + dt v, energy partial <a, v> per segment block
+// epilogue of step `step`: x_{t+1} = x_t + dt v, energy partial <a, v> of the group, planes of the next step
 template <int D>
-static __global__ void rag_shoot_combine_kernel(const RagSeg* __restrict__ segs, int nseg,
-                                                const double* __restrict__ part, double* __restrict__ xt,
-                                                const double* __restrict__ at, int T, int step, int d,
-                                                double* __restrict__ epart) {
-    // grid: blocks enumerate (segment, local block) pairs; eoff gives the first block of a segment
-    const int b = blockIdx.x;
-    int s = 0;
-    {
-        int lo = 0, hi = nseg - 1;
-        while (lo < hi) {
-            const int mid = (lo + hi + 1) >> 1;
-            if (segs[mid].eoff <= b) lo = mid; else hi = mid - 1;
+struct EpiRagShoot {
+    static constexpr bool NONE = false;
+    const RagSeg* segs;
+    double* xt;
+    const double* at;
+    int T, step, d;
+    RagPlanes nx;
+    long long tstride, sstride;
+    double* epart;
+    int op_rows;
+    template <int NOUT>
+    LDDMM_D void run(const SegDesc& sd, int row0, int rows, const double* red) const {
+        const RagSeg& g = segs[sd.id];
+        double e = 0.0;
+        for (int r = threadIdx.x; r < ((rows + 31) & ~31); r += blockDim.x) {   // whole warps: fold boxes
+            const bool valid = r < rows;
+            const long long i = row0 + r;
+            const double* x0 = xt + (((long long)(T + 1) * g.row0 + (long long)step * g.n + i) * d);
+            double* x1 = xt + (((long long)(T + 1) * g.row0 + (long long)(step + 1) * g.n + i) * d);
+            const double* a0 = at + (((long long)T * g.row0 + (long long)step * g.n + i) * d);
+            double xn[3] = {0, 0, 0};
+            for (int j = 0; j < d && valid; ++j) {
+                const double v = red[r * NOUT + j];
+                e += a0[j] * v;
+                xn[j] = x0[j] + g.extra * v;
+                x1[j] = xn[j];
+            }
+            if (step + 1 < T)
+                rag_shoot_row<D>(g, i, valid ? xn : nullptr, a0 + (long long)g.n * d, d, nx, tstride, sstride);
         }
-        s = lo;
+        e = block_sum_all(e);
+        if (threadIdx.x == 0) epart[g.eoff + row0 / op_rows] += e;
     }
-    const RagSeg& g = segs[s];
-    const int lb = b - (int)g.eoff;
-    double e = 0.0;
-    for (long long i = (long long)lb * blockDim.x + threadIdx.x; i < g.n; i += (long long)g.nb * blockDim.x) {
-        const double* x0 = xt + (((long long)(T + 1) * g.row0 + (long long)step * g.n + i) * d);
-        double* x1 = xt + (((long long)(T + 1) * g.row0 + (long long)(step + 1) * g.n + i) * d);
-        const double* a0 = at + (((long long)T * g.row0 + (long long)step * g.n + i) * d);
-        double v[D];
-        for (int j = 0; j < D; ++j) v[j] = 0.0;
-#pragma unroll 4
-        for (int k = 0; k < g.split; ++k) {
-            const double* pk = part + (g.part + (long long)k * g.n + i) * D;
-            for (int j = 0; j < D; ++j) v[j] += pk[j];
-        }
-        for (int j = 0; j < d; ++j) {
-            e += a0[j] * v[j];
-            x1[j] = x0[j] + g.extra * v[j];
-        }
-    }
-    const double r = rag_block_sum(e);
-    if (threadIdx.x == 0) epart[(long long)step * 0 + b] += r;
-}
+};
 
-// energy[s] = rw dt * sum of the segment's partials (fixed order)
+// energy[s] = rw dt * sum of the segment's partials (one warp per segment, fixed order)
 static __global__ void rag_energy_kernel(const RagSeg* __restrict__ segs, int nseg, const double* __restrict__ epart,
                                          double scale_by_dt, double* __restrict__ energy, int use_rw) {
-    const int s = blockIdx.x * blockDim.x + threadIdx.x;
+    const int s = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     if (s >= nseg) return;
     const RagSeg& g = segs[s];
     double v = 0.0;
-    for (int k = 0; k < g.nb; ++k) v += epart[g.eoff + k];
-    energy[s] = (use_rw ? g.rw * g.extra : scale_by_dt) * v;
+    for (int k = threadIdx.x & 31; k < g.nb; k += 32) v += epart[g.eoff + k];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
+    if ((threadIdx.x & 31) == 0) energy[s] = (use_rw ? g.rw * g.extra : scale_by_dt) * v;
 }
 
 static int rag_copy_table(const void* host, size_t bytes, void* dev, cudaStream_t st) {
@@ -300,11 +300,15 @@ int rag_shoot_impl(int nseg, const int64_t* v_off, int d, const double* x0, cons
     RagSeg* dsegs = ws.take<RagSeg>(nseg);
     SegDesc* ddesc = ws.take<SegDesc>(nseg);
     long long* dpad = ws.take<long long>(nseg + 1);
-    float4* tgt = ws.take<float4>((size_t)Op::PP * pl.tt);
-    float4* src = ws.take<float4>((size_t)Op::NS * pl.ss);
-    float4* boxes = ws.take<float4>(2 * (size_t)(pl.ss / kFold));
+    RagPlanes pn[2];
+    for (RagPlanes& p : pn) {
+        p.tgt = ws.take<float4>((size_t)Op::PP * pl.tt);
+        p.src = ws.take<float4>((size_t)Op::NS * pl.ss);
+        p.boxes = ws.take<float4>(2 * (size_t)(pl.ss / kFold));
+    }
     double* part = ws.take<double>((size_t)pl.parts * D);
-    double* epart = ws.take<double>((size_t)std::max<long long>(1, pl.eparts));
+    double* epart = ws.take<double>((size_t)pl.eparts + 1);   // and the groups' counters behind it
+    int* counters = ws.take<int>((size_t)pl.eparts + 1);
     if (ws.measuring()) return LDDMM_OK;
     for (int s = 0; s < nseg; ++s) {
         const KScale ks = kernel_scale(KIND, order, sigma[s], true);
@@ -317,102 +321,118 @@ int rag_shoot_impl(int nseg, const int64_t* v_off, int d, const double* x0, cons
     LDDMM_TRY(rag_copy_table(pl.segs.data(), sizeof(RagSeg) * nseg, dsegs, st));
     LDDMM_TRY(rag_copy_table(pl.desc.data(), sizeof(SegDesc) * nseg, ddesc, st));
     LDDMM_TRY(rag_copy_table(padoff.data(), sizeof(long long) * (nseg + 1), dpad, st));
-    LDDMM_TRY(cuda_check(cudaMemsetAsync(epart, 0, sizeof(double) * std::max<long long>(1, pl.eparts), st), "memset"));
+    LDDMM_TRY(cuda_check(cudaMemsetAsync(epart, 0, (size_t)((char*)(counters + pl.eparts + 1) - (char*)epart), st),
+                         "memset"));
     // xt[0] = x0 per request
     for (int s = 0; s < nseg; ++s)
         LDDMM_TRY(cuda_check(cudaMemcpyAsync(xt + (T + 1) * v_off[s] * d, x0 + v_off[s] * d, sizeof(double) * n[s] * d,
                                              cudaMemcpyDeviceToDevice, st), "ragged shoot copy"));
     rag_bbox_launch<false>(dsegs, nseg, nbb, x0, nullptr, d, 0, st);   // x0 rows [row0, row0 + n)
     KernelParams2 P{};
-    P.src4 = src;
     P.src_stride = pl.ss;
-    P.tgt4 = tgt;
     P.tgt_stride = pl.tt;
-    const KScale ks0 = kernel_scale(KIND, order, sigma[0], true);
-    for (int j = 0; j < 5; ++j) P.pkd[j] = dup_coeff(ks0.pk[j]);
-    for (int j = 0; j < 4; ++j) P.pqd[j] = dup_coeff(ks0.pq[j]);
+    set_poly(P, kernel_scale(KIND, order, sigma[0], true));
     SweepGrid grid{};
     grid.segs = ddesc;
     grid.nseg = nseg;
     grid.n_items = pl.items;
-    for (int t = 0; t < T; ++t) {
-        rag_shoot_pack_kernel<D><<<grid_for(padoff[nseg]), 256, 0, st>>>(dsegs, dpad, nseg, xt, at, T, t, d, tgt, pl.tt,
-                                                                        src, pl.ss, boxes);
-        sweep_kernel<Op><<<pl.items, 32 * kSweepWarps, 0, st>>>(grid, P, boxes, part);
-        rag_shoot_combine_kernel<D><<<(int)pl.eparts, kRagThreads, 0, st>>>(dsegs, nseg, part, xt, at, T, t, d, epart);
+    rag_shoot_pack_kernel<D><<<grid_for(padoff[nseg]), 256, 0, st>>>(dsegs, dpad, nseg, xt, at, T, d, pn[0], pn[1],
+                                                                    pl.tt, pl.ss);
+    for (int t = 0; t < T && pl.items > 0; ++t) {
+        P.tgt4 = pn[t & 1].tgt;
+        P.src4 = pn[t & 1].src;
+        const EpiRagShoot<D> E{dsegs, xt, at, T, t, d, pn[(t + 1) & 1], pl.tt, pl.ss, epart, op_group<Op>()};
+        sweep_kernel<Op, false, EpiRagShoot<D>><<<pl.items, 32 * kSweepWarps, 0, st>>>(grid, P, pn[t & 1].boxes, part,
+                                                                                      counters, E);
     }
-    if (energy) rag_energy_kernel<<<(nseg + 127) / 128, 128, 0, st>>>(dsegs, nseg, epart, 0.0, energy, 1);
+    if (energy) rag_energy_kernel<<<(nseg + 3) / 4, 128, 0, st>>>(dsegs, nseg, epart, 0.0, energy, 1);
     return cuda_check(cudaGetLastError(), "ragged shoot");
 }
 
 // ---- ragged covector ---------------------------------------------------------------
 // step t: targets (pos x_t, u = (p_{t+1} - 2 rw a_t, a_t)), sources (pos, v = (a_t, p_{t+1}))
 template <int D>
+LDDMM_D void rag_cov_row(const RagSeg& g, long long i, const double* x, const double* a, const double* p, int d,
+                         const RagPlanes& pl, long long tstride, long long sstride) {
+    float pos[3] = {0, 0, 0}, u[2 * D], v[3 * D];
+    for (int k = 0; k < 2 * D; ++k) u[k] = 0.f;
+    for (int k = 0; k < 3 * D; ++k) v[k] = 0.f;
+    if (x != nullptr)
+        for (int j = 0; j < d; ++j) {
+            pos[j] = (float)((x[j] - g.center[j]) * g.scale);
+            u[j] = (float)(p[j] - 2.0 * g.rw * a[j]);
+            u[D + j] = (float)a[j];
+            v[j] = pos[j];
+            v[D + j] = (float)a[j];
+            v[2 * D + j] = (float)p[j];
+        }
+    if (i < g.tpad) {
+        put_plain(pl.tgt, tstride, g.tgt + i, pos, 3, 1);
+        put_plain(pl.tgt + tstride, tstride, g.tgt + i, u, 2 * D, (2 * D + 3) / 4);
+    }
+    if (i < g.spad) {
+        put_plain(pl.src, sstride, g.src + i, v, 3 * D, (3 * D + 3) / 4);
+        rag_box<D>(pl.boxes, g.src + i, x != nullptr, v, 3 * D);
+    }
+}
+
+// planes of step T-1, the padding of both sets
+template <int D>
 static __global__ void rag_cov_pack_kernel(const RagSeg* __restrict__ segs, const long long* __restrict__ padoff,
                                            int nseg, const double* __restrict__ xt, const double* __restrict__ at,
-                                           const double* __restrict__ pxt, int T, int step, int d, float4* tgt,
-                                           long long tstride, float4* src, long long sstride, float4* boxes) {
+                                           const double* __restrict__ pxt, int T, int d, RagPlanes p0, RagPlanes p1,
+                                           long long tstride, long long sstride) {
     const long long total = padoff[nseg];
     for (long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x; q < total;
          q += (long long)gridDim.x * blockDim.x) {
         const int s = seg_lookup(padoff, nseg, q);
         const RagSeg& g = segs[s];
         const long long i = q - padoff[s];
-        float pos[3] = {0, 0, 0}, u[2 * D], v[3 * D];
-        for (int k = 0; k < 2 * D; ++k) u[k] = 0.f;
-        for (int k = 0; k < 3 * D; ++k) v[k] = 0.f;
+        const double *x = nullptr, *a = nullptr, *p = nullptr;
         if (i < g.n) {
-            const double* x = xt + (((long long)(T + 1) * g.row0 + (long long)step * g.n + i) * d);
-            const double* a = at + (((long long)T * g.row0 + (long long)step * g.n + i) * d);
-            const double* p = pxt + (((long long)(T + 1) * g.row0 + (long long)(step + 1) * g.n + i) * d);
-            for (int j = 0; j < d; ++j) {
-                pos[j] = (float)((x[j] - g.center[j]) * g.scale);
-                u[j] = (float)(p[j] - 2.0 * g.rw * a[j]);
-                u[D + j] = (float)a[j];
-                v[j] = pos[j];
-                v[D + j] = (float)a[j];
-                v[2 * D + j] = (float)p[j];
-            }
+            x = xt + (((long long)(T + 1) * g.row0 + (long long)(T - 1) * g.n + i) * d);
+            a = at + (((long long)T * g.row0 + (long long)(T - 1) * g.n + i) * d);
+            p = pxt + (((long long)(T + 1) * g.row0 + (long long)T * g.n + i) * d);
         }
-        if (i < g.tpad) {
-            put_plain(tgt, tstride, g.tgt + i, pos, 3, 1);
-            put_plain(tgt + tstride, tstride, g.tgt + i, u, 2 * D, (2 * D + 3) / 4);
-        }
-        if (i < g.spad) {
-            put_plain(src, sstride, g.src + i, v, 3 * D, (3 * D + 3) / 4);
-            rag_box<D>(boxes, g.src + i, i < g.n, v, 3 * D);
-        }
+        rag_cov_row<D>(g, i, x, a, p, d, p0, tstride, sstride);
+        rag_cov_row<D>(g, i, x, a, p, d, p1, tstride, sstride);
     }
 }
 
+// epilogue of step `step`: p_t = p_{t+1} + dt dscale sums, dat_t, planes of step - 1
 template <int D>
-static __global__ void rag_cov_combine_kernel(const RagSeg* __restrict__ segs, const long long* __restrict__ rowoff,
-                                              int nseg, const double* __restrict__ part, const double* __restrict__ at,
-                                              double* __restrict__ pxt, double* __restrict__ dat, int T, int step,
-                                              int d) {
-    const long long total = rowoff[nseg];
-    for (long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x; q < total;
-         q += (long long)gridDim.x * blockDim.x) {
-        const int s = seg_lookup(rowoff, nseg, q);
-        const RagSeg& g = segs[s];
-        const long long i = q - rowoff[s];
-        const double* pn = pxt + (((long long)(T + 1) * g.row0 + (long long)(step + 1) * g.n + i) * d);
-        double* pc = pxt + (((long long)(T + 1) * g.row0 + (long long)step * g.n + i) * d);
-        const double* a = at + (((long long)T * g.row0 + (long long)step * g.n + i) * d);
-        double* da = dat ? dat + (((long long)T * g.row0 + (long long)step * g.n + i) * d) : nullptr;
-        double f[D];
-        for (int j = 0; j < D; ++j) f[j] = 0.0;
-#pragma unroll 4
-        for (int k = 0; k < g.split; ++k) {
-            const double* pk = part + (g.part + (long long)k * g.n + i) * D;
-            for (int j = 0; j < D; ++j) f[j] += pk[j];
-        }
-        for (int j = 0; j < d; ++j) {
-            pc[j] = pn[j] + g.extra * (g.dscale * f[j]);
-            if (da) da[j] = 2.0 * g.rw * a[j] - pn[j];
+struct EpiRagCov {
+    static constexpr bool NONE = false;
+    const RagSeg* segs;
+    const double *xt, *at;
+    double *pxt, *dat;
+    int T, step, d;
+    RagPlanes nx;
+    long long tstride, sstride;
+    template <int NOUT>
+    LDDMM_D void run(const SegDesc& sd, int row0, int rows, const double* red) const {
+        const RagSeg& g = segs[sd.id];
+        const long long prev = (long long)g.n * d;
+        for (int r = threadIdx.x; r < ((rows + 31) & ~31); r += blockDim.x) {   // whole warps: fold boxes
+            const bool valid = r < rows;
+            const long long i = row0 + r;
+            const double* pn = pxt + (((long long)(T + 1) * g.row0 + (long long)(step + 1) * g.n + i) * d);
+            double* pc = pxt + (((long long)(T + 1) * g.row0 + (long long)step * g.n + i) * d);
+            const double* a = at + (((long long)T * g.row0 + (long long)step * g.n + i) * d);
+            double* da = dat ? dat + (((long long)T * g.row0 + (long long)step * g.n + i) * d) : nullptr;
+            double p[3] = {0, 0, 0};
+            for (int j = 0; j < d && valid; ++j) {
+                p[j] = pn[j] + g.extra * (g.dscale * red[r * NOUT + j]);
+                pc[j] = p[j];
+                if (da) da[j] = 2.0 * g.rw * a[j] - pn[j];
+            }
+            if (step > 0) {
+                const double* x = xt + (((long long)(T + 1) * g.row0 + (long long)(step - 1) * g.n + i) * d);
+                rag_cov_row<D>(g, i, valid ? x : nullptr, a - prev, p, d, nx, tstride, sstride);
+            }
         }
     }
-}
+};
 
 template <int KIND, int QDEG, int D>
 int rag_cov_impl(int nseg, const int64_t* v_off, int d, const double* xt, const double* at, int T,
@@ -424,19 +444,19 @@ int rag_cov_impl(int nseg, const int64_t* v_off, int d, const double* xt, const 
     std::vector<long long> n(nseg);
     for (int s = 0; s < nseg; ++s) n[s] = v_off[s + 1] - v_off[s];
     RagPlan<Op> pl = rag_plan<Op>(n, n);
-    std::vector<long long> padoff(nseg + 1, 0), rowoff(nseg + 1, 0);
-    for (int s = 0; s < nseg; ++s) {
-        padoff[s + 1] = padoff[s] + std::max(pl.segs[s].tpad, pl.segs[s].spad);
-        rowoff[s + 1] = rowoff[s] + n[s];
-    }
+    std::vector<long long> padoff(nseg + 1, 0);
+    for (int s = 0; s < nseg; ++s) padoff[s + 1] = padoff[s] + std::max(pl.segs[s].tpad, pl.segs[s].spad);
     RagSeg* dsegs = ws.take<RagSeg>(nseg);
     SegDesc* ddesc = ws.take<SegDesc>(nseg);
     long long* dpad = ws.take<long long>(nseg + 1);
-    long long* drow = ws.take<long long>(nseg + 1);
-    float4* tgt = ws.take<float4>((size_t)NT * pl.tt);
-    float4* src = ws.take<float4>((size_t)Op::NS * pl.ss);
-    float4* boxes = ws.take<float4>(2 * (size_t)(pl.ss / kFold));
+    RagPlanes pn[2];
+    for (RagPlanes& p : pn) {
+        p.tgt = ws.take<float4>((size_t)NT * pl.tt);
+        p.src = ws.take<float4>((size_t)Op::NS * pl.ss);
+        p.boxes = ws.take<float4>(2 * (size_t)(pl.ss / kFold));
+    }
     double* part = ws.take<double>((size_t)pl.parts * D);
+    int* counters = ws.take<int>((size_t)pl.eparts + 1);
     if (ws.measuring()) return LDDMM_OK;
     for (int s = 0; s < nseg; ++s) {
         const KScale ks = kernel_scale(KIND, order, sigma[s], true);
@@ -449,29 +469,27 @@ int rag_cov_impl(int nseg, const int64_t* v_off, int d, const double* xt, const 
     LDDMM_TRY(rag_copy_table(pl.segs.data(), sizeof(RagSeg) * nseg, dsegs, st));
     LDDMM_TRY(rag_copy_table(pl.desc.data(), sizeof(SegDesc) * nseg, ddesc, st));
     LDDMM_TRY(rag_copy_table(padoff.data(), sizeof(long long) * (nseg + 1), dpad, st));
-    LDDMM_TRY(rag_copy_table(rowoff.data(), sizeof(long long) * (nseg + 1), drow, st));
+    LDDMM_TRY(cuda_check(cudaMemsetAsync(counters, 0, sizeof(int) * ((size_t)pl.eparts + 1), st), "memset"));
     for (int s = 0; s < nseg; ++s)
         LDDMM_TRY(cuda_check(cudaMemcpyAsync(pxt + ((T + 1) * v_off[s] + (long long)T * n[s]) * d, px1 + v_off[s] * d,
                                              sizeof(double) * n[s] * d, cudaMemcpyDeviceToDevice, st), "cov copy"));
     rag_bbox_launch<true>(dsegs, nseg, nbb, xt, nullptr, d, T, st);   // x_0 of each trajectory block
     KernelParams2 P{};
-    P.src4 = src;
     P.src_stride = pl.ss;
-    P.tgt4 = tgt;
     P.tgt_stride = pl.tt;
-    const KScale ks0 = kernel_scale(KIND, order, sigma[0], true);
-    for (int j = 0; j < 5; ++j) P.pkd[j] = dup_coeff(ks0.pk[j]);
-    for (int j = 0; j < 4; ++j) P.pqd[j] = dup_coeff(ks0.pq[j]);
+    set_poly(P, kernel_scale(KIND, order, sigma[0], true));
     SweepGrid grid{};
     grid.segs = ddesc;
     grid.nseg = nseg;
     grid.n_items = pl.items;
-    for (int t = T - 1; t >= 0; --t) {
-        rag_cov_pack_kernel<D><<<grid_for(padoff[nseg]), 256, 0, st>>>(dsegs, dpad, nseg, xt, at, pxt, T, t, d, tgt,
-                                                                      pl.tt, src, pl.ss, boxes);
-        sweep_kernel<Op><<<pl.items, 32 * kSweepWarps, 0, st>>>(grid, P, boxes, part);
-        rag_cov_combine_kernel<D><<<grid_for(rowoff[nseg]), 256, 0, st>>>(dsegs, drow, nseg, part, at, pxt, dat, T, t,
-                                                                         d);
+    rag_cov_pack_kernel<D><<<grid_for(padoff[nseg]), 256, 0, st>>>(dsegs, dpad, nseg, xt, at, pxt, T, d,
+                                                                  pn[(T - 1) & 1], pn[T & 1], pl.tt, pl.ss);
+    for (int t = T - 1; t >= 0 && pl.items > 0; --t) {
+        P.tgt4 = pn[t & 1].tgt;
+        P.src4 = pn[t & 1].src;
+        const EpiRagCov<D> E{dsegs, xt, at, pxt, dat, T, t, d, pn[(t + 1) & 1], pl.tt, pl.ss};
+        sweep_kernel<Op, false, EpiRagCov<D>><<<pl.items, 32 * kSweepWarps, 0, st>>>(grid, P, pn[t & 1].boxes, part,
+                                                                                    counters, E);
     }
     return cuda_check(cudaGetLastError(), "ragged covector");
 }
@@ -509,26 +527,21 @@ static __global__ void rag_applyk_pack_kernel(const RagSeg* __restrict__ segs, c
     }
 }
 
-template <int DIMB>
-static __global__ void rag_applyk_combine_kernel(const RagSeg* __restrict__ segs, const long long* __restrict__ rowoff,
-                                                 int nseg, const double* __restrict__ part, int dimb,
-                                                 double* __restrict__ f) {
-    const long long total = rowoff[nseg];
-    for (long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x; q < total;
-         q += (long long)gridDim.x * blockDim.x) {
-        const int s = seg_lookup(rowoff, nseg, q);
-        const RagSeg& g = segs[s];
-        const long long i = q - rowoff[s];
-        double v[DIMB];
-        for (int c = 0; c < DIMB; ++c) v[c] = 0.0;
-#pragma unroll 4
-        for (int k = 0; k < g.split; ++k) {
-            const double* pk = part + (g.part + (long long)k * g.n + i) * DIMB;
-            for (int c = 0; c < DIMB; ++c) v[c] += pk[c];
+// f rows [rowoff[s], + n) of segment s
+struct EpiRagSum {
+    static constexpr bool NONE = false;
+    const long long* rowoff;
+    double* f;
+    int dimb;
+    template <int NOUT>
+    LDDMM_D void run(const SegDesc& sd, int row0, int rows, const double* red) const {
+        const long long q0 = rowoff[sd.id] + row0;
+        for (int i = threadIdx.x; i < rows * dimb; i += blockDim.x) {
+            const int r = i / dimb;
+            f[q0 * dimb + i] = red[r * NOUT + (i - r * dimb)];
         }
-        for (int c = 0; c < dimb && c < DIMB; ++c) f[q * dimb + c] = v[c];
     }
-}
+};
 
 template <int KIND, int DEG, int D, int DIMB>
 int rag_applyk_impl(int nseg, const int64_t* t_start, const int64_t* t_count, const int64_t* s_start,
@@ -556,6 +569,7 @@ int rag_applyk_impl(int nseg, const int64_t* t_start, const int64_t* t_count, co
     float4* src = ws.take<float4>((size_t)Op::NS * pl.ss);
     float4* boxes = ws.take<float4>(2 * (size_t)(pl.ss / kFold));
     double* part = ws.take<double>((size_t)pl.parts * DIMB);
+    int* counters = ws.take<int>((size_t)pl.eparts + 1);
     if (ws.measuring()) return LDDMM_OK;
     for (int s = 0; s < nseg; ++s) {
         const KScale ks = kernel_scale(KIND, order, sigma[s], true);
@@ -567,23 +581,23 @@ int rag_applyk_impl(int nseg, const int64_t* t_start, const int64_t* t_count, co
     LDDMM_TRY(rag_copy_table(pl.desc.data(), sizeof(SegDesc) * nseg, ddesc, st));
     LDDMM_TRY(rag_copy_table(padoff.data(), sizeof(long long) * (nseg + 1), dpad, st));
     LDDMM_TRY(rag_copy_table(rowoff.data(), sizeof(long long) * (nseg + 1), drow, st));
+    LDDMM_TRY(cuda_check(cudaMemsetAsync(counters, 0, sizeof(int) * ((size_t)pl.eparts + 1), st), "memset"));
     rag_bbox_launch<false>(dsegs, nseg, nbb, x, y, d, 0, st);
     KernelParams2 P{};
     P.src4 = src;
     P.src_stride = pl.ss;
     P.tgt4 = tgt;
     P.tgt_stride = pl.tt;
-    const KScale ks0 = kernel_scale(KIND, order, sigma[0], true);
-    for (int j = 0; j < 5; ++j) P.pkd[j] = dup_coeff(ks0.pk[j]);
-    for (int j = 0; j < 4; ++j) P.pqd[j] = dup_coeff(ks0.pq[j]);
+    set_poly(P, kernel_scale(KIND, order, sigma[0], true));
     SweepGrid grid{};
     grid.segs = ddesc;
     grid.nseg = nseg;
     grid.n_items = pl.items;
     rag_applyk_pack_kernel<D, DIMB><<<grid_for(padoff[nseg]), 256, 0, st>>>(dsegs, dpad, nseg, x, y, beta, d, dimb,
                                                                              tgt, pl.tt, src, pl.ss, boxes);
-    if (pl.items > 0) sweep_kernel<Op><<<pl.items, 32 * kSweepWarps, 0, st>>>(grid, P, boxes, part);
-    rag_applyk_combine_kernel<DIMB><<<grid_for(rowoff[nseg]), 256, 0, st>>>(dsegs, drow, nseg, part, dimb, f);
+    const EpiRagSum E{drow, f, dimb};
+    if (pl.items > 0)
+        sweep_kernel<Op, false, EpiRagSum><<<pl.items, 32 * kSweepWarps, 0, st>>>(grid, P, boxes, part, counters, E);
     return cuda_check(cudaGetLastError(), "ragged applyk");
 }
 
@@ -622,57 +636,45 @@ static __global__ void rag_dt_pack_kernel(const RagSeg* __restrict__ segs, const
     }
 }
 
-// energy partial of the segment's block: sum_k w1_k . z_k
-static __global__ void rag_dt_value_kernel(const RagSeg* __restrict__ segs, int nseg, int norm,
-                                           const double* __restrict__ part, int nout, const double* __restrict__ s1,
-                                           int d, double eps1, double* __restrict__ epart) {
-    const int b = blockIdx.x;
-    int lo = 0, hi = nseg - 1;
-    while (lo < hi) {
-        const int mid = (lo + hi + 1) >> 1;
-        if (segs[mid].eoff <= b) lo = mid; else hi = mid - 1;
+// energy partial of the group's cells
+struct EpiRagDtValue {
+    static constexpr bool NONE = false;
+    const RagSeg* segs;
+    int norm;
+    const double* s1;
+    int d;
+    double eps1;
+    double* epart;
+    int op_rows;
+    template <int NOUT>
+    LDDMM_D void run(const SegDesc& sd, int row0, int rows, const double* red) const {
+        const RagSeg& g = segs[sd.id];
+        double e = 0.0;
+        for (int r = threadIdx.x; r < rows; r += blockDim.x)
+            e += dt_value_row(norm, red + r * NOUT, s1 + (g.row0 + row0 + r) * d, d, eps1);
+        e = block_sum_all(e);
+        if (threadIdx.x == 0) epart[g.eoff + row0 / op_rows] = e;
     }
-    const RagSeg& g = segs[lo];
-    const int lb = b - (int)g.eoff;
-    double e = 0.0;
-    for (long long i = (long long)lb * blockDim.x + threadIdx.x; i < g.n; i += (long long)g.nb * blockDim.x) {
-        double z[4] = {0, 0, 0, 0};
-#pragma unroll 4
-        for (int k = 0; k < g.split; ++k) {
-            const double* pk = part + (g.part + (long long)k * g.n + i) * nout;
-            for (int c = 0; c < nout && c < 4; ++c) z[c] += pk[c];
-        }
-        const double* sv = s1 + (g.row0 + i) * d;
-        if (norm == NCURRENT) {
-            for (int j = 0; j < d; ++j) e += sv[j] * z[j];
-        } else {
-            e += vec_norm_eps(sv, d, eps1) * z[0];
-        }
-    }
-    const double r = rag_block_sum(e);
-    if (threadIdx.x == 0) epart[b] = r;
-}
+};
 
-static __global__ void rag_dt_grad_kernel(const RagSeg* __restrict__ segs, const long long* __restrict__ rowoff,
-                                          int nseg, int norm, const double* __restrict__ part, int nout,
-                                          const double* __restrict__ s1, int d, double eps1, double fac,
-                                          double* __restrict__ z1, double* __restrict__ dz1) {
-    const long long total = rowoff[nseg];
-    for (long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x; q < total;
-         q += (long long)gridDim.x * blockDim.x) {
-        const int sg = seg_lookup(rowoff, nseg, q);
-        const RagSeg& g = segs[sg];
-        const long long i = q - rowoff[sg];
-        double acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-#pragma unroll 2
-        for (int k = 0; k < g.split; ++k) {
-            const double* pk = part + (g.part + (long long)k * g.n + i) * nout;
-            for (int c = 0; c < nout && c < 8; ++c) acc[c] += pk[c];
+// per-cell z1, dz1
+struct EpiRagDtGrad {
+    static constexpr bool NONE = false;
+    const RagSeg* segs;
+    int norm;
+    const double* s1;
+    int d;
+    double eps1, fac;
+    double *z1, *dz1;
+    template <int NOUT>
+    LDDMM_D void run(const SegDesc& sd, int row0, int rows, const double* red) const {
+        const RagSeg& g = segs[sd.id];
+        for (int r = threadIdx.x; r < rows; r += blockDim.x) {
+            const long long q = (g.row0 + row0 + r) * d;
+            dt_grad_row(norm, red + r * NOUT, s1 + q, d, eps1, fac * g.dscale, z1 + q, dz1 + q);
         }
-        const long long r = g.row0 + i;
-        dt_grad_row(norm, acc, s1 + r * d, d, eps1, fac * g.dscale, z1 + r * d, dz1 + r * d);
     }
-}
+};
 
 struct RagDataArgs {
     int nseg;
@@ -695,11 +697,13 @@ struct RagDataArgs {
     double* px;
 };
 
-// SYM (values): each segment's cell-cell self part is evaluated once per
+// One sweep over all segments: energies into a.energy, or (GRAD) the cells' z1, dz1.
+// Values are SYM: each segment's cell-cell self part is evaluated once per
 // unordered pair (sweep_kernel<Op, true>); its target cells start at a fold.
-template <class Real, class Op, int TSLOTS, int SSLOTS, int NT, bool SYM = false>
-int rag_dt_sweep(const RagDataArgs& a, int kind, int grad, double sign2, const double* c1, const double* s1,
-                 Workspace& ws, cudaStream_t st, RagPlan<Op>& pl, RagSeg*& dsegs, long long*& drow, double*& part) {
+template <class Real, class Op, int TSLOTS, int SSLOTS, int NT, bool GRAD>
+int rag_dt_sweep(const RagDataArgs& a, int kind, const double* c1, const double* s1, Workspace& ws, cudaStream_t st,
+                 double* z1, double* dz1) {
+    constexpr bool SYM = !GRAD;
     const int nseg = a.nseg;
     std::vector<long long> n(nseg), m(nseg), n1s(nseg);
     for (int s = 0; s < nseg; ++s) {
@@ -707,24 +711,24 @@ int rag_dt_sweep(const RagDataArgs& a, int kind, int grad, double sign2, const d
         n1s[s] = SYM ? round_up(n[s], kFold) : n[s];
         m[s] = n1s[s] + (a.c2_off[s + 1] - a.c2_off[s]);
     }
-    pl = rag_plan<Op>(n, m);
+    RagPlan<Op> pl = rag_plan<Op>(n, m);
     for (int s = 0; s < nseg; ++s) pl.desc[s].sym_folds = SYM ? (int)(n1s[s] / kFold) : 0;
-    std::vector<long long> padoff(nseg + 1, 0), rowoff(nseg + 1, 0);
+    std::vector<long long> padoff(nseg + 1, 0);
     for (int s = 0; s < nseg; ++s) {
         pl.segs[s].row0 = a.c_off[s];
         pl.segs[s].m0 = a.c2_off[s];
         pl.segs[s].m = a.c2_off[s + 1] - a.c2_off[s];
         padoff[s + 1] = padoff[s] + std::max(pl.segs[s].tpad, pl.segs[s].spad);
-        rowoff[s + 1] = rowoff[s] + n[s];
     }
-    dsegs = ws.take<RagSeg>(nseg);
+    RagSeg* dsegs = ws.take<RagSeg>(nseg);
     SegDesc* ddesc = ws.take<SegDesc>(nseg);
     long long* dpad = ws.take<long long>(nseg + 1);
-    drow = ws.take<long long>(nseg + 1);
     float4* tgt = ws.take<float4>((size_t)NT * pl.tt);
     float4* src = ws.take<float4>((size_t)Op::NS * pl.ss);
     float4* boxes = ws.take<float4>(2 * (size_t)(pl.ss / kFold));
-    part = ws.take<double>((size_t)pl.parts * Op::NOUT);
+    double* part = ws.take<double>((size_t)pl.parts * Op::NOUT);
+    int* counters = ws.take<int>((size_t)pl.eparts + 1);
+    double* epart = ws.take<double>(GRAD ? 0 : (size_t)pl.eparts + 1);
     if (ws.measuring()) return LDDMM_OK;
     for (int s = 0; s < nseg; ++s) {
         const KScale ks = kernel_scale(kind, a.order, a.sigma[s], true);
@@ -737,23 +741,33 @@ int rag_dt_sweep(const RagDataArgs& a, int kind, int grad, double sign2, const d
     LDDMM_TRY(rag_copy_table(pl.segs.data(), sizeof(RagSeg) * nseg, dsegs, st));
     LDDMM_TRY(rag_copy_table(pl.desc.data(), sizeof(SegDesc) * nseg, ddesc, st));
     LDDMM_TRY(rag_copy_table(padoff.data(), sizeof(long long) * (nseg + 1), dpad, st));
-    LDDMM_TRY(rag_copy_table(rowoff.data(), sizeof(long long) * (nseg + 1), drow, st));
+    LDDMM_TRY(cuda_check(cudaMemsetAsync(counters, 0, sizeof(int) * ((size_t)pl.eparts + 1), st), "memset"));
     if (!a.frame) rag_bbox_launch<false>(dsegs, nseg, nbb, c1, a.c2, a.d, 0, st);
     typename Op::Params P{};
     P.src4 = src;
     P.src_stride = pl.ss;
     P.tgt4 = tgt;
     P.tgt_stride = pl.tt;
-    const KScale ks0 = kernel_scale(kind, a.order, a.sigma[0], true);
-    set_data_poly<Op, Real>(P, ks0);
+    set_poly(P, kernel_scale(kind, a.order, a.sigma[0], true));
     rag_dt_pack_kernel<Real><<<grid_for(padoff[nseg]), 256, 0, st>>>(
-        dsegs, dpad, nseg, a.norm, grad, c1, s1, a.c2, a.s2, a.d, a.eps1, a.eps2, sign2, tgt, pl.tt, NT, TSLOTS, src,
+        dsegs, dpad, nseg, a.norm, GRAD ? 1 : 0, c1, s1, a.c2, a.s2, a.d, a.eps1, a.eps2, GRAD ? -1.0 : -2.0, tgt, pl.tt, NT, TSLOTS, src,
         pl.ss, Op::NS, SSLOTS, op_list<Op>::value ? 1 : 0, SYM ? kFold : 0, boxes);
     SweepGrid grid{};
     grid.segs = ddesc;
     grid.nseg = nseg;
     grid.n_items = pl.items;
-    if (pl.items > 0) sweep_kernel<Op, SYM><<<pl.items, 32 * kSweepWarps, 0, st>>>(grid, P, boxes, part);
+    if constexpr (GRAD) {
+        const EpiRagDtGrad E{dsegs, a.norm, s1, a.d, a.eps1, a.ncorner == 3 ? 1.0 / 3.0 : 0.5, z1, dz1};
+        if (pl.items > 0)
+            sweep_kernel<Op, false, EpiRagDtGrad><<<pl.items, 32 * kSweepWarps, 0, st>>>(grid, P, boxes, part,
+                                                                                        counters, E);
+    } else {
+        const EpiRagDtValue E{dsegs, a.norm, s1, a.d, a.eps1, epart, op_group<Op>()};
+        if (pl.items > 0)
+            sweep_kernel<Op, true, EpiRagDtValue><<<pl.items, 32 * kSweepWarps, 0, st>>>(grid, P, boxes, part,
+                                                                                        counters, E);
+        rag_energy_kernel<<<(nseg + 3) / 4, 128, 0, st>>>(dsegs, nseg, epart, 1.0, a.energy, 0);
+    }
     return cuda_check(cudaGetLastError(), "ragged data sweep");
 }
 
@@ -767,78 +781,39 @@ int rag_dt_impl(const RagDataArgs& a, Workspace& ws, cudaStream_t st) {
     double* s1 = ws.take<double>((size_t)C * a.d);
     if (!ws.measuring())
         cell_geometry_kernel<<<grid_for(C), 256, 0, st>>>(a.ncorner, a.v, NV, a.d, a.cells, C, c1, s1);
+    constexpr bool PACK = sizeof(Real) == 4 && D == 3;   // FP32 surfaces: packed-pair operators with list records
     if (a.energy != nullptr) {
-        RagSeg* dsegs = nullptr;
-        long long* drow = nullptr;
-        double* part = nullptr;
-        int nout = 1, rc = LDDMM_OK;
-        long long eparts = 0;
         if (a.norm == NVARIFOLD) {
-            // FP32: packed-pair operator (two targets per slot, list records)
-            using Op = std::conditional_t<(sizeof(Real) == 4 && D == 3), OpVariValue2<KIND, PDEG>,
+            using Op = std::conditional_t<PACK, OpVariValue2<KIND, PDEG>,
                                           OpData<Real, KIND, PDEG, QDEG, D, M_VARI_VALUE>>;
-            RagPlan<Op> pl;
-            rc = rag_dt_sweep<Real, Op, 3, 4, PP + (3 + PW - 1) / PW, true>(a, KIND, 0, -2.0, c1, s1, ws, st, pl, dsegs,
-                                                                       drow, part);
-            nout = Op::NOUT;
-            eparts = pl.eparts;
+            LDDMM_TRY((rag_dt_sweep<Real, Op, 3, 4, PP + (3 + PW - 1) / PW, false>(a, KIND, c1, s1, ws, st, nullptr,
+                                                                                   nullptr)));
         } else if (a.norm == NCURRENT) {
             using Op = OpApplyK<Real, KIND, PDEG, D, D>;
-            RagPlan<Op> pl;
-            rc = rag_dt_sweep<Real, Op, 0, D, PP, true>(a, KIND, 0, -2.0, c1, s1, ws, st, pl, dsegs, drow, part);
-            nout = Op::NOUT;
-            eparts = pl.eparts;
+            LDDMM_TRY((rag_dt_sweep<Real, Op, 0, D, PP, false>(a, KIND, c1, s1, ws, st, nullptr, nullptr)));
         } else {
             using Op = OpApplyK<Real, KIND, PDEG, D, 1>;
-            RagPlan<Op> pl;
-            rc = rag_dt_sweep<Real, Op, 0, 1, PP, true>(a, KIND, 0, -2.0, c1, s1, ws, st, pl, dsegs, drow, part);
-            nout = Op::NOUT;
-            eparts = pl.eparts;
-        }
-        if (rc != LDDMM_OK) return rc;
-        double* epart = ws.take<double>((size_t)std::max<long long>(1, eparts));
-        if (!ws.measuring()) {
-            rag_dt_value_kernel<<<(int)eparts, kRagThreads, 0, st>>>(dsegs, a.nseg, a.norm, part, nout, s1, a.d,
-                                                                    a.eps1, epart);
-            rag_energy_kernel<<<(a.nseg + 127) / 128, 128, 0, st>>>(dsegs, a.nseg, epart, 1.0, a.energy, 0);
+            LDDMM_TRY((rag_dt_sweep<Real, Op, 0, 1, PP, false>(a, KIND, c1, s1, ws, st, nullptr, nullptr)));
         }
     }
     if (a.px != nullptr) {
-        RagSeg* dsegs = nullptr;
-        long long* drow = nullptr;
-        double* part = nullptr;
-        int nout = 1, rc = LDDMM_OK;
-        constexpr bool PACK = sizeof(Real) == 4 && D == 3;   // FP32 surfaces: packed-pair operators
+        double* z1 = ws.take<double>((size_t)C * a.d);
+        double* dz1 = ws.take<double>((size_t)C * a.d);
         if (a.norm == NVARIFOLD) {
             using Op = std::conditional_t<PACK, OpVariGrad2<KIND, PDEG, QDEG>,
                                           OpData<Real, KIND, PDEG, QDEG, D, M_VARI_GRAD>>;
-            RagPlan<Op> pl;
-            rc = rag_dt_sweep<Real, Op, 3, 4, PP + (3 + PW - 1) / PW>(a, KIND, 1, -1.0, c1, s1, ws, st, pl, dsegs,
-                                                                       drow, part);
-            nout = Op::NOUT;
+            LDDMM_TRY((rag_dt_sweep<Real, Op, 3, 4, PP + (3 + PW - 1) / PW, true>(a, KIND, c1, s1, ws, st, z1, dz1)));
         } else if (a.norm == NCURRENT) {
             using Op = std::conditional_t<PACK, OpCurGrad2<KIND, PDEG, QDEG>,
                                           OpData<Real, KIND, PDEG, QDEG, D, M_CUR_GRAD>>;
-            RagPlan<Op> pl;
-            rc = rag_dt_sweep<Real, Op, D, D, PP + (D + PW - 1) / PW>(a, KIND, 1, -1.0, c1, s1, ws, st, pl, dsegs,
-                                                                       drow, part);
-            nout = Op::NOUT;
+            LDDMM_TRY((rag_dt_sweep<Real, Op, D, D, PP + (D + PW - 1) / PW, true>(a, KIND, c1, s1, ws, st, z1, dz1)));
         } else {
             using Op = OpData<Real, KIND, PDEG, QDEG, D, M_MEAS_GRAD>;
-            RagPlan<Op> pl;
-            rc = rag_dt_sweep<Real, Op, 0, 1, PP>(a, KIND, 1, -1.0, c1, s1, ws, st, pl, dsegs, drow, part);
-            nout = Op::NOUT;
+            LDDMM_TRY((rag_dt_sweep<Real, Op, 0, 1, PP, true>(a, KIND, c1, s1, ws, st, z1, dz1)));
         }
-        if (rc != LDDMM_OK) return rc;
-        double* z1 = ws.take<double>((size_t)C * a.d);
-        double* dz1 = ws.take<double>((size_t)C * a.d);
-        if (!ws.measuring()) {
-            const double fac = a.ncorner == 3 ? 1.0 / 3.0 : 0.5;
-            rag_dt_grad_kernel<<<grid_for(C), 256, 0, st>>>(dsegs, drow, a.nseg, a.norm, part, nout, s1, a.d, a.eps1,
-                                                           fac, z1, dz1);
+        if (!ws.measuring())
             dt_gather_kernel<<<grid_for(NV), 256, 0, st>>>(a.ncorner, a.v, NV, a.d, a.cells, C, a.vptr, a.vidx, z1,
                                                            dz1, a.px);
-        }
     }
     if (ws.measuring()) return LDDMM_OK;
     return cuda_check(cudaGetLastError(), "ragged dataterm");

@@ -94,102 +94,100 @@ LDDMM_D void store_box(float4* boxes, long long i, bool valid, const double* x, 
     store_fold_box<Real>(boxes, i, valid, p, w);
 }
 
-// block-level FP64 sum with a fixed tree; thread 0 writes out[blockIdx.x]
-LDDMM_D void block_sum_store(double v, double* out) {
-    __shared__ double red[kCombineThreads];
-    red[threadIdx.x] = v;
-    __syncthreads();
-    for (int s = kCombineThreads / 2; s > 0; s >>= 1) {
-        if (threadIdx.x < s) red[threadIdx.x] += red[threadIdx.x + s];
-        __syncthreads();
-    }
-    if (threadIdx.x == 0) out[blockIdx.x] = red[0];
-}
-
-// kernel polynomials into either parameter block
-inline void set_poly(KernelParamsBase<double>& P, const KScale& ks) {
-    for (int j = 0; j < 5; ++j) P.pk[j] = ks.pk[j];
-    for (int j = 0; j < 4; ++j) P.pq[j] = ks.pq[j];
-}
-inline void set_poly(KernelParamsBase<float>& P, const KScale& ks) {
-    for (int j = 0; j < 5; ++j) P.pk[j] = (float)ks.pk[j];
-    for (int j = 0; j < 4; ++j) P.pq[j] = (float)ks.pq[j];
-}
-inline void set_poly(KernelParams2& P, const KScale& ks) {
-    for (int j = 0; j < 5; ++j) P.pkd[j] = dup_coeff(ks.pk[j]);
-    for (int j = 0; j < 4; ++j) P.pqd[j] = dup_coeff(ks.pq[j]);
-}
-
 // ---- shooting ---------------------------------------------------------------
-// Packs step-0 planes: targets (pos) and sources (pos, a).
+// Packed planes of one step: a sweep reads one set while its epilogue writes the other.
+struct StepPlanes {
+    float4 *tgt, *src, *boxes;
+};
+
+// Packs step-0 planes: targets (pos) and sources (pos, a); pads both sets, copies
+// x to xt[0], zeroes the counters.
 template <class Real, bool LIST>
 static __global__ void shoot_pack_kernel(const double* __restrict__ x, const double* __restrict__ a, long long n,
-                                         int d, double s, const double* __restrict__ c, float4* tgt,
-                                         long long tstride, float4* src, long long sstride, int pp, int nslots,
-                                         int ns, float4* boxes) {
+                                         int d, double s, const double* __restrict__ c, StepPlanes p0, StepPlanes p1,
+                                         long long tstride, long long sstride, int pp, int nslots, int ns,
+                                         double* __restrict__ xt0, int* __restrict__ counters, int n_counters) {
     const long long npad = tstride > sstride ? tstride : sstride;
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < npad;
          i += (long long)gridDim.x * blockDim.x) {
-        if (i < sstride) store_box<Real>(boxes, i, i < n, x + i * d, a + i * d, nullptr, d, s, c);
+        if (i < n_counters) counters[i] = 0;
+        if (i < sstride) store_box<Real>(p0.boxes, i, i < n, x + i * d, a + i * d, nullptr, d, s, c);
         if (i < n) {
-            if (i < tstride) store_point<Real>(tgt, tstride, i, x + i * d, d, s, c);
-            if (i < sstride) {
-                if constexpr (LIST) {
-                    store_list(src, sstride, i, x + i * d, d, nslots, s, c, a + i * d, d, nslots);
-                } else {
-                    store_point<Real>(src, sstride, i, x + i * d, d, s, c);
-                    store_vals<Real>(src, sstride, i, pp, a + i * d, d, nslots);
-                }
+            for (int j = 0; j < d; ++j) xt0[i * d + j] = x[i * d + j];
+            store_point<Real>(p0.tgt, tstride, i, x + i * d, d, s, c);
+            if constexpr (LIST) {
+                store_list(p0.src, sstride, i, x + i * d, d, nslots, s, c, a + i * d, d, nslots);
+            } else {
+                store_point<Real>(p0.src, sstride, i, x + i * d, d, s, c);
+                store_vals<Real>(p0.src, sstride, i, pp, a + i * d, d, nslots);
             }
         } else {
-            if (i < tstride) zero_record<Real>(tgt, tstride, i, pp);
-            if (i < sstride) zero_record<Real>(src, sstride, i, ns);
-        }
-    }
-}
-
-// v = sum of chunks; x1 = x0 + dt v; energy partial <a, v>; pack next step.
-template <class Real, bool LIST>
-static __global__ void shoot_combine_kernel(const double* __restrict__ part, long long n, int d, int dout,
-                                            int split, double dt, const double* __restrict__ x0,
-                                            const double* __restrict__ a0, double* __restrict__ x1,
-                                            const double* __restrict__ a1, double s, const double* __restrict__ c,
-                                            float4* tgt, long long tstride, float4* src, long long sstride, int pp,
-                                            int nslots, float4* boxes, double* __restrict__ epart) {
-    double e = 0.0;
-    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < sstride;   // whole warps: n padded to folds
-         i += (long long)gridDim.x * blockDim.x) {
-        const bool valid = i < n;
-        double xn[4];
-        for (int j = 0; j < d && valid; ++j) {
-            double v = 0.0;
-            for (int k = 0; k < split; ++k) v += part[((long long)k * n + i) * dout + j];
-            e += a0[i * d + j] * v;
-            xn[j] = x0[i * d + j] + dt * v;
-            x1[i * d + j] = xn[j];
-        }
-        if (a1 != nullptr) store_box<Real>(boxes, i, valid, xn, a1 + i * d, nullptr, d, s, c);
-        if (a1 != nullptr && valid) {
-            store_point<Real>(tgt, tstride, i, xn, d, s, c);
-            if constexpr (LIST) {
-                store_list(src, sstride, i, xn, d, nslots, s, c, a1 + i * d, d, nslots);
-            } else {
-                store_point<Real>(src, sstride, i, xn, d, s, c);
-                store_vals<Real>(src, sstride, i, pp, a1 + i * d, d, nslots);
+            if (i < tstride) {
+                zero_record<Real>(p0.tgt, tstride, i, pp);
+                zero_record<Real>(p1.tgt, tstride, i, pp);
+            }
+            if (i < sstride) {
+                zero_record<Real>(p0.src, sstride, i, ns);
+                zero_record<Real>(p1.src, sstride, i, ns);
             }
         }
     }
-    block_sum_store(e, epart);
 }
 
-// out = scale * sum(vals[0..count)) in a fixed order (single block)
-static __global__ void finalize_sum_kernel(const double* __restrict__ vals, long long count, double scale,
-                                           double* __restrict__ out) {
-    double v = 0.0;
-    for (long long i = threadIdx.x; i < count; i += blockDim.x) v += vals[i];
-    block_sum_store(v, out);
-    if (threadIdx.x == 0) out[0] = scale * out[0];
-}
+// v = the group's sums; x1 = x0 + dt v; energy partial <a, v>; pack next step.
+// The last step's last group adds the energy.
+template <class Real, bool LIST>
+struct EpiShoot {
+    static constexpr bool NONE = false;
+    int d, pp, nslots;
+    double dt, s;
+    const double* c;
+    const double *x0, *a0;
+    double* x1;
+    const double* a1;   // next step's momenta, NULL for the last step
+    StepPlanes nx;
+    long long tstride, sstride;
+    double* epart;      // this step's partials, one per group
+    // last step: energy = escale * (all steps' partials), if energy
+    double* energy;
+    const double* eall;
+    long long ecount;
+    double escale;
+    int* counter;
+    int groups, op_rows;   // groups, and rows of one
+    template <int NOUT>
+    LDDMM_D void run(const SegDesc&, int row0, int rows, const double* red) const {
+        double e = 0.0;
+        for (int r = threadIdx.x; r < ((rows + 31) & ~31); r += blockDim.x) {   // whole warps: fold boxes
+            const bool valid = r < rows;
+            const long long i = row0 + r;
+            double xn[3] = {0, 0, 0};
+            for (int j = 0; j < d && valid; ++j) {
+                const double v = red[r * NOUT + j];
+                e += a0[i * d + j] * v;
+                xn[j] = x0[i * d + j] + dt * v;
+                x1[i * d + j] = xn[j];
+            }
+            if (a1 == nullptr) continue;
+            store_box<Real>(nx.boxes, i, valid, xn, a1 + i * d, nullptr, d, s, c);
+            if (!valid) continue;
+            store_point<Real>(nx.tgt, tstride, i, xn, d, s, c);
+            if constexpr (LIST) {
+                store_list(nx.src, sstride, i, xn, d, nslots, s, c, a1 + i * d, d, nslots);
+            } else {
+                store_point<Real>(nx.src, sstride, i, xn, d, s, c);
+                store_vals<Real>(nx.src, sstride, i, pp, a1 + i * d, d, nslots);
+            }
+        }
+        e = block_sum_all(e);
+        if (threadIdx.x == 0) epart[row0 / op_rows] = e;
+        if (energy == nullptr || !last_block(counter, groups)) return;
+        double t = 0.0;
+        for (long long q = threadIdx.x; q < ecount; q += blockDim.x) t += __ldcg(eall + q);
+        t = block_sum_all(t);
+        if (threadIdx.x == 0) *energy = escale * t;
+    }
+};
 
 struct ShootArgs {
     const double* x0;
@@ -226,37 +224,40 @@ int shoot_impl(const ShootArgs& a, Workspace& ws, cudaStream_t st) {
     constexpr bool LIST = sizeof(Real) == 4;  // FP32: packed-pair operator with list records
     using Op = std::conditional_t<LIST, OpApplyK2<KIND, DEG, D, D, SMALL>, OpApplyK<Real, KIND, DEG, D, D, SMALL>>;
     const SinglePlan pl = plan_single<Op>(a.n, a.n);
-    float4* tgt = ws.take<float4>((size_t)Op::PP * pl.n_tpad);
-    float4* src = ws.take<float4>((size_t)Op::NS * pl.m_pad);
-    float4* boxes = ws.take<float4>(pl.box_words());
-    double* part = ws.take<double>((size_t)pl.split * a.n * D);
-    const int nb = combine_blocks(a.n);
-    double* epart = ws.take<double>((size_t)a.T * nb);
+    StepPlanes pn[2];
+    for (StepPlanes& p : pn) {
+        p.tgt = ws.take<float4>((size_t)Op::PP * pl.n_tpad);
+        p.src = ws.take<float4>((size_t)Op::NS * pl.m_pad);
+        p.boxes = ws.take<float4>(pl.box_words());
+    }
+    double* part = ws.take<double>(pl.part_doubles(a.n, D));
+    int* counters = ws.take<int>(pl.counters());
+    double* epart = ws.take<double>((size_t)a.T * pl.n_tb);
     double* center = ws.take<double>(kCenterWords);
     if (ws.measuring()) return LDDMM_OK;
     const KScale ks = kernel_scale(KIND, a.order, a.sigma, !pl.seq);
     typename Op::Params P{};
-    P.src4 = src;
     P.src_stride = pl.m_pad;
-    P.tgt4 = tgt;
     P.tgt_stride = pl.n_tpad;
     set_poly(P, ks);
     const long long N = a.n * a.d;
-    LDDMM_TRY(cuda_check(cudaMemcpyAsync(a.xt, a.x0, sizeof(double) * N, cudaMemcpyDeviceToDevice, st), "shoot copy"));
     launch_bbox_center(a.x0, a.n, nullptr, 0, a.d, center, st);
     shoot_pack_kernel<Real, LIST><<<grid_for(std::max(pl.n_tpad, pl.m_pad)), 256, 0, st>>>(
-        a.x0, a.at, a.n, a.d, ks.scale, center, tgt, pl.n_tpad, src, pl.m_pad, Op::PP, D, Op::NS, boxes);
+        a.x0, a.at, a.n, a.d, ks.scale, center, pn[0], pn[1], pl.n_tpad, pl.m_pad, Op::PP, D, Op::NS, a.xt, counters,
+        (int)pl.counters());
     const double dt = a.dt > 0 ? a.dt : 1.0 / a.T;
     for (int t = 0; t < a.T; ++t) {
-        LDDMM_TRY(launch_single<Op>(pl, a.n, P, boxes, part, st));
-        shoot_combine_kernel<Real, LIST><<<nb, kCombineThreads, 0, st>>>(
-            part, a.n, a.d, D, pl.split, dt, a.xt + t * N, a.at + t * N, a.xt + (t + 1) * N,
-            t + 1 < a.T ? a.at + (t + 1) * N : nullptr, ks.scale, center, tgt, pl.n_tpad, src, pl.m_pad, Op::PP,
-            D, boxes, epart + (long long)t * nb);
+        const StepPlanes& p = pn[t & 1];
+        P.tgt4 = p.tgt;
+        P.src4 = p.src;
+        const bool last = t + 1 == a.T;
+        EpiShoot<Real, LIST> E{a.d, Op::PP, D, dt, ks.scale, center, a.xt + t * N, a.at + t * N, a.xt + (t + 1) * N,
+                               last ? nullptr : a.at + (t + 1) * N, pn[(t + 1) & 1], pl.n_tpad, pl.m_pad,
+                               epart + (long long)t * pl.n_tb, last ? a.energy : nullptr, epart,
+                               (long long)a.T * pl.n_tb, a.rw * dt, counters + pl.n_tb, pl.n_tb, op_group<Op>()};
+        LDDMM_TRY((launch_single<Op, false>(pl, a.n, P, p.boxes, part, st, 0, counters, E)));
     }
-    if (a.energy != nullptr)
-        finalize_sum_kernel<<<1, kCombineThreads, 0, st>>>(epart, (long long)a.T * nb, a.rw * dt, a.energy);
-    return cuda_check(cudaGetLastError(), "shoot");
+    return LDDMM_OK;
 }
 
 // n <= kFusedMaxPoints (and d >= 2): all T steps in one cluster launch (fused_small.cuh)
@@ -345,52 +346,67 @@ LDDMM_D void cov_store(float4* tgt, long long tstride, float4* src, long long ss
     }
 }
 
+// Packs the planes of step T-1; pads both sets, copies p to pxt[T], zeroes the counters.
 template <class Real, bool LIST>
 static __global__ void cov_pack_kernel(const double* __restrict__ x, const double* __restrict__ a,
                                        const double* __restrict__ p, long long n, int d, double s,
-                                       const double* __restrict__ c, double rw, float4* tgt, long long tstride,
-                                       float4* src, long long sstride, int pp, int tplanes, int nplanes, int tw,
-                                       float4* boxes) {
+                                       const double* __restrict__ c, double rw, StepPlanes p0, StepPlanes p1,
+                                       long long tstride, long long sstride, int pp, int tplanes, int nplanes, int tw,
+                                       double* __restrict__ pT, int* __restrict__ counters, int n_counters) {
     const long long npad = tstride > sstride ? tstride : sstride;
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < npad;
          i += (long long)gridDim.x * blockDim.x) {
-        if (i < sstride) store_box<Real>(boxes, i, i < n, x + i * d, a + i * d, p + i * d, d, s, c);
+        if (i < n_counters) counters[i] = 0;
+        if (i < sstride) store_box<Real>(p0.boxes, i, i < n, x + i * d, a + i * d, p + i * d, d, s, c);
         if (i < n) {
-            cov_store<Real, LIST>(tgt, tstride, src, sstride, i, pp, x + i * d, a + i * d, p + i * d, d, s, c, rw, tw);
+            for (int j = 0; j < d; ++j) pT[i * d + j] = p[i * d + j];
+            cov_store<Real, LIST>(p0.tgt, tstride, p0.src, sstride, i, pp, x + i * d, a + i * d, p + i * d, d, s, c,
+                                  rw, tw);
         } else {
-            if (i < tstride) zero_record<Real>(tgt, tstride, i, tplanes);
-            if (i < sstride) zero_record<Real>(src, sstride, i, nplanes);
+            if (i < tstride) {
+                zero_record<Real>(p0.tgt, tstride, i, tplanes);
+                zero_record<Real>(p1.tgt, tstride, i, tplanes);
+            }
+            if (i < sstride) {
+                zero_record<Real>(p0.src, sstride, i, nplanes);
+                zero_record<Real>(p1.src, sstride, i, nplanes);
+            }
         }
     }
 }
 
-// p_t = p_{t+1} + dt * dscale * sum(chunks); dat_t = 2 rw a_t - p_{t+1}; pack step t-1.
+// p_t = p_{t+1} + dt * dscale * sums; dat_t = 2 rw a_t - p_{t+1}; pack step t-1.
 template <class Real, bool LIST>
-static __global__ void cov_combine_kernel(const double* __restrict__ part, long long n, int d, int dout, int split,
-                                          double dt, double dscale, double rw, const double* __restrict__ p_next,
-                                          const double* __restrict__ a_t, double* __restrict__ p_t,
-                                          double* __restrict__ dat_t, const double* __restrict__ x_prev,
-                                          const double* __restrict__ a_prev, double s, const double* __restrict__ c,
-                                          float4* tgt, long long tstride, float4* src, long long sstride, int pp,
-                                          int tw, float4* boxes) {
-    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < sstride;   // whole warps: n padded to folds
-         i += (long long)gridDim.x * blockDim.x) {
-        const bool valid = i < n;
-        double pn[4];
-        for (int j = 0; j < d && valid; ++j) {
-            double f = 0.0;
-            for (int k = 0; k < split; ++k) f += part[((long long)k * n + i) * dout + j];
-            const double pj = p_next[i * d + j];
-            pn[j] = pj + dt * (dscale * f);
-            p_t[i * d + j] = pn[j];
-            if (dat_t != nullptr) dat_t[i * d + j] = 2.0 * rw * a_t[i * d + j] - pj;
+struct EpiCov {
+    static constexpr bool NONE = false;
+    int d, pp, tw;
+    double dt, dscale, rw, s;
+    const double* c;
+    const double *p_next, *a_t;
+    double *p_t, *dat_t;
+    const double *x_prev, *a_prev;   // NULL for step 0
+    StepPlanes nx;
+    long long tstride, sstride;
+    template <int NOUT>
+    LDDMM_D void run(const SegDesc&, int row0, int rows, const double* red) const {
+        for (int r = threadIdx.x; r < ((rows + 31) & ~31); r += blockDim.x) {   // whole warps: fold boxes
+            const bool valid = r < rows;
+            const long long i = row0 + r;
+            double pn[3] = {0, 0, 0};
+            for (int j = 0; j < d && valid; ++j) {
+                const double pj = p_next[i * d + j];
+                pn[j] = pj + dt * (dscale * red[r * NOUT + j]);
+                p_t[i * d + j] = pn[j];
+                if (dat_t != nullptr) dat_t[i * d + j] = 2.0 * rw * a_t[i * d + j] - pj;
+            }
+            if (x_prev == nullptr) continue;
+            store_box<Real>(nx.boxes, i, valid, x_prev + i * d, a_prev + i * d, pn, d, s, c);
+            if (valid)
+                cov_store<Real, LIST>(nx.tgt, tstride, nx.src, sstride, i, pp, x_prev + i * d, a_prev + i * d, pn, d,
+                                      s, c, rw, tw);
         }
-        if (x_prev != nullptr) store_box<Real>(boxes, i, valid, x_prev + i * d, a_prev + i * d, pn, d, s, c);
-        if (x_prev != nullptr && valid)
-            cov_store<Real, LIST>(tgt, tstride, src, sstride, i, pp, x_prev + i * d, a_prev + i * d, pn, d, s, c, rw,
-                                 tw);
     }
-}
+};
 
 struct CovArgs {
     const double* xt;
@@ -414,38 +430,41 @@ int cov_impl(const CovArgs& a, Workspace& ws, cudaStream_t st) {
     using Op = std::conditional_t<LIST, OpDiffKT2<KIND, DEG, D, W, SMALL>, OpDiffKT<Real, KIND, DEG, D, W>>;
     constexpr int NT = LIST ? 1 + (W + 3) / 4 : Op::NS;  // target planes (standard layout)
     const SinglePlan pl = plan_single<Op>(a.n, a.n);
-    float4* tgt = ws.take<float4>((size_t)NT * pl.n_tpad);
-    float4* src = ws.take<float4>((size_t)Op::NS * pl.m_pad);
-    float4* boxes = ws.take<float4>(pl.box_words());
-    double* part = ws.take<double>((size_t)pl.split * a.n * D);
+    StepPlanes pn[2];
+    for (StepPlanes& p : pn) {
+        p.tgt = ws.take<float4>((size_t)NT * pl.n_tpad);
+        p.src = ws.take<float4>((size_t)Op::NS * pl.m_pad);
+        p.boxes = ws.take<float4>(pl.box_words());
+    }
+    double* part = ws.take<double>(pl.part_doubles(a.n, D));
+    int* counters = ws.take<int>(pl.counters());
     double* center = ws.take<double>(kCenterWords);
     if (ws.measuring()) return LDDMM_OK;
     const KScale ks = kernel_scale(KIND, a.order, a.sigma, !pl.seq);
     typename Op::Params P{};
-    P.src4 = src;
     P.src_stride = pl.m_pad;
-    P.tgt4 = tgt;
     P.tgt_stride = pl.n_tpad;
     set_poly(P, ks);
     const long long N = a.n * a.d;
     const double dt = a.dt > 0 ? a.dt : 1.0 / a.T;
-    LDDMM_TRY(cuda_check(cudaMemcpyAsync(a.pxt + (long long)a.T * N, a.px1, sizeof(double) * N,
-                                         cudaMemcpyDeviceToDevice, st), "covector copy"));
     const int T = a.T;
     launch_bbox_center(a.xt, a.n, nullptr, 0, a.d, center, st);
     cov_pack_kernel<Real, LIST><<<grid_for(std::max(pl.n_tpad, pl.m_pad)), 256, 0, st>>>(
         a.xt + (long long)(T - 1) * N, a.at + (long long)(T - 1) * N, a.px1, a.n, a.d, ks.scale, center, a.rw,
-        tgt, pl.n_tpad, src, pl.m_pad, Op::PP, NT, Op::NS, W, boxes);
-    const int nb = combine_blocks(a.n);
+        pn[(T - 1) & 1], pn[T & 1], pl.n_tpad, pl.m_pad, Op::PP, NT, Op::NS, W, a.pxt + (long long)T * N, counters,
+        (int)pl.counters());
     for (int t = T - 1; t >= 0; --t) {
-        LDDMM_TRY(launch_single<Op>(pl, a.n, P, boxes, part, st));
-        cov_combine_kernel<Real, LIST><<<nb, kCombineThreads, 0, st>>>(
-            part, a.n, a.d, D, pl.split, dt, ks.dscale, a.rw, a.pxt + (long long)(t + 1) * N,
-            a.at + (long long)t * N, a.pxt + (long long)t * N, a.dat ? a.dat + (long long)t * N : nullptr,
-            t > 0 ? a.xt + (long long)(t - 1) * N : nullptr, t > 0 ? a.at + (long long)(t - 1) * N : nullptr,
-            ks.scale, center, tgt, pl.n_tpad, src, pl.m_pad, Op::PP, W, boxes);
+        const StepPlanes& p = pn[t & 1];
+        P.tgt4 = p.tgt;
+        P.src4 = p.src;
+        EpiCov<Real, LIST> E{a.d, Op::PP, W, dt, ks.dscale, a.rw, ks.scale, center, a.pxt + (long long)(t + 1) * N,
+                             a.at + (long long)t * N, a.pxt + (long long)t * N,
+                             a.dat ? a.dat + (long long)t * N : nullptr,
+                             t > 0 ? a.xt + (long long)(t - 1) * N : nullptr,
+                             t > 0 ? a.at + (long long)(t - 1) * N : nullptr, pn[(t + 1) & 1], pl.n_tpad, pl.m_pad};
+        LDDMM_TRY((launch_single<Op, false>(pl, a.n, P, p.boxes, part, st, 0, counters, E)));
     }
-    return cuda_check(cudaGetLastError(), "covector");
+    return LDDMM_OK;
 }
 
 template <class Real, int KIND, int QDEG, int D>

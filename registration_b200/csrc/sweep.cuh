@@ -16,8 +16,13 @@
 // order, folded into a TwoSum-compensated (sum, err) pair (FP32 ops), or plain
 // FP64 sums.  The block adds its warps in order and writes doubles into
 //   part[(seg.part + chunk * seg.n_tgt + t) * Op::NOUT + c]
-// and a separate combine kernel adds the chunks in a fixed order, so results
-// do not depend on scheduling.
+// The block of a group that finishes last adds the chunks in their order and
+// hands the group's sums to the epilogue Epi (which scales and writes them, or
+// takes the Euler step and packs the next sweep's records), so results do not
+// depend on scheduling.  The groups' counters start at zero and are left at
+// zero.  A separate combine launch per sweep cost 4-10 us of a shot's step at a
+// few thousand points (13 blocks, each thread adding its row's chunks one after
+// the other).  EpiNone leaves the chunk sums in `part`.
 //
 // Far folds (operators with Op::lgk, `boxes` given).  The pack kernels leave
 // for each fold its bounding box and log2 of the sum of its weights.  With the
@@ -109,19 +114,30 @@ struct op_has_out_scale : std::false_type {};
 template <class Op>
 struct op_has_out_scale<Op, std::void_t<decltype(Op::out_scale(0))>> : std::true_type {};
 
-// Resident blocks per SM that the register budget is cut for, and the unrolling
-// of the source loop.  Measured at n = m = 131,072 (FP32) and 32,768 (FP64):
-// both run best with 128 registers (4 blocks) and 8 sources in flight (FP32
-// Gaussian applyK 2.69 -> 2.78e12 pairs/s against no bound and 4 sources,
-// Laplacian applyDiffKT 1.54 -> 1.62e12; FP64 applyK 6.35 -> 6.5e11, varifold
-// gradient 4.1 -> 4.2e11).  Operators with many outputs or wide records keep 168
-// registers (3 blocks) instead of spilling.
+// An operator may name the resident blocks per SM that its register budget is cut for.
+template <class Op, class = void>
+struct op_has_min_blocks : std::false_type {};
+template <class Op>
+struct op_has_min_blocks<Op, std::void_t<decltype(Op::MIN_BLOCKS)>> : std::true_type {};
+
+// Resident blocks per SM and the unrolling of the source loop.  Measured at
+// n = m = 131,072 (FP32) and 32,768 (FP64), 1e12 pairs/s:
+//   FP32, 8 / 16 / 32 sources unrolled, 128 registers (4 blocks):
+//     Gaussian applyK 2.93 / 3.07 / 3.07, Laplacian 1.97 / 2.00 / 2.02,
+//     adjoint 1.66 / 1.71 / 1.73, current gradient 1.63 / 1.62 / 1.66
+//   gradient sums with 168 registers (3 blocks), 32 sources: Gaussian 2.09 ->
+//     2.18, Laplacian 1.67 -> 1.72, adjoint 1.73 -> 1.74
+//   FP64, 8 / 16 / 32 sources: applyK 0.646 / 0.658 / 0.653, varifold gradient
+//     0.424 / 0.428 / 0.333
+// Operators with many outputs or wide records keep 168 registers as well.
 template <class Op>
 constexpr int op_min_blocks() {
-    return sizeof(typename Op::Real) == 4 ? (Op::NOUT * Op::R > 24 || Op::NS > 6 ? 3 : 4)
-                                          : (Op::NOUT > 4 || Op::NS > 5 ? 3 : 4);
+    if constexpr (op_has_min_blocks<Op>::value) return Op::MIN_BLOCKS;
+    else if constexpr (sizeof(typename Op::Real) == 4) return Op::NOUT * Op::R > 24 || Op::NS > 6 ? 3 : 4;
+    else return Op::NOUT > 4 || Op::NS > 5 ? 3 : 4;
 }
-constexpr int kSweepUnroll = 8;
+template <class Op>
+constexpr int op_unroll() { return sizeof(typename Op::Real) == 4 ? kFold : kFold / 2; }
 
 // Operators that bound their kernel factor (Op::lgk) can pass over far folds.
 template <class Op, class = void>
@@ -203,10 +219,62 @@ LDDMM_D void store_fold_box(float4* boxes, long long row, bool valid, const Real
     }
 }
 
-template <class Op, bool SYM = false>
+// Whether this block is the last of `total` to come here (all threads ask; what
+// the others wrote before is visible to the last one).  The counter goes back to
+// zero.
+LDDMM_D bool last_block(int* counter, int total) {
+    __shared__ int last;
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        last = atomicAdd(counter, 1) == total - 1;
+        if (last) *counter = 0;
+    }
+    __syncthreads();
+    const bool r = last != 0;
+    __threadfence();
+    return r;
+}
+
+// Sum over the block in a fixed tree; every thread gets it.
+LDDMM_D double block_sum_all(double v) {
+    __shared__ double ws[32];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
+    if ((threadIdx.x & 31) == 0) ws[threadIdx.x >> 5] = v;
+    __syncthreads();
+    double r = 0.0;
+    for (int w = 0; w < (int)(blockDim.x >> 5); ++w) r += ws[w];
+    __syncthreads();
+    return r;
+}
+
+// Epilogues: run() is called by all threads of a group's last block with the
+// group's sums red[row * NOUT + c], rows [row0, row0 + rows) of the segment.
+struct EpiNone {
+    static constexpr bool NONE = true;
+};
+
+// f[row, col0 + c] = scale * sum, c < ncols
+struct EpiSum {
+    static constexpr bool NONE = false;
+    double* f;
+    long long ld;
+    int col0, ncols;
+    double scale;
+    template <int NOUT>
+    LDDMM_D void run(const SegDesc&, int row0, int rows, const double* red) const {
+        for (int i = threadIdx.x; i < rows * ncols; i += blockDim.x) {
+            const int r = i / ncols, c = i - r * ncols;
+            f[(row0 + r) * ld + col0 + c] = scale * red[r * NOUT + c];
+        }
+    }
+};
+
+template <class Op, bool SYM, class Epi>
 __global__ void __launch_bounds__(32 * kSweepWarps, op_min_blocks<Op>())
-    sweep_kernel(const SweepGrid grid, const typename Op::Params P, const float4* __restrict__ boxes,
-                 double* __restrict__ part) {
+    sweep_kernel(const SweepGrid grid, const typename Op::Params P, const float4* __restrict__ boxes, double* part,
+                 int* counters, const Epi E) {
     constexpr int R = Op::R, TPS = Op::TPS, NS = Op::NS, NOUT = Op::NOUT, GT = op_group<Op>();
     constexpr int STAGE = NS * kFold;   // 16-byte words of one fold
     constexpr int STAGES = NS > 6 ? 2 : 3;   // folds of a warp's ring (at most 48 KB for the block)
@@ -214,12 +282,13 @@ __global__ void __launch_bounds__(32 * kSweepWarps, op_min_blocks<Op>())
     constexpr int RED = (GT * NOUT * 8 + 15) / 16;
     __shared__ __align__(16) float4 smem[RING > RED ? RING : RED];
     __shared__ float sbox[kSweepWarps][7];
+    __shared__ Box wbox;   // the group's box
 
     const int item = blockIdx.x;
     const SegDesc sg = find_segment(grid, item);
     const int local = item - sg.item0;
-    const int tb = local % sg.n_tb;
-    const int chunk = local / sg.n_tb;
+    const int tb = local / sg.split;
+    const int chunk = local - tb * sg.split;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 
     // targets of this lane: t = tb*GT + r*32 + lane (rows are padded); an
@@ -245,7 +314,6 @@ __global__ void __launch_bounds__(32 * kSweepWarps, op_min_blocks<Op>())
     }
 
     // the group's box and the threshold below which a fold is passed over
-    Box wb{};
     float thr = 0.f;
     bool cull = false;
     const float4* fbox = nullptr;
@@ -282,6 +350,7 @@ __global__ void __launch_bounds__(32 * kSweepWarps, op_min_blocks<Op>())
                 }
             }
             cull = !__syncthreads_or(bad);
+            Box wb;
 #pragma unroll
             for (int j = 0; j < 3; ++j) {
                 wb.lo[j] = sbox[0][j];
@@ -313,6 +382,7 @@ __global__ void __launch_bounds__(32 * kSweepWarps, op_min_blocks<Op>())
             }
             lgl = warp_max(lgl);
             if (lane == 0) sbox[warp][6] = lgl;
+            if (threadIdx.x == 0) wbox = wb;
             __syncthreads();
             for (int w = 0; w < kSweepWarps; ++w) lgl = fmaxf(lgl, sbox[w][6]);
             constexpr float kMargin = sizeof(Real) == 4 ? 36.f : 58.f;
@@ -333,7 +403,7 @@ __global__ void __launch_bounds__(32 * kSweepWarps, op_min_blocks<Op>())
                 if (cull && act) {
                     float d0, d1;
                     const float4 bl = fbox[2 * f];
-                    box_dist2(wb, bl, fbox[2 * f + 1], d0, d1);
+                    box_dist2(wbox, bl, fbox[2 * f + 1], d0, d1);
                     float u = bl.w + Op::lgk(P, d0);
                     if (Op::GRADX) u += 0.5f * __log2f(fmaxf(1.f, d1));
                     act = !(u <= thr);
@@ -375,7 +445,7 @@ __global__ void __launch_bounds__(32 * kSweepWarps, op_min_blocks<Op>())
         const float4* S = ring + st * STAGE;
 #pragma unroll
         for (int q = 0; q < SLOTS; ++q) acc[q].begin_fold();
-#pragma unroll kSweepUnroll
+#pragma unroll op_unroll<Op>()
         for (int j = 0; j < kFold; ++j) {
             typename Op::Src s;
             Op::load_source(S, j, s);
@@ -419,33 +489,54 @@ __global__ void __launch_bounds__(32 * kSweepWarps, op_min_blocks<Op>())
     }
     const int rows = min(GT, sg.n_tgt - tb * GT);
     double* dst = part + (sg.part + (long long)chunk * sg.n_tgt + (long long)tb * GT) * NOUT;
-    for (int i = threadIdx.x; i < rows * NOUT; i += 32 * kSweepWarps) dst[i] = red[i];
+    if constexpr (Epi::NONE) {
+        for (int i = threadIdx.x; i < rows * NOUT; i += 32 * kSweepWarps) dst[i] = red[i];
+    } else {
+        if (sg.split > 1) {
+            for (int i = threadIdx.x; i < rows * NOUT; i += 32 * kSweepWarps) dst[i] = red[i];
+            if (!last_block(counters + sg.cnt + tb, sg.split)) return;
+            const double* p0 = part + (sg.part + (long long)tb * GT) * NOUT;
+            const long long step = (long long)sg.n_tgt * NOUT;
+            for (int i = threadIdx.x; i < rows * NOUT; i += 32 * kSweepWarps) {
+                double v = 0.0;
+                for (int k0 = 0; k0 < sg.split; k0 += 16) {   // 16 loads in flight
+                    double q[16];
+#pragma unroll
+                    for (int j = 0; j < 16; ++j) q[j] = k0 + j < sg.split ? __ldcg(p0 + (k0 + j) * step + i) : 0.0;
+#pragma unroll
+                    for (int j = 0; j < 16; ++j) v += q[j];
+                }
+                red[i] = v;
+            }
+            __syncthreads();
+        }
+        E.template run<NOUT>(sg, tb * GT, rows, red);
+    }
 }
 
 // FP64 sums over at most kSeqFolds folds: one thread per target adds all sources
 // in their order, as the reference's loop does.  An optimiser run on a few
 // hundred points amplifies the last bits of its FP64 sums by 1e7 over 50
 // iterations, so these keep the reference's order to the bit; the sums are too
-// small for the split of the sweep above to gain anything (256 x 256 points: 8
-// blocks, one source after the other, 10 us).
+// small for the split of the sweep above to gain anything.
 constexpr int kSeqFolds = 15;
-template <class Op>
-__global__ void __launch_bounds__(32) sweep_seq_kernel(const SegDesc sg, const typename Op::Params P,
-                                                       double* __restrict__ part) {
+template <class Op, class Epi>
+__global__ void __launch_bounds__(op_group<Op>()) sweep_seq_kernel(const SegDesc sg, const typename Op::Params P,
+                                                                   double* part, const Epi E) {
     static_assert(Op::TPS == 1, "unpacked operators");
-    constexpr int NS = Op::NS, NOUT = Op::NOUT;
+    constexpr int NS = Op::NS, NOUT = Op::NOUT, GT = op_group<Op>();
     __shared__ __align__(16) float4 S[NS * kFold];
-    const long long t = (long long)blockIdx.x * 32 + threadIdx.x;   // rows are padded to whole groups
+    __shared__ double red[GT * NOUT];
+    const int t = blockIdx.x * GT + threadIdx.x;   // rows are padded to whole groups
     typename Op::Tgt tg;
     Op::load_target(P, sg.tgt + t, tg);
     typename Op::Acc acc;
     acc.zero();
     for (int f = 0; f < sg.n_folds; ++f) {
-        const float4* g = P.src4 + sg.src + (long long)f * kFold + threadIdx.x;
-        __syncwarp();
-#pragma unroll
-        for (int w = 0; w < NS; ++w) S[w * kFold + threadIdx.x] = g[(long long)w * P.src_stride];
-        __syncwarp();
+        const float4* g = P.src4 + sg.src + (long long)f * kFold;
+        __syncthreads();
+        for (int i = threadIdx.x; i < NS * kFold; i += GT) S[i] = g[(long long)(i / kFold) * P.src_stride + i % kFold];
+        __syncthreads();
 #pragma unroll 4
         for (int j = 0; j < kFold; ++j) {
             typename Op::Src s;
@@ -453,8 +544,14 @@ __global__ void __launch_bounds__(32) sweep_seq_kernel(const SegDesc sg, const t
             Op::template pair<true>(P, tg, s, acc);
         }
     }
-    if (t < sg.n_tgt)
-        for (int c = 0; c < NOUT; ++c) part[(sg.part + t) * NOUT + c] = acc.value(c);
+    if constexpr (Epi::NONE) {
+        if (t < sg.n_tgt)
+            for (int c = 0; c < NOUT; ++c) part[(sg.part + t) * NOUT + c] = acc.value(c);
+    } else {
+        for (int c = 0; c < NOUT; ++c) red[threadIdx.x * NOUT + c] = acc.value(c);
+        __syncthreads();
+        E.template run<NOUT>(sg, blockIdx.x * GT, min(GT, sg.n_tgt - (int)blockIdx.x * GT), red);
+    }
 }
 
 // ---------------------------------------------------------------------------

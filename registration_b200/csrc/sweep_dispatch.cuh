@@ -4,20 +4,13 @@
 #include <type_traits>
 
 #include "host.h"
-#include "ops.cuh"
+#include "ops2.cuh"
 #include "sweep.cuh"
 
 namespace lddmm {
 
 template <int V>
 using IC = std::integral_constant<int, V>;
-
-// Nominal resident blocks of a sweep on the whole device (8 per SM for every
-// operator, so plans and workspaces do not depend on register allocation).
-template <class Op>
-int sweep_slots() {
-    return 8 * device_info().sms;
-}
 
 // Problems with at most this many targets use the SMALL shape of the operators
 // that have one (groups of 64 targets: more, smaller items).
@@ -30,28 +23,34 @@ struct SinglePlan {
     long long n_tpad, m_pad;
     int n_tb, n_folds, split;
     bool seq;   // FP64 sums over few sources: sweep_seq_kernel, coordinates in the x/s frame (kfun.cuh)
+    // chunk sums (doubles) of a sweep with an epilogue: none where a group has one chunk
+    size_t part_doubles(long long n, int nout) const { return split > 1 ? (size_t)split * n * nout : 0; }
+    size_t counters() const { return (size_t)n_tb + 1; }
     size_t box_words() const { return 2 * (size_t)(m_pad / kFold); }   // float4 words of the fold boxes
 };
 
 template <class Op>
-SinglePlan plan_single(long long n, long long m, int split_cap = 0) {
+SinglePlan plan_single(long long n, long long m, int split_cap = 0, bool shared = false) {
     SinglePlan p;
     const long long per_group = op_group<Op>();
     p.n_tb = (int)((n + per_group - 1) / per_group);
     p.n_tpad = (long long)std::max(p.n_tb, 1) * per_group;
     p.n_folds = (int)((m + kFold - 1) / kFold);
     p.m_pad = (long long)std::max(p.n_folds, 1) * kFold;
-    p.split = choose_split(p.n_tb, p.n_folds, sweep_slots<Op>());
-    p.seq = sizeof(typename Op::Real) == 8 && p.n_folds <= kSeqFolds;   // split is 1 for so few folds
+    const int sms = device_info().sms;
+    p.split = choose_split(p.n_tb, p.n_folds, sms, sms * op_min_blocks<Op>(), shared);
+    p.seq = sizeof(typename Op::Real) == 8 && p.n_folds <= kSeqFolds;
+    if (p.seq) p.split = 1;
     if (split_cap > 0 && p.split > split_cap) p.split = split_cap;
     return p;
 }
 
 // boxes: fold boxes written with the packed sources, or NULL (every fold counts).
-// SYM: symmetric sweep over sym_folds own folds (see sweep_kernel<Op, true>)
-template <class Op, bool SYM = false>
+// SYM: symmetric sweep over sym_folds own folds (see sweep_kernel<Op, true>).
+// Epi: what is done with a group's sums; counters: n_tb + 1 zeros (see sweep_kernel).
+template <class Op, bool SYM = false, class Epi = EpiNone>
 int launch_single(const SinglePlan& pl, long long n, const typename Op::Params& P, const float4* boxes, double* part,
-                  cudaStream_t st, int sym_folds = 0) {
+                  cudaStream_t st, int sym_folds = 0, int* counters = nullptr, const Epi& E = Epi()) {
     SweepGrid g{};
     g.seg0.n_tgt = (int)n;
     g.seg0.n_folds = pl.n_folds;
@@ -63,11 +62,11 @@ int launch_single(const SinglePlan& pl, long long n, const typename Op::Params& 
     if (g.n_items <= 0) return LDDMM_OK;
     if constexpr (sizeof(typename Op::Real) == 8) {
         if (pl.seq) {
-            sweep_seq_kernel<Op><<<(unsigned)((n + 31) / 32), 32, 0, st>>>(g.seg0, P, part);
+            sweep_seq_kernel<Op, Epi><<<pl.n_tb, op_group<Op>(), 0, st>>>(g.seg0, P, part, E);
             return cuda_check(cudaGetLastError(), "sweep launch");
         }
     }
-    sweep_kernel<Op, SYM><<<g.n_items, 32 * kSweepWarps, 0, st>>>(g, P, boxes, part);
+    sweep_kernel<Op, SYM, Epi><<<g.n_items, 32 * kSweepWarps, 0, st>>>(g, P, boxes, part, counters, E);
     return cuda_check(cudaGetLastError(), "sweep launch");
 }
 
@@ -101,6 +100,20 @@ inline KScale kernel_scale(int kind, int order, double sigma, bool base2, bool e
     }
     k.dscale = -1.0 / (sigma * sigma * k.scale);
     return k;
+}
+
+// kernel polynomials into either parameter block
+inline void set_poly(KernelParamsBase<double>& P, const KScale& ks) {
+    for (int j = 0; j < 5; ++j) P.pk[j] = ks.pk[j];
+    for (int j = 0; j < 4; ++j) P.pq[j] = ks.pq[j];
+}
+inline void set_poly(KernelParamsBase<float>& P, const KScale& ks) {
+    for (int j = 0; j < 5; ++j) P.pk[j] = (float)ks.pk[j];
+    for (int j = 0; j < 4; ++j) P.pq[j] = (float)ks.pq[j];
+}
+inline void set_poly(KernelParams2& P, const KScale& ks) {
+    for (int j = 0; j < 5; ++j) P.pkd[j] = dup_coeff(ks.pk[j]);
+    for (int j = 0; j < 4; ++j) P.pqd[j] = dup_coeff(ks.pq[j]);
 }
 
 // order > 4: Gaussian; otherwise Laplacian with polynomial degree = order (K)
