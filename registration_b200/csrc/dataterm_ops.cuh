@@ -496,16 +496,18 @@ struct EpiDtValue {
     int d;
     double eps1;
     double* epart;
-    int groups, op_rows;   // groups, and rows of one
+    int groups;
     int* counter;
     double* energy;
-    template <int NOUT>
-    LDDMM_D void run(const SegDesc&, int row0, int rows, const double* red) const {
+    template <int GT, int NOUT>
+    LDDMM_D void run(const SegDesc& sg, int tb, const int* srow, const double* red) const {
         double e = 0.0;
-        for (int r = threadIdx.x; r < rows; r += blockDim.x)
-            e += dt_value_row(norm, red + r * NOUT, s1 + (long long)(row0 + r) * d, d, eps1);
+        for (int r = threadIdx.x; r < GT; r += blockDim.x) {
+            const long long i = srow[r];
+            if (i < sg.n_tgt) e += dt_value_row(norm, red + r * NOUT, s1 + i * d, d, eps1);
+        }
         e = block_sum_all(e);
-        if (threadIdx.x == 0) epart[row0 / op_rows] = e;
+        if (threadIdx.x == 0) epart[tb] = e;
         if (!last_block(counter, groups)) return;
         e = 0.0;
         for (int q = threadIdx.x; q < groups; q += blockDim.x) e += __ldcg(epart + q);
@@ -522,10 +524,11 @@ struct EpiDtGrad {
     int d;
     double eps1, dzscale;
     double *z1, *dz1;
-    template <int NOUT>
-    LDDMM_D void run(const SegDesc&, int row0, int rows, const double* red) const {
-        for (int r = threadIdx.x; r < rows; r += blockDim.x) {
-            const long long q = (long long)(row0 + r) * d;
+    template <int GT, int NOUT>
+    LDDMM_D void run(const SegDesc& sg, int, const int* srow, const double* red) const {
+        for (int r = threadIdx.x; r < GT; r += blockDim.x) {
+            const long long i = srow[r], q = i * d;
+            if (i >= sg.n_tgt) continue;
             dt_grad_row(norm, red + r * NOUT, s1 + q, d, eps1, dzscale, z1 + q, dz1 + q);
         }
     }

@@ -72,7 +72,7 @@ int dt_sweep(const DataArgs& a, Workspace& ws, cudaStream_t st, const double* c1
     float4* tgt = ws.take<float4>((size_t)Op::NT_ * pl.n_tpad);
     float4* src = ws.take<float4>((size_t)Op::NS * pl.m_pad);
     float4* boxes = ws.take<float4>(pl.box_words());
-    double* part = ws.take<double>(pl.part_doubles(a.nc, Op::NOUT));
+    double* part = ws.take<double>(pl.part_doubles(Op::NOUT));
     int* counters = ws.take<int>(pl.counters());
     double* epart = ws.take<double>(GRAD ? 0 : pl.n_tb);
     if (ws.measuring()) return LDDMM_OK;
@@ -91,7 +91,7 @@ int dt_sweep(const DataArgs& a, Workspace& ws, cudaStream_t st, const double* c1
         const EpiDtGrad E{a.norm, s1, a.d, a.eps1, fac * ks.dscale, z1, dz1};
         return launch_single<Op, false>(pl, a.nc, P, boxes, part, st, 0, counters, E);
     } else {
-        const EpiDtValue E{a.norm, s1, a.d, a.eps1, epart, pl.n_tb, op_group<Op>(), counters + pl.n_tb, a.energy};
+        const EpiDtValue E{a.norm, s1, a.d, a.eps1, epart, pl.n_tb, counters + pl.n_tb, a.energy};
         return launch_single<Op, true>(pl, a.nc, P, boxes, part, st, (int)(n1s / kFold), counters, E);
     }
 }

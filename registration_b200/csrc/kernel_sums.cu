@@ -36,8 +36,10 @@ int applyk_group(const ApplyKArgs& a, int col0, Workspace& ws, cudaStream_t st) 
     float4* tgt = ws.take<float4>((size_t)Op::PP * pl.n_tpad);
     float4* src = ws.take<float4>((size_t)Op::NS * pl.m_pad);
     float4* boxes = a.boxed ? ws.take<float4>(pl.box_words()) : nullptr;
-    double* part = ws.take<double>(pl.part_doubles(a.n, DIMB));
+    double* part = ws.take<double>(pl.part_doubles(DIMB));
     int* counters = ws.take<int>(pl.split > 1 ? pl.counters() : 0);
+    // sums over the targets' own points (the query cannot know: room for the order whenever n == m)
+    OrderRows order = a.boxed && a.n == a.m ? take_order_rows(ws, pl) : OrderRows{};
     double* center = ws.take<double>(kCenterWords);
     if (ws.measuring()) return LDDMM_OK;
     if (ws.overflow()) {
@@ -61,9 +63,11 @@ int applyk_group(const ApplyKArgs& a, int col0, Workspace& ws, cudaStream_t st) 
     pack_sum_kernel<Real, sizeof(Real) == 4><<<grid_for(pl.n_tpad + pl.m_pad), 256, 0, st>>>(
         a.x, a.n, Gather{}, 0, tgt, pl.n_tpad, a.y, a.m, g, D, DIMB, src, pl.m_pad, a.d, ks.scale, center, boxes,
         counters, pl.split > 1 ? (int)pl.counters() : 0);
+    if (a.x != a.y) order.perm = nullptr;
+    LDDMM_TRY((launch_order_rows<Real>(order, tgt, a.n, pl, st)));
     // the epilogue writes only the group's own columns
     const EpiSum E{a.f, a.dimb, col0, g.nvals, 1.0};
-    return launch_single<Op, false>(pl, a.n, P, boxes, part, st, 0, counters, E);
+    return launch_single<Op, false>(pl, a.n, P, boxes, part, st, 0, counters, E, order.perm);
 }
 
 template <class Real>
@@ -166,8 +170,9 @@ int difft_impl(const DiffKTArgs& a, Workspace& ws, cudaStream_t st) {
     float4* tgt = ws.take<float4>((size_t)NT * pl.n_tpad);
     float4* src = ws.take<float4>((size_t)Op::NS * pl.m_pad);
     float4* boxes = ws.take<float4>(pl.box_words());
-    double* part = ws.take<double>(pl.part_doubles(a.n, D));
+    double* part = ws.take<double>(pl.part_doubles(D));
     int* counters = ws.take<int>(pl.counters());
+    OrderRows order = a.n == a.m ? take_order_rows(ws, pl) : OrderRows{};
     double* center = ws.take<double>(kCenterWords);
     if (ws.measuring()) return LDDMM_OK;
     const KScale ks = kernel_scale(KIND, a.order, a.sigma, !pl.seq);
@@ -193,8 +198,10 @@ int difft_impl(const DiffKTArgs& a, Workspace& ws, cudaStream_t st) {
     pack_sum_kernel<Real, sizeof(Real) == 4><<<grid_for(pl.n_tpad + pl.m_pad), 256, 0, st>>>(
         a.x, a.n, gu, W, tgt, pl.n_tpad, a.y, a.m, gv, D, W, src, pl.m_pad, a.d, ks.scale, center, boxes, counters,
         (int)pl.counters());
+    if (a.x != a.y) order.perm = nullptr;
+    LDDMM_TRY((launch_order_rows<Real>(order, tgt, a.n, pl, st)));
     const EpiSum E{a.f, a.d, 0, a.d, ks.dscale};   // D may exceed d (d == 1 runs as D == 2)
-    return launch_single<Op, false>(pl, a.n, P, boxes, part, st, 0, counters, E);
+    return launch_single<Op, false>(pl, a.n, P, boxes, part, st, 0, counters, E, order.perm);
 }
 
 template <class Real>
@@ -275,7 +282,7 @@ int div_impl(const ApplyKArgs& a, Workspace& ws, cudaStream_t st) {
     const SinglePlan pl = plan_single<Op>(a.n, a.m);
     float4* tgt = ws.take<float4>((size_t)Op::PP * pl.n_tpad);
     float4* src = ws.take<float4>((size_t)Op::NS * pl.m_pad);
-    double* part = ws.take<double>(pl.part_doubles(a.n, 1));
+    double* part = ws.take<double>(pl.part_doubles(1));
     int* counters = ws.take<int>(pl.counters());
     double* center = ws.take<double>(kCenterWords);
     if (ws.measuring()) return LDDMM_OK;

@@ -185,6 +185,143 @@ static __global__ void pack_sum_kernel(const double* __restrict__ x, long long n
     }
 }
 
+// Fold boxes of packed source rows (list records of D + V values, or standard
+// planes with V values).
+template <class Real, bool LIST>
+static __global__ void fold_boxes_kernel(const float4* __restrict__ src, long long m_pad, long long n, int D, int V,
+                                         float4* __restrict__ boxes) {
+    constexpr int PW = Traits<Real>::PER_WORD;
+    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < m_pad;
+         i += (long long)gridDim.x * blockDim.x) {
+        Real p[3] = {0, 0, 0}, w = 0;
+        const int first = LIST ? D : 4, total = first + V;
+        for (int k = 0; k * PW < total; ++k) {
+            const float4 word = src[(long long)k * m_pad + i];
+            for (int q = 0; q < PW; ++q) {
+                const int j = k * PW + q;
+                const Real v = word_get<Real>(&word, q);
+                if (j < 3 && j < D) p[j] = v;
+                if (j >= first && j < total) w = max_nan(w, v);
+            }
+        }
+        store_fold_box<Real>(boxes, i, i < n, p, w);
+    }
+}
+
+// Order of the target rows by cells of a 32 x 32 x 32 grid over the packed points,
+// the cells along a Morton curve, the rows of a cell as they lie: a counting sort
+// whose result does not depend on scheduling (counts are whole numbers; the rows
+// that the scatter leaves in any order within a cell are ranked by their number).
+// Where the points crowd into a few cells (over kOrderCrowd rows in one) the rows
+// keep their order.  On a sphere of 40,962 subdivided vertices at sigma 0.05 the
+// groups' boxes let a sweep pass over 73% of the pairs instead of 55%.
+constexpr int kOrderCells = 32768, kOrderCrowd = 2048;
+LDDMM_D unsigned morton_spread(unsigned v) {   // 5 bits to every third
+    v = (v | (v << 8)) & 0x0000100Fu;
+    v = (v | (v << 4)) & 0x000010C3u;
+    return (v | (v << 2)) & 0x00001249u;
+}
+// info[0]: bits of the largest finite |coordinate|
+template <class Real>
+static __global__ void __launch_bounds__(1024) order_extent_kernel(const float4* __restrict__ tgt, long long stride,
+                                                                   long long n, int* __restrict__ info) {
+    __shared__ float sm[32];
+    float m = 0.f;
+#pragma unroll 4
+    for (long long i = threadIdx.x; i < n; i += 1024) {
+        Real x[3];
+        load_vals<Real, 3>(tgt, stride, i, 0, x);
+        for (int j = 0; j < 3; ++j) {
+            const float v = fabsf((float)x[j]);
+            if (v < INFINITY) m = fmaxf(m, v);
+        }
+    }
+    m = warp_max(m);
+    if ((threadIdx.x & 31) == 0) sm[threadIdx.x >> 5] = m;
+    __syncthreads();
+    if (threadIdx.x < 32) {
+        m = warp_max(sm[threadIdx.x]);
+        if (threadIdx.x == 0) info[0] = __float_as_int(m);
+    }
+}
+template <class Real>
+static __global__ void order_cells_kernel(const float4* __restrict__ tgt, long long stride, long long n,
+                                          const int* __restrict__ info, int* __restrict__ hist,
+                                          int* __restrict__ cell) {
+    const float m = __int_as_float(info[0]);
+    const float unit = m > 0.f ? 15.99f / m : 0.f;
+    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n;
+         i += (long long)gridDim.x * blockDim.x) {
+        Real x[3];
+        load_vals<Real, 3>(tgt, stride, i, 0, x);
+        unsigned k = 0;
+        for (int j = 0; j < 3; ++j) {
+            const float q = 16.f + (float)x[j] * unit;   // NaN and infinities: the first or the last cell
+            k |= morton_spread((unsigned)fminf(fmaxf(q, 0.f), 31.f)) << j;
+        }
+        cell[i] = (int)k;
+        atomicAdd(hist + k, 1);
+    }
+}
+// hist: counts -> starts, and a copy of them behind (the scatter's cursors); info[0]: the largest count
+static __global__ void __launch_bounds__(1024) order_scan_kernel(int* __restrict__ hist, int* __restrict__ info) {
+    __shared__ int ws[32], wm[32];
+    constexpr int PER = kOrderCells / 1024;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    int c[PER], sum = 0, big = 0;
+#pragma unroll
+    for (int q = 0; q < PER; ++q) {
+        c[q] = hist[threadIdx.x * PER + q];
+        sum += c[q];
+        big = max(big, c[q]);
+    }
+    int incl = sum;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int v = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += v;
+        big = max(big, __shfl_xor_sync(0xffffffffu, big, o));
+    }
+    if (lane == 31) ws[warp] = incl;
+    if (lane == 0) wm[warp] = big;
+    __syncthreads();
+    int at = incl - sum;
+    for (int w = 0; w < 32; ++w) {
+        if (w < warp) at += ws[w];
+        big = max(big, wm[w]);
+    }
+#pragma unroll
+    for (int q = 0; q < PER; ++q) {
+        hist[threadIdx.x * PER + q] = at;
+        hist[kOrderCells + threadIdx.x * PER + q] = at;
+        at += c[q];
+    }
+    if (threadIdx.x == 0) info[0] = big;
+}
+static __global__ void order_scatter_kernel(const int* __restrict__ cell, long long n, int* __restrict__ cursor,
+                                            int* __restrict__ tmp) {
+    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n;
+         i += (long long)gridDim.x * blockDim.x)
+        tmp[atomicAdd(cursor + cell[i], 1)] = (int)i;
+}
+static __global__ void order_rank_kernel(const int* __restrict__ tmp, const int* __restrict__ cell,
+                                         const int* __restrict__ start, const int* __restrict__ info, long long n,
+                                         long long n_pad, int* __restrict__ perm) {
+    const bool crowd = info[0] > kOrderCrowd;
+    for (long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x; q < n_pad;
+         q += (long long)gridDim.x * blockDim.x) {
+        if (crowd || q >= n) {
+            perm[q] = (int)q;
+            continue;
+        }
+        const int i = tmp[q], c = cell[i];
+        const int b = start[c], e = c + 1 < kOrderCells ? start[c + 1] : (int)n;
+        int rank = 0;
+        for (int j = b; j < e; ++j) rank += tmp[j] < i;
+        perm[b + rank] = i;
+    }
+}
+
 inline int grid_for(long long work, int block = 256, int max_blocks = 148 * 16) {
     long long b = (work + block - 1) / block;
     if (b < 1) b = 1;

@@ -102,7 +102,7 @@ RagPlan<Op> rag_plan(const std::vector<long long>& n, const std::vector<long lon
         p.items += pl.n_tb * pl.split;
         p.tt += pl.n_tpad;
         p.ss += pl.m_pad;
-        p.parts += (long long)pl.split * n[s];
+        p.parts += (long long)pl.split * pl.n_tpad;
         p.eparts += g.nb;
         row += n[s];
         mrow += m[s];
@@ -244,14 +244,14 @@ struct EpiRagShoot {
     RagPlanes nx;
     long long tstride, sstride;
     double* epart;
-    int op_rows;
-    template <int NOUT>
-    LDDMM_D void run(const SegDesc& sd, int row0, int rows, const double* red) const {
+    template <int GT, int NOUT>
+    LDDMM_D void run(const SegDesc& sd, int tb, const int* srow, const double* red) const {
         const RagSeg& g = segs[sd.id];
         double e = 0.0;
-        for (int r = threadIdx.x; r < ((rows + 31) & ~31); r += blockDim.x) {   // whole warps: fold boxes
-            const bool valid = r < rows;
-            const long long i = row0 + r;
+        for (int r = threadIdx.x; r < GT; r += blockDim.x) {
+            const long long i = srow[r];
+            const bool valid = i < g.n;
+            if (srow[r & ~31] >= g.n) continue;   // whole warps: fold boxes
             const double* x0 = xt + (((long long)(T + 1) * g.row0 + (long long)step * g.n + i) * d);
             double* x1 = xt + (((long long)(T + 1) * g.row0 + (long long)(step + 1) * g.n + i) * d);
             const double* a0 = at + (((long long)T * g.row0 + (long long)step * g.n + i) * d);
@@ -266,7 +266,7 @@ struct EpiRagShoot {
                 rag_shoot_row<D>(g, i, valid ? xn : nullptr, a0 + (long long)g.n * d, d, nx, tstride, sstride);
         }
         e = block_sum_all(e);
-        if (threadIdx.x == 0) epart[g.eoff + row0 / op_rows] += e;
+        if (threadIdx.x == 0) epart[g.eoff + tb] += e;
     }
 };
 
@@ -341,7 +341,7 @@ int rag_shoot_impl(int nseg, const int64_t* v_off, int d, const double* x0, cons
     for (int t = 0; t < T && pl.items > 0; ++t) {
         P.tgt4 = pn[t & 1].tgt;
         P.src4 = pn[t & 1].src;
-        const EpiRagShoot<D> E{dsegs, xt, at, T, t, d, pn[(t + 1) & 1], pl.tt, pl.ss, epart, op_group<Op>()};
+        const EpiRagShoot<D> E{dsegs, xt, at, T, t, d, pn[(t + 1) & 1], pl.tt, pl.ss, epart};
         sweep_kernel<Op, false, EpiRagShoot<D>><<<pl.items, 32 * kSweepWarps, 0, st>>>(grid, P, pn[t & 1].boxes, part,
                                                                                       counters, E);
     }
@@ -409,13 +409,14 @@ struct EpiRagCov {
     int T, step, d;
     RagPlanes nx;
     long long tstride, sstride;
-    template <int NOUT>
-    LDDMM_D void run(const SegDesc& sd, int row0, int rows, const double* red) const {
+    template <int GT, int NOUT>
+    LDDMM_D void run(const SegDesc& sd, int, const int* srow, const double* red) const {
         const RagSeg& g = segs[sd.id];
         const long long prev = (long long)g.n * d;
-        for (int r = threadIdx.x; r < ((rows + 31) & ~31); r += blockDim.x) {   // whole warps: fold boxes
-            const bool valid = r < rows;
-            const long long i = row0 + r;
+        for (int r = threadIdx.x; r < GT; r += blockDim.x) {
+            const long long i = srow[r];
+            const bool valid = i < g.n;
+            if (srow[r & ~31] >= g.n) continue;   // whole warps: fold boxes
             const double* pn = pxt + (((long long)(T + 1) * g.row0 + (long long)(step + 1) * g.n + i) * d);
             double* pc = pxt + (((long long)(T + 1) * g.row0 + (long long)step * g.n + i) * d);
             const double* a = at + (((long long)T * g.row0 + (long long)step * g.n + i) * d);
@@ -533,12 +534,11 @@ struct EpiRagSum {
     const long long* rowoff;
     double* f;
     int dimb;
-    template <int NOUT>
-    LDDMM_D void run(const SegDesc& sd, int row0, int rows, const double* red) const {
-        const long long q0 = rowoff[sd.id] + row0;
-        for (int i = threadIdx.x; i < rows * dimb; i += blockDim.x) {
-            const int r = i / dimb;
-            f[q0 * dimb + i] = red[r * NOUT + (i - r * dimb)];
+    template <int GT, int NOUT>
+    LDDMM_D void run(const SegDesc& sd, int, const int* srow, const double* red) const {
+        for (int i = threadIdx.x; i < GT * dimb; i += blockDim.x) {
+            const int r = i / dimb, c = i - r * dimb, row = srow[r];
+            if (row < sd.n_tgt) f[(rowoff[sd.id] + row) * dimb + c] = red[r * NOUT + c];
         }
     }
 };
@@ -645,15 +645,16 @@ struct EpiRagDtValue {
     int d;
     double eps1;
     double* epart;
-    int op_rows;
-    template <int NOUT>
-    LDDMM_D void run(const SegDesc& sd, int row0, int rows, const double* red) const {
+    template <int GT, int NOUT>
+    LDDMM_D void run(const SegDesc& sd, int tb, const int* srow, const double* red) const {
         const RagSeg& g = segs[sd.id];
         double e = 0.0;
-        for (int r = threadIdx.x; r < rows; r += blockDim.x)
-            e += dt_value_row(norm, red + r * NOUT, s1 + (g.row0 + row0 + r) * d, d, eps1);
+        for (int r = threadIdx.x; r < GT; r += blockDim.x) {
+            const long long i = srow[r];
+            if (i < g.n) e += dt_value_row(norm, red + r * NOUT, s1 + (g.row0 + i) * d, d, eps1);
+        }
         e = block_sum_all(e);
-        if (threadIdx.x == 0) epart[g.eoff + row0 / op_rows] = e;
+        if (threadIdx.x == 0) epart[g.eoff + tb] = e;
     }
 };
 
@@ -666,11 +667,12 @@ struct EpiRagDtGrad {
     int d;
     double eps1, fac;
     double *z1, *dz1;
-    template <int NOUT>
-    LDDMM_D void run(const SegDesc& sd, int row0, int rows, const double* red) const {
+    template <int GT, int NOUT>
+    LDDMM_D void run(const SegDesc& sd, int, const int* srow, const double* red) const {
         const RagSeg& g = segs[sd.id];
-        for (int r = threadIdx.x; r < rows; r += blockDim.x) {
-            const long long q = (g.row0 + row0 + r) * d;
+        for (int r = threadIdx.x; r < GT; r += blockDim.x) {
+            const long long i = srow[r], q = (g.row0 + i) * d;
+            if (i >= g.n) continue;
             dt_grad_row(norm, red + r * NOUT, s1 + q, d, eps1, fac * g.dscale, z1 + q, dz1 + q);
         }
     }
@@ -762,7 +764,7 @@ int rag_dt_sweep(const RagDataArgs& a, int kind, const double* c1, const double*
             sweep_kernel<Op, false, EpiRagDtGrad><<<pl.items, 32 * kSweepWarps, 0, st>>>(grid, P, boxes, part,
                                                                                         counters, E);
     } else {
-        const EpiRagDtValue E{dsegs, a.norm, s1, a.d, a.eps1, epart, op_group<Op>()};
+        const EpiRagDtValue E{dsegs, a.norm, s1, a.d, a.eps1, epart};
         if (pl.items > 0)
             sweep_kernel<Op, true, EpiRagDtValue><<<pl.items, 32 * kSweepWarps, 0, st>>>(grid, P, boxes, part,
                                                                                         counters, E);

@@ -154,13 +154,14 @@ struct EpiShoot {
     long long ecount;
     double escale;
     int* counter;
-    int groups, op_rows;   // groups, and rows of one
-    template <int NOUT>
-    LDDMM_D void run(const SegDesc&, int row0, int rows, const double* red) const {
+    int groups;
+    template <int GT, int NOUT>
+    LDDMM_D void run(const SegDesc& sg, int tb, const int* srow, const double* red) const {
         double e = 0.0;
-        for (int r = threadIdx.x; r < ((rows + 31) & ~31); r += blockDim.x) {   // whole warps: fold boxes
-            const bool valid = r < rows;
-            const long long i = row0 + r;
+        for (int r = threadIdx.x; r < GT; r += blockDim.x) {
+            const long long i = srow[r];
+            const bool valid = i < sg.n_tgt;
+            if (sg.perm == nullptr && srow[r & ~31] >= sg.n_tgt) continue;   // whole warps: fold boxes
             double xn[3] = {0, 0, 0};
             for (int j = 0; j < d && valid; ++j) {
                 const double v = red[r * NOUT + j];
@@ -169,7 +170,7 @@ struct EpiShoot {
                 x1[i * d + j] = xn[j];
             }
             if (a1 == nullptr) continue;
-            store_box<Real>(nx.boxes, i, valid, xn, a1 + i * d, nullptr, d, s, c);
+            if (sg.perm == nullptr) store_box<Real>(nx.boxes, i, valid, xn, a1 + i * d, nullptr, d, s, c);
             if (!valid) continue;
             store_point<Real>(nx.tgt, tstride, i, xn, d, s, c);
             if constexpr (LIST) {
@@ -180,7 +181,7 @@ struct EpiShoot {
             }
         }
         e = block_sum_all(e);
-        if (threadIdx.x == 0) epart[row0 / op_rows] = e;
+        if (threadIdx.x == 0) epart[tb] = e;
         if (energy == nullptr || !last_block(counter, groups)) return;
         double t = 0.0;
         for (long long q = threadIdx.x; q < ecount; q += blockDim.x) t += __ldcg(eall + q);
@@ -230,8 +231,9 @@ int shoot_impl(const ShootArgs& a, Workspace& ws, cudaStream_t st) {
         p.src = ws.take<float4>((size_t)Op::NS * pl.m_pad);
         p.boxes = ws.take<float4>(pl.box_words());
     }
-    double* part = ws.take<double>(pl.part_doubles(a.n, D));
+    double* part = ws.take<double>(pl.part_doubles(D));
     int* counters = ws.take<int>(pl.counters());
+    OrderRows order = take_order_rows(ws, pl);
     double* epart = ws.take<double>((size_t)a.T * pl.n_tb);
     double* center = ws.take<double>(kCenterWords);
     if (ws.measuring()) return LDDMM_OK;
@@ -245,6 +247,7 @@ int shoot_impl(const ShootArgs& a, Workspace& ws, cudaStream_t st) {
     shoot_pack_kernel<Real, LIST><<<grid_for(std::max(pl.n_tpad, pl.m_pad)), 256, 0, st>>>(
         a.x0, a.at, a.n, a.d, ks.scale, center, pn[0], pn[1], pl.n_tpad, pl.m_pad, Op::PP, D, Op::NS, a.xt, counters,
         (int)pl.counters());
+    LDDMM_TRY((launch_order_rows<Real>(order, pn[0].tgt, a.n, pl, st)));
     const double dt = a.dt > 0 ? a.dt : 1.0 / a.T;
     for (int t = 0; t < a.T; ++t) {
         const StepPlanes& p = pn[t & 1];
@@ -254,8 +257,11 @@ int shoot_impl(const ShootArgs& a, Workspace& ws, cudaStream_t st) {
         EpiShoot<Real, LIST> E{a.d, Op::PP, D, dt, ks.scale, center, a.xt + t * N, a.at + t * N, a.xt + (t + 1) * N,
                                last ? nullptr : a.at + (t + 1) * N, pn[(t + 1) & 1], pl.n_tpad, pl.m_pad,
                                epart + (long long)t * pl.n_tb, last ? a.energy : nullptr, epart,
-                               (long long)a.T * pl.n_tb, a.rw * dt, counters + pl.n_tb, pl.n_tb, op_group<Op>()};
-        LDDMM_TRY((launch_single<Op, false>(pl, a.n, P, p.boxes, part, st, 0, counters, E)));
+                               (long long)a.T * pl.n_tb, a.rw * dt, counters + pl.n_tb, pl.n_tb};
+        LDDMM_TRY((launch_single<Op, false>(pl, a.n, P, p.boxes, part, st, 0, counters, E, order.perm)));
+        if (order.perm != nullptr && !last)   // the epilogue's rows are not whole folds
+            fold_boxes_kernel<Real, LIST><<<grid_for(pl.m_pad), 256, 0, st>>>(
+                pn[(t + 1) & 1].src, pl.m_pad, a.n, D, D, pn[(t + 1) & 1].boxes);
     }
     return LDDMM_OK;
 }
@@ -387,11 +393,12 @@ struct EpiCov {
     const double *x_prev, *a_prev;   // NULL for step 0
     StepPlanes nx;
     long long tstride, sstride;
-    template <int NOUT>
-    LDDMM_D void run(const SegDesc&, int row0, int rows, const double* red) const {
-        for (int r = threadIdx.x; r < ((rows + 31) & ~31); r += blockDim.x) {   // whole warps: fold boxes
-            const bool valid = r < rows;
-            const long long i = row0 + r;
+    template <int GT, int NOUT>
+    LDDMM_D void run(const SegDesc& sg, int, const int* srow, const double* red) const {
+        for (int r = threadIdx.x; r < GT; r += blockDim.x) {
+            const long long i = srow[r];
+            const bool valid = i < sg.n_tgt;
+            if (sg.perm == nullptr && srow[r & ~31] >= sg.n_tgt) continue;   // whole warps: fold boxes
             double pn[3] = {0, 0, 0};
             for (int j = 0; j < d && valid; ++j) {
                 const double pj = p_next[i * d + j];
@@ -400,7 +407,8 @@ struct EpiCov {
                 if (dat_t != nullptr) dat_t[i * d + j] = 2.0 * rw * a_t[i * d + j] - pj;
             }
             if (x_prev == nullptr) continue;
-            store_box<Real>(nx.boxes, i, valid, x_prev + i * d, a_prev + i * d, pn, d, s, c);
+            if (sg.perm == nullptr)
+                store_box<Real>(nx.boxes, i, valid, x_prev + i * d, a_prev + i * d, pn, d, s, c);
             if (valid)
                 cov_store<Real, LIST>(nx.tgt, tstride, nx.src, sstride, i, pp, x_prev + i * d, a_prev + i * d, pn, d,
                                       s, c, rw, tw);
@@ -436,8 +444,9 @@ int cov_impl(const CovArgs& a, Workspace& ws, cudaStream_t st) {
         p.src = ws.take<float4>((size_t)Op::NS * pl.m_pad);
         p.boxes = ws.take<float4>(pl.box_words());
     }
-    double* part = ws.take<double>(pl.part_doubles(a.n, D));
+    double* part = ws.take<double>(pl.part_doubles(D));
     int* counters = ws.take<int>(pl.counters());
+    OrderRows order = take_order_rows(ws, pl);
     double* center = ws.take<double>(kCenterWords);
     if (ws.measuring()) return LDDMM_OK;
     const KScale ks = kernel_scale(KIND, a.order, a.sigma, !pl.seq);
@@ -453,6 +462,7 @@ int cov_impl(const CovArgs& a, Workspace& ws, cudaStream_t st) {
         a.xt + (long long)(T - 1) * N, a.at + (long long)(T - 1) * N, a.px1, a.n, a.d, ks.scale, center, a.rw,
         pn[(T - 1) & 1], pn[T & 1], pl.n_tpad, pl.m_pad, Op::PP, NT, Op::NS, W, a.pxt + (long long)T * N, counters,
         (int)pl.counters());
+    LDDMM_TRY((launch_order_rows<Real>(order, pn[(T - 1) & 1].tgt, a.n, pl, st)));
     for (int t = T - 1; t >= 0; --t) {
         const StepPlanes& p = pn[t & 1];
         P.tgt4 = p.tgt;
@@ -462,7 +472,10 @@ int cov_impl(const CovArgs& a, Workspace& ws, cudaStream_t st) {
                              a.dat ? a.dat + (long long)t * N : nullptr,
                              t > 0 ? a.xt + (long long)(t - 1) * N : nullptr,
                              t > 0 ? a.at + (long long)(t - 1) * N : nullptr, pn[(t + 1) & 1], pl.n_tpad, pl.m_pad};
-        LDDMM_TRY((launch_single<Op, false>(pl, a.n, P, p.boxes, part, st, 0, counters, E)));
+        LDDMM_TRY((launch_single<Op, false>(pl, a.n, P, p.boxes, part, st, 0, counters, E, order.perm)));
+        if (order.perm != nullptr && t > 0)   // the epilogue's rows are not whole folds
+            fold_boxes_kernel<Real, LIST><<<grid_for(pl.m_pad), 256, 0, st>>>(
+                pn[(t + 1) & 1].src, pl.m_pad, a.n, D, W, pn[(t + 1) & 1].boxes);
     }
     return LDDMM_OK;
 }

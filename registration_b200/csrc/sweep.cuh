@@ -15,7 +15,7 @@
 // Per-target accumulators: FP32 partials over the 32 sources of a fold, in
 // order, folded into a TwoSum-compensated (sum, err) pair (FP32 ops), or plain
 // FP64 sums.  The block adds its warps in order and writes doubles into
-//   part[(seg.part + chunk * seg.n_tgt + t) * Op::NOUT + c]
+//   part[(seg.part + chunk * seg.n_tb * GT + tb * GT + t) * Op::NOUT + c]
 // The block of a group that finishes last adds the chunks in their order and
 // hands the group's sums to the epilogue Epi (which scales and writes them, or
 // takes the Euler step and packs the next sweep's records), so results do not
@@ -40,6 +40,11 @@
 // varifold gradient of a 20,480-cell sphere at sigma 0.1 0.97 -> 0.47 ms, its
 // FP64 value 1.63 -> 0.81 ms, the value of 98,000 cells at sigma 0.05 6.2 ->
 // 1.9 ms.  Where no fold is far (uniform random points) the test costs 0.5%.
+//
+// perm (SegDesc): the target rows in an order that puts neighbours into the same
+// group (launch_order_rows, pack.cuh).  The sum of a target does not depend on
+// its group, but the group's box does: 128 consecutive vertices of a subdivided
+// mesh are strung out along its coarser edges.
 //
 // SYM (symmetric sums, used for energies <S,S> - 2 <S,T> whose summand is
 // symmetric in the target and the source): the first seg.sym_folds folds hold
@@ -250,7 +255,8 @@ LDDMM_D double block_sum_all(double v) {
 }
 
 // Epilogues: run() is called by all threads of a group's last block with the
-// group's sums red[row * NOUT + c], rows [row0, row0 + rows) of the segment.
+// group's sums red[r * NOUT + c], r < GT; sum r belongs to the segment's row
+// srow[r] where that is below seg.n_tgt.
 struct EpiNone {
     static constexpr bool NONE = true;
 };
@@ -262,11 +268,11 @@ struct EpiSum {
     long long ld;
     int col0, ncols;
     double scale;
-    template <int NOUT>
-    LDDMM_D void run(const SegDesc&, int row0, int rows, const double* red) const {
-        for (int i = threadIdx.x; i < rows * ncols; i += blockDim.x) {
-            const int r = i / ncols, c = i - r * ncols;
-            f[(row0 + r) * ld + col0 + c] = scale * red[r * NOUT + c];
+    template <int GT, int NOUT>
+    LDDMM_D void run(const SegDesc& sg, int, const int* srow, const double* red) const {
+        for (int i = threadIdx.x; i < GT * ncols; i += blockDim.x) {
+            const int r = i / ncols, c = i - r * ncols, row = srow[r];
+            if (row < sg.n_tgt) f[row * ld + col0 + c] = scale * red[r * NOUT + c];
         }
     }
 };
@@ -291,16 +297,25 @@ __global__ void __launch_bounds__(32 * kSweepWarps, op_min_blocks<Op>())
     const int chunk = local - tb * sg.split;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 
-    // targets of this lane: t = tb*GT + r*32 + lane (rows are padded); an
+    // targets of this lane: rows r*32 + lane of the group (rows are padded); an
     // operator with TPS == 2 keeps two of them per slot (packed FP32 pairs)
     constexpr int SLOTS = R / TPS;
     static_assert(R % TPS == 0, "R must be a multiple of TPS");
+    __shared__ int srow[GT];
     typename Op::Tgt tg[SLOTS];
+    {
+        int row[R];
 #pragma unroll
-    for (int q = 0; q < SLOTS; ++q) {
-        const long long row = sg.tgt + (long long)tb * GT + (q * TPS) * 32 + lane;
-        if constexpr (TPS == 1) Op::load_target(P, row, tg[q]);
-        else Op::load_target(P, row, row + 32, tg[q]);
+        for (int q = 0; q < R; ++q) {
+            const int r = tb * GT + q * 32 + lane;
+            row[q] = sg.perm != nullptr ? sg.perm[r] : r;
+            if (warp == 0) srow[q * 32 + lane] = row[q];
+        }
+#pragma unroll
+        for (int q = 0; q < SLOTS; ++q) {
+            if constexpr (TPS == 1) Op::load_target(P, sg.tgt + row[q], tg[q]);
+            else Op::load_target(P, sg.tgt + row[q * TPS], sg.tgt + row[q * TPS + 1], tg[q]);
+        }
     }
     typename Op::Acc acc[SLOTS];
 #pragma unroll
@@ -323,9 +338,11 @@ __global__ void __launch_bounds__(32 * kSweepWarps, op_min_blocks<Op>())
             using Real = typename Op::Real;
             float lo[3] = {INFINITY, INFINITY, INFINITY}, hi[3] = {-INFINITY, -INFINITY, -INFINITY};
             bool bad = false;
-            if (threadIdx.x < GT && tb * GT + (int)threadIdx.x < sg.n_tgt) {
+            const int br = tb * GT + (int)threadIdx.x;
+            const int brow = threadIdx.x >= GT ? sg.n_tgt : sg.perm != nullptr ? sg.perm[br] : br;
+            if (brow < sg.n_tgt) {
                 Real x[3];
-                load_vals<Real, 3>(P.tgt4, P.tgt_stride, sg.tgt + (long long)tb * GT + threadIdx.x, 0, x);
+                load_vals<Real, 3>(P.tgt4, P.tgt_stride, sg.tgt + brow, 0, x);
 #pragma unroll
                 for (int j = 0; j < 3; ++j) {
                     if constexpr (sizeof(Real) == 4) {
@@ -372,8 +389,8 @@ __global__ void __launch_bounds__(32 * kSweepWarps, op_min_blocks<Op>())
                 if (bl.w < INFINITY) lgl = fmaxf(lgl, bl.w + Op::lgk(P, d1));
             }
             {
-                const int f = tb * (GT / kFold) + (int)threadIdx.x;
-                if (step > 1 && threadIdx.x < GT / kFold && f < n_folds) {
+                const int f = lane == 0 && brow < sg.n_tgt ? brow / kFold : n_folds;
+                if (step > 1 && f < n_folds) {
                     float d0, d1;
                     const float4 bl = fbox[2 * f];
                     box_dist2(wb, bl, fbox[2 * f + 1], d0, d1);
@@ -487,17 +504,17 @@ __global__ void __launch_bounds__(32 * kSweepWarps, op_min_blocks<Op>())
         }
         __syncthreads();
     }
-    const int rows = min(GT, sg.n_tgt - tb * GT);
-    double* dst = part + (sg.part + (long long)chunk * sg.n_tgt + (long long)tb * GT) * NOUT;
     if constexpr (Epi::NONE) {
+        const int rows = min(GT, sg.n_tgt - tb * GT);   // (targets as they lie)
+        double* dst = part + (sg.part + (long long)chunk * sg.n_tgt + (long long)tb * GT) * NOUT;
         for (int i = threadIdx.x; i < rows * NOUT; i += 32 * kSweepWarps) dst[i] = red[i];
     } else {
         if (sg.split > 1) {
-            for (int i = threadIdx.x; i < rows * NOUT; i += 32 * kSweepWarps) dst[i] = red[i];
+            const long long step = (long long)sg.n_tb * GT * NOUT;
+            double* p0 = part + (sg.part + (long long)tb * GT) * NOUT;
+            for (int i = threadIdx.x; i < GT * NOUT; i += 32 * kSweepWarps) p0[chunk * step + i] = red[i];
             if (!last_block(counters + sg.cnt + tb, sg.split)) return;
-            const double* p0 = part + (sg.part + (long long)tb * GT) * NOUT;
-            const long long step = (long long)sg.n_tgt * NOUT;
-            for (int i = threadIdx.x; i < rows * NOUT; i += 32 * kSweepWarps) {
+            for (int i = threadIdx.x; i < GT * NOUT; i += 32 * kSweepWarps) {
                 double v = 0.0;
                 for (int k0 = 0; k0 < sg.split; k0 += 16) {   // 16 loads in flight
                     double q[16];
@@ -510,7 +527,7 @@ __global__ void __launch_bounds__(32 * kSweepWarps, op_min_blocks<Op>())
             }
             __syncthreads();
         }
-        E.template run<NOUT>(sg, tb * GT, rows, red);
+        E.template run<GT, NOUT>(sg, tb, srow, red);
     }
 }
 
@@ -548,9 +565,11 @@ __global__ void __launch_bounds__(op_group<Op>()) sweep_seq_kernel(const SegDesc
         if (t < sg.n_tgt)
             for (int c = 0; c < NOUT; ++c) part[(sg.part + t) * NOUT + c] = acc.value(c);
     } else {
+        __shared__ int srow[GT];
+        srow[threadIdx.x] = t;
         for (int c = 0; c < NOUT; ++c) red[threadIdx.x * NOUT + c] = acc.value(c);
         __syncthreads();
-        E.template run<NOUT>(sg, blockIdx.x * GT, min(GT, sg.n_tgt - (int)blockIdx.x * GT), red);
+        E.template run<GT, NOUT>(sg, blockIdx.x, srow, red);
     }
 }
 

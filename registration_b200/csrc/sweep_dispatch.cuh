@@ -24,7 +24,7 @@ struct SinglePlan {
     int n_tb, n_folds, split;
     bool seq;   // FP64 sums over few sources: sweep_seq_kernel, coordinates in the x/s frame (kfun.cuh)
     // chunk sums (doubles) of a sweep with an epilogue: none where a group has one chunk
-    size_t part_doubles(long long n, int nout) const { return split > 1 ? (size_t)split * n * nout : 0; }
+    size_t part_doubles(int nout) const { return split > 1 ? (size_t)split * n_tpad * nout : 0; }
     size_t counters() const { return (size_t)n_tb + 1; }
     size_t box_words() const { return 2 * (size_t)(m_pad / kFold); }   // float4 words of the fold boxes
 };
@@ -45,18 +45,52 @@ SinglePlan plan_single(long long n, long long m, int split_cap = 0, bool shared 
     return p;
 }
 
+// Order of the target rows of a sum over its own points (perm NULL: as they lie),
+// from 32,768 points on: the five launches (15 us) and a shot's box launch per step
+// (3 us) are 1-4% of sums that take 350 us each when nothing is far, and save a
+// third where the kernel is narrow (launch_order_rows).
+struct OrderRows {
+    int *perm = nullptr, *hist = nullptr, *cell = nullptr, *tmp = nullptr;
+};
+constexpr long long kOrderRowsMin = 32768;
+inline OrderRows take_order_rows(Workspace& ws, const SinglePlan& pl) {
+    OrderRows o;
+    if (pl.seq || (long long)pl.n_folds * kFold < kOrderRowsMin) return o;
+    o.perm = ws.take<int>(pl.n_tpad);
+    o.hist = ws.take<int>(2 * kOrderCells + 1);
+    o.cell = ws.take<int>(pl.n_tpad);
+    o.tmp = ws.take<int>(pl.n_tpad);
+    if (ws.measuring()) o.perm = nullptr;
+    return o;
+}
+template <class Real>
+int launch_order_rows(const OrderRows& o, const float4* tgt, long long n, const SinglePlan& pl, cudaStream_t st) {
+    if (o.perm == nullptr) return LDDMM_OK;
+    LDDMM_TRY(cuda_check(cudaMemsetAsync(o.hist, 0, sizeof(int) * kOrderCells, st), "order memset"));
+    const int blocks = grid_for(pl.n_tpad);
+    order_extent_kernel<Real><<<1, 1024, 0, st>>>(tgt, pl.n_tpad, n, o.hist + 2 * kOrderCells);
+    order_cells_kernel<Real><<<blocks, 256, 0, st>>>(tgt, pl.n_tpad, n, o.hist + 2 * kOrderCells, o.hist, o.cell);
+    order_scan_kernel<<<1, 1024, 0, st>>>(o.hist, o.hist + 2 * kOrderCells);
+    order_scatter_kernel<<<blocks, 256, 0, st>>>(o.cell, n, o.hist + kOrderCells, o.tmp);
+    order_rank_kernel<<<blocks, 256, 0, st>>>(o.tmp, o.cell, o.hist, o.hist + 2 * kOrderCells, n, pl.n_tpad, o.perm);
+    return cuda_check(cudaGetLastError(), "order rows");
+}
+
 // boxes: fold boxes written with the packed sources, or NULL (every fold counts).
 // SYM: symmetric sweep over sym_folds own folds (see sweep_kernel<Op, true>).
-// Epi: what is done with a group's sums; counters: n_tb + 1 zeros (see sweep_kernel).
+// Epi: what is done with a group's sums; counters: n_tb + 1 zeros; perm: order of the
+// targets' sets of 32 rows, or NULL (see sweep_kernel).
 template <class Op, bool SYM = false, class Epi = EpiNone>
 int launch_single(const SinglePlan& pl, long long n, const typename Op::Params& P, const float4* boxes, double* part,
-                  cudaStream_t st, int sym_folds = 0, int* counters = nullptr, const Epi& E = Epi()) {
+                  cudaStream_t st, int sym_folds = 0, int* counters = nullptr, const Epi& E = Epi(),
+                  const int* perm = nullptr) {
     SweepGrid g{};
     g.seg0.n_tgt = (int)n;
     g.seg0.n_folds = pl.n_folds;
     g.seg0.n_tb = pl.n_tb;
     g.seg0.split = pl.split;
     g.seg0.sym_folds = sym_folds;
+    g.seg0.perm = perm;
     g.nseg = 0;
     g.n_items = pl.n_tb * pl.split;
     if (g.n_items <= 0) return LDDMM_OK;

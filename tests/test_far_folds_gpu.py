@@ -120,3 +120,54 @@ def test_data_terms_of_narrow_kernels(oracle_lib, precision, tol, norm, level):
     assert abs(getattr(sf, norm + "NormDef")(S, T, K) - want) <= tol * vmag
     g, gw = getattr(sf, norm + "NormGradient")(S, T, K), getattr(ref, norm + "NormGradient" + sfx)(RS, RT, RK)
     assert np.linalg.norm(g - gw) <= tol * 6 * np.linalg.norm(gmag)
+
+
+@pytest.mark.parametrize("precision", ["fp32c", "fp64"])
+@pytest.mark.parametrize("d,cloud", [(3, "sphere"), (2, "square"), (3, "crowd")])
+def test_ordered_target_rows_change_nothing(precision, d, cloud):
+    """From 32,768 points on a sum over its own points groups its targets by cells of a grid (or, where over 2,048
+    rows share a cell, as they lie).  Same terms and same FP32 partial sums: against the sum with separate targets
+    only the far folds left out (2^-36 of the absolute terms) may differ, 1e-9 of the largest row."""
+    import torch
+    from registration_b200 import kernelFunctions as kf
+    from registration_b200 import pointEvolution as evol
+    n = 33001
+    rng = np.random.default_rng(5)
+    x = rng.standard_normal((n, d))
+    if cloud == "sphere":
+        x /= np.linalg.norm(x, axis=1, keepdims=True)
+    elif cloud == "square":
+        x = np.stack([np.arange(n) % 182, np.arange(n) // 182], axis=1) / 182.0
+    else:
+        x *= 0.01
+        x[7] = 30.0
+    a = rng.standard_normal((n, d))
+    K = kf.Kernel(name="gauss", sigma=0.04, precision=precision)
+    xd, ad = torch.from_numpy(x).cuda(), torch.from_numpy(a).cuda()
+    for got, want in ((K.applyK(xd, ad), K.applyK(xd, ad, firstVar=xd.clone())),
+                      (K.applyDiffKT(xd, [ad], [ad]), K.applyDiffKT(xd, [ad], [ad], firstVar=xd.clone()))):
+        assert float((got - want).abs().max()) <= 1e-9 * float(want.abs().max())
+    # steps of a shot and of its adjoint against the separate sums.  FP32c: one step (later ones are packed in the
+    # first step's frame, the separate sums in their own), and two steps against FP64 within the 1e-5 of its shots
+    # (not for the crowd, whose outlier at 750 widths costs FP32 coordinates ten bits)
+    T = 2 if precision == "fp64" else 1
+    at = torch.stack([ad, 0.5 * ad])[:T] * 1e-3
+    xt, _ = evol.shoot(xd, at, K, dt=0.5)
+    want = xd
+    for t in range(T):
+        step = 0.5 * K.applyK(want, at[t], firstVar=want.clone())
+        want = want + step
+        assert float((xt[t + 1] - want).abs().max()) <= 1e-8 * float(step.abs().max())
+    pxt, _ = evol.covector(xt, at, ad, K, 1.0, dt=0.5)
+    p = ad
+    for t in reversed(range(T)):
+        step = 0.5 * K.applyDiffKT(xt[t], [p - 2 * at[t], at[t]], [at[t], p], firstVar=xt[t].clone())
+        p = p + step
+        assert float((pxt[t] - p).abs().max()) <= 1e-8 * float(step.abs().max())
+    if precision == "fp32c" and cloud != "crowd":
+        K64 = kf.Kernel(name="gauss", sigma=0.04, precision="fp64")
+        at = torch.stack([ad, 0.5 * ad]) * 1e-3
+        got, want = evol.shoot(xd, at, K)[0], evol.shoot(xd, at, K64)[0]
+        assert float((got - want).norm()) <= 1e-5 * float((want - xd).norm())
+        got, ref64 = (evol.covector(want, at, ad, k, 1.0)[0] for k in (K, K64))
+        assert float((got - ref64).norm()) <= 1e-5 * float((ref64 - ad).norm())
