@@ -100,6 +100,8 @@ int launch_single(const SinglePlan& pl, long long n, const typename Op::Params& 
             return cuda_check(cudaGetLastError(), "sweep launch");
         }
     }
+    // up to 1,024 sources no warp has more than a few folds: bounding them costs more than it saves
+    if (pl.n_folds <= 32) boxes = nullptr;
     sweep_kernel<Op, SYM, Epi><<<g.n_items, 32 * kSweepWarps, 0, st>>>(g, P, boxes, part, counters, E);
     return cuda_check(cudaGetLastError(), "sweep launch");
 }
