@@ -52,7 +52,7 @@ OPS = [  # name, kernel, op, flops/pair, FMA-pipe instr/pair, XU ops/pair (per-p
     ("applyDiffKT_lap3", "laplacian", "DKT", 28, 19, 2),
 ]
 # bounding box (init, keys, finish), target / source packs (+1 target value pack for DKT), sweep, combine
-LAUNCHES_PER_OP = {"K": 7, "DKT": 8}
+LAUNCHES_PER_OP = {"K": 4, "DKT": 4}
 # DRAM bytes (dram__bytes_read.sum + dram__bytes_write.sum) of one sweep launch
 # at N = M = 2^20, from one ncu metrics capture of this workload's sweep kernels
 TRAFFIC_1M = {"applyK_gauss": 87339264 + 89124864, "applyDiffKT_gauss": 148929024 + 94077952,

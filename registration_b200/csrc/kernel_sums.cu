@@ -10,6 +10,33 @@
 
 namespace lddmm {
 
+// FP64 sums may add their sources in any order, so large ones order both point
+// sets by cells (launch_order_rows): folds and groups are then compact wherever the
+// points come from.  From 2^30 pairs on (1.6 ms; the twelve launches take 35 us).
+// B200, 65,536 x 65,536 points uniform in the unit cube, sigma 0.05: 6.55 -> 4.37 ms.
+struct Ordered64 {
+    OrderRows t, s;
+    float4* src = nullptr;
+    bool taken = false;
+};
+template <class Op>
+Ordered64 take_ordered64(Workspace& ws, const SinglePlan& pl, long long n, long long m) {
+    Ordered64 o;
+    if (sizeof(typename Op::Real) != 8 || pl.seq || n < 2048 || m < 2048 || n < (1LL << 30) / m) return o;
+    o.taken = true;
+    o.t = take_order(ws, pl.n_tpad);
+    o.s = take_order(ws, pl.m_pad);
+    o.src = ws.take<float4>((size_t)Op::NS * pl.m_pad);
+    return o;
+}
+inline int launch_ordered64(const Ordered64& o, const float4* tgt, const float4* src, const SinglePlan& pl,
+                            long long n, long long m, int V, float4* boxes, cudaStream_t st) {
+    LDDMM_TRY(launch_order_rows<double>(o.t, tgt, n, pl.n_tpad, st));
+    LDDMM_TRY(launch_order_rows<double>(o.s, src, m, pl.m_pad, st));
+    permute_records_kernel<<<grid_for(pl.m_pad), 256, 0, st>>>(src, o.s.perm, pl.m_pad, m, V, o.src, boxes);
+    return cuda_check(cudaGetLastError(), "ordered sum");
+}
+
 // ---------------------------------------------------------------------------
 // applyk
 // ---------------------------------------------------------------------------
@@ -39,7 +66,8 @@ int applyk_group(const ApplyKArgs& a, int col0, Workspace& ws, cudaStream_t st) 
     double* part = ws.take<double>(pl.part_doubles(DIMB));
     int* counters = ws.take<int>(pl.split > 1 ? pl.counters() : 0);
     // sums over the targets' own points (the query cannot know: room for the order whenever n == m)
-    OrderRows order = a.boxed && a.n == a.m ? take_order_rows(ws, pl) : OrderRows{};
+    const Ordered64 both = take_ordered64<Op>(ws, pl, a.n, a.m);
+    OrderRows order = a.boxed && !both.taken && a.n == a.m ? take_order_rows(ws, pl) : OrderRows{};
     double* center = ws.take<double>(kCenterWords);
     if (ws.measuring()) return LDDMM_OK;
     if (ws.overflow()) {
@@ -64,7 +92,12 @@ int applyk_group(const ApplyKArgs& a, int col0, Workspace& ws, cudaStream_t st) 
         a.x, a.n, Gather{}, 0, tgt, pl.n_tpad, a.y, a.m, g, D, DIMB, src, pl.m_pad, a.d, ks.scale, center, boxes,
         counters, pl.split > 1 ? (int)pl.counters() : 0);
     if (a.x != a.y) order.perm = nullptr;
-    LDDMM_TRY((launch_order_rows<Real>(order, tgt, a.n, pl, st)));
+    LDDMM_TRY((launch_order_rows<Real>(order, tgt, a.n, pl.n_tpad, st)));
+    if (both.taken) {
+        LDDMM_TRY(launch_ordered64(both, tgt, src, pl, a.n, a.m, DIMB, boxes, st));
+        P.src4 = both.src;
+        order = both.t;
+    }
     // the epilogue writes only the group's own columns
     const EpiSum E{a.f, a.dimb, col0, g.nvals, 1.0};
     return launch_single<Op, false>(pl, a.n, P, boxes, part, st, 0, counters, E, order.perm);
@@ -172,7 +205,8 @@ int difft_impl(const DiffKTArgs& a, Workspace& ws, cudaStream_t st) {
     float4* boxes = ws.take<float4>(pl.box_words());
     double* part = ws.take<double>(pl.part_doubles(D));
     int* counters = ws.take<int>(pl.counters());
-    OrderRows order = a.n == a.m ? take_order_rows(ws, pl) : OrderRows{};
+    const Ordered64 both = take_ordered64<Op>(ws, pl, a.n, a.m);
+    OrderRows order = !both.taken && a.n == a.m ? take_order_rows(ws, pl) : OrderRows{};
     double* center = ws.take<double>(kCenterWords);
     if (ws.measuring()) return LDDMM_OK;
     const KScale ks = kernel_scale(KIND, a.order, a.sigma, !pl.seq);
@@ -199,7 +233,12 @@ int difft_impl(const DiffKTArgs& a, Workspace& ws, cudaStream_t st) {
         a.x, a.n, gu, W, tgt, pl.n_tpad, a.y, a.m, gv, D, W, src, pl.m_pad, a.d, ks.scale, center, boxes, counters,
         (int)pl.counters());
     if (a.x != a.y) order.perm = nullptr;
-    LDDMM_TRY((launch_order_rows<Real>(order, tgt, a.n, pl, st)));
+    LDDMM_TRY((launch_order_rows<Real>(order, tgt, a.n, pl.n_tpad, st)));
+    if (both.taken) {
+        LDDMM_TRY(launch_ordered64(both, tgt, src, pl, a.n, a.m, W, boxes, st));
+        P.src4 = both.src;
+        order = both.t;
+    }
     const EpiSum E{a.f, a.d, 0, a.d, ks.dscale};   // D may exceed d (d == 1 runs as D == 2)
     return launch_single<Op, false>(pl, a.n, P, boxes, part, st, 0, counters, E, order.perm);
 }

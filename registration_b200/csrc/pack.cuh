@@ -208,6 +208,27 @@ static __global__ void fold_boxes_kernel(const float4* __restrict__ src, long lo
     }
 }
 
+// Standard FP64 records in the order of perm, with V values each, and their fold boxes.
+static __global__ void permute_records_kernel(const float4* __restrict__ src, const int* __restrict__ perm,
+                                              long long m_pad, long long m, int V, float4* __restrict__ out,
+                                              float4* __restrict__ boxes) {
+    for (long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x; q < m_pad;
+         q += (long long)gridDim.x * blockDim.x) {
+        const long long i = perm[q];
+        double p[4] = {0, 0, 0, 0}, w = 0;
+        for (int k = 0; k < 2 + (V + 1) / 2; ++k) {
+            const float4 word = src[(long long)k * m_pad + i];
+            out[(long long)k * m_pad + q] = word;
+            for (int h = 0; h < 2; ++h) {
+                const double v = word_get<double>(&word, h);
+                if (k < 2) p[2 * k + h] = v;
+                else if (2 * (k - 2) + h < V) w = max_nan(w, v);
+            }
+        }
+        store_fold_box<double>(boxes, q, i < m, p, w);
+    }
+}
+
 // Order of the target rows by cells of a 32 x 32 x 32 grid over the packed points,
 // the cells along a Morton curve, the rows of a cell as they lie: a counting sort
 // whose result does not depend on scheduling (counts are whole numbers; the rows

@@ -247,7 +247,7 @@ int shoot_impl(const ShootArgs& a, Workspace& ws, cudaStream_t st) {
     shoot_pack_kernel<Real, LIST><<<grid_for(std::max(pl.n_tpad, pl.m_pad)), 256, 0, st>>>(
         a.x0, a.at, a.n, a.d, ks.scale, center, pn[0], pn[1], pl.n_tpad, pl.m_pad, Op::PP, D, Op::NS, a.xt, counters,
         (int)pl.counters());
-    LDDMM_TRY((launch_order_rows<Real>(order, pn[0].tgt, a.n, pl, st)));
+    LDDMM_TRY((launch_order_rows<Real>(order, pn[0].tgt, a.n, pl.n_tpad, st)));
     const double dt = a.dt > 0 ? a.dt : 1.0 / a.T;
     for (int t = 0; t < a.T; ++t) {
         const StepPlanes& p = pn[t & 1];
@@ -462,7 +462,7 @@ int cov_impl(const CovArgs& a, Workspace& ws, cudaStream_t st) {
         a.xt + (long long)(T - 1) * N, a.at + (long long)(T - 1) * N, a.px1, a.n, a.d, ks.scale, center, a.rw,
         pn[(T - 1) & 1], pn[T & 1], pl.n_tpad, pl.m_pad, Op::PP, NT, Op::NS, W, a.pxt + (long long)T * N, counters,
         (int)pl.counters());
-    LDDMM_TRY((launch_order_rows<Real>(order, pn[(T - 1) & 1].tgt, a.n, pl, st)));
+    LDDMM_TRY((launch_order_rows<Real>(order, pn[(T - 1) & 1].tgt, a.n, pl.n_tpad, st)));
     for (int t = T - 1; t >= 0; --t) {
         const StepPlanes& p = pn[t & 1];
         P.tgt4 = p.tgt;

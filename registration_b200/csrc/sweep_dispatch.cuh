@@ -53,26 +53,31 @@ struct OrderRows {
     int *perm = nullptr, *hist = nullptr, *cell = nullptr, *tmp = nullptr;
 };
 constexpr long long kOrderRowsMin = 32768;
-inline OrderRows take_order_rows(Workspace& ws, const SinglePlan& pl) {
+inline OrderRows take_order(Workspace& ws, long long n_pad) {
     OrderRows o;
-    if (pl.seq || (long long)pl.n_folds * kFold < kOrderRowsMin) return o;
-    o.perm = ws.take<int>(pl.n_tpad);
+    o.perm = ws.take<int>(n_pad);
     o.hist = ws.take<int>(2 * kOrderCells + 1);
-    o.cell = ws.take<int>(pl.n_tpad);
-    o.tmp = ws.take<int>(pl.n_tpad);
+    o.cell = ws.take<int>(n_pad);
+    o.tmp = ws.take<int>(n_pad);
     if (ws.measuring()) o.perm = nullptr;
     return o;
 }
+inline OrderRows take_order_rows(Workspace& ws, const SinglePlan& pl) {
+    if (pl.seq || (long long)pl.n_folds * kFold < kOrderRowsMin) return OrderRows{};
+    return take_order(ws, pl.n_tpad);
+}
+// o.perm of the n rows packed in `planes` (n_pad of them, positions first)
 template <class Real>
-int launch_order_rows(const OrderRows& o, const float4* tgt, long long n, const SinglePlan& pl, cudaStream_t st) {
+int launch_order_rows(const OrderRows& o, const float4* planes, long long n, long long n_pad, cudaStream_t st) {
     if (o.perm == nullptr) return LDDMM_OK;
     LDDMM_TRY(cuda_check(cudaMemsetAsync(o.hist, 0, sizeof(int) * kOrderCells, st), "order memset"));
-    const int blocks = grid_for(pl.n_tpad);
-    order_extent_kernel<Real><<<1, 1024, 0, st>>>(tgt, pl.n_tpad, n, o.hist + 2 * kOrderCells);
-    order_cells_kernel<Real><<<blocks, 256, 0, st>>>(tgt, pl.n_tpad, n, o.hist + 2 * kOrderCells, o.hist, o.cell);
-    order_scan_kernel<<<1, 1024, 0, st>>>(o.hist, o.hist + 2 * kOrderCells);
+    const int blocks = grid_for(n_pad);
+    int* info = o.hist + 2 * kOrderCells;
+    order_extent_kernel<Real><<<1, 1024, 0, st>>>(planes, n_pad, n, info);
+    order_cells_kernel<Real><<<blocks, 256, 0, st>>>(planes, n_pad, n, info, o.hist, o.cell);
+    order_scan_kernel<<<1, 1024, 0, st>>>(o.hist, info);
     order_scatter_kernel<<<blocks, 256, 0, st>>>(o.cell, n, o.hist + kOrderCells, o.tmp);
-    order_rank_kernel<<<blocks, 256, 0, st>>>(o.tmp, o.cell, o.hist, o.hist + 2 * kOrderCells, n, pl.n_tpad, o.perm);
+    order_rank_kernel<<<blocks, 256, 0, st>>>(o.tmp, o.cell, o.hist, info, n, n_pad, o.perm);
     return cuda_check(cudaGetLastError(), "order rows");
 }
 

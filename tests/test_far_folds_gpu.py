@@ -172,3 +172,28 @@ def test_ordered_target_rows_change_nothing(precision, d, cloud):
         assert float((got - want).norm()) <= 1e-5 * float((want - xd).norm())
         got, ref64 = (evol.covector(want, at, ad, k, 1.0)[0] for k in (K, K64))
         assert float((got - ref64).norm()) <= 1e-5 * float((ref64 - ad).norm())
+
+
+@pytest.mark.parametrize("name,order", [("gauss", 10), ("laplacian", 3)])
+@pytest.mark.parametrize("cloud", ["uniform", "crowd"])
+def test_ordered_fp64_sums_equal_unordered_ones(name, order, cloud):
+    """FP64 sums of 2^30 pairs and more order both point sets; two halves of the targets stay below that.  The same
+    terms in another order: 40,000 roundings of 2^-53 at random signs, 1e-12 of the largest row."""
+    import torch
+    from registration_b200 import kernelFunctions as kf
+    n, m = 33001, 40007
+    g = torch.Generator(device="cuda").manual_seed(3)
+    opt = dict(dtype=torch.float64, device="cuda", generator=g)
+    x, y = torch.rand((n, 3), **opt), torch.rand((m, 3), **opt)
+    if cloud == "crowd":
+        x, y = 0.01 * x, 0.01 * y
+        x[5], y[11] = 2.0, -2.0
+    a, p = torch.randn((m, 3), **opt), torch.randn((n, 3), **opt)
+    K = kf.Kernel(name=name, sigma=0.05, order=order, precision="fp64")
+    h = n // 2
+    f = K.applyK(y, a, firstVar=x)
+    want = torch.cat([K.applyK(y, a, firstVar=x[:h]), K.applyK(y, a, firstVar=x[h:])])
+    assert float((f - want).abs().max()) <= 1e-12 * float(want.abs().max())
+    f = K.applyDiffKT(y, [p], [a], firstVar=x)
+    want = torch.cat([K.applyDiffKT(y, [p[:h]], [a], firstVar=x[:h]), K.applyDiffKT(y, [p[h:]], [a], firstVar=x[h:])])
+    assert float((f - want).abs().max()) <= 1e-12 * float(want.abs().max())
