@@ -51,12 +51,12 @@ OPS = [  # name, kernel, op, flops/pair, FMA-pipe instr/pair, XU ops/pair (per-p
     ("applyK_lap3", "laplacian", "K", 24, 16, 2),
     ("applyDiffKT_lap3", "laplacian", "DKT", 28, 19, 2),
 ]
-# bounding box (init, keys, finish), target / source packs (+1 target value pack for DKT), sweep, combine
+# bounding box (blocks' keys, centre), pack of targets and sources, sweep with its epilogue
 LAUNCHES_PER_OP = {"K": 4, "DKT": 4}
 # DRAM bytes (dram__bytes_read.sum + dram__bytes_write.sum) of one sweep launch
 # at N = M = 2^20, from one ncu metrics capture of this workload's sweep kernels
-TRAFFIC_1M = {"applyK_gauss": 87339264 + 89124864, "applyDiffKT_gauss": 148929024 + 94077952,
-              "applyK_lap3": 88632576 + 84919296, "applyDiffKT_lap3": 170131712 + 133973760}
+TRAFFIC_1M = {"applyK_gauss": 56410624 + 50727424, "applyDiffKT_gauss": 75705600 + 51765504,
+              "applyK_lap3": 57260800 + 48904448, "applyDiffKT_lap3": 75033088 + 52696064}
 
 
 def parse():

@@ -51,7 +51,6 @@ struct ApplyKArgs {
     int order;
     double* f;
     int split_cap;  // 0: no cap on the number of source chunks
-    bool boxed;     // keep fold boxes in the workspace (far folds are passed over)
 };
 
 template <class Real, int KIND, int DEG, int D, int DIMB>
@@ -62,12 +61,12 @@ int applyk_group(const ApplyKArgs& a, int col0, Workspace& ws, cudaStream_t st) 
     const SinglePlan pl = plan_single<Op>(a.n, a.m, a.split_cap);
     float4* tgt = ws.take<float4>((size_t)Op::PP * pl.n_tpad);
     float4* src = ws.take<float4>((size_t)Op::NS * pl.m_pad);
-    float4* boxes = a.boxed ? ws.take<float4>(pl.box_words()) : nullptr;
+    float4* boxes = ws.take<float4>(pl.box_words());
     double* part = ws.take<double>(pl.part_doubles(DIMB));
     int* counters = ws.take<int>(pl.split > 1 ? pl.counters() : 0);
     // sums over the targets' own points (the query cannot know: room for the order whenever n == m)
     const Ordered64 both = take_ordered64<Op>(ws, pl, a.n, a.m);
-    OrderRows order = a.boxed && !both.taken && a.n == a.m ? take_order_rows(ws, pl) : OrderRows{};
+    OrderRows order = !both.taken && a.n == a.m ? take_order_rows(ws, pl) : OrderRows{};
     double* center = ws.take<double>(kCenterWords);
     if (ws.measuring()) return LDDMM_OK;
     if (ws.overflow()) {
@@ -148,7 +147,7 @@ static int applyk_validate(const ApplyKArgs& a) {
 
 template <class Real>
 size_t applyk_ws(int64_t n, int64_t m, int d, int dimb) {
-    ApplyKArgs a{nullptr, n, nullptr, m, nullptr, d, dimb, 1.0, 10, nullptr, 0, true};
+    ApplyKArgs a{nullptr, n, nullptr, m, nullptr, d, dimb, 1.0, 10, nullptr, 0};
     if (n <= 0 || m <= 0 || d < 1 || d > 3 || dimb < 1) return 0;
     Workspace ws;
     applyk_run<Real>(a, ws, 0);
@@ -360,7 +359,7 @@ int div_run(const ApplyKArgs& a, Workspace& ws, cudaStream_t st) {
 template <class Real>
 size_t div_ws(int64_t n, int64_t m, int d) {
     if (n <= 0 || m <= 0 || d < 1 || d > 3) return 0;
-    ApplyKArgs a{nullptr, n, nullptr, m, nullptr, d, d, 1.0, 10, nullptr, 0, true};
+    ApplyKArgs a{nullptr, n, nullptr, m, nullptr, d, d, 1.0, 10, nullptr, 0};
     Workspace ws;
     div_run<Real>(a, ws, 0);
     return ws.off + 256;
@@ -388,9 +387,9 @@ int div_entry(const ApplyKArgs& a, void* wsp, size_t wsb, cudaStream_t st) {
     return div_run<Real>(a, ws, st);
 }
 
-size_t applyk_f32c_scratch_bytes(int64_t n, int64_t m, int d, int dimb, int split_cap, bool boxed) {
+size_t applyk_f32c_scratch_bytes(int64_t n, int64_t m, int d, int dimb, int split_cap) {
     if (n <= 0 || m <= 0 || d < 1 || d > 3 || dimb < 1) return 0;
-    ApplyKArgs a{nullptr, n, nullptr, m, nullptr, d, dimb, 1.0, 10, nullptr, split_cap, boxed};
+    ApplyKArgs a{nullptr, n, nullptr, m, nullptr, d, dimb, 1.0, 10, nullptr, split_cap};
     size_t best = 0;
     for (int order : {10, 3}) {  // Gaussian and Laplacian plans
         a.order = order;
@@ -403,8 +402,8 @@ size_t applyk_f32c_scratch_bytes(int64_t n, int64_t m, int d, int dimb, int spli
 
 int applyk_f32c_in_workspace(const double* x, int64_t n, const double* y, int64_t m, const double* beta, int d,
                              int dimb, double sigma, int order, double* f, void* workspace, size_t workspace_bytes,
-                             cudaStream_t stream, int split_cap, bool boxed) {
-    ApplyKArgs a{x, n, y, m, beta, d, dimb, sigma, order, f, split_cap, boxed};
+                             cudaStream_t stream, int split_cap) {
+    ApplyKArgs a{x, n, y, m, beta, d, dimb, sigma, order, f, split_cap};
     return applyk_entry<float>(a, workspace, workspace_bytes, stream);
 }
 
@@ -420,14 +419,14 @@ size_t lddmm_applyk_f64_workspace(int64_t n, int64_t m, int d, int dimb) { retur
 int lddmm_applyk_f32c(const double* x, int64_t n, const double* y, int64_t m, const double* beta, int d, int dimb,
                       double sigma, int order, double* f, void* workspace, size_t workspace_bytes,
                       lddmm_stream_t stream) {
-    ApplyKArgs a{x, n, y, m, beta, d, dimb, sigma, order, f, 0, true};
+    ApplyKArgs a{x, n, y, m, beta, d, dimb, sigma, order, f, 0};
     return applyk_entry<float>(a, workspace, workspace_bytes, (cudaStream_t)stream);
 }
 
 int lddmm_applyk_f64(const double* x, int64_t n, const double* y, int64_t m, const double* beta, int d, int dimb,
                      double sigma, int order, double* f, void* workspace, size_t workspace_bytes,
                      lddmm_stream_t stream) {
-    ApplyKArgs a{x, n, y, m, beta, d, dimb, sigma, order, f, 0, true};
+    ApplyKArgs a{x, n, y, m, beta, d, dimb, sigma, order, f, 0};
     return applyk_entry<double>(a, workspace, workspace_bytes, (cudaStream_t)stream);
 }
 
@@ -457,13 +456,13 @@ size_t lddmm_applydiv_f64_workspace(int64_t n, int64_t m, int d) { return div_ws
 
 int lddmm_applydiv_f32c(const double* x, int64_t n, const double* y, int64_t m, const double* a, int d, double sigma,
                         int order, double* f, void* workspace, size_t workspace_bytes, lddmm_stream_t stream) {
-    ApplyKArgs q{x, n, y, m, a, d, d, sigma, order, f, 0, true};
+    ApplyKArgs q{x, n, y, m, a, d, d, sigma, order, f, 0};
     return div_entry<float>(q, workspace, workspace_bytes, (cudaStream_t)stream);
 }
 
 int lddmm_applydiv_f64(const double* x, int64_t n, const double* y, int64_t m, const double* a, int d, double sigma,
                        int order, double* f, void* workspace, size_t workspace_bytes, lddmm_stream_t stream) {
-    ApplyKArgs q{x, n, y, m, a, d, d, sigma, order, f, 0, true};
+    ApplyKArgs q{x, n, y, m, a, d, d, sigma, order, f, 0};
     return div_entry<double>(q, workspace, workspace_bytes, (cudaStream_t)stream);
 }
 

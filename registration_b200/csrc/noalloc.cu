@@ -59,6 +59,19 @@ static int noalloc_scratch(void** out) {
     return LDDMM_OK;
 }
 
+// The size that decides which shapes are taken: scratch of a one-chunk sum whose
+// records hold every value twice and whose chunk sums are kept beside the result
+// (n = m = 400,000 at dimb <= 4).  The sweep's own one-chunk scratch (single
+// values, no chunk sums, fold boxes, row order) is always smaller, so every shape
+// taken fits.
+static size_t noalloc_limit_bytes(int64_t n, int64_t m, int d, int dimb) {
+    const size_t D = d <= 2 ? 2 : 3, g = std::min(dimb, 4), words = (D + g + 1) / 2;
+    size_t off = 16 * (size_t)round_up(std::max<int64_t>(n, 1), 512);
+    off = (size_t)round_up((long long)off, 256) + 16 * words * (size_t)round_up(std::max<int64_t>(m, 1), 128);
+    off = (size_t)round_up((long long)off, 256) + 8 * (size_t)n * g;
+    return (size_t)round_up((long long)off, 256) + 128 + 256;
+}
+
 }  // namespace lddmm
 
 extern "C" LDDMM_API int lddmm_applyk_f32c_noalloc(const double* x, int64_t n, const double* y, int64_t m,
@@ -75,14 +88,9 @@ extern "C" LDDMM_API int lddmm_applyk_f32c_noalloc(const double* x, int64_t n, c
         return LDDMM_ERR_ARG;
     }
     int cap = 0;
-    bool boxed = true;   // without the fold boxes where only they would not fit
     if (n > 0 && m > 0) {
         // largest chunk count whose workspace fits the static scratch
-        size_t one = applyk_f32c_scratch_bytes(n, m, d, dimb, 1, boxed);
-        if (one > kNoAllocScratchBytes) {
-            boxed = false;
-            one = applyk_f32c_scratch_bytes(n, m, d, dimb, 1, boxed);
-        }
+        const size_t one = noalloc_limit_bytes(n, m, d, dimb);
         if (one == 0 || one > kNoAllocScratchBytes) {
             set_error("applyk_noalloc: n=%lld, m=%lld, dimb=%d needs %zu bytes of scratch; the static scratch holds "
                       "%zu (use lddmm_applyk_f32c with a workspace)",
@@ -90,11 +98,11 @@ extern "C" LDDMM_API int lddmm_applyk_f32c_noalloc(const double* x, int64_t n, c
             return LDDMM_ERR_WORKSPACE;
         }
         const size_t per_chunk = (size_t)n * (size_t)std::min(dimb, 4) * sizeof(double) + 256;
-        cap = 1 + (int)std::min<size_t>((kNoAllocScratchBytes - one) / per_chunk, 1 << 20);
-        while (cap > 1 && applyk_f32c_scratch_bytes(n, m, d, dimb, cap, boxed) > kNoAllocScratchBytes) --cap;
+        cap = 1 + (int)std::min<size_t>(kNoAllocScratchBytes / per_chunk, 1 << 20);
+        while (cap > 1 && applyk_f32c_scratch_bytes(n, m, d, dimb, cap) > kNoAllocScratchBytes) --cap;
     }
     void* scratch = nullptr;
     LDDMM_TRY(noalloc_scratch(&scratch));
     return applyk_f32c_in_workspace(x, n, y, m, beta, d, dimb, sigma, order, f, scratch, kNoAllocScratchBytes,
-                                    (cudaStream_t)stream, cap, boxed);
+                                    (cudaStream_t)stream, cap);
 }

@@ -10,16 +10,17 @@
 //             values per 16-byte word; splat2 makes the packed operand (v, v) of
 //             the f32x2 instructions from each.
 //
-// A record read by a warp returns its words to all 32 lanes at 128 bytes per
-// clock and SM, broadcast or not: a record of values stored twice (v, v), which
-// needs no splat, took 3 words = 12 clocks for the 128 pairs of a Gaussian applyK
-// whose FP32 arithmetic takes 9, so the sweep was bound by shared memory.  Two
-// words (6 values) take 8.  Measured at n = m = 131,072 (pairs/s, before ->
-// after): Gaussian applyK 2.78 -> 3.02e12, Laplacian 1.84 -> 1.93e12, Gaussian
+// Records that hold each value twice, (v, v), need no splat but three words
+// instead of two for a Gaussian applyK (four instead of two for the varifold
+// operators): more shared-memory reads and more registers in flight per source.
+// Measured at n = m = 131,072 (pairs/s, doubled -> single values, 8 sources
+// unrolled): Gaussian applyK 2.78 -> 3.02e12, Laplacian 1.84 -> 1.93e12, Gaussian
 // applyDiffKT 2.02 -> 2.15e12, adjoint (W = 6) 1.62 -> 1.73e12, varifold value
 // 2.36 -> 2.47e12, varifold gradient 1.25 -> 1.33e12, current gradient 1.51 ->
 // 1.63e12.  Eight targets per thread instead of four gain nothing more and make
-// the groups coarser.
+// the groups coarser.  What bounds the sweeps now is the FMA pipe, 80% (Gaussian)
+// and 74-76% (Laplacian, with the XU 74-87%) busy, math-pipe throttle the first
+// stall.
 #pragma once
 #include <cstring>
 

@@ -9,8 +9,8 @@
 // follows the shape) spread evenly over them.  A warp streams its folds
 // through its own cp.async ring: it waits for nobody but itself
 // (`__syncwarp`), every lane reads the same record (shared-memory broadcast).
-// One fold is 4096 pairs against 1.5-2 KB from L2, about 5 bytes per clock
-// and SM, so sharing a tile between the warps would save nothing that counts.
+// One fold is 4096 pairs against 1-2 KB from L2, about 5 bytes per clock and SM,
+// so sharing a tile between the warps would save nothing that counts.
 //
 // Per-target accumulators: FP32 partials over the 32 sources of a fold, in
 // order, folded into a TwoSum-compensated (sum, err) pair (FP32 ops), or plain
