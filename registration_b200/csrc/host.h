@@ -62,12 +62,16 @@ inline int choose_split(int n_tb, int n_folds, int sms, int resident, bool share
     const long long want = (64LL * sms + n_tb - 1) / n_tb;
     const long long many = std::max(1LL, std::min<long long>(want, n_folds / (4 * (shared ? 8 : 16))));
     if (shared || many * n_tb >= 4LL * resident) return (int)many;
+    // for each number of waves the most chunks that fit, then the fewest with as few folds per warp
+    const long long cap = (n_folds + 3) / 4;
     long long best = 1, best_cost = -1;
-    for (long long s = 1; s <= (n_folds + 3) / 4 && s * n_tb <= 4LL * resident + n_tb; ++s) {
-        const long long waves = (s * n_tb + resident - 1) / resident;
-        const long long cost = waves * ((n_folds + 4 * s - 1) / (4 * s) + kBlockFolds);
+    for (long long waves = 1; waves <= 5; ++waves) {
+        const long long fit = std::min(cap, waves * resident / n_tb);
+        if (fit < 1) continue;
+        const long long folds = (n_folds + 4 * fit - 1) / (4 * fit);
+        const long long cost = waves * (folds + kBlockFolds);
         if (best_cost < 0 || cost < best_cost) {
-            best = s;
+            best = (n_folds + 4 * folds - 1) / (4 * folds);
             best_cost = cost;
         }
     }
