@@ -131,8 +131,12 @@ LDDMM_D double exp2neg(double x) {
     return __hiloint2double(big ? (hx > 0x7FF00000u ? (int)hx : 0) : hi, big ? 0 : __double2loint(p));
 }
 
-// a < b for non-negative doubles, compared as integers (the FP64 pipe is the scarce one)
-LDDMM_D bool less_nonneg(double a, double b) { return __double_as_longlong(a) < __double_as_longlong(b); }
+// a < b for a >= 0 or NaN and b > 0, compared as integers (the FP64 pipe is the scarce
+// one).  Unsigned, so that a NaN of either sign is not below b: inf - inf has its sign
+// bit set, and as a signed integer it would be.
+LDDMM_D bool less_nonneg(double a, double b) {
+    return (unsigned long long)__double_as_longlong(a) < (unsigned long long)__double_as_longlong(b);
+}
 
 // the zero-distance thresholds in the base-2 frame
 static constexpr double kLog2e = 1.4426950408889634;
