@@ -371,6 +371,8 @@ LDDMM_D void dt_pack_record(int norm, int grad, bool is_t, const double* c, cons
         for (int j = 0; j < 3; ++j) bp[j] = (Real)pos[j];
         if (norm == NCURRENT)
             for (int j = 0; j < d; ++j) w = max_nan(w, (Real)(s[j] * sign));
+        if (norm == NVARIFOLD)   // 0 / 0 of a cell without area: never passed over, though it weighs nothing
+            for (int j = 0; j < 3; ++j) w = max_nan(w, (Real)(s[j] / a) * (Real)0);
         *bw = max_nan((Real)0, w);
     }
     if (sizeof(Real) == 4 && list) {

@@ -104,3 +104,22 @@ def test_data_terms_keep_non_finite_vertices(norm, bad):
     g = g.cpu().numpy() if hasattr(g, "cpu") else np.asarray(g)
     near = np.unique(f[(f == 3).any(axis=1)])
     assert not np.isfinite(g[near]).all(axis=1).any()
+
+
+@pytest.mark.parametrize("precision", ["fp32c", "fp64"])
+def test_varifold_normals_of_cells_without_area(precision):
+    """Without a floor under the areas the unit normal of a cell without area is 0 / 0 and reaches every cell's sum,
+    also those of cells so far away that other folds of that size are passed over (5,120 cells, sigma 0.05)."""
+    import torch
+    from registration_b200 import _dataterm as dt
+    from registration_b200 import geometry as geo
+    from registration_b200 import kernelFunctions as kf
+    from registration_b200 import surfaces as sf
+    v, whole = geo.icosphere(4)
+    f = whole.copy()
+    f[3000] = f[3000, 0]
+    K = kf.Kernel(name="gauss", sigma=0.05, precision=precision)
+    S, T = sf.Surface(FV=[f, torch.from_numpy(v).cuda()]), sf.Surface(FV=[whole, 1.01 * v])
+    val, g = dt.dataterm("varifold", S.vertices, S.device_shape(), T.centers, T.surfel, K, grad=True, eps1=0.0, eps2=0.0)
+    assert not np.isfinite(float(val))
+    assert not torch.isfinite(g).all(dim=1).any()
