@@ -30,7 +30,8 @@
  *   _f64  : plain FP64 arithmetic with the Fortran's branches.
  * Sources are summed in sets of 32; sets so far from a group of targets that all
  * of them together stay below 2^-36 (_f32c) or 2^-58 (_f64) of the sum of the
- * absolute terms of every target of the group are passed over.
+ * absolute terms of every output (each column, each component) of every target of
+ * the group are passed over.
  */
 #ifndef LDDMM_B200_H
 #define LDDMM_B200_H

@@ -30,6 +30,7 @@ struct SegDesc {
     int sym_folds;    // > 0: the first sym_folds folds are the targets' own records and the
                       // sum is symmetric in (target, source): see sweep_kernel<Op, true>
     int id;           // segment number (ragged launches)
+    int self;         // the first sources are the targets, in their order
     int cnt;          // first counter of this segment's groups (see sweep_kernel)
     const int* perm;  // order of the target rows (n_tb * 32 R of them), or NULL: as they lie
 };

@@ -44,6 +44,66 @@ struct DataLayout {
                                                       : D + 1;
 };
 
+// Bounds of the data-term sweeps (see op_culls, sweep.cuh).  Weight columns: the weight
+// (varifold value, measure), the components of the vector (current), or those of the
+// weighted normal and the weight (varifold gradient).
+constexpr int dt_weights(int mode, int D) { return mode == M_VARI_GRAD ? D + 1 : mode == M_CUR_GRAD ? D : 1; }
+
+// What the sums of a target with values u hold at least.  Varifold gradient: its sums
+// 0..D-1 and D meet in z1_j = a_j + a_D u_j, so what is left out of either has to be small
+// against |a_j| + |a_D u_j| (near flat pieces a_D is next to nothing by itself).
+template <int MODE, int D, class Real>
+LDDMM_D void dt_lower(const Real* u, const Real* a, Real norm1, Real* lo) {
+    if constexpr (MODE == M_VARI_GRAD) {
+        lo[D] = -1;
+#pragma unroll
+        for (int j = 0; j < D; ++j) {
+            const Real n = u[j] < (Real)0 ? -u[j] : u[j];
+            lo[j] = a[j] + a[D] * n;
+            if (n != (Real)0) {
+                const Real q = lo[j] / n;
+                if (!(lo[D] >= (Real)0) || !(q >= lo[D])) lo[D] = lo[D] != lo[D] ? lo[D] : q;
+            }
+            lo[D + 1 + j] = a[D + 1 + j];
+        }
+    } else {
+#pragma unroll
+        for (int b = 0; b < DataLayout<MODE, D>::NOUT; ++b) lo[b] = a[b];
+        if constexpr (MODE == M_CUR_GRAD)
+#pragma unroll
+            for (int j = 0; j < D; ++j) lo[D + j] = norm1 == (Real)0 ? (Real)-1 : a[D + j] / norm1;
+    }
+}
+template <int MODE, int D>
+LDDMM_D void dt_upper(const float* lgw, float lgv, float lk, const float* lext, float* u) {
+    if constexpr (MODE == M_VARI_VALUE) {
+        u[0] = lgw[0] + lk + 1.f;                       // 1 + <n, n'>^2 <= 2
+    } else if constexpr (MODE == M_VARI_GRAD) {
+#pragma unroll
+        for (int j = 0; j < D; ++j) {
+            u[j] = lgw[j] + lk + 2.f;                   // 2 <n, n'>, and half of what z1_j may lose
+            u[D + 1 + j] = lgw[D] + lk + 1.f + lext[j];
+        }
+        u[D] = lgw[D] + lk + 1.f;                       // the other half
+    } else if constexpr (MODE == M_CUR_GRAD) {
+#pragma unroll
+        for (int j = 0; j < D; ++j) {
+            u[j] = lgw[j] + lk;
+            u[D + j] = lgv + lk + lext[j];
+        }
+    } else {
+        u[0] = lgw[0] + lk;
+#pragma unroll
+        for (int j = 0; j < D; ++j) u[1 + j] = lgw[0] + lk + lext[j];
+    }
+}
+// the half h of N packed values
+template <int N>
+LDDMM_D void halves2(const f2* v, int h, float* out) {
+#pragma unroll
+    for (int j = 0; j < N; ++j) out[j] = half2(v[j], h);
+}
+
 template <class Real_, int KIND, int PDEG, int QDEG, int D, int MODE>
 struct OpData {
     using Real = Real_;
@@ -60,8 +120,9 @@ struct OpData {
     static constexpr int NOUT = L::NOUT;
     using Params = KernelParamsBase<Real>;
     using Acc = typename AccFor<Real>::template type<NOUT>;
+    using Abs = AccAbs<Real, NOUT>;
+    static constexpr int NW = dt_weights(MODE, D), NB = NOUT, DOT = MODE == M_CUR_GRAD ? D : 0;
     // K bounds the factor of K' as well (its polynomial Q is below P term by term)
-    static constexpr bool GRADX = MODE != M_VARI_VALUE;
     static LDDMM_D float lgk(const Params& P, float d2) { return lg_factor<KIND, PDEG>(P.pk, d2); }
     struct Tgt {
         Real x[D];
@@ -71,6 +132,12 @@ struct OpData {
         Real y[D];
         Real v[L::SV];
     };
+    static LDDMM_D Real coord(const Tgt& t, int, int j) { return j < D ? t.x[j < D ? j : 0] : (Real)0; }
+    static LDDMM_D Real dot_val(const Tgt& t, int, int w) { return t.u[w]; }
+    static LDDMM_D void lower(const Tgt& t, int, const Real* a, Real norm1, Real* lo) { dt_lower<MODE, D>(t.u, a, norm1, lo); }
+    static LDDMM_D void upper(const float* lgw, float lgv, float lk, const float* lext, float* u) {
+        dt_upper<MODE, D>(lgw, lgv, lk, lext, u);
+    }
     static LDDMM_D void load_target(const Params& P, long long row, Tgt& t) {
         load_vals<Real, D>(P.tgt4, P.tgt_stride, row, 0, t.x);
         if constexpr (L::TV > 0) load_vals<Real, L::TV>(P.tgt4, P.tgt_stride, row, PP, t.u);
@@ -79,8 +146,8 @@ struct OpData {
         load_vals_smem<Real, D>(S, j, 0, s.y);
         load_vals_smem<Real, L::SV>(S, j, PP, s.v);
     }
-    template <bool LIB = false>
-    static LDDMM_D void pair(const Params& P, const Tgt& t, const Src& s, Acc& acc) {
+    template <bool LIB = false, class A>
+    static LDDMM_D void pair(const Params& P, const Tgt& t, const Src& s, A& acc) {
         Real dx[D], r2 = 0;
 #pragma unroll
         for (int j = 0; j < D; ++j) {
@@ -142,7 +209,8 @@ struct OpVariValue2 {
     static constexpr int NOUT = 1;
     using Params = KernelParams2;
     using Acc = AccF32C2<1>;
-    static constexpr bool GRADX = false;
+    using Abs = AccAbs2<NOUT>;
+    static constexpr int NW = dt_weights(M_VARI_VALUE, 3), NB = NOUT, DOT = 0;
     static LDDMM_D float lgk(const Params& P, float d2) { return lg_factor<KIND, PDEG>(P.pkd, d2); }
     struct Tgt {
         f2 x[3];
@@ -151,12 +219,23 @@ struct OpVariValue2 {
     struct Src {
         f2 val[NV];
     };
+    static LDDMM_D float coord(const Tgt& t, int h, int j) { return half2(t.x[j], h); }
+    static LDDMM_D float dot_val(const Tgt& t, int h, int w) { return half2(t.u[w], h); }
+    static LDDMM_D void lower(const Tgt& t, int h, const float* a, float norm1, float* lo) {
+        float u[3];
+        halves2<3>(t.u, h, u);
+        dt_lower<M_VARI_VALUE, 3>(u, a, norm1, lo);
+    }
+    static LDDMM_D void upper(const float* lgw, float lgv, float lk, const float* lext, float* u) {
+        dt_upper<M_VARI_VALUE, 3>(lgw, lgv, lk, lext, u);
+    }
     static LDDMM_D void load_target(const Params& P, long long ra, long long rb, Tgt& t) {
         load_target_pair<3>(P.tgt4, P.tgt_stride, ra, rb, 0, t.x);
         load_target_pair<3>(P.tgt4, P.tgt_stride, ra, rb, 1, t.u);
     }
     static LDDMM_D void load_source(const float4* S, int j, Src& s) { load_list_source<NV>(S, j, s.val); }
-    static LDDMM_D void pair(const Params& P, const Tgt& t, const Src& s, Acc& a) {
+    template <class A>
+    static LDDMM_D void pair(const Params& P, const Tgt& t, const Src& s, A& a) {
         f2 r2;
 #pragma unroll
         for (int j = 0; j < 3; ++j) {
@@ -193,7 +272,8 @@ struct OpVariGrad2 {
     static constexpr int NOUT = 7;
     using Params = KernelParams2;
     using Acc = AccF32C2<NOUT>;
-    static constexpr bool GRADX = true;
+    using Abs = AccAbs2<NOUT>;
+    static constexpr int NW = dt_weights(M_VARI_GRAD, 3), NB = NOUT, DOT = 0;
     static LDDMM_D float lgk(const Params& P, float d2) { return lg_factor<KIND, PDEG>(P.pkd, d2); }
     struct Tgt {
         f2 x[3];
@@ -202,12 +282,23 @@ struct OpVariGrad2 {
     struct Src {
         f2 val[NV];
     };
+    static LDDMM_D float coord(const Tgt& t, int h, int j) { return half2(t.x[j], h); }
+    static LDDMM_D float dot_val(const Tgt& t, int h, int w) { return half2(t.u[w], h); }
+    static LDDMM_D void lower(const Tgt& t, int h, const float* a, float norm1, float* lo) {
+        float u[3];
+        halves2<3>(t.u, h, u);
+        dt_lower<M_VARI_GRAD, 3>(u, a, norm1, lo);
+    }
+    static LDDMM_D void upper(const float* lgw, float lgv, float lk, const float* lext, float* u) {
+        dt_upper<M_VARI_GRAD, 3>(lgw, lgv, lk, lext, u);
+    }
     static LDDMM_D void load_target(const Params& P, long long ra, long long rb, Tgt& t) {
         load_target_pair<3>(P.tgt4, P.tgt_stride, ra, rb, 0, t.x);
         load_target_pair<3>(P.tgt4, P.tgt_stride, ra, rb, 1, t.u);
     }
     static LDDMM_D void load_source(const float4* S, int j, Src& s) { load_list_source<NV>(S, j, s.val); }
-    static LDDMM_D void pair(const Params& P, const Tgt& t, const Src& s, Acc& a) {
+    template <class A>
+    static LDDMM_D void pair(const Params& P, const Tgt& t, const Src& s, A& a) {
         f2 dx[3], r2;
 #pragma unroll
         for (int j = 0; j < 3; ++j) {
@@ -254,7 +345,8 @@ struct OpCurGrad2 {
     static constexpr int NOUT = 6;
     using Params = KernelParams2;
     using Acc = AccF32C2<NOUT>;
-    static constexpr bool GRADX = true;
+    using Abs = AccAbs2<NOUT>;
+    static constexpr int NW = dt_weights(M_CUR_GRAD, 3), NB = NOUT, DOT = 3;
     static LDDMM_D float lgk(const Params& P, float d2) { return lg_factor<KIND, PDEG>(P.pkd, d2); }
     struct Tgt {
         f2 x[3];
@@ -263,12 +355,23 @@ struct OpCurGrad2 {
     struct Src {
         f2 val[NV];
     };
+    static LDDMM_D float coord(const Tgt& t, int h, int j) { return half2(t.x[j], h); }
+    static LDDMM_D float dot_val(const Tgt& t, int h, int w) { return half2(t.u[w], h); }
+    static LDDMM_D void lower(const Tgt& t, int h, const float* a, float norm1, float* lo) {
+        float u[3];
+        halves2<3>(t.u, h, u);
+        dt_lower<M_CUR_GRAD, 3>(u, a, norm1, lo);
+    }
+    static LDDMM_D void upper(const float* lgw, float lgv, float lk, const float* lext, float* u) {
+        dt_upper<M_CUR_GRAD, 3>(lgw, lgv, lk, lext, u);
+    }
     static LDDMM_D void load_target(const Params& P, long long ra, long long rb, Tgt& t) {
         load_target_pair<3>(P.tgt4, P.tgt_stride, ra, rb, 0, t.x);
         load_target_pair<3>(P.tgt4, P.tgt_stride, ra, rb, 1, t.u);
     }
     static LDDMM_D void load_source(const float4* S, int j, Src& s) { load_list_source<NV>(S, j, s.val); }
-    static LDDMM_D void pair(const Params& P, const Tgt& t, const Src& s, Acc& a) {
+    template <class A>
+    static LDDMM_D void pair(const Params& P, const Tgt& t, const Src& s, A& a) {
         f2 dx[3], r2;
 #pragma unroll
         for (int j = 0; j < 3; ++j) {
@@ -351,7 +454,7 @@ LDDMM_D double vec_norm_eps(const double* s, int d, double eps) {
 //   norm measure : target -, source a*sign              (value and gradient)
 //   norm varifold: target n, source (n, a*sign)         (value and gradient)
 // c == nullptr writes a zero (padding) record of nplanes planes.
-// bp, bw (sources): the packed position and the weight that bounds what the record adds (fold boxes).
+// bp, bw (sources): the packed position and the columns that bound what the record adds (dt_weights of them).
 template <class Real>
 LDDMM_D void dt_pack_record(int norm, int grad, bool is_t, const double* c, const double* s, int d, double eps,
                             double sign, double scale, const double* center, float4* planes, long long stride,
@@ -359,7 +462,10 @@ LDDMM_D void dt_pack_record(int norm, int grad, bool is_t, const double* c, cons
                             Real* bw = nullptr) {
     constexpr int PP = PointPlanes<Real>::N;
     if (c == nullptr) {
-        if (bp != nullptr) bp[0] = bp[1] = bp[2] = *bw = 0;
+        if (bp != nullptr) {
+            for (int j = 0; j < 3; ++j) bp[j] = 0;
+            for (int j = 0; j < 4; ++j) bw[j] = 0;
+        }
         for (int p = 0; p < nplanes; ++p) planes[(long long)p * stride + i] = make_float4(0.f, 0.f, 0.f, 0.f);
         return;
     }
@@ -367,13 +473,18 @@ LDDMM_D void dt_pack_record(int norm, int grad, bool is_t, const double* c, cons
     double pos[4] = {0, 0, 0, 0};
     for (int j = 0; j < d; ++j) pos[j] = (c[j] - center[j]) * scale;
     if (bp != nullptr) {
-        Real w = (Real)(norm == NCURRENT ? 0.0 : a * sign);
         for (int j = 0; j < 3; ++j) bp[j] = (Real)pos[j];
-        if (norm == NCURRENT)
-            for (int j = 0; j < d; ++j) w = max_nan(w, (Real)(s[j] * sign));
-        if (norm == NVARIFOLD)   // 0 / 0 of a cell without area: never passed over, though it weighs nothing
-            for (int j = 0; j < 3; ++j) w = max_nan(w, (Real)(s[j] / a) * (Real)0);
-        *bw = max_nan((Real)0, w);
+        for (int j = 0; j < 4; ++j) bw[j] = 0;
+        if (norm == NCURRENT) {
+            for (int j = 0; j < d; ++j) bw[j] = (Real)(s[j] * sign);
+        } else if (norm == NVARIFOLD && grad) {
+            for (int j = 0; j < 3; ++j) bw[j] = (Real)(s[j] / a) * (Real)(a * sign);
+            bw[3] = (Real)(a * sign);
+        } else {
+            bw[0] = (Real)(a * sign);
+            // 0 / 0 of a cell without area: never passed over, though it weighs nothing
+            if (norm == NVARIFOLD) bw[0] += (Real)(s[0] / a + s[1] / a + s[2] / a) * (Real)0;
+        }
     }
     if (sizeof(Real) == 4 && list) {
         // list source record [pos0 pos1 pos2 vals...] (see ops2.cuh)
@@ -437,7 +548,7 @@ static __global__ void dt_pack_kernel(int norm, int grad, const double* __restri
                                       long long n2, int d, double eps1, double eps2, double sign2, double scale,
                                       const double* __restrict__ center, float4* tgt, long long tstride, int tplanes,
                                       int tslots, float4* src, long long sstride, int splanes, int sslots,
-                                      int list, long long n1s, float4* boxes, int* __restrict__ counters,
+                                      int list, long long n1s, float4* boxes, int nw, int* __restrict__ counters,
                                       int n_counters) {
     // set-2 sources start at row n1s (n1 rounded up to a fold for symmetric sweeps)
     const long long npad = tstride > sstride ? tstride : sstride;
@@ -451,10 +562,10 @@ static __global__ void dt_pack_kernel(int norm, int grad, const double* __restri
             const bool first = i < n1, second = i >= n1s && i < n1s + n2;
             const double* c = first ? c1 + i * d : (second ? c2 + (i - n1s) * d : nullptr);
             const double* sv = first ? s1 + i * d : (second ? s2 + (i - n1s) * d : nullptr);
-            Real bp[3], bw;
+            Real bp[3], bw[4];
             dt_pack_record<Real>(norm, grad, false, c, sv, d, first ? eps1 : eps2, first ? 1.0 : sign2, scale, center,
-                                 src, sstride, i, splanes, sslots, list != 0, bp, &bw);
-            store_fold_box<Real>(boxes, i, c != nullptr, bp, bw);
+                                 src, sstride, i, splanes, sslots, list != 0, bp, bw);
+            store_fold_box<Real, 4>(boxes, i, c != nullptr, bp, bw, nw);
         }
     }
 }

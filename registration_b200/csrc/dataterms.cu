@@ -71,7 +71,7 @@ int dt_sweep(const DataArgs& a, Workspace& ws, cudaStream_t st, const double* c1
     pl.seq = false;   // shapes of so few cells take the single-cluster kernels
     float4* tgt = ws.take<float4>((size_t)Op::NT_ * pl.n_tpad);
     float4* src = ws.take<float4>((size_t)Op::NS * pl.m_pad);
-    float4* boxes = ws.take<float4>(pl.box_words());
+    float4* boxes = ws.take<float4>(pl.box_words<Op>());
     double* part = ws.take<double>(pl.part_doubles(Op::NOUT));
     int* counters = ws.take<int>(pl.counters());
     double* epart = ws.take<double>(GRAD ? 0 : pl.n_tb);
@@ -85,7 +85,7 @@ int dt_sweep(const DataArgs& a, Workspace& ws, cudaStream_t st, const double* c1
     dt_pack_kernel<Real><<<grid_for(std::max(pl.n_tpad, pl.m_pad)), 256, 0, st>>>(
         a.norm, GRAD ? 1 : 0, c1, s1, a.nc, a.c2, a.s2, a.nc2, a.d, a.eps1, a.eps2, GRAD ? -1.0 : -2.0, ks.scale,
         center, tgt, pl.n_tpad, Op::NT_, Op::TSLOTS, src, pl.m_pad, Op::NS, Op::SSLOTS, op_list<Op>::value ? 1 : 0,
-        n1s, boxes, counters, (int)pl.counters());
+        n1s, boxes, Op::NW, counters, (int)pl.counters());
     if constexpr (GRAD) {
         const double fac = a.ncorner == 3 ? 1.0 / 3.0 : 0.5;
         const EpiDtGrad E{a.norm, s1, a.d, a.eps1, fac * ks.dscale, z1, dz1};

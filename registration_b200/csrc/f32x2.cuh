@@ -19,6 +19,11 @@ LDDMM_D f2 pk2(float lo, float hi) {
     return r;
 }
 LDDMM_D void upk2(f2 a, float& lo, float& hi) { asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(a.v)); }
+LDDMM_D float half2(f2 a, int lane) {
+    float lo, hi;
+    upk2(a, lo, hi);
+    return lane == 0 ? lo : hi;
+}
 LDDMM_D f2 add2(f2 a, f2 b) {
     f2 r;
     asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
@@ -92,6 +97,18 @@ struct AccF32C2 {
         upk2(e[c], e0, e1);
         return lane == 0 ? (double)s0 + (double)e0 : (double)s1 + (double)e1;
     }
+};
+
+// Sums of the terms' absolute values, lane by lane.
+template <int N>
+struct AccAbs2 {
+    f2 a[N];
+    LDDMM_D void zero() {
+#pragma unroll
+        for (int c = 0; c < N; ++c) a[c] = splat2(0.f);
+    }
+    LDDMM_D void fma(int c, f2 x, f2 y) { a[c] = add2(a[c], f2{mul2(x, y).v & 0x7FFFFFFF7FFFFFFFull}); }
+    LDDMM_D float value(int c, int lane) const { return half2(a[c], lane); }
 };
 
 // Horner on packed lanes; c holds each coefficient duplicated as a pair.

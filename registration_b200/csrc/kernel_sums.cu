@@ -61,7 +61,7 @@ int applyk_group(const ApplyKArgs& a, int col0, Workspace& ws, cudaStream_t st) 
     const SinglePlan pl = plan_single<Op>(a.n, a.m, a.split_cap);
     float4* tgt = ws.take<float4>((size_t)Op::PP * pl.n_tpad);
     float4* src = ws.take<float4>((size_t)Op::NS * pl.m_pad);
-    float4* boxes = ws.take<float4>(pl.box_words());
+    float4* boxes = ws.take<float4>(pl.box_words<Op>());
     double* part = ws.take<double>(pl.part_doubles(DIMB));
     int* counters = ws.take<int>(pl.split > 1 ? pl.counters() : 0);
     // sums over the targets' own points (the query cannot know: room for the order whenever n == m)
@@ -99,7 +99,7 @@ int applyk_group(const ApplyKArgs& a, int col0, Workspace& ws, cudaStream_t st) 
     }
     // the epilogue writes only the group's own columns
     const EpiSum E{a.f, a.dimb, col0, g.nvals, 1.0};
-    return launch_single<Op, false>(pl, a.n, P, boxes, part, st, 0, counters, E, order.perm);
+    return launch_single<Op, false>(pl, a.n, P, boxes, part, st, 0, counters, E, order.perm, a.x == a.y && !both.taken);
 }
 
 template <class Real>
@@ -201,7 +201,7 @@ int difft_impl(const DiffKTArgs& a, Workspace& ws, cudaStream_t st) {
     const SinglePlan pl = plan_single<Op>(a.n, a.m);
     float4* tgt = ws.take<float4>((size_t)NT * pl.n_tpad);
     float4* src = ws.take<float4>((size_t)Op::NS * pl.m_pad);
-    float4* boxes = ws.take<float4>(pl.box_words());
+    float4* boxes = ws.take<float4>(pl.box_words<Op>());
     double* part = ws.take<double>(pl.part_doubles(D));
     int* counters = ws.take<int>(pl.counters());
     const Ordered64 both = take_ordered64<Op>(ws, pl, a.n, a.m);
@@ -239,7 +239,7 @@ int difft_impl(const DiffKTArgs& a, Workspace& ws, cudaStream_t st) {
         order = both.t;
     }
     const EpiSum E{a.f, a.d, 0, a.d, ks.dscale};   // D may exceed d (d == 1 runs as D == 2)
-    return launch_single<Op, false>(pl, a.n, P, boxes, part, st, 0, counters, E, order.perm);
+    return launch_single<Op, false>(pl, a.n, P, boxes, part, st, 0, counters, E, order.perm, a.x == a.y && !both.taken);
 }
 
 template <class Real>

@@ -74,7 +74,8 @@ struct OpApplyK {
     static constexpr int NOUT = DIMB;
     using Params = KernelParamsBase<Real>;
     using Acc = typename AccFor<Real>::template type<DIMB>;
-    static constexpr bool GRADX = false;
+    using Abs = AccAbs<Real, DIMB>;
+    static constexpr int NW = DIMB, NB = DIMB, DOT = 0;   // bounds: the columns
     static LDDMM_D float lgk(const Params& P, float d2) { return lg_factor<KIND, DEG>(P.pk, d2); }
     struct Tgt {
         Real x[D];
@@ -83,6 +84,15 @@ struct OpApplyK {
         Real y[D];
         Real b[DIMB];
     };
+    static LDDMM_D Real coord(const Tgt& t, int, int j) { return j < D ? t.x[j < D ? j : 0] : (Real)0; }
+    static LDDMM_D void lower(const Tgt&, int, const Real* a, Real, Real* lo) {
+#pragma unroll
+        for (int c = 0; c < DIMB; ++c) lo[c] = a[c];
+    }
+    static LDDMM_D void upper(const float* lgw, float, float lk, const float*, float* u) {
+#pragma unroll
+        for (int c = 0; c < DIMB; ++c) u[c] = lgw[c] + lk;
+    }
     static LDDMM_D void load_target(const Params& P, long long row, Tgt& t) {
         load_vals<Real, D>(P.tgt4, P.tgt_stride, row, 0, t.x);
     }
@@ -90,8 +100,8 @@ struct OpApplyK {
         load_vals_smem<Real, D>(S, j, 0, s.y);
         load_vals_smem<Real, DIMB>(S, j, PP, s.b);
     }
-    template <bool LIB = false>
-    static LDDMM_D void pair(const Params& P, const Tgt& t, const Src& s, Acc& a) {
+    template <bool LIB = false, class A>
+    static LDDMM_D void pair(const Params& P, const Tgt& t, const Src& s, A& a) {
         Real r2 = 0;
 #pragma unroll
         for (int j = 0; j < D; ++j) {
@@ -119,7 +129,8 @@ struct OpDiffKT {
     static constexpr int NOUT = D;
     using Params = KernelParamsBase<Real>;
     using Acc = typename AccFor<Real>::template type<D>;
-    static constexpr bool GRADX = true;
+    using Abs = AccAbs<Real, D>;
+    static constexpr int NW = W, NB = D, DOT = W;   // bounds: the components
     static LDDMM_D float lgk(const Params& P, float d2) { return lg_factor<KIND, DEG>(P.pq, d2); }
     struct Tgt {
         Real x[D];
@@ -129,6 +140,16 @@ struct OpDiffKT {
         Real y[D];
         Real v[W];
     };
+    static LDDMM_D Real coord(const Tgt& t, int, int j) { return j < D ? t.x[j < D ? j : 0] : (Real)0; }
+    static LDDMM_D Real dot_val(const Tgt& t, int, int w) { return t.u[w]; }
+    static LDDMM_D void lower(const Tgt&, int, const Real* a, Real norm1, Real* lo) {
+#pragma unroll
+        for (int j = 0; j < D; ++j) lo[j] = norm1 == (Real)0 ? (Real)-1 : a[j] / norm1;
+    }
+    static LDDMM_D void upper(const float*, float lgv, float lk, const float* lext, float* u) {
+#pragma unroll
+        for (int j = 0; j < D; ++j) u[j] = lgv + lk + lext[j];
+    }
     static LDDMM_D void load_target(const Params& P, long long row, Tgt& t) {
         load_vals<Real, D>(P.tgt4, P.tgt_stride, row, 0, t.x);
         load_vals<Real, W>(P.tgt4, P.tgt_stride, row, PP, t.u);
@@ -137,8 +158,8 @@ struct OpDiffKT {
         load_vals_smem<Real, D>(S, j, 0, s.y);
         load_vals_smem<Real, W>(S, j, PP, s.v);
     }
-    template <bool LIB = false>
-    static LDDMM_D void pair(const Params& P, const Tgt& t, const Src& s, Acc& a) {
+    template <bool LIB = false, class A>
+    static LDDMM_D void pair(const Params& P, const Tgt& t, const Src& s, A& a) {
         Real dx[D];
         Real r2 = 0;
 #pragma unroll

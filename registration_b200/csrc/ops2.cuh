@@ -106,7 +106,8 @@ struct OpApplyK2 {
     static constexpr int NOUT = DIMB;
     using Params = KernelParams2;
     using Acc = AccF32C2<DIMB>;
-    static constexpr bool GRADX = false;
+    using Abs = AccAbs2<DIMB>;
+    static constexpr int NW = DIMB, NB = DIMB, DOT = 0;   // bounds: the columns
     static LDDMM_D float lgk(const Params& P, float d2) { return lg_factor<KIND, DEG>(P.pkd, d2); }
     struct Tgt {
         f2 x[D];
@@ -114,11 +115,21 @@ struct OpApplyK2 {
     struct Src {
         f2 val[NV];
     };
+    static LDDMM_D float coord(const Tgt& t, int h, int j) { return j < D ? half2(t.x[j < D ? j : 0], h) : 0.f; }
+    static LDDMM_D void lower(const Tgt&, int, const float* a, float, float* lo) {
+#pragma unroll
+        for (int c = 0; c < DIMB; ++c) lo[c] = a[c];
+    }
+    static LDDMM_D void upper(const float* lgw, float, float lk, const float*, float* u) {
+#pragma unroll
+        for (int c = 0; c < DIMB; ++c) u[c] = lgw[c] + lk;
+    }
     static LDDMM_D void load_target(const Params& P, long long ra, long long rb, Tgt& t) {
         load_target_pair<D>(P.tgt4, P.tgt_stride, ra, rb, 0, t.x);
     }
     static LDDMM_D void load_source(const float4* S, int j, Src& s) { load_list_source<NV>(S, j, s.val); }
-    static LDDMM_D void pair(const Params& P, const Tgt& t, const Src& s, Acc& a) {
+    template <class A>
+    static LDDMM_D void pair(const Params& P, const Tgt& t, const Src& s, A& a) {
         f2 r2;
 #pragma unroll
         for (int j = 0; j < D; ++j) {
@@ -146,7 +157,8 @@ struct OpDiffKT2 {
     static constexpr int NOUT = D;
     using Params = KernelParams2;
     using Acc = AccF32C2<D>;
-    static constexpr bool GRADX = true;
+    using Abs = AccAbs2<D>;
+    static constexpr int NW = W, NB = D, DOT = W;   // bounds: the components
     static LDDMM_D float lgk(const Params& P, float d2) { return lg_factor<KIND, DEG>(P.pqd, d2); }
     struct Tgt {
         f2 x[D];
@@ -155,12 +167,23 @@ struct OpDiffKT2 {
     struct Src {
         f2 val[NV];
     };
+    static LDDMM_D float coord(const Tgt& t, int h, int j) { return j < D ? half2(t.x[j < D ? j : 0], h) : 0.f; }
+    static LDDMM_D float dot_val(const Tgt& t, int h, int w) { return half2(t.u[w], h); }
+    static LDDMM_D void lower(const Tgt&, int, const float* a, float norm1, float* lo) {
+#pragma unroll
+        for (int j = 0; j < D; ++j) lo[j] = norm1 == 0.f ? -1.f : __fdividef(a[j], norm1);
+    }
+    static LDDMM_D void upper(const float*, float lgv, float lk, const float* lext, float* u) {
+#pragma unroll
+        for (int j = 0; j < D; ++j) u[j] = lgv + lk + lext[j];
+    }
     static LDDMM_D void load_target(const Params& P, long long ra, long long rb, Tgt& t) {
         load_target_pair<D>(P.tgt4, P.tgt_stride, ra, rb, 0, t.x);
         load_target_pair<W>(P.tgt4, P.tgt_stride, ra, rb, 1, t.u);
     }
     static LDDMM_D void load_source(const float4* S, int j, Src& s) { load_list_source<NV>(S, j, s.val); }
-    static LDDMM_D void pair(const Params& P, const Tgt& t, const Src& s, Acc& a) {
+    template <class A>
+    static LDDMM_D void pair(const Params& P, const Tgt& t, const Src& s, A& a) {
         f2 dx[D], r2;
 #pragma unroll
         for (int j = 0; j < D; ++j) {

@@ -145,16 +145,13 @@ LDDMM_D void pack_row(const double* __restrict__ x, long long n, int d, double s
                       const double* __restrict__ center, const Gather& g, int D, int V, float4* __restrict__ out,
                       long long stride, long long i, float4* boxes) {
     constexpr int PW = Traits<Real>::PER_WORD;
-    Real v[16], w = 0;
+    Real v[16];
 #pragma unroll
     for (int q = 0; q < 16; ++q) v[q] = 0;
     const int V0 = LIST ? D : 4;   // first value
     if (i < n) {
         for (int j = 0; j < d && j < 3; ++j) v[j] = (Real)((x[i * d + j] - center[j]) * scale);
-        for (int q = 0; q < V && q < g.nvals; ++q) {
-            v[V0 + q] = (Real)(g.src[i * g.row_stride + g.off[q]] * g.mult);
-            w = max_nan(w, v[V0 + q]);
-        }
+        for (int q = 0; q < V && q < g.nvals; ++q) v[V0 + q] = (Real)(g.src[i * g.row_stride + g.off[q]] * g.mult);
     }
     const int nwords = LIST ? (D + V + PW - 1) / PW : 4 / PW + (V + PW - 1) / PW;
     for (int k = 0; k < nwords; ++k) {
@@ -164,7 +161,7 @@ LDDMM_D void pack_row(const double* __restrict__ x, long long n, int d, double s
     }
     if (boxes != nullptr) {
         const Real p[3] = {v[0], v[1], D > 2 ? v[2] : (Real)0};
-        store_fold_box<Real>(boxes, i, i < n, p, w);
+        store_fold_box<Real, 12>(boxes, i, i < n, p, v + V0, V);
     }
 }
 
@@ -193,7 +190,7 @@ static __global__ void fold_boxes_kernel(const float4* __restrict__ src, long lo
     constexpr int PW = Traits<Real>::PER_WORD;
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < m_pad;
          i += (long long)gridDim.x * blockDim.x) {
-        Real p[3] = {0, 0, 0}, w = 0;
+        Real p[3] = {0, 0, 0}, w[12];
         const int first = LIST ? D : 4, total = first + V;
         for (int k = 0; k * PW < total; ++k) {
             const float4 word = src[(long long)k * m_pad + i];
@@ -201,10 +198,10 @@ static __global__ void fold_boxes_kernel(const float4* __restrict__ src, long lo
                 const int j = k * PW + q;
                 const Real v = word_get<Real>(&word, q);
                 if (j < 3 && j < D) p[j] = v;
-                if (j >= first && j < total) w = max_nan(w, v);
+                if (j >= first && j < total) w[j - first] = v;
             }
         }
-        store_fold_box<Real>(boxes, i, i < n, p, w);
+        store_fold_box<Real, 12>(boxes, i, i < n, p, w, V);
     }
 }
 
@@ -215,17 +212,17 @@ static __global__ void permute_records_kernel(const float4* __restrict__ src, co
     for (long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x; q < m_pad;
          q += (long long)gridDim.x * blockDim.x) {
         const long long i = perm[q];
-        double p[4] = {0, 0, 0, 0}, w = 0;
+        double p[4] = {0, 0, 0, 0}, w[12];
         for (int k = 0; k < 2 + (V + 1) / 2; ++k) {
             const float4 word = src[(long long)k * m_pad + i];
             out[(long long)k * m_pad + q] = word;
             for (int h = 0; h < 2; ++h) {
                 const double v = word_get<double>(&word, h);
                 if (k < 2) p[2 * k + h] = v;
-                else if (2 * (k - 2) + h < V) w = max_nan(w, v);
+                else if (2 * (k - 2) + h < V) w[2 * (k - 2) + h] = v;
             }
         }
-        store_fold_box<double>(boxes, q, i < m, p, w);
+        store_fold_box<double, 12>(boxes, q, i < m, p, w, V);
     }
 }
 

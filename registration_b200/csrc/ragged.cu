@@ -67,7 +67,7 @@ struct RagPlan {
 };
 
 template <class Op>
-RagPlan<Op> rag_plan(const std::vector<long long>& n, const std::vector<long long>& m) {
+RagPlan<Op> rag_plan(const std::vector<long long>& n, const std::vector<long long>& m, bool self) {
     RagPlan<Op> p;
     const int nseg = (int)n.size();
     p.segs.resize(nseg);
@@ -98,6 +98,7 @@ RagPlan<Op> rag_plan(const std::vector<long long>& n, const std::vector<long lon
         d.split = pl.split;
         d.item0 = p.items;
         d.id = s;
+        d.self = self;
         d.cnt = (int)p.eparts;
         p.items += pl.n_tb * pl.split;
         p.tt += pl.n_tpad;
@@ -180,13 +181,11 @@ LDDMM_D void put_plain(float4* planes, long long stride, long long i, const floa
     }
 }
 
-// fold box of a packed source row: position v[0..D), weights v[D..NV) (whole warps: segments are padded to folds)
-template <int D>
-LDDMM_D void rag_box(float4* boxes, long long row, bool valid, const float* v, int NV) {
+// fold box of a packed source row: position v[0..D), values v[D..NV) (whole warps: segments are padded to folds)
+template <int D, int NV>
+LDDMM_D void rag_box(float4* boxes, long long row, bool valid, const float* v) {
     const float p[3] = {v[0], v[1], D > 2 ? v[2] : 0.f};
-    float w = 0.f;
-    for (int k = D; k < NV; ++k) w = max_nan(w, v[k]);
-    store_fold_box<float>(boxes, row, valid, p, w);
+    store_fold_box<float, NV - D>(boxes, row, valid, p, v + D, NV - D);
 }
 
 // ---- ragged shooting ---------------------------------------------------------------
@@ -210,7 +209,7 @@ LDDMM_D void rag_shoot_row(const RagSeg& g, long long i, const double* x, const 
     if (i < g.tpad) put_plain(p.tgt, tstride, g.tgt + i, pos, 3, 1);
     if (i < g.spad) {
         put_plain(p.src, sstride, g.src + i, vals, 2 * D, (2 * D + 3) / 4);
-        rag_box<D>(p.boxes, g.src + i, x != nullptr, vals, 2 * D);
+        rag_box<D, 2 * D>(p.boxes, g.src + i, x != nullptr, vals);
     }
 }
 
@@ -294,7 +293,7 @@ int rag_shoot_impl(int nseg, const int64_t* v_off, int d, const double* x0, cons
     using Op = OpApplyK2<KIND, DEG, D, D>;
     std::vector<long long> n(nseg);
     for (int s = 0; s < nseg; ++s) n[s] = v_off[s + 1] - v_off[s];
-    RagPlan<Op> pl = rag_plan<Op>(n, n);
+    RagPlan<Op> pl = rag_plan<Op>(n, n, true);
     std::vector<long long> padoff(nseg + 1, 0);
     for (int s = 0; s < nseg; ++s) padoff[s + 1] = padoff[s] + std::max(pl.segs[s].tpad, pl.segs[s].spad);
     RagSeg* dsegs = ws.take<RagSeg>(nseg);
@@ -304,7 +303,7 @@ int rag_shoot_impl(int nseg, const int64_t* v_off, int d, const double* x0, cons
     for (RagPlanes& p : pn) {
         p.tgt = ws.take<float4>((size_t)Op::PP * pl.tt);
         p.src = ws.take<float4>((size_t)Op::NS * pl.ss);
-        p.boxes = ws.take<float4>(2 * (size_t)(pl.ss / kFold));
+        p.boxes = ws.take<float4>((size_t)fold_box_words(Op::NW) * (size_t)(pl.ss / kFold));
     }
     double* part = ws.take<double>((size_t)pl.parts * D);
     double* epart = ws.take<double>((size_t)pl.eparts + 1);   // and the groups' counters behind it
@@ -372,7 +371,7 @@ LDDMM_D void rag_cov_row(const RagSeg& g, long long i, const double* x, const do
     }
     if (i < g.spad) {
         put_plain(pl.src, sstride, g.src + i, v, 3 * D, (3 * D + 3) / 4);
-        rag_box<D>(pl.boxes, g.src + i, x != nullptr, v, 3 * D);
+        rag_box<D, 3 * D>(pl.boxes, g.src + i, x != nullptr, v);
     }
 }
 
@@ -444,7 +443,7 @@ int rag_cov_impl(int nseg, const int64_t* v_off, int d, const double* xt, const 
     constexpr int NT = 1 + (W + 3) / 4;
     std::vector<long long> n(nseg);
     for (int s = 0; s < nseg; ++s) n[s] = v_off[s + 1] - v_off[s];
-    RagPlan<Op> pl = rag_plan<Op>(n, n);
+    RagPlan<Op> pl = rag_plan<Op>(n, n, true);
     std::vector<long long> padoff(nseg + 1, 0);
     for (int s = 0; s < nseg; ++s) padoff[s + 1] = padoff[s] + std::max(pl.segs[s].tpad, pl.segs[s].spad);
     RagSeg* dsegs = ws.take<RagSeg>(nseg);
@@ -454,7 +453,7 @@ int rag_cov_impl(int nseg, const int64_t* v_off, int d, const double* xt, const 
     for (RagPlanes& p : pn) {
         p.tgt = ws.take<float4>((size_t)NT * pl.tt);
         p.src = ws.take<float4>((size_t)Op::NS * pl.ss);
-        p.boxes = ws.take<float4>(2 * (size_t)(pl.ss / kFold));
+        p.boxes = ws.take<float4>((size_t)fold_box_words(Op::NW) * (size_t)(pl.ss / kFold));
     }
     double* part = ws.take<double>((size_t)pl.parts * D);
     int* counters = ws.take<int>((size_t)pl.eparts + 1);
@@ -523,7 +522,7 @@ static __global__ void rag_applyk_pack_kernel(const RagSeg* __restrict__ segs, c
                 for (int c = 0; c < dimb && c < DIMB; ++c) v[D + c] = (float)beta[(g.m0 + i) * dimb + c];
             }
             put_plain(src, sstride, g.src + i, v, D + DIMB, (D + DIMB + 3) / 4);
-            rag_box<D>(boxes, g.src + i, i < g.m, v, D + DIMB);
+            rag_box<D, D + DIMB>(boxes, g.src + i, i < g.m, v);
         }
     }
 }
@@ -553,7 +552,7 @@ int rag_applyk_impl(int nseg, const int64_t* t_start, const int64_t* t_count, co
         n[s] = t_count[s];
         m[s] = s_count[s];
     }
-    RagPlan<Op> pl = rag_plan<Op>(n, m);
+    RagPlan<Op> pl = rag_plan<Op>(n, m, false);
     std::vector<long long> padoff(nseg + 1, 0), rowoff(nseg + 1, 0);
     for (int s = 0; s < nseg; ++s) {
         pl.segs[s].row0 = t_start[s];
@@ -567,7 +566,7 @@ int rag_applyk_impl(int nseg, const int64_t* t_start, const int64_t* t_count, co
     long long* drow = ws.take<long long>(nseg + 1);
     float4* tgt = ws.take<float4>((size_t)Op::PP * pl.tt);
     float4* src = ws.take<float4>((size_t)Op::NS * pl.ss);
-    float4* boxes = ws.take<float4>(2 * (size_t)(pl.ss / kFold));
+    float4* boxes = ws.take<float4>((size_t)fold_box_words(Op::NW) * (size_t)(pl.ss / kFold));
     double* part = ws.take<double>((size_t)pl.parts * DIMB);
     int* counters = ws.take<int>((size_t)pl.eparts + 1);
     if (ws.measuring()) return LDDMM_OK;
@@ -611,7 +610,7 @@ static __global__ void rag_dt_pack_kernel(const RagSeg* __restrict__ segs, const
                                           const double* __restrict__ s2, int d, double eps1, double eps2,
                                           double sign2, float4* tgt, long long tstride, int tplanes, int tslots,
                                           float4* src, long long sstride, int splanes, int sslots, int list,
-                                          int sym_align, float4* boxes) {
+                                          int sym_align, float4* boxes, int nw) {
     const long long total = padoff[nseg];
     for (long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x; q < total;
          q += (long long)gridDim.x * blockDim.x) {
@@ -628,10 +627,10 @@ static __global__ void rag_dt_pack_kernel(const RagSeg* __restrict__ segs, const
             const bool first = i < g.n, second = i >= n1s && i < n1s + g.m;
             const double* c = first ? c1 + (g.row0 + i) * d : (second ? c2 + (g.m0 + i - n1s) * d : nullptr);
             const double* sv = first ? s1 + (g.row0 + i) * d : (second ? s2 + (g.m0 + i - n1s) * d : nullptr);
-            Real bp[3], bw;
+            Real bp[3], bw[4];
             dt_pack_record<Real>(norm, grad, false, c, sv, d, first ? eps1 : eps2, first ? 1.0 : sign2, g.scale,
-                                 g.center, src, sstride, g.src + i, splanes, sslots, list != 0, bp, &bw);
-            store_fold_box<Real>(boxes, g.src + i, c != nullptr, bp, bw);
+                                 g.center, src, sstride, g.src + i, splanes, sslots, list != 0, bp, bw);
+            store_fold_box<Real, 4>(boxes, g.src + i, c != nullptr, bp, bw, nw);
         }
     }
 }
@@ -713,7 +712,7 @@ int rag_dt_sweep(const RagDataArgs& a, int kind, const double* c1, const double*
         n1s[s] = SYM ? round_up(n[s], kFold) : n[s];
         m[s] = n1s[s] + (a.c2_off[s + 1] - a.c2_off[s]);
     }
-    RagPlan<Op> pl = rag_plan<Op>(n, m);
+    RagPlan<Op> pl = rag_plan<Op>(n, m, true);
     for (int s = 0; s < nseg; ++s) pl.desc[s].sym_folds = SYM ? (int)(n1s[s] / kFold) : 0;
     std::vector<long long> padoff(nseg + 1, 0);
     for (int s = 0; s < nseg; ++s) {
@@ -727,7 +726,7 @@ int rag_dt_sweep(const RagDataArgs& a, int kind, const double* c1, const double*
     long long* dpad = ws.take<long long>(nseg + 1);
     float4* tgt = ws.take<float4>((size_t)NT * pl.tt);
     float4* src = ws.take<float4>((size_t)Op::NS * pl.ss);
-    float4* boxes = ws.take<float4>(2 * (size_t)(pl.ss / kFold));
+    float4* boxes = ws.take<float4>((size_t)fold_box_words(Op::NW) * (size_t)(pl.ss / kFold));
     double* part = ws.take<double>((size_t)pl.parts * Op::NOUT);
     int* counters = ws.take<int>((size_t)pl.eparts + 1);
     double* epart = ws.take<double>(GRAD ? 0 : (size_t)pl.eparts + 1);
@@ -753,7 +752,7 @@ int rag_dt_sweep(const RagDataArgs& a, int kind, const double* c1, const double*
     set_poly(P, kernel_scale(kind, a.order, a.sigma[0], true));
     rag_dt_pack_kernel<Real><<<grid_for(padoff[nseg]), 256, 0, st>>>(
         dsegs, dpad, nseg, a.norm, GRAD ? 1 : 0, c1, s1, a.c2, a.s2, a.d, a.eps1, a.eps2, GRAD ? -1.0 : -2.0, tgt, pl.tt, NT, TSLOTS, src,
-        pl.ss, Op::NS, SSLOTS, op_list<Op>::value ? 1 : 0, SYM ? kFold : 0, boxes);
+        pl.ss, Op::NS, SSLOTS, op_list<Op>::value ? 1 : 0, SYM ? kFold : 0, boxes, Op::NW);
     SweepGrid grid{};
     grid.segs = ddesc;
     grid.nseg = nseg;

@@ -79,19 +79,17 @@ LDDMM_D void store_list(float4* planes, long long stride, long long i, const dou
         planes[(long long)w * stride + i] = make_float4(v[4 * w], v[4 * w + 1], v[4 * w + 2], v[4 * w + 3]);
 }
 
-// Fold box of source row i (whole warps, see store_fold_box): packed position
-// of x and the largest of the values of a and (if given) b.
-template <class Real>
-LDDMM_D void store_box(float4* boxes, long long i, bool valid, const double* x, const double* a, const double* b,
-                       int d, double s, const double* c) {
-    Real p[3] = {0, 0, 0}, w = 0;
+// Fold box of source row i (whole warps, see store_fold_box): packed position of x, the
+// values v[0..nv) of its NW columns.
+template <class Real, int NW>
+LDDMM_D void store_box(float4* boxes, long long i, bool valid, const double* x, const double* v, int nv, int nw, int d,
+                       double s, const double* c) {
+    Real p[3] = {0, 0, 0}, w[NW];
     if (valid)
-        for (int j = 0; j < d; ++j) {
-            p[j] = (Real)((x[j] - c[j]) * s);
-            w = max_nan(w, (Real)a[j]);
-            if (b != nullptr) w = max_nan(w, (Real)b[j]);
-        }
-    store_fold_box<Real>(boxes, i, valid, p, w);
+        for (int j = 0; j < d; ++j) p[j] = (Real)((x[j] - c[j]) * s);
+#pragma unroll
+    for (int j = 0; j < NW; ++j) w[j] = valid && j < nv ? (Real)v[j] : (Real)0;
+    store_fold_box<Real, NW>(boxes, i, valid, p, w, nw);
 }
 
 // ---- shooting ---------------------------------------------------------------
@@ -111,7 +109,7 @@ static __global__ void shoot_pack_kernel(const double* __restrict__ x, const dou
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < npad;
          i += (long long)gridDim.x * blockDim.x) {
         if (i < n_counters) counters[i] = 0;
-        if (i < sstride) store_box<Real>(p0.boxes, i, i < n, x + i * d, a + i * d, nullptr, d, s, c);
+        if (i < sstride) store_box<Real, 3>(p0.boxes, i, i < n, x + i * d, a + i * d, d, nslots, d, s, c);
         if (i < n) {
             for (int j = 0; j < d; ++j) xt0[i * d + j] = x[i * d + j];
             store_point<Real>(p0.tgt, tstride, i, x + i * d, d, s, c);
@@ -170,7 +168,7 @@ struct EpiShoot {
                 x1[i * d + j] = xn[j];
             }
             if (a1 == nullptr) continue;
-            if (sg.perm == nullptr) store_box<Real>(nx.boxes, i, valid, xn, a1 + i * d, nullptr, d, s, c);
+            if (sg.perm == nullptr) store_box<Real, 3>(nx.boxes, i, valid, xn, a1 + i * d, d, nslots, d, s, c);
             if (!valid) continue;
             store_point<Real>(nx.tgt, tstride, i, xn, d, s, c);
             if constexpr (LIST) {
@@ -229,7 +227,7 @@ int shoot_impl(const ShootArgs& a, Workspace& ws, cudaStream_t st) {
     for (StepPlanes& p : pn) {
         p.tgt = ws.take<float4>((size_t)Op::PP * pl.n_tpad);
         p.src = ws.take<float4>((size_t)Op::NS * pl.m_pad);
-        p.boxes = ws.take<float4>(pl.box_words());
+        p.boxes = ws.take<float4>(pl.box_words<Op>());
     }
     double* part = ws.take<double>(pl.part_doubles(D));
     int* counters = ws.take<int>(pl.counters());
@@ -352,6 +350,17 @@ LDDMM_D void cov_store(float4* tgt, long long tstride, float4* src, long long ss
     }
 }
 
+template <class Real>
+LDDMM_D void cov_box(float4* boxes, long long i, bool valid, const double* x, const double* a, const double* p, int d,
+                     double s, const double* c, int tw) {
+    double v[6] = {0, 0, 0, 0, 0, 0};
+    for (int j = 0; j < d && valid; ++j) {
+        v[j] = a[j];
+        v[d + j] = p[j];
+    }
+    store_box<Real, 6>(boxes, i, valid, x, v, 2 * d, tw, d, s, c);
+}
+
 // Packs the planes of step T-1; pads both sets, copies p to pxt[T], zeroes the counters.
 template <class Real, bool LIST>
 static __global__ void cov_pack_kernel(const double* __restrict__ x, const double* __restrict__ a,
@@ -363,7 +372,7 @@ static __global__ void cov_pack_kernel(const double* __restrict__ x, const doubl
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < npad;
          i += (long long)gridDim.x * blockDim.x) {
         if (i < n_counters) counters[i] = 0;
-        if (i < sstride) store_box<Real>(p0.boxes, i, i < n, x + i * d, a + i * d, p + i * d, d, s, c);
+        if (i < sstride) cov_box<Real>(p0.boxes, i, i < n, x + i * d, a + i * d, p + i * d, d, s, c, tw);
         if (i < n) {
             for (int j = 0; j < d; ++j) pT[i * d + j] = p[i * d + j];
             cov_store<Real, LIST>(p0.tgt, tstride, p0.src, sstride, i, pp, x + i * d, a + i * d, p + i * d, d, s, c,
@@ -408,7 +417,7 @@ struct EpiCov {
             }
             if (x_prev == nullptr) continue;
             if (sg.perm == nullptr)
-                store_box<Real>(nx.boxes, i, valid, x_prev + i * d, a_prev + i * d, pn, d, s, c);
+                cov_box<Real>(nx.boxes, i, valid, x_prev + i * d, a_prev + i * d, pn, d, s, c, tw);
             if (valid)
                 cov_store<Real, LIST>(nx.tgt, tstride, nx.src, sstride, i, pp, x_prev + i * d, a_prev + i * d, pn, d,
                                       s, c, rw, tw);
@@ -442,7 +451,7 @@ int cov_impl(const CovArgs& a, Workspace& ws, cudaStream_t st) {
     for (StepPlanes& p : pn) {
         p.tgt = ws.take<float4>((size_t)NT * pl.n_tpad);
         p.src = ws.take<float4>((size_t)Op::NS * pl.m_pad);
-        p.boxes = ws.take<float4>(pl.box_words());
+        p.boxes = ws.take<float4>(pl.box_words<Op>());
     }
     double* part = ws.take<double>(pl.part_doubles(D));
     int* counters = ws.take<int>(pl.counters());

@@ -24,22 +24,28 @@
 // few thousand points (13 blocks, each thread adding its row's chunks one after
 // the other).  EpiNone leaves the chunk sums in `part`.
 //
-// Far folds (operators with Op::lgk, `boxes` given).  The pack kernels leave
-// for each fold its bounding box and log2 of the sum of its weights.  With the
-// box of the target group these bound what a fold can add to any target of
-// the group, U = W_F K(dmin) (times dmax where the summand carries x - y), and
-// from below what the sum is made of, L = max_F W_F K(dmax).  A fold with
-//   U <= L 2^-MARGIN / (number of folds)
-// is passed over: all such folds together stay below 2^-MARGIN of the sum of
-// absolute terms of every target of the group, MARGIN = 36 for FP32 pairs (whose
-// own rounding is 2^-22 to 2^-24 of it) and 58 for FP64 (2^-53).  The test is
-// done in log2, so it holds as well for targets far from every source, where
-// the whole sum is tiny.  A fold or group with a non-finite coordinate or weight
-// is never passed over.  A lane tests one fold, a warp 32 at a time.
-// Measured against the sweep over every pair that this replaces (B200): FP32c
-// varifold gradient of a 20,480-cell sphere at sigma 0.1 0.97 -> 0.47 ms, its
-// FP64 value 1.63 -> 0.81 ms, the value of 98,000 cells at sigma 0.05 6.2 ->
-// 1.9 ms.  Where no fold is far (uniform random points) the test costs 0.5%.
+// Far folds (operators with Op::lgk, `boxes` given, more than kBoundFolds folds).  The
+// pack kernels leave for each fold its bounding box and, by weight column, log2 of the
+// sum of its weights.  With the box of the target group these bound what a fold can add
+// to an output of any target of the group, U = W_F K(dmin), times max |x_j - y_j| where
+// the term carries x - y and |u_k|_1 where it carries <u_k, v_l>.  What the outputs
+// hold at least is measured: each warp adds up the absolute terms of all targets of the
+// group over eight records of one fold, and L, by output, is the least over the targets
+// (per unit of |u_k|_1), of the warps the best.  A fold with
+//   U <= L 2^-MARGIN / (number of folds)   for every output
+// is passed over: all such folds together stay below 2^-MARGIN of the sum of absolute
+// terms of every output of every target, MARGIN = 36 for FP32 pairs (whose own rounding
+// is 2^-22 to 2^-24 of it) and 58 for FP64 (2^-53).  A bound by boxes alone would not do:
+// near records may add nothing to an output, because they coincide with the target,
+// weigh in other columns or are orthogonal to u_k.  The test is done in log2, so it holds
+// as well for targets far from every source, where the whole sum is tiny.  A fold with a
+// non-finite coordinate or value is never passed over, nor is any by a group with a
+// non-finite target; nor where L is 0 or overflows.  A lane tests one fold, a warp 32 at
+// a time.
+// Measured against the sweep over every pair (B200): FP32c varifold gradient of a
+// 20,480-cell sphere at sigma 0.1 0.97 -> 0.41 ms, its FP64 value 1.63 -> 0.58 ms, the
+// value of 98,000 cells at sigma 0.05 6.2 -> 1.6 ms.  Where no fold is far it costs 3% of
+// a shot and adjoint of 10,242 points (1384 -> 1430 us), less of longer sweeps.
 //
 // perm (SegDesc): the target rows in an order that puts neighbours into the same
 // group (launch_order_rows, pack.cuh).  The sum of a target does not depend on
@@ -54,6 +60,7 @@
 // each unordered pair is evaluated once: the per-target partial sums are no
 // longer the per-target sums, their weighted total is.
 #pragma once
+#include <cfloat>
 #include <type_traits>
 
 #include "common.cuh"
@@ -144,22 +151,50 @@ constexpr int op_min_blocks() {
 template <class Op>
 constexpr int op_unroll() { return sizeof(typename Op::Real) == 4 ? kFold : kFold / 2; }
 
-// Operators that bound their kernel factor (Op::lgk) can pass over far folds.
+// Operators that can pass over far folds.  They give, with h the half of a packed slot:
+//   NW               weight columns of a source record that bound its terms
+//   NB               bounds: what a fold adds is compared bound by bound
+//   coord(t, h, j)   packed coordinate j of target t
+//   DOT, dot_val     columns of the inner product <u_k, v_l> in some terms (0: none), u_k
+//   lgk(P, d2)       log2 of the kernel factor at a squared distance (falls with it)
+//   lower(t, h, a, norm1, lo)   what target t's sums hold at least, one value per bound,
+//                    from a, its sums of absolute terms over some records; per unit of
+//                    norm1 = |u_k|_1 where the terms carry <u_k, v_l>; -1: any fold may go
+//   upper(lgw, lgv, lk, lext, u)  log2 of what a fold adds to any target, per bound:
+//                    lgw its weights by column, lgv of the inner product per unit of
+//                    norm1, lk of the kernel factor, lext of |x_j - y_j|
 template <class Op, class = void>
 struct op_culls : std::false_type {};
 template <class Op>
 struct op_culls<Op, std::void_t<decltype(&Op::lgk)>> : std::true_type {};
+template <class Op>
+constexpr int op_weights() {
+    if constexpr (op_culls<Op>::value) return Op::NW;
+    else return 0;
+}
+
+// Up to this many folds (6,144 sources) a sweep is so short that bounding its folds costs
+// what it saves.  Shot and adjoint of ten steps at 1,500 / 3,166 / 6,000 / 10,242 points of a
+// sphere, us, FP32: every fold 251 / 389 / 677 / 1384; bounded, sigma 0.05 291 / 427 / 720 /
+// 1294, sigma 0.2 292 / 429 / 745 / 1430.
+constexpr int kBoundFolds = 192;
+
+// float4 words of a fold's box: (lo, lgw[0]), (hi, lgw[1]), (lgw[2..5]), ...
+constexpr __host__ __device__ int fold_box_words(int nw) { return 2 + (nw > 2 ? (nw + 1) / 4 : 0); }
+
+// log2 of a sum of n values at most, per value
+constexpr LDDMM_D float lg_columns(int n) { return n <= 1 ? 0.f : n <= 2 ? 1.f : n <= 4 ? 2.f : n <= 8 ? 3.f : 4.f; }
 
 // Targets of one group.
 template <class Op>
 constexpr int op_group() { return 32 * Op::R; }
 
-// Squared distances between two boxes: the smallest and the largest, with
-// slack for the rounding of the pairs' own distances.
+// Squared distances between two boxes: the smallest and the largest, and the largest
+// |x_j - y_j|, with slack for the rounding of the pairs' own distances.
 struct Box {
     float lo[3], hi[3];
 };
-LDDMM_D void box_dist2(const Box& a, const float4 lo, const float4 hi, float& dmin2, float& dmax2) {
+LDDMM_D void box_dist2(const Box& a, const float4 lo, const float4 hi, float& dmin2, float& dmax2, float (&ext)[3]) {
     const float l[3] = {lo.x, lo.y, lo.z}, h[3] = {hi.x, hi.y, hi.z};
     float mn = 0.f, mx = 0.f;
 #pragma unroll
@@ -168,6 +203,7 @@ LDDMM_D void box_dist2(const Box& a, const float4 lo, const float4 hi, float& dm
         const float f = fmaxf(h[j] - a.lo[j], a.hi[j] - l[j]);
         mn = fmaf(g, g, mn);
         mx = fmaf(f, f, mx);
+        ext[j] = f * (1.f + 1.f / 65536.f);
     }
     dmin2 = mn * (1.f - 1.f / 65536.f);
     dmax2 = mx * (1.f + 1.f / 65536.f);
@@ -184,21 +220,24 @@ LDDMM_D float warp_max(float v) {
     return v;
 }
 
-// max(w, |v|) that keeps a NaN
-template <class Real>
-LDDMM_D Real max_nan(Real w, Real v) {
-    const Real a = v < (Real)0 ? -v : v;
-    return (a > w || !(a == a)) ? a : w;
+LDDMM_D float lg_float(float v) { return log2f(v); }
+LDDMM_D float lg_float(double v) {   // (log2 of the FP32 part and the exponent: a few 2^-24)
+    if (!(v > 0.0)) return -INFINITY;
+    if (!(v < INFINITY)) return (float)v;
+    int e;
+    const double m = frexp(v, &e);
+    return log2f((float)m) + (float)e;
 }
 
-// The box of a fold of packed source records and log2 of the sum of its
-// weights, written to boxes[2 fold] = (lo, lgw), boxes[2 fold + 1] = (hi, 0).
-// Called by whole warps, lane i holding record `row` = 32 fold + i; `valid`:
-// a real record (padding has none), p its packed position, w >= 0 its weight.
-// A non-finite value makes lgw +inf: such a fold is never passed over.
-template <class Real>
-LDDMM_D void store_fold_box(float4* boxes, long long row, bool valid, const Real* p, Real w) {
-    float lo[3], hi[3];
+// The box of a fold of packed source records and log2 of the sums of its weights by
+// column (see fold_box_words).  Called by whole warps, lane i holding record `row` = 32
+// fold + i; `valid`: a real record (padding has none), p its packed position, w[0..nw)
+// its values (nw <= NW).  A non-finite value makes all lgw +inf: such a fold is never
+// passed over.
+template <class Real, int NW>
+LDDMM_D void store_fold_box(float4* boxes, long long row, bool valid, const Real* p, const Real* w, int nw) {
+    constexpr int WORDS = fold_box_words(NW);
+    float lo[3], hi[3], lg[4 * WORDS - 6];
     bool bad = false;
 #pragma unroll
     for (int j = 0; j < 3; ++j) {
@@ -212,15 +251,29 @@ LDDMM_D void store_fold_box(float4* boxes, long long row, bool valid, const Real
         lo[j] = warp_min(valid ? lo[j] : INFINITY);
         hi[j] = warp_max(valid ? hi[j] : -INFINITY);
     }
-    bad = bad || !(w < (Real)INFINITY);
-    Real sum = valid ? w : (Real)0;
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+    for (int c = 0; c < 4 * WORDS - 6; ++c) {
+        lg[c] = -INFINITY;
+        if (c < NW && c < nw) {
+            const Real v = w[c] < (Real)0 ? -w[c] : w[c];
+            bad = bad || !(v < (Real)INFINITY);
+            Real sum = valid ? v : (Real)0;
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+            lg[c] = lg_float(sum);
+        }
+    }
     const bool any = __any_sync(0xffffffffu, valid && bad);
     if ((threadIdx.x & 31) == 0) {
-        const float lgw = any ? INFINITY : (sizeof(Real) == 4 ? log2f((float)sum) : (float)log2((double)sum));
-        boxes[2 * (row / kFold)] = make_float4(lo[0], lo[1], lo[2], lgw);
-        boxes[2 * (row / kFold) + 1] = make_float4(hi[0], hi[1], hi[2], 0.f);
+        const int words = fold_box_words(nw);
+        float4* o = boxes + words * (row / kFold);
+#pragma unroll
+        for (int c = 0; c < 4 * WORDS - 6; ++c) lg[c] = any ? INFINITY : lg[c];
+        o[0] = make_float4(lo[0], lo[1], lo[2], lg[0]);
+        o[1] = make_float4(hi[0], hi[1], hi[2], lg[1]);
+#pragma unroll
+        for (int k = 2; k < WORDS; ++k)
+            if (k < words) o[k] = make_float4(lg[4 * k - 6], lg[4 * k - 5], lg[4 * k - 4], lg[4 * k - 3]);
     }
 }
 
@@ -287,8 +340,9 @@ __global__ void __launch_bounds__(32 * kSweepWarps, op_min_blocks<Op>())
     constexpr int RING = kSweepWarps * STAGES * STAGE;
     constexpr int RED = (GT * NOUT * 8 + 15) / 16;
     __shared__ __align__(16) float4 smem[RING > RED ? RING : RED];
-    __shared__ float sbox[kSweepWarps][7];
-    __shared__ Box wbox;   // the group's box
+    __shared__ Box wbox;                                             // the group's box
+    __shared__ float sthr[kSweepWarps][8], sthr_w[kSweepWarps][8];   // log2 of what a fold may add, by bound
+    __shared__ unsigned slive_w[kSweepWarps];
 
     const int item = blockIdx.x;
     const SegDesc sg = find_segment(grid, item);
@@ -303,109 +357,198 @@ __global__ void __launch_bounds__(32 * kSweepWarps, op_min_blocks<Op>())
     static_assert(R % TPS == 0, "R must be a multiple of TPS");
     __shared__ int srow[GT];
     typename Op::Tgt tg[SLOTS];
-    {
-        int row[R];
+    unsigned valid = 0;   // which of the rows are targets
+    int row[R];
 #pragma unroll
-        for (int q = 0; q < R; ++q) {
-            const int r = tb * GT + q * 32 + lane;
-            row[q] = sg.perm != nullptr ? sg.perm[r] : r;
-            if (warp == 0) srow[q * 32 + lane] = row[q];
-        }
+    for (int q = 0; q < R; ++q) {
+        const int r = tb * GT + q * 32 + lane;
+        row[q] = sg.perm != nullptr ? sg.perm[r] : r;
+        if (warp == 0) srow[q * 32 + lane] = row[q];
+        if (row[q] < sg.n_tgt) valid |= 1u << q;
+    }
+    const int n_folds = sg.n_folds;
+
+    // source words: Op lays a record out as NS planes of 16-byte words, plane
+    // p of record j at P.src4[p * P.src_stride + j]; a fold's stage is plane-major
+    float4* ring = smem + warp * STAGES * STAGE;
+    auto load_fold = [&](int f, int st) {
+        if (f >= 0) {
+            const float4* g = P.src4 + sg.src + (long long)f * kFold + lane;
 #pragma unroll
-        for (int q = 0; q < SLOTS; ++q) {
-            if constexpr (TPS == 1) Op::load_target(P, sg.tgt + row[q], tg[q]);
-            else Op::load_target(P, sg.tgt + row[q * TPS], sg.tgt + row[q * TPS + 1], tg[q]);
+            for (int w = 0; w < NS; ++w) cp_async16(ring + st * STAGE + w * kFold + lane, g + (long long)w * P.src_stride);
         }
+        cp_async_commit();
+    };
+
+    // far folds: a fold of the group's own rows, another one for each warp where it has as many
+    const bool bounded = op_culls<Op>::value && boxes != nullptr && n_folds > kBoundFolds;
+    int own_fold = -1;
+    if (bounded && sg.self) {
+        int own = -1;
+#pragma unroll
+        for (int q = 0; q < R; ++q)
+            if (q == warp % R && (valid & (1u << q))) own = row[q];
+        own = __shfl_sync(0xffffffffu, own, warp / R * 16 % 32);
+        if (own < 0) own = __shfl_sync(0xffffffffu, row[0], 0);   // (a group has one target at least)
+        own_fold = min(own / kFold, n_folds - 1);
+        load_fold(own_fold, 0);
+    }
+#pragma unroll
+    for (int q = 0; q < SLOTS; ++q) {
+        if constexpr (TPS == 1) Op::load_target(P, sg.tgt + row[q], tg[q]);
+        else Op::load_target(P, sg.tgt + row[q * TPS], sg.tgt + row[q * TPS + 1], tg[q]);
     }
     typename Op::Acc acc[SLOTS];
 #pragma unroll
     for (int q = 0; q < SLOTS; ++q) acc[q].zero();
 
-    const int n_folds = sg.n_folds;
     int f_lo = 0, diag_hi = 0;   // SYM: own folds at or after diag_hi (and before sym_folds) count twice
     if constexpr (SYM) {
         f_lo = min(tb * (GT / kFold), sg.sym_folds);
         diag_hi = tb * (GT / kFold) + GT / kFold;
     }
 
-    // the group's box and the threshold below which a fold is passed over
-    float thr = 0.f;
+    // the group's box and, by bound, what a fold may add at most to be passed over
     bool cull = false;
+    constexpr int BW = fold_box_words(op_weights<Op>());
     const float4* fbox = nullptr;
     if constexpr (op_culls<Op>::value) {
-        if (boxes != nullptr) {
-            fbox = boxes + 2 * (sg.src / kFold);
+        if (bounded) {
+            fbox = boxes + BW * (sg.src / kFold);
             using Real = typename Op::Real;
-            float lo[3] = {INFINITY, INFINITY, INFINITY}, hi[3] = {-INFINITY, -INFINITY, -INFINITY};
+            constexpr int NB = Op::NB;
+            // every warp holds all targets of the group: the box needs no exchange
+            Box wb{{INFINITY, INFINITY, INFINITY}, {-INFINITY, -INFINITY, -INFINITY}};
             bool bad = false;
-            const int br = tb * GT + (int)threadIdx.x;
-            const int brow = threadIdx.x >= GT ? sg.n_tgt : sg.perm != nullptr ? sg.perm[br] : br;
-            if (brow < sg.n_tgt) {
-                Real x[3];
-                load_vals<Real, 3>(P.tgt4, P.tgt_stride, sg.tgt + brow, 0, x);
+#pragma unroll
+            for (int q = 0; q < R; ++q) {
+                if (!(valid & (1u << q))) continue;
 #pragma unroll
                 for (int j = 0; j < 3; ++j) {
+                    const Real x = Op::coord(tg[q / TPS], q % TPS, j);
+                    float l, h;
                     if constexpr (sizeof(Real) == 4) {
-                        lo[j] = hi[j] = x[j];
+                        l = h = x;
                     } else {
-                        lo[j] = __double2float_rd(x[j]);
-                        hi[j] = __double2float_ru(x[j]);
+                        l = __double2float_rd(x);
+                        h = __double2float_ru(x);
                     }
-                    bad = bad || !(fabsf(lo[j]) < INFINITY) || !(fabsf(hi[j]) < INFINITY);
+                    bad = bad || !(fabsf(l) < INFINITY) || !(fabsf(h) < INFINITY);
+                    wb.lo[j] = fminf(wb.lo[j], l);
+                    wb.hi[j] = fmaxf(wb.hi[j], h);
                 }
             }
+            cull = !__any_sync(0xffffffffu, bad);
 #pragma unroll
             for (int j = 0; j < 3; ++j) {
-                lo[j] = warp_min(lo[j]);
-                hi[j] = warp_max(hi[j]);
+                wb.lo[j] = warp_min(wb.lo[j]);
+                wb.hi[j] = warp_max(wb.hi[j]);
             }
-            if (lane == 0) {
+            // a fold whose records the targets' sums are compared with: of the group's own rows, or else
+            // the one that adds most by its box, of 512 spread over the range (each warp its share)
+            int bf = own_fold;
+            if (!sg.self) {
+                constexpr int PER = 4, LANES = 32 * kSweepWarps;
+                const int step = (n_folds + PER * LANES - 1) / (PER * LANES);
+                float best = -INFINITY;
+                float4 bx[PER][BW];
+                int fs[PER];
 #pragma unroll
-                for (int j = 0; j < 3; ++j) {
-                    sbox[warp][j] = lo[j];
-                    sbox[warp][3 + j] = hi[j];
-                }
-            }
-            cull = !__syncthreads_or(bad);
-            Box wb;
+                for (int k = 0; k < PER; ++k) {   // all loads before the first use
+                    fs[k] = min((k * LANES + (int)threadIdx.x) * step, n_folds - 1);
 #pragma unroll
-            for (int j = 0; j < 3; ++j) {
-                wb.lo[j] = sbox[0][j];
-                wb.hi[j] = sbox[0][3 + j];
-                for (int w = 1; w < kSweepWarps; ++w) {
-                    wb.lo[j] = fminf(wb.lo[j], sbox[w][j]);
-                    wb.hi[j] = fmaxf(wb.hi[j], sbox[w][3 + j]);
+                    for (int w = 0; w < BW; ++w) bx[k][w] = fbox[BW * fs[k] + w];
+                }
+#pragma unroll
+                for (int k = 0; k < PER; ++k) {
+                    float d0, d1, ext[3];
+                    box_dist2(wb, bx[k][0], bx[k][1], d0, d1, ext);
+                    float lw = fmaxf(bx[k][0].w, bx[k][1].w);
+#pragma unroll
+                    for (int w = 2; w < BW; ++w)
+                        lw = fmaxf(lw, fmaxf(fmaxf(bx[k][w].x, bx[k][w].y), fmaxf(bx[k][w].z, bx[k][w].w)));
+                    const float v = lw + Op::lgk(P, d1);
+                    if (lw < INFINITY && v > best) {
+                        best = v;
+                        bf = fs[k];
+                    }
+                }
+                const float top = warp_max(best);
+                bf = __reduce_max_sync(0xffffffffu, best == top ? bf : -1);
+                if (bf >= 0) load_fold(bf, 0);
+            }
+            // the targets' sums of absolute terms over a quarter of its records: what their sums over all
+            // sources hold at least; the least over the group, 0 where nothing may be passed over
+            Real least[NB];
+#pragma unroll
+            for (int b = 0; b < NB; ++b) least[b] = (Real)INFINITY;
+            unsigned live = 0;
+            if (bf >= 0) {
+                cp_async_wait<0>();
+                __syncwarp();
+                typename Op::Abs sum[SLOTS];
+#pragma unroll
+                for (int q = 0; q < SLOTS; ++q) sum[q].zero();
+#pragma unroll 2
+                for (int j = warp; j < kFold; j += kSweepWarps) {
+                    typename Op::Src s;
+                    Op::load_source(ring, j, s);
+#pragma unroll
+                    for (int q = 0; q < SLOTS; ++q) Op::pair(P, tg[q], s, sum[q]);
+                }
+                __syncwarp();
+#pragma unroll
+                for (int q = 0; q < R; ++q) {
+                    if (!(valid & (1u << q))) continue;
+                    Real a[NOUT], lo[NB], norm1 = 0;
+#pragma unroll
+                    for (int c = 0; c < NOUT; ++c) {
+                        a[c] = sum[q / TPS].value(c, q % TPS);
+                        if constexpr (op_has_out_scale<Op>::value) a[c] *= (Real)Op::out_scale(c);
+                    }
+                    if constexpr (Op::DOT > 0) {
+#pragma unroll
+                        for (int w = 0; w < Op::DOT; ++w) {
+                            const Real u = Op::dot_val(tg[q / TPS], q % TPS, w);
+                            norm1 += u < (Real)0 ? -u : u;
+                            if (u != (Real)0) live |= 1u << w;
+                        }
+                    }
+                    Op::lower(tg[q / TPS], q % TPS, a, norm1, lo);
+#pragma unroll
+                    for (int b = 0; b < NB; ++b) {
+                        if (lo[b] == (Real)-1) continue;
+                        if (!(lo[b] < least[b])) lo[b] = lo[b] < (Real)INFINITY ? least[b] : (Real)0;
+                        least[b] = lo[b];
+                    }
                 }
             }
-            // L from at most kLSamples folds spread over the range and the group's own rows (any fold
-            // gives a valid lower bound; the nearest heavy one gives a good one)
-            constexpr int kLSamples = 512;
-            float lgl = -INFINITY;
-            const int step = max(1, n_folds / kLSamples);
-            for (int f = threadIdx.x * step; f < n_folds; f += 32 * kSweepWarps * step) {
-                float d0, d1;
-                const float4 bl = fbox[2 * f];
-                box_dist2(wb, bl, fbox[2 * f + 1], d0, d1);
-                if (bl.w < INFINITY) lgl = fmaxf(lgl, bl.w + Op::lgk(P, d1));
+#pragma unroll
+            for (int b = 0; b < NB; ++b) {
+                float l = bf >= 0 ? lg_float(least[b]) : -INFINITY;
+                l = warp_min(l);
+                if (lane == 0) sthr_w[warp][b] = l;
             }
-            {
-                const int f = lane == 0 && brow < sg.n_tgt ? brow / kFold : n_folds;
-                if (step > 1 && f < n_folds) {
-                    float d0, d1;
-                    const float4 bl = fbox[2 * f];
-                    box_dist2(wb, bl, fbox[2 * f + 1], d0, d1);
-                    if (bl.w < INFINITY) lgl = fmaxf(lgl, bl.w + Op::lgk(P, d1));
-                }
+            if constexpr (Op::DOT > 0) {
+                live = __reduce_or_sync(0xffffffffu, live);   // (the same in every warp that has a fold)
+                if (lane == 0) slive_w[warp] = live;
             }
-            lgl = warp_max(lgl);
-            if (lane == 0) sbox[warp][6] = lgl;
             if (threadIdx.x == 0) wbox = wb;
             __syncthreads();
-            for (int w = 0; w < kSweepWarps; ++w) lgl = fmaxf(lgl, sbox[w][6]);
-            constexpr float kMargin = sizeof(Real) == 4 ? 36.f : 58.f;
-            thr = lgl - kMargin - log2f((float)n_folds) - (SYM ? 1.f : 0.f);
+            if (lane < NB) {
+                float l = sthr_w[0][lane];
+                for (int w = 1; w < kSweepWarps; ++w) l = fmaxf(l, sthr_w[w][lane]);
+                constexpr float kMargin = sizeof(Real) == 4 ? 36.1f : 58.1f;
+                sthr[warp][lane] = fminf(l, FLT_MAX) - kMargin - log2f((float)n_folds) - (SYM ? 1.f : 0.f);
+            }
+            __syncwarp();
         }
     }
+    unsigned live = 0;   // columns of the inner product that some target of the group has
+    if constexpr (op_culls<Op>::value)
+        if constexpr (Op::DOT > 0)
+            if (cull)
+                for (int w = 0; w < kSweepWarps; ++w) live |= slive_w[w];
 
     // this warp's folds: f_lo + c, f_lo + c + C, ...; next() gives the next one that counts, -1 after the last
     const int C = sg.split * kSweepWarps;
@@ -418,12 +561,27 @@ __global__ void __launch_bounds__(32 * kSweepWarps, op_min_blocks<Op>())
             bool act = f < n_folds;
             if constexpr (op_culls<Op>::value) {
                 if (cull && act) {
-                    float d0, d1;
-                    const float4 bl = fbox[2 * f];
-                    box_dist2(wbox, bl, fbox[2 * f + 1], d0, d1);
-                    float u = bl.w + Op::lgk(P, d0);
-                    if (Op::GRADX) u += 0.5f * __log2f(fmaxf(1.f, d1));
-                    act = !(u <= thr);
+                    float d0, d1, ext[3], lgw[4 * BW - 6], u[Op::NB];
+                    const float4 bl = fbox[BW * f], bh = fbox[BW * f + 1];
+                    box_dist2(wbox, bl, bh, d0, d1, ext);
+                    lgw[0] = bl.w;
+                    lgw[1] = bh.w;
+#pragma unroll
+                    for (int k = 2; k < BW; ++k) {
+                        const float4 q = fbox[BW * f + k];
+                        lgw[4 * k - 6] = q.x, lgw[4 * k - 5] = q.y, lgw[4 * k - 4] = q.z, lgw[4 * k - 3] = q.w;
+                    }
+                    float lgv = -INFINITY;   // sum over the records of max |v_w| over the columns in use
+#pragma unroll
+                    for (int w = 0; w < Op::DOT; ++w)
+                        if (live & (1u << w)) lgv = fmaxf(lgv, lgw[w]);
+                    lgv += lg_columns(Op::DOT);
+#pragma unroll
+                    for (int j = 0; j < 3; ++j) ext[j] = __log2f(ext[j]);
+                    Op::upper(lgw, lgv, Op::lgk(P, d0), ext, u);
+                    act = !(lgw[0] < INFINITY);
+#pragma unroll
+                    for (int b = 0; b < Op::NB; ++b) act = act || !(u[b] <= sthr[warp][b]);
                 }
             }
             f_mask = __ballot_sync(0xffffffffu, act);
@@ -433,18 +591,6 @@ __global__ void __launch_bounds__(32 * kSweepWarps, op_min_blocks<Op>())
         const int b = __ffs(f_mask) - 1;
         f_mask &= f_mask - 1;
         return f_cur + b * C;
-    };
-
-    // source words: Op lays a record out as NS planes of 16-byte words, plane
-    // p of record j at P.src4[p * P.src_stride + j]; a fold's stage is plane-major
-    float4* ring = smem + warp * STAGES * STAGE;
-    auto load_fold = [&](int f, int st) {
-        if (f >= 0) {
-            const float4* g = P.src4 + sg.src + (long long)f * kFold + lane;
-#pragma unroll
-            for (int w = 0; w < NS; ++w) cp_async16(ring + st * STAGE + w * kFold + lane, g + (long long)w * P.src_stride);
-        }
-        cp_async_commit();
     };
 
     int fa = next(), fb = -1;   // the fold to do, and (three stages) the one after it
@@ -599,6 +745,19 @@ struct AccF32C {
     LDDMM_D void add(int c, float v) { p[c] += v; }
     LDDMM_D void fma(int c, float a, float b) { p[c] = fmaf(a, b, p[c]); }
     LDDMM_D double value(int c) const { return (double)s[c] + (double)e[c]; }
+};
+
+// Sums of the terms' absolute values (one target).
+template <class Real, int N>
+struct AccAbs {
+    Real a[N];
+    LDDMM_D void zero() {
+#pragma unroll
+        for (int c = 0; c < N; ++c) a[c] = 0;
+    }
+    LDDMM_D void add(int c, Real v) { a[c] += v < (Real)0 ? -v : v; }
+    LDDMM_D void fma(int c, Real x, Real y) { add(c, x * y); }
+    LDDMM_D Real value(int c, int) const { return a[c]; }
 };
 
 // Plain FP64 accumulation (the uncompensated FP64 comparator path).

@@ -26,7 +26,9 @@ struct SinglePlan {
     // chunk sums (doubles) of a sweep with an epilogue: none where a group has one chunk
     size_t part_doubles(int nout) const { return split > 1 ? (size_t)split * n_tpad * nout : 0; }
     size_t counters() const { return (size_t)n_tb + 1; }
-    size_t box_words() const { return 2 * (size_t)(m_pad / kFold); }   // float4 words of the fold boxes
+    // float4 words of the fold boxes
+    template <class Op>
+    size_t box_words() const { return (size_t)fold_box_words(op_weights<Op>()) * (size_t)(m_pad / kFold); }
 };
 
 template <class Op>
@@ -83,12 +85,13 @@ int launch_order_rows(const OrderRows& o, const float4* planes, long long n, lon
 
 // boxes: fold boxes written with the packed sources, or NULL (every fold counts).
 // SYM: symmetric sweep over sym_folds own folds (see sweep_kernel<Op, true>).
+// self: the first sources are the targets, in their order (a hint: see the far folds).
 // Epi: what is done with a group's sums; counters: n_tb + 1 zeros; perm: order of the
-// targets' sets of 32 rows, or NULL (see sweep_kernel).
+// target rows, or NULL (see sweep_kernel).
 template <class Op, bool SYM = false, class Epi = EpiNone>
 int launch_single(const SinglePlan& pl, long long n, const typename Op::Params& P, const float4* boxes, double* part,
                   cudaStream_t st, int sym_folds = 0, int* counters = nullptr, const Epi& E = Epi(),
-                  const int* perm = nullptr) {
+                  const int* perm = nullptr, bool self = true) {
     SweepGrid g{};
     g.seg0.n_tgt = (int)n;
     g.seg0.n_folds = pl.n_folds;
@@ -96,6 +99,7 @@ int launch_single(const SinglePlan& pl, long long n, const typename Op::Params& 
     g.seg0.split = pl.split;
     g.seg0.sym_folds = sym_folds;
     g.seg0.perm = perm;
+    g.seg0.self = self;
     g.nseg = 0;
     g.n_items = pl.n_tb * pl.split;
     if (g.n_items <= 0) return LDDMM_OK;
@@ -105,8 +109,6 @@ int launch_single(const SinglePlan& pl, long long n, const typename Op::Params& 
             return cuda_check(cudaGetLastError(), "sweep launch");
         }
     }
-    // up to 1,024 sources no warp has more than a few folds: bounding them costs more than it saves
-    if (pl.n_folds <= 32) boxes = nullptr;
     sweep_kernel<Op, SYM, Epi><<<g.n_items, 32 * kSweepWarps, 0, st>>>(g, P, boxes, part, counters, E);
     return cuda_check(cudaGetLastError(), "sweep launch");
 }
