@@ -18,8 +18,8 @@
 //
 // FP64 sweeps: the same base-2 frame and exponential exp2neg below, with the
 // zero-distance branch kept as in the Fortran.  FP64 sums that keep the
-// reference's order to the bit (single-cluster kernels, sums over fewer than
-// 512 sources; LIB): x' = x/s, u = |x'-y'|^2 (Gaussian) or |x'-y'| (Laplacian)
+// reference's order to the bit (single-cluster kernels, sums over at most 384
+// sources; LIB): x' = x/s, u = |x'-y'|^2 (Gaussian) or |x'-y'| (Laplacian)
 // and exp() from the CUDA math library.
 #pragma once
 #include "common.cuh"

@@ -677,12 +677,13 @@ __global__ void __launch_bounds__(32 * kSweepWarps, op_min_blocks<Op>())
     }
 }
 
-// FP64 sums over at most kSeqFolds folds: one thread per target adds all sources
-// in their order, as the reference's loop does.  An optimiser run on a few
-// hundred points amplifies the last bits of its FP64 sums by 1e7 over 50
-// iterations, so these keep the reference's order to the bit; the sums are too
-// small for the split of the sweep above to gain anything.
-constexpr int kSeqFolds = 15;
+// FP64 sums over at most kSeqFolds folds (384 sources): one thread per target adds all
+// sources in their order, as the reference's loop does.  An optimiser run on a few
+// hundred points amplifies the last bits of its FP64 sums by 1e7 over 50 iterations, so
+// these keep the reference's order to the bit.  A thread's chain of 480 terms takes
+// 64-73 us however many targets there are, the split sweep 18 us (64 x 480 points,
+// B200), so the line is where the longest such chain was before there was a choice.
+constexpr int kSeqFolds = 12;
 template <class Op, class Epi>
 __global__ void __launch_bounds__(op_group<Op>()) sweep_seq_kernel(const SegDesc sg, const typename Op::Params P,
                                                                    double* part, const Epi E) {
