@@ -109,6 +109,7 @@ struct OpData {
     using Real = Real_;
     using L = DataLayout<MODE, D>;
     static constexpr bool F32 = sizeof(Real) == 4;
+    static constexpr int FAMILY = KIND;
     static constexpr int TPS = 1;
     static constexpr int R = 2;
     static constexpr int PP = PointPlanes<Real>::N;

@@ -66,6 +66,7 @@ template <class Real_, int KIND, int DEG, int D, int DIMB, bool SMALL = false>
 struct OpApplyK {
     using Real = Real_;
     static constexpr bool F32 = sizeof(Real) == 4;
+    static constexpr int FAMILY = KIND;
     static constexpr int TPS = 1;
     static constexpr int R = (F32 && !SMALL) ? 4 : 2;
     static constexpr int PP = PointPlanes<Real>::N;
@@ -121,6 +122,7 @@ template <class Real_, int KIND, int DEG, int D, int W>
 struct OpDiffKT {
     using Real = Real_;
     static constexpr bool F32 = sizeof(Real) == 4;
+    static constexpr int FAMILY = KIND;
     static constexpr int TPS = 1;
     static constexpr int R = 2;
     static constexpr int PP = PointPlanes<Real>::N;
@@ -184,6 +186,7 @@ template <class Real_, int KIND, int DEG, int D>
 struct OpDivergence {
     using Real = Real_;
     static constexpr bool F32 = sizeof(Real) == 4;
+    static constexpr int FAMILY = KIND;
     static constexpr int TPS = 1;
     static constexpr int R = 4;
     static constexpr int PP = PointPlanes<Real>::N;

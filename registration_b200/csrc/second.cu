@@ -75,6 +75,7 @@ struct OpSecond {
     using Real = Real_;
     using L = SecondLayout<MODE, D>;
     static constexpr bool F32 = sizeof(Real) == 4;
+    static constexpr int FAMILY = KIND;
     static constexpr int TPS = 1;
     static constexpr int R = 2;
     static constexpr int PP = PointPlanes<Real>::N;

@@ -522,6 +522,7 @@ template <class Real_, int KIND, int PDEG, int QDEG, int D>
 struct OpEPDiff {
     using Real = Real_;
     static constexpr bool F32 = sizeof(Real) == 4;
+    static constexpr int FAMILY = KIND;
     static constexpr int TPS = 1;
     static constexpr int R = 2;
     static constexpr int PP = PointPlanes<Real>::N;

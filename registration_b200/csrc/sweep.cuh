@@ -141,6 +141,9 @@ struct op_has_min_blocks<Op, std::void_t<decltype(Op::MIN_BLOCKS)>> : std::true_
 //     2.18, Laplacian 1.67 -> 1.72, adjoint 1.73 -> 1.74
 //   FP64, 8 / 16 / 32 sources: applyK 0.646 / 0.658 / 0.653, varifold gradient
 //     0.424 / 0.428 / 0.333
+//   FP64 Laplacian, whose square roots each carry a rare branch, 2 / 4 / 8 / 16 sources
+//     at 40,000: applyK 0.323 / 0.327 / 0.325 / 0.278, applyDiffKT 0.306 / 0.308 /
+//     0.305 / 0.255, divergence 0.348 / 0.348 / 0.320 / 0.222 (5 to 8 blocks: less)
 // Operators with many outputs or wide records keep 168 registers as well.
 template <class Op>
 constexpr int op_min_blocks() {
@@ -149,7 +152,10 @@ constexpr int op_min_blocks() {
     else return Op::NOUT > 4 || Op::NS > 5 ? 3 : 4;
 }
 template <class Op>
-constexpr int op_unroll() { return sizeof(typename Op::Real) == 4 ? kFold : kFold / 2; }
+constexpr int op_unroll() {
+    if constexpr (sizeof(typename Op::Real) == 4) return kFold;
+    else return Op::FAMILY == KLAP ? 4 : kFold / 2;
+}
 
 // Operators that can pass over far folds.  They give, with h the half of a packed slot:
 //   NW               weight columns of a source record that bound its terms
