@@ -45,8 +45,10 @@ int occupancy_blocks(const void* kernel, int block, size_t dyn_smem = 0);
 // of 32 sources; `resident` blocks fit the device at once, a block's four warps
 // share the folds of its chunk.  A function of the operator, the shape and the
 // SM count only (workspace queries run the same code).
-//   Many blocks (four waves and more): up to 64 blocks per SM, at least 16 folds
-// per warp, so that groups whose far folds are passed over balance out.
+//   Many blocks (four waves and more): up to 64 blocks per SM, at least 32 folds
+// per warp, so that groups whose far folds are passed over balance out.  (With 16 every
+// group measures its bounds twice as often: FP64 varifold value of 20,480 cells 576 ->
+// 555 us, FP32c current gradient of 30,000 edges, nothing far, 971 -> 940 us.)
 //   Fewer: waves count.  The chunks that make ceil(blocks / resident) (folds per
 // warp + kBlockFolds) smallest, kBlockFolds being what a block's start and end
 // cost in folds (3,166 points, 11 / 8 / 5 chunks: 404 / 392 / 420 us per shot and
@@ -60,7 +62,7 @@ constexpr int kBlockFolds = 3;
 inline int choose_split(int n_tb, int n_folds, int sms, int resident, bool shared) {
     if (n_tb <= 0 || n_folds <= 0) return 1;
     const long long want = (64LL * sms + n_tb - 1) / n_tb;
-    const long long many = std::max(1LL, std::min<long long>(want, n_folds / (4 * (shared ? 8 : 16))));
+    const long long many = std::max(1LL, std::min<long long>(want, n_folds / (4 * (shared ? 8 : 32))));
     if (shared || many * n_tb >= 4LL * resident) return (int)many;
     // for each number of waves the most chunks that fit, then the fewest with as few folds per warp
     const long long cap = (n_folds + 3) / 4;
