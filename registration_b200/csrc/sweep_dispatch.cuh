@@ -72,10 +72,10 @@ inline OrderRows take_order_rows(Workspace& ws, const SinglePlan& pl) {
 template <class Real>
 int launch_order_rows(const OrderRows& o, const float4* planes, long long n, long long n_pad, cudaStream_t st) {
     if (o.perm == nullptr) return LDDMM_OK;
-    LDDMM_TRY(cuda_check(cudaMemsetAsync(o.hist, 0, sizeof(int) * kOrderCells, st), "order memset"));
+    LDDMM_TRY(cuda_check(cudaMemsetAsync(o.hist, 0, sizeof(int) * (2 * kOrderCells + 1), st), "order memset"));
     const int blocks = grid_for(n_pad);
     int* info = o.hist + 2 * kOrderCells;
-    order_extent_kernel<Real><<<1, 1024, 0, st>>>(planes, n_pad, n, info);
+    order_extent_kernel<Real><<<(blocks + 7) / 8, 256, 0, st>>>(planes, n_pad, n, info);
     order_cells_kernel<Real><<<blocks, 256, 0, st>>>(planes, n_pad, n, info, o.hist, o.cell);
     order_scan_kernel<<<1, 1024, 0, st>>>(o.hist, info);
     order_scatter_kernel<<<blocks, 256, 0, st>>>(o.cell, n, o.hist + kOrderCells, o.tmp);
