@@ -566,7 +566,7 @@ static __global__ void dt_pack_kernel(int norm, int grad, const double* __restri
             Real bp[3], bw[4];
             dt_pack_record<Real>(norm, grad, false, c, sv, d, first ? eps1 : eps2, first ? 1.0 : sign2, scale, center,
                                  src, sstride, i, splanes, sslots, list != 0, bp, bw);
-            store_fold_box<Real, 4>(boxes, i, c != nullptr, bp, bw, nw);
+            if (boxes != nullptr) store_fold_box<Real, 4>(boxes, i, c != nullptr, bp, bw, nw);
         }
     }
 }

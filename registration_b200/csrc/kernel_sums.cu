@@ -63,7 +63,7 @@ int applyk_group(const ApplyKArgs& a, int col0, Workspace& ws, cudaStream_t st) 
     const SinglePlan pl = plan_single<Op>(a.n, a.m, a.split_cap);
     float4* tgt = ws.take<float4>((size_t)Op::PP * pl.n_tpad);
     float4* src = ws.take<float4>((size_t)Op::NS * pl.m_pad);
-    float4* boxes = ws.take<float4>(pl.box_words<Op>());
+    float4* boxes = pl.take_boxes<Op>(ws);
     double* part = ws.take<double>(pl.part_doubles(DIMB));
     int* counters = ws.take<int>(pl.split > 1 ? pl.counters() : 0);
     // sums over the targets' own points (the query cannot know: room for the order whenever n == m)
@@ -203,7 +203,7 @@ int difft_impl(const DiffKTArgs& a, Workspace& ws, cudaStream_t st) {
     const SinglePlan pl = plan_single<Op>(a.n, a.m);
     float4* tgt = ws.take<float4>((size_t)NT * pl.n_tpad);
     float4* src = ws.take<float4>((size_t)Op::NS * pl.m_pad);
-    float4* boxes = ws.take<float4>(pl.box_words<Op>());
+    float4* boxes = pl.take_boxes<Op>(ws);
     double* part = ws.take<double>(pl.part_doubles(D));
     int* counters = ws.take<int>(pl.counters());
     const Ordered64 both = take_ordered64<Op>(ws, pl, a.n, a.m);

@@ -181,6 +181,9 @@ LDDMM_D void put_plain(float4* planes, long long stride, long long i, const floa
     }
 }
 
+// whether the sweep bounds the segment's folds (sweep_kernel)
+LDDMM_D bool rag_bounded(const RagSeg& g) { return g.spad > (long long)kBoundFolds * kFold; }
+
 // fold box of a packed source row: position v[0..D), values v[D..NV) (whole warps: segments are padded to folds)
 template <int D, int NV>
 LDDMM_D void rag_box(float4* boxes, long long row, bool valid, const float* v) {
@@ -209,7 +212,7 @@ LDDMM_D void rag_shoot_row(const RagSeg& g, long long i, const double* x, const 
     if (i < g.tpad) put_plain(p.tgt, tstride, g.tgt + i, pos, 3, 1);
     if (i < g.spad) {
         put_plain(p.src, sstride, g.src + i, vals, 2 * D, (2 * D + 3) / 4);
-        rag_box<D, 2 * D>(p.boxes, g.src + i, x != nullptr, vals);
+        if (rag_bounded(g)) rag_box<D, 2 * D>(p.boxes, g.src + i, x != nullptr, vals);
     }
 }
 
@@ -371,7 +374,7 @@ LDDMM_D void rag_cov_row(const RagSeg& g, long long i, const double* x, const do
     }
     if (i < g.spad) {
         put_plain(pl.src, sstride, g.src + i, v, 3 * D, (3 * D + 3) / 4);
-        rag_box<D, 3 * D>(pl.boxes, g.src + i, x != nullptr, v);
+        if (rag_bounded(g)) rag_box<D, 3 * D>(pl.boxes, g.src + i, x != nullptr, v);
     }
 }
 
@@ -522,7 +525,7 @@ static __global__ void rag_applyk_pack_kernel(const RagSeg* __restrict__ segs, c
                 for (int c = 0; c < dimb && c < DIMB; ++c) v[D + c] = (float)beta[(g.m0 + i) * dimb + c];
             }
             put_plain(src, sstride, g.src + i, v, D + DIMB, (D + DIMB + 3) / 4);
-            rag_box<D, D + DIMB>(boxes, g.src + i, i < g.m, v);
+            if (rag_bounded(g)) rag_box<D, D + DIMB>(boxes, g.src + i, i < g.m, v);
         }
     }
 }
@@ -630,7 +633,7 @@ static __global__ void rag_dt_pack_kernel(const RagSeg* __restrict__ segs, const
             Real bp[3], bw[4];
             dt_pack_record<Real>(norm, grad, false, c, sv, d, first ? eps1 : eps2, first ? 1.0 : sign2, g.scale,
                                  g.center, src, sstride, g.src + i, splanes, sslots, list != 0, bp, bw);
-            store_fold_box<Real, 4>(boxes, g.src + i, c != nullptr, bp, bw, nw);
+            if (rag_bounded(g)) store_fold_box<Real, 4>(boxes, g.src + i, c != nullptr, bp, bw, nw);
         }
     }
 }

@@ -84,6 +84,7 @@ LDDMM_D void store_list(float4* planes, long long stride, long long i, const dou
 template <class Real, int NW>
 LDDMM_D void store_box(float4* boxes, long long i, bool valid, const double* x, const double* v, int nv, int nw, int d,
                        double s, const double* c) {
+    if (boxes == nullptr) return;
     Real p[3] = {0, 0, 0}, w[NW];
     if (valid)
         for (int j = 0; j < d; ++j) p[j] = (Real)((x[j] - c[j]) * s);
@@ -227,7 +228,7 @@ int shoot_impl(const ShootArgs& a, Workspace& ws, cudaStream_t st) {
     for (StepPlanes& p : pn) {
         p.tgt = ws.take<float4>((size_t)Op::PP * pl.n_tpad);
         p.src = ws.take<float4>((size_t)Op::NS * pl.m_pad);
-        p.boxes = ws.take<float4>(pl.box_words<Op>());
+        p.boxes = pl.take_boxes<Op>(ws);
     }
     double* part = ws.take<double>(pl.part_doubles(D));
     int* counters = ws.take<int>(pl.counters());
@@ -353,6 +354,7 @@ LDDMM_D void cov_store(float4* tgt, long long tstride, float4* src, long long ss
 template <class Real>
 LDDMM_D void cov_box(float4* boxes, long long i, bool valid, const double* x, const double* a, const double* p, int d,
                      double s, const double* c, int tw) {
+    if (boxes == nullptr) return;
     double v[6] = {0, 0, 0, 0, 0, 0};
     for (int j = 0; j < d && valid; ++j) {
         v[j] = a[j];
@@ -451,7 +453,7 @@ int cov_impl(const CovArgs& a, Workspace& ws, cudaStream_t st) {
     for (StepPlanes& p : pn) {
         p.tgt = ws.take<float4>((size_t)NT * pl.n_tpad);
         p.src = ws.take<float4>((size_t)Op::NS * pl.m_pad);
-        p.boxes = ws.take<float4>(pl.box_words<Op>());
+        p.boxes = pl.take_boxes<Op>(ws);
     }
     double* part = ws.take<double>(pl.part_doubles(D));
     int* counters = ws.take<int>(pl.counters());
