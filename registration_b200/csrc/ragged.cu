@@ -44,8 +44,6 @@ struct RagSeg {
     long long tgt;       // first packed target row
     long long src;       // first packed source row
     long long tpad, spad;  // packed rows of this segment (targets, sources)
-    long long part;      // first row of the partial-sum buffer
-    int split;
     int nb;              // target groups of this segment (one energy partial each)
     long long eoff;      // first energy partial of this segment
     double scale;        // coordinate prescale
@@ -84,14 +82,12 @@ RagPlan<Op> rag_plan(const std::vector<long long>& n, const std::vector<long lon
         g.src = p.ss;
         g.tpad = pl.n_tpad;
         g.spad = pl.m_pad;
-        g.part = p.parts;
-        g.split = pl.split;
         g.nb = pl.n_tb;
         g.eoff = p.eparts;
         SegDesc& d = p.desc[s];
         d.tgt = g.tgt;
         d.src = g.src;
-        d.part = g.part;
+        d.part = p.parts;
         d.n_tgt = (int)n[s];
         d.n_folds = pl.n_folds;
         d.n_tb = pl.n_tb;
@@ -216,7 +212,7 @@ LDDMM_D void rag_shoot_row(const RagSeg& g, long long i, const double* x, const 
     }
 }
 
-// planes of step 0, the padding of both sets
+// planes of step 0, the padding of both sets (the epilogue writes the folds that hold real rows)
 template <int D>
 static __global__ void rag_shoot_pack_kernel(const RagSeg* __restrict__ segs, const long long* __restrict__ padoff,
                                              int nseg, const double* __restrict__ xt, const double* __restrict__ at,
@@ -231,7 +227,7 @@ static __global__ void rag_shoot_pack_kernel(const RagSeg* __restrict__ segs, co
         const double* x = i < g.n ? xt + ((long long)(T + 1) * g.row0 + i) * d : nullptr;
         const double* a = i < g.n ? at + ((long long)T * g.row0 + i) * d : nullptr;
         rag_shoot_row<D>(g, i, x, a, d, p0, tstride, sstride);
-        rag_shoot_row<D>(g, i, x, a, d, p1, tstride, sstride);
+        if (i >= (g.n & ~31LL)) rag_shoot_row<D>(g, i, nullptr, nullptr, d, p1, tstride, sstride);
     }
 }
 
@@ -378,7 +374,7 @@ LDDMM_D void rag_cov_row(const RagSeg& g, long long i, const double* x, const do
     }
 }
 
-// planes of step T-1, the padding of both sets
+// planes of step T-1, the padding of both sets (the epilogue writes the folds that hold real rows)
 template <int D>
 static __global__ void rag_cov_pack_kernel(const RagSeg* __restrict__ segs, const long long* __restrict__ padoff,
                                            int nseg, const double* __restrict__ xt, const double* __restrict__ at,
@@ -397,7 +393,7 @@ static __global__ void rag_cov_pack_kernel(const RagSeg* __restrict__ segs, cons
             p = pxt + (((long long)(T + 1) * g.row0 + (long long)T * g.n + i) * d);
         }
         rag_cov_row<D>(g, i, x, a, p, d, p0, tstride, sstride);
-        rag_cov_row<D>(g, i, x, a, p, d, p1, tstride, sstride);
+        if (i >= (g.n & ~31LL)) rag_cov_row<D>(g, i, nullptr, nullptr, nullptr, d, p1, tstride, sstride);
     }
 }
 
