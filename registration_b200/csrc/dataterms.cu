@@ -96,7 +96,7 @@ int dt_sweep(const DataArgs& a, Workspace& ws, cudaStream_t st, const double* c1
     }
 }
 
-// SMALL: the small groups of OpApplyK (few target cells); the other operators have one shape.
+// SMALL: the small groups of the FP32 OpApplyK (few target cells); the other operators have one shape.
 template <class Real, int KIND, int PDEG, int QDEG, int D, bool SMALL = false>
 int dt_impl(const DataArgs& a, Workspace& ws, cudaStream_t st) {
     constexpr int PW = Traits<Real>::PER_WORD;
@@ -117,10 +117,10 @@ int dt_impl(const DataArgs& a, Workspace& ws, cudaStream_t st) {
                                                PP + (3 + PW - 1) / PW>>;
             LDDMM_TRY((dt_sweep<Op, Real, false>(a, ws, st, c1, s1, ks, center, nullptr, nullptr)));
         } else if (a.norm == NCURRENT) {
-            using Op = DtOp<OpApplyK<Real, KIND, PDEG, D, D, SMALL>, 0, D, PP>;
+            using Op = DtOp<OpApplyK<Real, KIND, PDEG, D, D, SMALL && sizeof(Real) == 4>, 0, D, PP>;
             LDDMM_TRY((dt_sweep<Op, Real, false>(a, ws, st, c1, s1, ks, center, nullptr, nullptr)));
         } else {
-            using Op = DtOp<OpApplyK<Real, KIND, PDEG, D, 1, SMALL>, 0, 1, PP>;
+            using Op = DtOp<OpApplyK<Real, KIND, PDEG, D, 1, SMALL && sizeof(Real) == 4>, 0, 1, PP>;
             LDDMM_TRY((dt_sweep<Op, Real, false>(a, ws, st, c1, s1, ks, center, nullptr, nullptr)));
         }
     }

@@ -222,7 +222,7 @@ static __global__ void trial_momenta_kernel(const double* __restrict__ at, const
 template <class Real, int KIND, int DEG, int D, bool SMALL = false>
 int shoot_impl(const ShootArgs& a, Workspace& ws, cudaStream_t st) {
     constexpr bool LIST = sizeof(Real) == 4;  // FP32: packed-pair operator with list records
-    using Op = std::conditional_t<LIST, OpApplyK2<KIND, DEG, D, D, SMALL>, OpApplyK<Real, KIND, DEG, D, D, SMALL>>;
+    using Op = std::conditional_t<LIST, OpApplyK2<KIND, DEG, D, D, SMALL>, OpApplyK<Real, KIND, DEG, D, D>>;
     const SinglePlan pl = plan_single<Op>(a.n, a.n);
     StepPlanes pn[2];
     for (StepPlanes& p : pn) {
