@@ -7,7 +7,7 @@
 //   K = P_p(u) e^-u, K' = -Q_p(u) e^-u / (2 s^2), u = |x-y|/s          (:41-47, :101-107)
 // with the polynomial tables c_ (P) and c1_ (Q).  Constant factors
 // (-1/(2 s^2), the 2 of the gradient and the coordinate prescale) are applied
-// once per target in the combine step, not per pair.
+// once per target when its sums are written, not per pair.
 //
 // FP32 prescaling (done when points are packed):
 //   Gaussian:  x' = x * sqrt(log2(e)/2)/s  ->  K  = 2^(-|x'-y'|^2)

@@ -116,7 +116,7 @@ struct OpApplyK {
 };
 
 // ---------------------------------------------------------------------------
-// f_k = sum_l K'(x_k,y_l) 2 (x_k - y_l) <u_k, v_l>     (up to the combine scale)
+// f_k = sum_l K'(x_k,y_l) 2 (x_k - y_l) <u_k, v_l>     (up to the epilogue's scale)
 // ---------------------------------------------------------------------------
 template <class Real_, int KIND, int DEG, int D, int W>
 struct OpDiffKT {
@@ -179,7 +179,7 @@ struct OpDiffKT {
 };
 
 // ---------------------------------------------------------------------------
-// div_k = sum_l K'(x_k,y_l) 2 <x_k - y_l, a_l>      (up to the combine scale)
+// div_k = sum_l K'(x_k,y_l) 2 <x_k - y_l, a_l>      (up to the epilogue's scale)
 // py-lddmm/kernelFunctions.py:510-530 (applyDivergence)
 // ---------------------------------------------------------------------------
 template <class Real_, int KIND, int DEG, int D>

@@ -1,5 +1,5 @@
-// Packing kernels (FP64 user arrays -> prescaled FP32/FP64 planes) and the
-// deterministic combine of per-chunk partial sums.
+// Packing kernels (FP64 user arrays -> prescaled FP32/FP64 planes), the packing
+// centre, and the order of rows by cells.
 #pragma once
 #include "common.cuh"
 #include "ops.cuh"

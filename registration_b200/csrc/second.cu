@@ -15,7 +15,8 @@
 // reads c2_(ord-1,.) out of bounds for orders 0 and 1): those orders are
 // rejected, as order 0 is for the first-derivative loops.
 //
-// Same sweep as the kernel sums (tiled, chunked, deterministic combine) with
+// Same sweep as the kernel sums (folds, chunks; a combine kernel adds the chunks in
+// their order), every pair counted, with
 // FP32-compensated (_f32c) or FP64 (_f64) pair arithmetic on prescaled
 // coordinates x' = scale x:  K' 2 dx = dscale F dx',  K'' 4 <dx,v> dx =
 // d2scale G <dx',v> dx',  K' 2 = c1s F, with F = Q e, G = R e the polynomial

@@ -14,11 +14,11 @@
 //   <p_k,a_l> + <a_k,p_l> - 2 rw <a_k,a_l> = <p_k - 2 rw a_k, a_l> + <a_k, p_l>,
 // a 2d-wide dot (u_k = (p_k - 2 rw a_k, a_k), v_l = (a_l, p_l)).
 //
-// One time step = one sweep over (target block, source chunk) items + one
-// combine kernel that adds the chunks in a fixed order, applies the Euler (or
-// adjoint) update in FP64, writes the packed planes of the next step and the
-// step's energy partials (one per combine block; the grid size depends only on
-// n, so the reduction order is fixed).
+// One time step of a shot or adjoint = one sweep over (target group, source chunk)
+// items, whose epilogue adds a group's chunks in a fixed order, applies the Euler
+// (or adjoint) update in FP64 and writes the packed planes of the next step and the
+// step's energy partials (one per group, so the reduction order is fixed).  EPDiff
+// keeps a combine kernel per step.
 #include "dataterm_fused.cuh"
 #include "fused_small.cuh"
 #include "host.h"

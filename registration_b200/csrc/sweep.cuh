@@ -22,7 +22,8 @@
 // depend on scheduling.  The groups' counters start at zero and are left at
 // zero.  A separate combine launch per sweep cost 4-10 us of a shot's step at a
 // few thousand points (13 blocks, each thread adding its row's chunks one after
-// the other).  EpiNone leaves the chunk sums in `part`.
+// the other).  EpiNone leaves the chunk sums in `part`, chunk by chunk with seg.n_tgt
+// rows each.
 //
 // Far folds (operators with Op::lgk, `boxes` given, more than kBoundFolds folds).  The
 // pack kernels leave for each fold its bounding box and, by weight column, log2 of the
