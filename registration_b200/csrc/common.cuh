@@ -31,6 +31,7 @@ struct SegDesc {
                       // sum is symmetric in (target, source): see sweep_kernel<Op, true>
     int id;           // segment number (ragged launches)
     int self;         // the first sources are the targets, in their order
+    int bound;        // far folds are looked for (see sweep_kernel)
     int cnt;          // first counter of this segment's groups (see sweep_kernel)
     const int* perm;  // order of the target rows (n_tb * 32 R of them), or NULL: as they lie
 };

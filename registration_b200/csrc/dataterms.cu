@@ -71,7 +71,8 @@ int dt_sweep(const DataArgs& a, Workspace& ws, cudaStream_t st, const double* c1
     pl.seq = false;   // shapes of so few cells take the single-cluster kernels
     float4* tgt = ws.take<float4>((size_t)Op::NT_ * pl.n_tpad);
     float4* src = ws.take<float4>((size_t)Op::NS * pl.m_pad);
-    float4* boxes = pl.take_boxes<Op>(ws);
+    const bool packed = GRAD && sizeof(Real) == 4 && a.norm == NVARIFOLD;
+    float4* boxes = pl.take_boxes<Op>(ws, packed ? kBoundFoldsPacked : kBoundFolds);
     double* part = ws.take<double>(pl.part_doubles(Op::NOUT));
     int* counters = ws.take<int>(pl.counters());
     double* epart = ws.take<double>(GRAD ? 0 : pl.n_tb);

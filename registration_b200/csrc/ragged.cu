@@ -46,6 +46,7 @@ struct RagSeg {
     long long tpad, spad;  // packed rows of this segment (targets, sources)
     int nb;              // target groups of this segment (one energy partial each)
     long long eoff;      // first energy partial of this segment
+    int bound;           // far folds are looked for (fold boxes)
     double scale;        // coordinate prescale
     double dscale;       // derivative constant
     double center[3];
@@ -95,6 +96,7 @@ RagPlan<Op> rag_plan(const std::vector<long long>& n, const std::vector<long lon
         d.item0 = p.items;
         d.id = s;
         d.self = self;
+        d.bound = g.bound = pl.n_folds > kBoundFolds;
         d.cnt = (int)p.eparts;
         p.items += pl.n_tb * pl.split;
         p.tt += pl.n_tpad;
@@ -177,9 +179,6 @@ LDDMM_D void put_plain(float4* planes, long long stride, long long i, const floa
     }
 }
 
-// whether the sweep bounds the segment's folds (sweep_kernel)
-LDDMM_D bool rag_bounded(const RagSeg& g) { return g.spad > (long long)kBoundFolds * kFold; }
-
 // fold box of a packed source row: position v[0..D), values v[D..NV) (whole warps: segments are padded to folds)
 template <int D, int NV>
 LDDMM_D void rag_box(float4* boxes, long long row, bool valid, const float* v) {
@@ -208,7 +207,7 @@ LDDMM_D void rag_shoot_row(const RagSeg& g, long long i, const double* x, const 
     if (i < g.tpad) put_plain(p.tgt, tstride, g.tgt + i, pos, 3, 1);
     if (i < g.spad) {
         put_plain(p.src, sstride, g.src + i, vals, 2 * D, (2 * D + 3) / 4);
-        if (rag_bounded(g)) rag_box<D, 2 * D>(p.boxes, g.src + i, x != nullptr, vals);
+        if (g.bound) rag_box<D, 2 * D>(p.boxes, g.src + i, x != nullptr, vals);
     }
 }
 
@@ -370,7 +369,7 @@ LDDMM_D void rag_cov_row(const RagSeg& g, long long i, const double* x, const do
     }
     if (i < g.spad) {
         put_plain(pl.src, sstride, g.src + i, v, 3 * D, (3 * D + 3) / 4);
-        if (rag_bounded(g)) rag_box<D, 3 * D>(pl.boxes, g.src + i, x != nullptr, v);
+        if (g.bound) rag_box<D, 3 * D>(pl.boxes, g.src + i, x != nullptr, v);
     }
 }
 
@@ -521,7 +520,7 @@ static __global__ void rag_applyk_pack_kernel(const RagSeg* __restrict__ segs, c
                 for (int c = 0; c < dimb && c < DIMB; ++c) v[D + c] = (float)beta[(g.m0 + i) * dimb + c];
             }
             put_plain(src, sstride, g.src + i, v, D + DIMB, (D + DIMB + 3) / 4);
-            if (rag_bounded(g)) rag_box<D, D + DIMB>(boxes, g.src + i, i < g.m, v);
+            if (g.bound) rag_box<D, D + DIMB>(boxes, g.src + i, i < g.m, v);
         }
     }
 }
@@ -629,7 +628,7 @@ static __global__ void rag_dt_pack_kernel(const RagSeg* __restrict__ segs, const
             Real bp[3], bw[4];
             dt_pack_record<Real>(norm, grad, false, c, sv, d, first ? eps1 : eps2, first ? 1.0 : sign2, g.scale,
                                  g.center, src, sstride, g.src + i, splanes, sslots, list != 0, bp, bw);
-            if (rag_bounded(g)) store_fold_box<Real, 4>(boxes, g.src + i, c != nullptr, bp, bw, nw);
+            if (g.bound) store_fold_box<Real, 4>(boxes, g.src + i, c != nullptr, bp, bw, nw);
         }
     }
 }

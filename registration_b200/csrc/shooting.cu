@@ -228,7 +228,7 @@ int shoot_impl(const ShootArgs& a, Workspace& ws, cudaStream_t st) {
     for (StepPlanes& p : pn) {
         p.tgt = ws.take<float4>((size_t)Op::PP * pl.n_tpad);
         p.src = ws.take<float4>((size_t)Op::NS * pl.m_pad);
-        p.boxes = pl.take_boxes<Op>(ws);
+        p.boxes = pl.take_boxes<Op>(ws, LIST ? kBoundFoldsPacked : kBoundFolds);
     }
     double* part = ws.take<double>(pl.part_doubles(D));
     int* counters = ws.take<int>(pl.counters());
@@ -453,7 +453,7 @@ int cov_impl(const CovArgs& a, Workspace& ws, cudaStream_t st) {
     for (StepPlanes& p : pn) {
         p.tgt = ws.take<float4>((size_t)NT * pl.n_tpad);
         p.src = ws.take<float4>((size_t)Op::NS * pl.m_pad);
-        p.boxes = pl.take_boxes<Op>(ws);
+        p.boxes = pl.take_boxes<Op>(ws, LIST ? kBoundFoldsPacked : kBoundFolds);
     }
     double* part = ws.take<double>(pl.part_doubles(D));
     int* counters = ws.take<int>(pl.counters());

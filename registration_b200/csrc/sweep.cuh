@@ -25,9 +25,9 @@
 // the other).  EpiNone leaves the chunk sums in `part`, chunk by chunk with seg.n_tgt
 // rows each.
 //
-// Far folds (operators with Op::lgk, `boxes` given, more than kBoundFolds folds).  The
-// pack kernels leave for each fold its bounding box and, by weight column, log2 of the
-// sum of its weights.  With the box of the target group these bound what a fold can add
+// Far folds (operators with Op::lgk, seg.bound: more than kBoundFolds folds).  The pack
+// kernels leave for each fold its bounding box and, by weight column, log2 of the sum of
+// its weights.  With the box of the target group these bound what a fold can add
 // to an output of any target of the group, U = W_F K(dmin), times max |x_j - y_j| where
 // the term carries x - y and |u_k|_1 where it carries <u_k, v_l>.  What the outputs
 // hold at least is measured: each warp adds up the absolute terms of all targets of the
@@ -45,8 +45,8 @@
 // a time.
 // Measured against the sweep over every pair (B200): FP32c varifold gradient of a
 // 20,480-cell sphere at sigma 0.1 0.97 -> 0.41 ms, its FP64 value 1.63 -> 0.58 ms, the
-// value of 98,000 cells at sigma 0.05 6.2 -> 1.6 ms.  Where no fold is far it costs 3% of
-// a shot and adjoint of 10,242 points (1384 -> 1430 us), less of longer sweeps.
+// value of 98,000 cells at sigma 0.05 6.2 -> 1.6 ms.  Where no fold is far it costs 5% of
+// a shot and adjoint of 12,300 points (1.8 -> 1.9 ms), less of longer sweeps.
 //
 // perm (SegDesc): the target rows in an order that puts neighbours into the same
 // group (launch_order_rows, pack.cuh).  The sum of a target does not depend on
@@ -181,10 +181,17 @@ constexpr int op_weights() {
 }
 
 // Up to this many folds (6,144 sources) a sweep is so short that bounding its folds costs
-// what it saves.  Shot and adjoint of ten steps at 1,500 / 3,166 / 6,000 / 10,242 points of a
-// sphere, us, FP32: every fold 251 / 389 / 677 / 1384; bounded, sigma 0.05 291 / 427 / 720 /
-// 1294, sigma 0.2 292 / 429 / 745 / 1430.
-constexpr int kBoundFolds = 192;
+// what it saves; FP32 shots, adjoints and varifold gradients of one problem, a wave or two
+// of blocks, up to twice as many (segments of a ragged launch have the others beside them).
+// B200, every fold / bounded, us, sigma 0.05 / 0.1 (0.12 of the shots) / 0.2:
+//   shot and adjoint of ten steps, FP32, 8,000 points of a sphere 872 / 874 / 875 and
+//     909 / 959 / 965, 10,242 points 1344 / 1345 / 1345 and 1284 / 1411 / 1430, 12,000 points
+//     1793 / 1791 / 1795 and 1685 / 1884 / 1891
+//   varifold gradient, FP32, 3,920 cells 82 / 82 / 82 and 84 / 86 / 86, 5,120 cells
+//     100 / 100 / 100 and 97 / 105 / 105, 5,831 cells 117 / 117 / 117 and 115 / 120 / 122
+//   varifold value and gradient, FP64, 5,120 cells 150 / 150 / 151 and 106 / 129 / 154,
+//     186 / 186 / 186 and 121 / 172 / 194; current gradient, FP32, 84 / 84 and 63 / 71
+constexpr int kBoundFolds = 192, kBoundFoldsPacked = 384;
 
 // float4 words of a fold's box: (lo, lgw[0]), (hi, lgw[1]), (lgw[2..5]), ...
 constexpr __host__ __device__ int fold_box_words(int nw) { return 2 + (nw > 2 ? (nw + 1) / 4 : 0); }
@@ -388,7 +395,7 @@ __global__ void __launch_bounds__(32 * kSweepWarps, op_min_blocks<Op>())
     };
 
     // far folds: a fold of the group's own rows, another one for each warp where it has as many
-    const bool bounded = op_culls<Op>::value && boxes != nullptr && n_folds > kBoundFolds;
+    const bool bounded = op_culls<Op>::value && sg.bound;
     int own_fold = -1;
     if (bounded && sg.self) {
         int own = -1;

@@ -30,8 +30,8 @@ struct SinglePlan {
     // (Formed all the same they cost a shot and adjoint of 1,000 / 2,000 points 248 / 291 us
     // instead of 216 / 253.)
     template <class Op>
-    float4* take_boxes(Workspace& ws) const {
-        if (n_folds <= kBoundFolds) return nullptr;
+    float4* take_boxes(Workspace& ws, int unbounded = kBoundFolds) const {
+        if (n_folds <= unbounded) return nullptr;
         return ws.take<float4>((size_t)fold_box_words(op_weights<Op>()) * (size_t)(m_pad / kFold));
     }
 };
@@ -105,6 +105,7 @@ int launch_single(const SinglePlan& pl, long long n, const typename Op::Params& 
     g.seg0.sym_folds = sym_folds;
     g.seg0.perm = perm;
     g.seg0.self = self;
+    g.seg0.bound = boxes != nullptr;
     g.nseg = 0;
     g.n_items = pl.n_tb * pl.split;
     if (g.n_items <= 0) return LDDMM_OK;

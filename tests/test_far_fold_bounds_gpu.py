@@ -214,3 +214,30 @@ def test_curve_terms_of_narrow_kernels(oracle_lib, precision, tol, norm):
     d = np.linalg.norm(C.centers[:, None] - y[None], axis=2)
     gmag = (np.abs(k1) * d * w).sum(axis=1) * length + 2 * (k @ w)
     assert np.abs(got - gw).max() <= tol * 4 * gmag.max()
+
+
+# FP32 shots and adjoints look for far folds from 12,289 points on
+@pytest.mark.parametrize("n", [12288, 12289])
+def test_large_fp32_shots_of_narrow_kernels(oracle_lib, n):
+    test_shots_of_narrow_kernels(oracle_lib, "fp32c", 2e-5, n)
+
+
+def test_adjoint_of_large_orthogonal_clusters():
+    """As test_adjoint_of_orthogonal_clusters; every 37th row is compared."""
+    import torch
+    from registration_b200 import pointEvolution as evol
+    n = 12801
+    rng = np.random.default_rng(n)
+    x, _ = _near_and_far(n, 2, 0, rng)
+    h = n // 2
+    x[h:, 0] += 11 * SIGMA
+    a, p = np.zeros((n, 3)), np.zeros((n, 3))
+    a[:h, 1], p[h:, 1] = rng.uniform(0.5, 2, h), rng.uniform(0.5, 2, n - h)
+    p[:h, 2], a[h:, 2] = rng.uniform(0.5, 2, h), rng.uniform(0.5, 2, n - h)
+    xd, ad, pd = _dev(x, a, p)
+    pxt, _ = evol.covector(torch.stack([xd, xd]), ad[None], pd, _kernel("gauss", "fp32c"), 0.0)
+    got = pxt[0].cpu().numpy()[::37, 0]
+    y, u, v = x[::37], p[::37], a[::37]
+    _, k1 = _factors("gauss", y, x)
+    t = k1 * (u @ a.T + v @ p.T) * (y[:, None, 0] - x[None, :, 0])
+    assert (np.abs(got - t.sum(axis=1)) <= ORACLE_TOL["fp32c"] * np.abs(t).sum(axis=1)).all()
